@@ -32,6 +32,7 @@
 #include <cstdio>
 
 #include "common.cuh"
+#include "gemm_few.cuh"
 #include "ptx.cuh"
 #include "tmap.cuh"
 
@@ -58,8 +59,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int id)
     atomicExch(&g_gemm_status, 1 + id);
     return false;
 }
-enum { GEMM_OUT_FM = 0, GEMM_OUT_TM = 1, GEMM_OUT_TM_ADD = 2 };   // output layouts, see the kernel
-
 // Epilogue store of one 32-token block of a thread's row (v = 32 fp32 accumulator values), in the
 // layout out_mode asks for.  m = this thread's row, mbase = first row of its 128-row tile,
 // nb = first token of the block.  `piece` counts the token-major staging pieces of this column
@@ -700,6 +699,12 @@ int launch_nvfp4_gemmtc_v5(const uint8_t* d_weight_packed, const uint8_t* d_weig
     if (M <= 0 || N <= 0 || K <= 0 || K % 16 != 0) return NVFP4_ERR_SHAPE;
     if (!d_weight_packed || !d_weight_scales || !d_activation || !d_output) return NVFP4_ERR_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
+    if (N % 8 == 0 && (((uintptr_t)d_activation | (uintptr_t)d_output) & 15) == 0 &&
+        gemm_few_takes(d_weight_packed, d_weight_scales, N, K)) {
+        const int rc = gemm_few_launch(d_weight_packed, d_weight_scales, d_activation, N, false, d_output, N,
+                                       M, N, N, K, GEMM_OUT_FM, st);
+        if (rc != -3) return rc;
+    }
     const bool tc_ok = (K % 64 == 0) && (N % 8 == 0) &&
                        (((uintptr_t)d_weight_packed & 15) == 0) &&
                        (((uintptr_t)d_weight_scales & 3) == 0) &&
@@ -754,6 +759,12 @@ int launch_nvfp4_gemm_w4a16_ex(const uint8_t* d_weight_packed, const uint8_t* d_
         return NVFP4_ERR_SHAPE;
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return -3;
+    const int mode = !out_tm ? GEMM_OUT_FM : add ? GEMM_OUT_TM_ADD : GEMM_OUT_TM;
+    __half* o = static_cast<__half*>(out);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (gemm_few_takes(d_weight_packed, d_weight_scales, N8, K))
+        return gemm_few_launch(d_weight_packed, d_weight_scales, static_cast<const __half*>(act), ld_act, in_tm,
+                               o, (int)ld_out, M, N8, n_tokens, K, mode, st);
     // token count the kernel's bounds use: feature-major sides are padded to 8
     const int N = (in_tm && out_tm) ? n_tokens : N8;
     CUtensorMap map;
@@ -776,9 +787,6 @@ int launch_nvfp4_gemm_w4a16_ex(const uint8_t* d_weight_packed, const uint8_t* d_
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
     if (r != CUDA_SUCCESS) return -3;
-    const int mode = !out_tm ? GEMM_OUT_FM : add ? GEMM_OUT_TM_ADD : GEMM_OUT_TM;
-    __half* o = static_cast<__half*>(out);
-    cudaStream_t st = (cudaStream_t)stream;
     const cudaError_t e = in_tm ? launch_tc_any<true>(map, d_weight_packed, d_weight_scales, o, M, N, K,
                                                       (int)ld_out, mode, n_tokens, st)
                                 : launch_tc_any<false>(map, d_weight_packed, d_weight_scales, o, M, N, K,
@@ -830,6 +838,8 @@ int nvfp4_gemm_status(int reset) {
     }
     const int f = nvfp4_gemm_fp4_status(reset);   // the FP4 kernel's waits: ids 100 + its own
     if (v == 0 && f != 0) v = (f < 0) ? f : 100 + f;
+    const int few = nvfp4::gemm_few_status(reset);  // the few-token kernel's: 200 + its own
+    if (v == 0 && few != 0) v = (few < 0) ? few : 200 + few;
     return v;
 }
 

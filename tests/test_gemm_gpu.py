@@ -485,3 +485,40 @@ def test_fp4_cta_pair_kernel_equals_the_single_cta_kernel(lib, M, n, K):
     if M * n <= 1 << 19:
         ref = oc.decode_f64(p, s) @ oc.decode_f64(ap, asc).T
         assert oc.rel_error_floored(outs[1].cpu().numpy(), ref).max() <= 2e-3 * max(1.0, (K / 4096) ** 0.5)
+
+
+@pytest.mark.parametrize("M,n,K", [
+    (128, 1, 256), (129, 16, 256), (100, 17, 512), (640, 33, 2304), (1000, 65, 1280), (260, 128, 17408),
+    (40000, 5, 512), (10240, 48, 1792),
+])
+def test_few_token_kernel_against_the_oracle(lib, M, n, K):
+    # at most 128 tokens: K split over clusters (1 to 8 CTAs: K = 256 has one stage, 40000 rows fill
+    # the GPU unsplit), ragged rows, every token tile (16, 32, 64, 128) at its edges; in every
+    # layout.  Bound: fp32 accumulation and the fp16 output, as for the other GEMM kernels.
+    rng = np.random.default_rng(M + n + K)
+    p = rng.integers(0, 256, size=(M, K // 2), dtype=np.uint8)
+    s = rng.integers(118, 123, size=(M, K // 16), dtype=np.uint8)
+    act = rng.standard_normal((n, K)).astype(np.float16)
+    resid = rng.standard_normal((n, M)).astype(np.float16)
+    N8 = (n + 7) // 8 * 8
+    d_p, d_s, d_a = dev(p), dev(s), dev(act)
+    lib.nvfp4_gemm_status(1)
+    rows = np.arange(M) if M <= 1024 else np.unique(np.r_[0, M - 1, rng.integers(0, M, 500)])
+    ref = oc.decode(p[rows], s[rows]).astype(np.float64) @ act.T.astype(np.float64)
+    outs = []
+    for flags in (1, 3, 7):
+        ld = N8 if flags == 1 else M
+        out = torch.full(((M * N8 if flags == 1 else n * M) + 16,), float("nan"), dtype=torch.float16, device="cuda")
+        if flags == 7:
+            out[:n * M] = dev(resid).view(-1)
+        assert lib.launch_nvfp4_gemm_w4a16_ex(ptr(d_p), ptr(d_s), ptr(d_a), K, ptr(out), ld, M, n, K, flags,
+                                              stream()) == 0
+        torch.cuda.synchronize()
+        o = out.cpu().numpy()
+        assert np.isnan(o[-16:]).all(), "wrote past the output"
+        outs.append(o[:-16].reshape(M, N8)[:, :n] if flags == 1 else o[:-16].reshape(n, M).T)
+    assert lib.nvfp4_gemm_status(0) == 0, "a bounded wait inside the kernel ran out"
+    fm, tm, add = outs
+    assert np.array_equal(fm, tm)
+    assert np.array_equal(add, (resid.T.astype(np.float32) + tm.astype(np.float32)).astype(np.float16))
+    assert oc.rel_error_floored(tm[rows], ref).max() <= 2e-3 * max(1.0, (K / 4096) ** 0.5)
