@@ -222,44 +222,42 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap act_map,
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            // instruction descriptor: D fp32, A fp16 K-major, B fp16 MN-major, N = BN, M = 128
-            const uint32_t idesc = (1u << 4) | (IN_TM ? 0u : (1u << 16)) | ((uint32_t)(BN >> 3) << 17) |
-                                   ((uint32_t)(GEMM_BM >> 4) << 24);
-            // stage index, phase and operand addresses are kept by increment (no division, no
-            // address arithmetic from scratch in this one-thread loop)
-            int s = 0;
-            uint32_t ph = 0;
-            uint32_t a_base = smem_u32(smem_a), b_base = smem_u32(smem_b);
-            uint32_t bar_f = smem_u32(&bar_full[0]), bar_e = smem_u32(&bar_empty[0]);
-            for (int it = 0; it < ksteps; it++) {
-                if (!mbar_wait(bar_f, ph, 1)) break;
-                tcgen05_fence_after();
+        // instruction descriptor: D fp32, A fp16 K-major, B fp16 MN-major, N = BN, M = 128
+        const uint32_t idesc = (1u << 4) | (IN_TM ? 0u : (1u << 16)) | ((uint32_t)(BN >> 3) << 17) |
+                               ((uint32_t)(GEMM_BM >> 4) << 24);
+        // stage index, phase and operand addresses are kept by increment (no division, no
+        // address arithmetic from scratch in this one-thread loop)
+        int s = 0;
+        uint32_t ph = 0;
+        uint32_t a_base = smem_u32(smem_a), b_base = smem_u32(smem_b);
+        uint32_t bar_f = smem_u32(&bar_full[0]), bar_e = smem_u32(&bar_empty[0]);
+        for (int it = 0; it < ksteps; it++) {
+            if (!mbar_wait(bar_f, ph, 1)) break;
+            tcgen05_fence_after();
 #pragma unroll
-                for (int kk = 0; kk < GEMM_BK / 16; kk++) {
-                    // A, K-major: 16 k = 32 bytes further along the 128-byte row; 8-row groups
-                    // are 1024 bytes apart.  B, MN-major: 16 k = two groups of 8 k rows (1024
-                    // bytes each); 64-token atoms are one box (8 KB) apart.
-                    // (token-major activations: a K-major tile of BN token rows, like A)
-                    const uint64_t bdesc = IN_TM ? make_desc_sw128(b_base + kk * 32, 16, 1024)
-                                                 : make_desc_sw128(b_base + kk * 2048, B_BOX, 1024);
+            for (int kk = 0; kk < GEMM_BK / 16; kk++) {
+                // A, K-major: 16 k = 32 bytes further along the 128-byte row; 8-row groups
+                // are 1024 bytes apart.  B, MN-major: 16 k = two groups of 8 k rows (1024
+                // bytes each); 64-token atoms are one box (8 KB) apart.
+                // (token-major activations: a K-major tile of BN token rows, like A)
+                const uint64_t bdesc = IN_TM ? make_desc_sw128(b_base + kk * 32, 16, 1024)
+                                             : make_desc_sw128(b_base + kk * 2048, B_BOX, 1024);
 #pragma unroll
-                    for (int mt = 0; mt < MT; mt++) {
-                        const uint64_t adesc = make_desc_sw128(a_base + mt * A_TILE + kk * 32, 16, 1024);
-                        tcgen05_mma_f16(tmem + (uint32_t)(mt * BN), adesc, bdesc, idesc,
-                                        (it | kk) != 0 ? 1u : 0u);
-                    }
-                }
-                tcgen05_commit(bar_e);                     // stage reusable when these MMAs retire
-                a_base += A_BYTES; b_base += B_BYTES; bar_f += 8; bar_e += 8;
-                if (++s == ST) {
-                    s = 0; ph ^= 1u;
-                    a_base = smem_u32(smem_a); b_base = smem_u32(smem_b);
-                    bar_f = smem_u32(&bar_full[0]); bar_e = smem_u32(&bar_empty[0]);
+                for (int mt = 0; mt < MT; mt++) {
+                    const uint64_t adesc = make_desc_sw128(a_base + mt * A_TILE + kk * 32, 16, 1024);
+                    tcgen05_mma_f16(tmem + (uint32_t)(mt * BN), adesc, bdesc, idesc,
+                                    (it | kk) != 0 ? 1u : 0u);
                 }
             }
-            tcgen05_commit(smem_u32(&bar_accum));
+            tcgen05_commit(bar_e);                     // stage reusable when these MMAs retire
+            a_base += A_BYTES; b_base += B_BYTES; bar_f += 8; bar_e += 8;
+            if (++s == ST) {
+                s = 0; ph ^= 1u;
+                a_base = smem_u32(smem_a); b_base = smem_u32(smem_b);
+                bar_f = smem_u32(&bar_full[0]); bar_e = smem_u32(&bar_empty[0]);
+            }
         }
+        tcgen05_commit(smem_u32(&bar_accum));
     } else {
         // ---------------- weight producers (two threads per weight row), then epilogue ----------------
         const int pt = threadIdx.x - 64;                 // 0..255

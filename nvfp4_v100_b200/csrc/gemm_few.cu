@@ -68,9 +68,7 @@ __device__ __forceinline__ bool few_wait(uint32_t bar, uint32_t parity, int id) 
     return false;
 }
 
-// Issued by a whole converged warp; the instruction itself by its elected lane.  With a branch on
-// the lane index around the loop instead, the compiler has to move every operand from a general to
-// a uniform register before each MMA (about 78 cycles per instruction).
+// A operand in tensor memory; called by a whole converged warp (see tcgen05_mma_f16)
 __device__ __forceinline__ void few_mma(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n.reg .pred p, e;\n"
@@ -78,13 +76,6 @@ __device__ __forceinline__ void few_mma(uint32_t d, uint32_t a, uint64_t bdesc, 
         "setp.ne.u32 p, %4, 0;\n"
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d), "r"(a), "l"(bdesc),
         "r"(idesc), "r"(acc)
-        : "memory");
-}
-__device__ __forceinline__ void few_commit(uint32_t bar) {
-    asm volatile(
-        "{\n.reg .pred e;\n"
-        "elect.sync _|e, 0xffffffff;\n"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar)
         : "memory");
 }
 __device__ __forceinline__ void few_st_x16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -246,10 +237,10 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
                                              : make_desc_sw128(bb + (kk & 3) * 2048, 8192, 1024);
                 few_mma(tmem, a + (uint32_t)(kk * 8), bdesc, idesc, (i | kk) != 0 ? 1u : 0u);
             }
-            few_commit(smem_u32(&bar_free[u]));
+            tcgen05_commit(smem_u32(&bar_free[u]));
             if (++u == NU) { u = 0; ph ^= 1u; }
         }
-        few_commit(smem_u32(&bar_accum));
+        tcgen05_commit(smem_u32(&bar_accum));
     } else if (warp >= 4) {
         const int q = warp & 3, grp = (warp - 4) >> 2;         // lane quarter; which units of a stage
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;

@@ -54,9 +54,10 @@ __device__ __forceinline__ void tcgen05_mma_fp4_block16(uint32_t taddr, uint64_t
                                                         uint32_t idesc, uint32_t sfa, uint32_t sfb,
                                                         uint32_t accumulate) {
     asm volatile(
-        "{\n.reg .pred p;\n"
+        "{\n.reg .pred p, e;\n"
+        "elect.sync _|e, 0xffffffff;\n"
         "setp.ne.u32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::
+        "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::
             "r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
         : "memory");
 }
@@ -189,39 +190,37 @@ gemm_fp4_block_scaled_kernel(const __grid_constant__ CUtensorMap w_map,
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // block-scaled instruction descriptor: A and B E2M1 (code 1) K-major, N = BN, scale
-            // type E8M0, M = 128, scale-factor ids 0 (a block-16 MMA consumes all four bytes of a
-            // column), K = 64
-            const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | (1u << 23) |
-                                   ((uint32_t)(F4_BM >> 4) << 24);
-            int s = 0, ti = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ti++) {
-                // the epilogue of the tile before must have read the accumulator
-                if (ti > 0 && !f4_wait(smem_u32(&bar_acc_free), (uint32_t)(ti - 1) & 1u, 5)) break;
+        // block-scaled instruction descriptor: A and B E2M1 (code 1) K-major, N = BN, scale
+        // type E8M0, M = 128, scale-factor ids 0 (a block-16 MMA consumes all four bytes of a
+        // column), K = 64
+        const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | (1u << 23) |
+                               ((uint32_t)(F4_BM >> 4) << 24);
+        int s = 0, ti = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ti++) {
+            // the epilogue of the tile before must have read the accumulator
+            if (ti > 0 && !f4_wait(smem_u32(&bar_acc_free), (uint32_t)(ti - 1) & 1u, 5)) break;
+            tcgen05_fence_after();
+            for (int it = 0; it < ksteps; it++) {
+                // (the scale writers arrive only after they saw the stage's copies land)
+                if (!f4_wait(smem_u32(&bar_sf[s]), ph, 1)) { ok = false; break; }
                 tcgen05_fence_after();
-                for (int it = 0; it < ksteps; it++) {
-                    // (the scale writers arrive only after they saw the stage's copies land)
-                    if (!f4_wait(smem_u32(&bar_sf[s]), ph, 1)) { ok = false; break; }
-                    tcgen05_fence_after();
-                    const uint32_t a_base = smem_u32(smem_a + s * A_BYTES);
-                    const uint32_t b_base = smem_u32(smem_b + s * B_BYTES);
-                    const uint32_t sf = tmem_sf + (uint32_t)(s * SF_COLS);
+                const uint32_t a_base = smem_u32(smem_a + s * A_BYTES);
+                const uint32_t b_base = smem_u32(smem_b + s * B_BYTES);
+                const uint32_t sf = tmem_sf + (uint32_t)(s * SF_COLS);
 #pragma unroll
-                    for (int kk = 0; kk < 4; kk++) {
-                        // 64 elements of K = 32 bytes further along the swizzled 128-byte row
-                        const uint64_t adesc = make_desc_sw128(a_base + kk * 32, 16, 1024);
-                        const uint64_t bdesc = make_desc_sw128(b_base + kk * 32, 16, 1024);
-                        tcgen05_mma_fp4_block16(tmem, adesc, bdesc, idesc, sf + (uint32_t)(kk * 4),
-                                                sf + (uint32_t)(SFA_COLS + kk * NBC), (it | kk) != 0 ? 1u : 0u);
-                    }
-                    tcgen05_commit(smem_u32(&bar_empty[s]));
-                    if (++s == ST) { s = 0; ph ^= 1u; }
+                for (int kk = 0; kk < 4; kk++) {
+                    // 64 elements of K = 32 bytes further along the swizzled 128-byte row
+                    const uint64_t adesc = make_desc_sw128(a_base + kk * 32, 16, 1024);
+                    const uint64_t bdesc = make_desc_sw128(b_base + kk * 32, 16, 1024);
+                    tcgen05_mma_fp4_block16(tmem, adesc, bdesc, idesc, sf + (uint32_t)(kk * 4),
+                                            sf + (uint32_t)(SFA_COLS + kk * NBC), (it | kk) != 0 ? 1u : 0u);
                 }
-                tcgen05_commit(smem_u32(&bar_accum));
+                tcgen05_commit(smem_u32(&bar_empty[s]));
+                if (++s == ST) { s = 0; ph ^= 1u; }
             }
+            tcgen05_commit(smem_u32(&bar_accum));
         }
     } else {
         // ---------------- scale-factor writers ----------------

@@ -34,9 +34,10 @@
 //               kernel in the stream has finished (programmatic dependent launch: weights are
 //               constants); the others once the activation loads have been issued, because those
 //               would queue behind the weight requests in the SM's request path.
-//   warp 1      MMA issuer (one thread): 4 x tcgen05.mma M128 N16 K64 per stage into one of two
-//               accumulators.  All its stage counters are kept by increment: this thread runs one
-//               instruction at a time, a division per stage would cost more than the MMAs.
+//   warp 1      MMA issuer: 4 x tcgen05.mma M128 N16 K64 per stage into one of two accumulators.
+//               The whole warp runs the loop and an elected lane issues (operands stay in uniform
+//               registers; as one thread's loop it cost a launch 0.9 us: 17408 x 5120 10.4 -> 9.5,
+//               5120 x 17408 11.4 -> 10.5).  All its stage counters are kept by increment.
 //   warps 2..5  scale writers: weight scale bytes shared memory -> tensor memory (tcgen05.st; lane
 //               r % 32, column r / 32, replicated in the four lane quarters) and the digit columns'
 //               scale bytes, one 32-column store per stage.
@@ -90,9 +91,10 @@ __device__ __forceinline__ bool tc_wait_poll(uint32_t bar, uint32_t parity, int 
 __device__ __forceinline__ void tc_mma(uint32_t taddr, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                        uint32_t sfa, uint32_t sfb, uint32_t accumulate) {
     asm volatile(
-        "{\n.reg .pred p;\n"
+        "{\n.reg .pred p, e;\n"
+        "elect.sync _|e, 0xffffffff;\n"
         "setp.ne.u32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::
+        "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::
             "r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
         : "memory");
 }
@@ -270,9 +272,9 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     // (the launcher keeps total * (G + 1) below 2^32: 32-bit divisions)
     const unsigned total = (unsigned)ntiles * (unsigned)nk;
     const unsigned g0 = (unsigned)b * total / (unsigned)G, g1 = (unsigned)(b + 1) * total / (unsigned)G;
-    // the loops below count stages with 32-bit counters kept by increment: the single-thread roles
-    // (copy issue, MMA issue) run one instruction at a time, a division per stage would cost them
-    // more than the stage's four MMAs
+    // the loops below count stages with 32-bit counters kept by increment: the roles that
+    // issue copies and MMAs run one instruction at a time, a division per stage would cost them more
+    // than the stage's four MMAs
     const int nst = (int)(g1 - g0);                  // stages of this CTA
     const int tile0 = (int)(g0 / nk), ks0 = (int)(g0 % nk);
 
@@ -397,45 +399,43 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         }
         if (warp == 1) {
             // ---------------- MMA issuer ----------------
-            if (lane == 0) {
-                // A, B E2M1 K-major; N = 16; E8M0 scales; M = 128
-                const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(16 >> 3) << 17) | (1u << 23) |
-                                       ((uint32_t)(TC_BM >> 4) << 24);
-                // descriptors: +1 in the low word = 16 bytes further in shared memory
-                const uint64_t a_desc0 = make_desc_sw128(smem_u32(smem_a), 16, 1024);
-                const uint64_t b_desc0 = make_desc_sw128(smem_u32(smem_b), 16, 1024);
-                int s = 0, ks = ks0, seg = 0, bs = 0;
-                uint32_t ph = 0;
-                bool first = true;
-                for (int i = 0; i < nst; i++) {
-                    const int buf = seg & 1;
-                    if (first &&  // the flush warps must have drained this accumulator's previous use
-                        !tc_wait_poll(smem_u32(&bar_acc_empty[buf]), (((uint32_t)seg >> 1) & 1u) ^ 1u, 1))
-                        break;
-                    // the scale writers arrive here only after they saw the stage's copies land and
-                    // its digit planes written
-                    if (!tc_wait_poll(smem_u32(&bar_ready[s]), ph, 3)) break;
-                    tcgen05_fence_after();
-                    if (rec && i == 0) atomicMax(dbg + 5, tc_now());
-                    const uint64_t adesc = a_desc0 + (uint64_t)(s * (TC_A_BYTES >> 4));
-                    const uint64_t bdesc = b_desc0 + (uint64_t)(bs * (TC_B_BYTES >> 4));
-                    const uint32_t sf = tmem_sf + (uint32_t)(s * TC_SF_COLS);
-                    const uint32_t d = tmem + (uint32_t)(buf * 16);
-                    tc_mma(d, adesc, bdesc, idesc, sf, sf + 16, first ? 0u : 1u);
-                    tc_mma(d, adesc + 2, bdesc + 2, idesc, sf + 4, sf + 20, 1u);
-                    tc_mma(d, adesc + 4, bdesc + 4, idesc, sf + 8, sf + 24, 1u);
-                    tc_mma(d, adesc + 6, bdesc + 6, idesc, sf + 12, sf + 28, 1u);
-                    tcgen05_commit(smem_u32(&bar_empty[s]));
-                    tcgen05_commit(smem_u32(&bar_bempty[bs]));
-                    first = false;
-                    if (++s == ST) { s = 0; ph ^= 1u; }
-                    bs = (bs + 1) & (NB - 1);
-                    if (++ks == nk || i == nst - 1) {       // the segment ends with this stage
-                        tcgen05_commit(smem_u32(&bar_acc_full[buf]));
-                        seg++;
-                        first = true;
-                        ks = 0;
-                    }
+            // A, B E2M1 K-major; N = 16; E8M0 scales; M = 128
+            const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(16 >> 3) << 17) | (1u << 23) |
+                                   ((uint32_t)(TC_BM >> 4) << 24);
+            // descriptors: +1 in the low word = 16 bytes further in shared memory
+            const uint64_t a_desc0 = make_desc_sw128(smem_u32(smem_a), 16, 1024);
+            const uint64_t b_desc0 = make_desc_sw128(smem_u32(smem_b), 16, 1024);
+            int s = 0, ks = ks0, seg = 0, bs = 0;
+            uint32_t ph = 0;
+            bool first = true;
+            for (int i = 0; i < nst; i++) {
+                const int buf = seg & 1;
+                if (first &&  // the flush warps must have drained this accumulator's previous use
+                    !tc_wait_poll(smem_u32(&bar_acc_empty[buf]), (((uint32_t)seg >> 1) & 1u) ^ 1u, 1))
+                    break;
+                // the scale writers arrive here only after they saw the stage's copies land and
+                // its digit planes written
+                if (!tc_wait_poll(smem_u32(&bar_ready[s]), ph, 3)) break;
+                tcgen05_fence_after();
+                if (rec && i == 0 && lane == 0) atomicMax(dbg + 5, tc_now());
+                const uint64_t adesc = a_desc0 + (uint64_t)(s * (TC_A_BYTES >> 4));
+                const uint64_t bdesc = b_desc0 + (uint64_t)(bs * (TC_B_BYTES >> 4));
+                const uint32_t sf = tmem_sf + (uint32_t)(s * TC_SF_COLS);
+                const uint32_t d = tmem + (uint32_t)(buf * 16);
+                tc_mma(d, adesc, bdesc, idesc, sf, sf + 16, first ? 0u : 1u);
+                tc_mma(d, adesc + 2, bdesc + 2, idesc, sf + 4, sf + 20, 1u);
+                tc_mma(d, adesc + 4, bdesc + 4, idesc, sf + 8, sf + 24, 1u);
+                tc_mma(d, adesc + 6, bdesc + 6, idesc, sf + 12, sf + 28, 1u);
+                tcgen05_commit(smem_u32(&bar_empty[s]));
+                tcgen05_commit(smem_u32(&bar_bempty[bs]));
+                first = false;
+                if (++s == ST) { s = 0; ph ^= 1u; }
+                bs = (bs + 1) & (NB - 1);
+                if (++ks == nk || i == nst - 1) {       // the segment ends with this stage
+                    tcgen05_commit(smem_u32(&bar_acc_full[buf]));
+                    seg++;
+                    first = true;
+                    ks = 0;
                 }
             }
         } else if (warp < 6) {
@@ -800,46 +800,44 @@ gemv_tc_mlp_kernel(const __grid_constant__ CUtensorMap w_map0, const __grid_cons
         }
         if (warp == 1) {
             // ---------------- MMA issuer: both phases, one stage sequence ----------------
-            if (lane == 0) {
-                const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(16 >> 3) << 17) | (1u << 23) |
-                                       ((uint32_t)(TC_BM >> 4) << 24);
-                const uint64_t a_desc0 = make_desc_sw128(smem_u32(smem_a), 16, 1024);
-                const uint64_t b_desc0 = make_desc_sw128(smem_u32(smem_b), 16, 1024);
-                int s = 0, seg = 0, bs = 0;
-                uint32_t ph = 0;
-                bool ok = true;
-                for (int p = 0; p < 2 && ok; p++) {
-                    const int nst = p ? R1.nst : R0.nst, nk = p ? R1.nk : R0.nk;
-                    int ks = p ? R1.ks0 : R0.ks0;
-                    bool first = true;
-                    for (int i = 0; i < nst; i++) {
-                        const int buf = seg & 1;
-                        if (first &&
-                            !tc_wait_poll(smem_u32(&bar_acc_empty[buf]), (((uint32_t)seg >> 1) & 1u) ^ 1u, 1)) {
-                            ok = false;
-                            break;
-                        }
-                        if (!tc_wait_poll(smem_u32(&bar_ready[s]), ph, 3)) { ok = false; break; }
-                        tcgen05_fence_after();
-                        const uint64_t adesc = a_desc0 + (uint64_t)(s * (TC_A_BYTES >> 4));
-                        const uint64_t bdesc = b_desc0 + (uint64_t)(bs * (TC_B_BYTES >> 4));
-                        const uint32_t sf = tmem_sf + (uint32_t)(s * TC_SF_COLS);
-                        const uint32_t d = tmem + (uint32_t)(buf * 16);
-                        tc_mma(d, adesc, bdesc, idesc, sf, sf + 16, first ? 0u : 1u);
-                        tc_mma(d, adesc + 2, bdesc + 2, idesc, sf + 4, sf + 20, 1u);
-                        tc_mma(d, adesc + 4, bdesc + 4, idesc, sf + 8, sf + 24, 1u);
-                        tc_mma(d, adesc + 6, bdesc + 6, idesc, sf + 12, sf + 28, 1u);
-                        tcgen05_commit(smem_u32(&bar_empty[s]));
-                        tcgen05_commit(smem_u32(&bar_bempty[bs]));
-                        first = false;
-                        if (++s == ST) { s = 0; ph ^= 1u; }
-                        bs = (bs + 1) & (NB - 1);
-                        if (++ks == nk || i == nst - 1) {
-                            tcgen05_commit(smem_u32(&bar_acc_full[buf]));
-                            seg++;
-                            first = true;
-                            ks = 0;
-                        }
+            const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(16 >> 3) << 17) | (1u << 23) |
+                                   ((uint32_t)(TC_BM >> 4) << 24);
+            const uint64_t a_desc0 = make_desc_sw128(smem_u32(smem_a), 16, 1024);
+            const uint64_t b_desc0 = make_desc_sw128(smem_u32(smem_b), 16, 1024);
+            int s = 0, seg = 0, bs = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int p = 0; p < 2 && ok; p++) {
+                const int nst = p ? R1.nst : R0.nst, nk = p ? R1.nk : R0.nk;
+                int ks = p ? R1.ks0 : R0.ks0;
+                bool first = true;
+                for (int i = 0; i < nst; i++) {
+                    const int buf = seg & 1;
+                    if (first &&
+                        !tc_wait_poll(smem_u32(&bar_acc_empty[buf]), (((uint32_t)seg >> 1) & 1u) ^ 1u, 1)) {
+                        ok = false;
+                        break;
+                    }
+                    if (!tc_wait_poll(smem_u32(&bar_ready[s]), ph, 3)) { ok = false; break; }
+                    tcgen05_fence_after();
+                    const uint64_t adesc = a_desc0 + (uint64_t)(s * (TC_A_BYTES >> 4));
+                    const uint64_t bdesc = b_desc0 + (uint64_t)(bs * (TC_B_BYTES >> 4));
+                    const uint32_t sf = tmem_sf + (uint32_t)(s * TC_SF_COLS);
+                    const uint32_t d = tmem + (uint32_t)(buf * 16);
+                    tc_mma(d, adesc, bdesc, idesc, sf, sf + 16, first ? 0u : 1u);
+                    tc_mma(d, adesc + 2, bdesc + 2, idesc, sf + 4, sf + 20, 1u);
+                    tc_mma(d, adesc + 4, bdesc + 4, idesc, sf + 8, sf + 24, 1u);
+                    tc_mma(d, adesc + 6, bdesc + 6, idesc, sf + 12, sf + 28, 1u);
+                    tcgen05_commit(smem_u32(&bar_empty[s]));
+                    tcgen05_commit(smem_u32(&bar_bempty[bs]));
+                    first = false;
+                    if (++s == ST) { s = 0; ph ^= 1u; }
+                    bs = (bs + 1) & (NB - 1);
+                    if (++ks == nk || i == nst - 1) {
+                        tcgen05_commit(smem_u32(&bar_acc_full[buf]));
+                        seg++;
+                        first = true;
+                        ks = 0;
                     }
                 }
             }

@@ -75,18 +75,27 @@ __device__ __forceinline__ void tcgen05_fence_before() {
 __device__ __forceinline__ void tcgen05_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 }
+// MMA and commit instructions are called by a whole converged warp and executed by one elected lane.
+// With `if (lane == 0)` around the issuing loop instead, the loop's control flow is not uniform for
+// the compiler, which then moves every operand from general to uniform registers before each MMA:
+// measured 78 cycles per MMA and 85 per commit, more than a narrow MMA takes.  (The CTA-pair forms
+// below are issued by one thread: their MMAs take longer than that, and 32 lanes polling the pair's
+// barriers made those kernels 6 % slower.)
 __device__ __forceinline__ void tcgen05_mma_f16(uint32_t taddr, uint64_t adesc, uint64_t bdesc,
                                                 uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n.reg .pred p;\n"
+        "{\n.reg .pred p, e;\n"
+        "elect.sync _|e, 0xffffffff;\n"
         "setp.ne.u32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(taddr),
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(taddr),
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void tcgen05_commit(uint32_t bar) {
     asm volatile(
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar)
+        "{\n.reg .pred e;\n"
+        "elect.sync _|e, 0xffffffff;\n"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar)
         : "memory");
 }
 __device__ __forceinline__ void tcgen05_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32]) {
