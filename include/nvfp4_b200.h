@@ -310,7 +310,9 @@ int launch_allreduce_residual(void* h, const void* const* bufs, int rank, int wo
  *                          pos0 (host int); qkv token-major, ld halves per row; q_out/gate_out
  *                          token-major [n_tokens][hq*256]; token i writes cache row pos0 + i
  *   launch_attn_prefill    causal attention, decode arithmetic: token i attends to cache rows
- *                          [0, len0 + i); q, gate, out token-major [n_tokens][hq*256]
+ *                          [0, len0 + i); q, gate, out token-major [n_tokens][hq*256].  Small chunks
+ *                          are bit-identical to the decode kernel; larger ones run on the tensor
+ *                          cores with fp32 sums in another order
  *   launch_dn_prefill      one Gated-DeltaNet layer over n tokens: x token-major [n][ld], row =
  *                          [mixed | z | b | a]; conv window and recurrent state carried in
  *                          conv_state / state; out token-major [n][nv*128]; work: 256-byte aligned

@@ -11,6 +11,7 @@
 // the last bit before the final fp16 rounding.
 #include <cstdio>
 
+#include "attn_prefill_tc.cuh"
 #include "common.cuh"
 
 namespace nvfp4 {
@@ -755,7 +756,9 @@ static int attn_decode_launch(const void* q, const void* keys, const void* value
 
 // Causal attention of a prefill chunk with the decode kernel's arithmetic: token i of the chunk
 // (i < n_tokens) attends to cache rows [0, len0 + i), which must already hold the chunk's own
-// keys and values.  q, gate, out: token-major [n_tokens][hq * 256].  Grid (hq, n_tokens).
+// keys and values.  q, gate, out: token-major [n_tokens][hq * 256].  Chunks of ATTN_TC_MIN_PAIRS
+// (token, key) pairs and more run on the tensor cores (attn_prefill_tc.cu): the same formulas and
+// fp16 rounding points with fp32 sums in another order.
 int launch_attn_prefill(const void* q, const void* keys, const void* values, int len0,
                         int n_tokens, const void* gate, void* out, int max_len, int hq, int hkv,
                         float scale, void* stream) {
@@ -768,6 +771,12 @@ int launch_attn_prefill(const void* q, const void* keys, const void* values, int
     const int lcap = len0 + n_tokens - 1;
     const int smem = ATT_G * lcap * (int)sizeof(float);
     if (smem > 150 * 1024) return -2;
+    if (nvfp4::attn_prefill_tc_takes(q, keys, values, gate, out, len0, n_tokens, hq, hkv)) {
+        const int rc = nvfp4::attn_prefill_tc_launch((const __half*)q, (const __half*)keys, (const __half*)values, len0,
+                                                     n_tokens, (const __half*)gate, (__half*)out, max_len, hq, hkv,
+                                                     scale, (cudaStream_t)stream);
+        if (rc != -3) return rc;     // -3: no tensor maps from this driver
+    }
     if (smem > 8 * 1024 && smem > smem_set[dev]) {
         if (cudaFuncSetAttribute(nvfp4::attn_prefill_group_kernel,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)

@@ -31,6 +31,7 @@
 
 #include <cstdio>
 
+#include "attn_prefill_tc.cuh"
 #include "common.cuh"
 #include "gemm_few.cuh"
 #include "ptx.cuh"
@@ -838,6 +839,8 @@ int nvfp4_gemm_status(int reset) {
     if (v == 0 && f != 0) v = (f < 0) ? f : 100 + f;
     const int few = nvfp4::gemm_few_status(reset);  // the few-token kernel's: 200 + its own
     if (v == 0 && few != 0) v = (few < 0) ? few : 200 + few;
+    const int atc = nvfp4::attn_prefill_tc_status(reset);   // the chunk attention kernel's: 300 + its own
+    if (v == 0 && atc != 0) v = (atc < 0) ? atc : 300 + atc;
     return v;
 }
 

@@ -68,25 +68,6 @@ __device__ __forceinline__ bool few_wait(uint32_t bar, uint32_t parity, int id) 
     return false;
 }
 
-// A operand in tensor memory; called by a whole converged warp (see tcgen05_mma_f16)
-__device__ __forceinline__ void few_mma(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n.reg .pred p, e;\n"
-        "elect.sync _|e, 0xffffffff;\n"
-        "setp.ne.u32 p, %4, 0;\n"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d), "r"(a), "l"(bdesc),
-        "r"(idesc), "r"(acc)
-        : "memory");
-}
-__device__ __forceinline__ void few_st_x16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
-__device__ __forceinline__ void few_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void few_ld_x8(uint32_t taddr, uint32_t* r) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
@@ -235,7 +216,7 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
                 const uint32_t bb = b + (kk >> 2) * (BN * 128);
                 const uint64_t bdesc = IN_TM ? make_desc_sw128(bb + (kk & 3) * 32, 16, 1024)
                                              : make_desc_sw128(bb + (kk & 3) * 2048, 8192, 1024);
-                few_mma(tmem, a + (uint32_t)(kk * 8), bdesc, idesc, (i | kk) != 0 ? 1u : 0u);
+                tcgen05_mma_f16_ta(tmem, a + (uint32_t)(kk * 8), bdesc, idesc, (i | kk) != 0 ? 1u : 0u);
             }
             tcgen05_commit(smem_u32(&bar_free[u]));
             if (++u == NU) { u = 0; ph ^= 1u; }
@@ -263,11 +244,11 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
             for (int c = 0; c < 4; c++) {
                 uint32_t o[16];
                 few_dequant(p[c], (c < 2 ? sc.x : sc.y) >> (16 * (c & 1)), o);
-                few_st_x16(a + (uint32_t)(c * 16), o);
+                tcgen05_st_32x32b_x16(a + (uint32_t)(c * 16), o);
             }
             __syncwarp();                                      // every lane's reads of the stage are done
             if (lane == 0) mbar_arrive(smem_u32(&bar_empty[s]));
-            few_wait_st();
+            tcgen05_wait_st();
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bar_ready[u]));

@@ -78,9 +78,6 @@ __device__ __forceinline__ void tcgen05_mma_fp4_block16_pair(uint32_t taddr, uin
             "r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
         : "memory");
 }
-__device__ __forceinline__ void tcgen05_wait_st() {
-    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
-}
 // tcgen05.st, shape 32x32b: lane l of the warp writes NR consecutive 32-bit columns of its own lane
 template <int NR>
 __device__ __forceinline__ void tcgen05_st_32x32b(uint32_t taddr, const uint32_t* r) {

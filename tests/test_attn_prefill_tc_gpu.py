@@ -1,0 +1,85 @@
+"""Chunk attention on the tensor cores against float64 and, for infinities and NaN, against the
+decode kernel run once per token."""
+import numpy as np
+import pytest
+import torch
+
+from tests.gpu_util import ptr, stream
+
+pytestmark = pytest.mark.gpu
+D = 256
+
+
+def _inputs(n, p0, hq, hkv, max_len, seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    q, gate = r(n, hq * D).half(), r(n, hq * D).half()
+    keys, vals = r(hkv, max_len, D).half(), r(hkv, max_len, D).half()
+    # rows no token of the chunk may see hold whatever was there before
+    keys[:, p0 + n:] = float("nan")
+    vals[:, p0 + n:] = float("inf")
+    return q, gate, keys, vals
+
+
+def _run(lib, q, keys, vals, p0, n, gate, hq, hkv, scale):
+    out = torch.full((n, hq * D), 7.0, dtype=torch.float16, device="cuda")
+    rc = lib.launch_attn_prefill(ptr(q), ptr(keys), ptr(vals), p0 + 1, n, ptr(gate), ptr(out),
+                                 keys.shape[1], hq, hkv, scale, stream())
+    torch.cuda.synchronize()
+    assert rc == 0 and lib.nvfp4_gemm_status(0) == 0
+    return out
+
+
+@pytest.mark.parametrize("n,p0,hq,hkv,max_len,scale", [
+    (64, 0, 2, 1, 64, 1 / 16),          # one key step, half masked
+    (65, 63, 2, 1, 200, 1 / 16),        # one token past a tile; last key = first of a step
+    (21, 235, 24, 4, 256, 1 / 16),      # one tile of 126 rows, keys split in two
+    (22, 300, 24, 4, 512, 1 / 4),       # ragged second tile; peaked weights, growing maxima
+    (1, 4095, 24, 4, 4096, 1 / 16),     # one token, keys split as far as they go
+    (130, 0, 5, 5, 130, 1 / 16),        # no shared heads: 128 + 2 tokens
+    (43, 1000, 9, 3, 1100, 1.0),        # 42 tokens a tile; weights on very few keys
+    (512, 3488, 24, 4, 4100, 1 / 16),   # the last chunk of a long document
+    (1024, 0, 6, 1, 1024, 1 / 16),
+])
+def test_against_float64(lib, n, p0, hq, hkv, max_len, scale):
+    q, gate, keys, vals = _inputs(n, p0, hq, hkv, max_len, n + p0)
+    out = _run(lib, q, keys, vals, p0, n, gate, hq, hkv, scale)
+    again = _run(lib, q, keys, vals, p0, n, gate, hq, hkv, scale)
+    assert torch.equal(out, again)
+    L = p0 + n
+    mask = torch.arange(L, device="cuda")[None, :] > (p0 + torch.arange(n, device="cuda"))[:, None]
+    for h in range(hq):
+        k, v = keys[h // (hq // hkv), :L].double(), vals[h // (hq // hkv), :L].double()
+        s = (q[:, h * D:(h + 1) * D].double() @ k.T * scale).masked_fill(mask, -float("inf"))
+        o = torch.softmax(s, -1) @ v
+        sg = torch.sigmoid(gate[:, h * D:(h + 1) * D].double()).half()
+        want = (o.half().double() * sg.double())
+        got = out[:, h * D:(h + 1) * D].double()
+        # one fp16 step in the rounded sum and one in the product, and the fp32 sums: a score of
+        # size |s| carries |s| 2^-22, which moves its weight by as much
+        bound = want.abs() * 2 ** -9 + v.abs().max() * (2 ** -20 + s[~mask].abs().max() * 2 ** -21)
+        assert ((got - want).abs() <= bound).all(), (h, ((got - want).abs() / bound).max().item())
+
+
+def test_infinities_and_nan_as_the_decode_kernel(lib):
+    # a later token's value never reaches an earlier one, an unmasked one does as in fp32
+    n, p0, hq, hkv, scale = 70, 130, 6, 2, 1 / 16
+    q, gate, keys, vals = _inputs(n, p0, hq, hkv, 256, 3)
+    vals[0, 150, 3] = float("inf")
+    vals[0, 170, 5] = -float("inf")
+    vals[1, 190, 7] = float("nan")
+    keys[1, 160, 0] = float("inf")
+    keys[1, 180] = 60000.0
+    out = _run(lib, q, keys, vals, p0, n, gate, hq, hkv, scale).cpu().numpy()
+    for t in range(n):
+        ln = torch.tensor([p0 + t + 1], dtype=torch.int64, device="cuda")
+        o = torch.zeros(hq * D, dtype=torch.float16, device="cuda")
+        qt, gt = q[t].contiguous(), gate[t].contiguous()
+        assert lib.launch_attn_decode_heads(ptr(qt), ptr(keys), ptr(vals), ptr(ln), ptr(gt), ptr(o), 256,
+                                            hq, hkv, scale, stream()) == 0
+        want = o.cpu().numpy()
+        assert np.array_equal(np.isnan(out[t]), np.isnan(want)), t
+        assert np.array_equal(np.isinf(out[t]), np.isinf(want)), t
+        fin = np.isfinite(want)
+        assert np.allclose(out[t][fin].astype(np.float64), want[fin].astype(np.float64), rtol=2 ** -9, atol=2 ** -14), t
