@@ -33,6 +33,7 @@
 #include <cuda.h>
 
 #include "attn_prefill_tc.cuh"
+#include "common.cuh"
 #include "ptx.cuh"
 #include "tmap.cuh"
 
