@@ -26,9 +26,9 @@
 // Every wait is bounded and reported through nvfp4_gemm_status.
 //
 // Measured, 24 query / 4 KV heads, us (before: attn_prefill_group_kernel), tokens after context:
-//   512 after 0      30.3 (386)     512 after 3488  119.6 (3596)     26 after 1500  19.1 (143)
-//   512 after 512    45.2 (859)     512 after 9000  253 (8670)      100 after 0     21.4 (45.7)
-// i.e. 23 us fixed and 26 us per 1024 keys of 512 tokens: 100 CTAs, 3072 cycles of MMAs per step.
+//   512 after 0      27.1 (386)     512 after 3488  123 (3596)     26 after 511   16.2 (58.9)
+//   512 after 512    41.1 (859)     512 after 9000  253 (8670)    100 after 0    17.6 (45.7)
+// i.e. 20 us fixed and 26 us per 1024 keys of 512 tokens: 100 CTAs, 3072 cycles of MMAs per step.
 // Relative error against float64 unchanged (3.5e-4: the fp16 rounding of the output).
 #include <cuda.h>
 
@@ -371,70 +371,86 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     if (split > 1) cluster_sync_all();
 
     // ---- weighted sum over the cluster, gate, output: a warp takes a row, a lane 4 + 4 dims ----
-    for (int r = rank + split * warp; r < bt * gqa; r += split * (ATC_THREADS / 32)) {
-        const int tok = t0 + r / gqa, h = kv * gqa + r % gqa;
-        if (tok >= n_tokens) break;
-        float o[8], l;
-        if (split == 1) {
-            const float* t = reinterpret_cast<const float*>(smem) + r * ATC_LD + lane * 4;
-            const float4 x = *reinterpret_cast<const float4*>(t), y = *reinterpret_cast<const float4*>(t + 128);
-            o[0] = x.x; o[1] = x.y; o[2] = x.z; o[3] = x.w;
-            o[4] = y.x; o[5] = y.y; o[6] = y.z; o[7] = y.w;
-            l = s_l[0][r] + s_l[1][r];
-        } else {
-            const uint32_t am = smem_u32(&s_m[r]), al = smem_u32(&s_l[0][r]), ah = smem_u32(&s_l[1][r]);
-            const uint32_t ao = smem_u32(smem) + (uint32_t)(r * ATC_LD + lane * 4) * 4u;
-            float mc[ATC_MAX_SPLIT], mm = ATC_NO_MAX;
+    // The gates of OUT_ROWS rows are requested together: with one row at a time a warp waited for
+    // memory eleven times in a row (64 tokens 21.4 -> 17.6 us, 512 tokens 30.9 -> 27.1).
+    constexpr int OUT_ROWS = 4;
+    const int stride = split * (ATC_THREADS / 32);
+    for (int r0 = rank + split * warp; r0 < bt * gqa; r0 += OUT_ROWS * stride) {
+        uint2 gw[OUT_ROWS][2];
 #pragma unroll
-            for (int c = 0; c < ATC_MAX_SPLIT; c++) {
-                mc[c] = c < split ? atc_ld_cluster(cluster_map_shared(am, (uint32_t)c)) : ATC_NO_MAX;
-                mm = fmaxf(mm, mc[c]);
-            }
-            l = 0.0f;
+        for (int u = 0; u < OUT_ROWS; u++) {
+            const int r = r0 + u * stride, tok = t0 + r / gqa;
+            const bool row = r < bt * gqa && tok < n_tokens;
+            const size_t at = ((size_t)tok * hq + kv * gqa + r % gqa) * ATC_D;
 #pragma unroll
-            for (int j = 0; j < 8; j++) o[j] = 0.0f;
+            for (int g = 0; g < 2; g++)
+                gw[u][g] = row ? *reinterpret_cast<const uint2*>(gate + at + g * 128 + lane * 4) : make_uint2(0u, 0u);
+        }
 #pragma unroll
-            for (int c = 0; c < ATC_MAX_SPLIT; c++)
-                if (c < split) {
-                    const float w = expf(mc[c] - mm);
-                    l = fmaf(w, atc_ld_cluster(cluster_map_shared(al, (uint32_t)c)) +
-                                    atc_ld_cluster(cluster_map_shared(ah, (uint32_t)c)), l);
-                    const float4 x = atc_ld_cluster4(cluster_map_shared(ao, (uint32_t)c));
-                    const float4 y = atc_ld_cluster4(cluster_map_shared(ao + 512u, (uint32_t)c));
-                    o[0] = fmaf(w, x.x, o[0]); o[1] = fmaf(w, x.y, o[1]);
-                    o[2] = fmaf(w, x.z, o[2]); o[3] = fmaf(w, x.w, o[3]);
-                    o[4] = fmaf(w, y.x, o[4]); o[5] = fmaf(w, y.y, o[5]);
-                    o[6] = fmaf(w, y.z, o[6]); o[7] = fmaf(w, y.w, o[7]);
+        for (int u = 0; u < OUT_ROWS; u++) {
+            const int r = r0 + u * stride, tok = t0 + r / gqa, h = kv * gqa + r % gqa;
+            if (r >= bt * gqa || tok >= n_tokens) continue;
+            float o[8], l;
+            if (split == 1) {
+                const float* t = reinterpret_cast<const float*>(smem) + r * ATC_LD + lane * 4;
+                const float4 x = *reinterpret_cast<const float4*>(t), y = *reinterpret_cast<const float4*>(t + 128);
+                o[0] = x.x; o[1] = x.y; o[2] = x.z; o[3] = x.w;
+                o[4] = y.x; o[5] = y.y; o[6] = y.z; o[7] = y.w;
+                l = s_l[0][r] + s_l[1][r];
+            } else {
+                const uint32_t am = smem_u32(&s_m[r]), al = smem_u32(&s_l[0][r]), ah = smem_u32(&s_l[1][r]);
+                const uint32_t ao = smem_u32(smem) + (uint32_t)(r * ATC_LD + lane * 4) * 4u;
+                float mc[ATC_MAX_SPLIT], mm = ATC_NO_MAX;
+#pragma unroll
+                for (int c = 0; c < ATC_MAX_SPLIT; c++) {
+                    mc[c] = c < split ? atc_ld_cluster(cluster_map_shared(am, (uint32_t)c)) : ATC_NO_MAX;
+                    mm = fmaxf(mm, mc[c]);
                 }
-        }
-        const float inv = 1.0f / l;
-        bool finite = true;
+                l = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            o[j] = o[j] * (1.0f / ATC_P_SCALE) * inv;
-            finite = finite && (fabsf(o[j]) <= 3.4e38f);
-        }
-        const size_t at = ((size_t)tok * hq + h) * ATC_D;
-        if (!__all_sync(0xffffffffu, finite)) {
-            const size_t base = (size_t)kv * (size_t)max_len * ATC_D;
-            atc_row_plain(q + at, keys + base, values + base, len0 + tok, scale, gate + at, out + at);
-            continue;
-        }
+                for (int j = 0; j < 8; j++) o[j] = 0.0f;
 #pragma unroll
-        for (int g = 0; g < 2; g++) {
-            const uint2 gw = *reinterpret_cast<const uint2*>(gate + at + g * 128 + lane * 4);
-            const float2 g0 = __half22float2(*reinterpret_cast<const __half2*>(&gw.x));
-            const float2 g1 = __half22float2(*reinterpret_cast<const __half2*>(&gw.y));
-            const float gt[4] = {g0.x, g0.y, g1.x, g1.y};
-            float f[4];
+                for (int c = 0; c < ATC_MAX_SPLIT; c++)
+                    if (c < split) {
+                        const float w = expf(mc[c] - mm);
+                        l = fmaf(w, atc_ld_cluster(cluster_map_shared(al, (uint32_t)c)) +
+                                        atc_ld_cluster(cluster_map_shared(ah, (uint32_t)c)), l);
+                        const float4 x = atc_ld_cluster4(cluster_map_shared(ao, (uint32_t)c));
+                        const float4 y = atc_ld_cluster4(cluster_map_shared(ao + 512u, (uint32_t)c));
+                        o[0] = fmaf(w, x.x, o[0]); o[1] = fmaf(w, x.y, o[1]);
+                        o[2] = fmaf(w, x.z, o[2]); o[3] = fmaf(w, x.w, o[3]);
+                        o[4] = fmaf(w, y.x, o[4]); o[5] = fmaf(w, y.y, o[5]);
+                        o[6] = fmaf(w, y.z, o[6]); o[7] = fmaf(w, y.w, o[7]);
+                    }
+            }
+            const float inv = 1.0f / l;
+            bool finite = true;
 #pragma unroll
-            for (int j = 0; j < 4; j++)
-                f[j] = round_f16(o[4 * g + j]) * round_f16(1.0f / (1.0f + expf(-gt[j])));
-            const __half2 w0 = __floats2half2_rn(f[0], f[1]), w1 = __floats2half2_rn(f[2], f[3]);
-            uint2 w;
-            w.x = *reinterpret_cast<const uint32_t*>(&w0);
-            w.y = *reinterpret_cast<const uint32_t*>(&w1);
-            *reinterpret_cast<uint2*>(out + at + g * 128 + lane * 4) = w;
+            for (int j = 0; j < 8; j++) {
+                o[j] = o[j] * (1.0f / ATC_P_SCALE) * inv;
+                finite = finite && (fabsf(o[j]) <= 3.4e38f);
+            }
+            const size_t at = ((size_t)tok * hq + h) * ATC_D;
+            if (!__all_sync(0xffffffffu, finite)) {
+                const size_t base = (size_t)kv * (size_t)max_len * ATC_D;
+                atc_row_plain(q + at, keys + base, values + base, len0 + tok, scale, gate + at, out + at);
+                continue;
+            }
+#pragma unroll
+            for (int g = 0; g < 2; g++) {
+                const float2 g0 = __half22float2(*reinterpret_cast<const __half2*>(&gw[u][g].x));
+                const float2 g1 = __half22float2(*reinterpret_cast<const __half2*>(&gw[u][g].y));
+                const float gt[4] = {g0.x, g0.y, g1.x, g1.y};
+                float f[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    f[j] = round_f16(o[4 * g + j]) * round_f16(1.0f / (1.0f + expf(-gt[j])));
+                const __half2 w0 = __floats2half2_rn(f[0], f[1]), w1 = __floats2half2_rn(f[2], f[3]);
+                uint2 w;
+                w.x = *reinterpret_cast<const uint32_t*>(&w0);
+                w.y = *reinterpret_cast<const uint32_t*>(&w1);
+                *reinterpret_cast<uint2*>(out + at + g * 128 + lane * 4) = w;
+            }
         }
     }
     if (split > 1) cluster_sync_all();       // nobody leaves while a peer still reads its shared memory

@@ -5,8 +5,8 @@
 namespace nvfp4 {
 
 // (token, key) pairs of a chunk from which the tensor-core kernel is the faster one: 64 tokens of an
-// empty cache 25.4 -> 21.4 us, 40 tokens after 64 22.6 -> 21.3; 26 after 64 (2340 pairs) take 20.4 us
-// on the one-query-at-a-time kernel, 16 after 64 11.2.
+// empty cache 25.4 -> 17.6 us, 8 tokens after 511 30.7 -> 11.8; below it the one-query-at-a-time kernel
+// takes 8 to 20 us (16 after 64: 11.2, 26 after 64: 20.4) except for a handful of tokens deep in a context.
 constexpr long long ATTN_TC_MIN_PAIRS = 4096;
 
 // Whether the tensor-core kernel takes this call (sizes and alignment).
