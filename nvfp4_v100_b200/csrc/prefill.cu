@@ -11,11 +11,11 @@
 //   transpose_f16 / add_transposed   layout changes (the second fused with the residual add)
 //   embed_rows                       token ids -> embedding rows
 //   silu_mul_rows                    gate/up rows (interleaved by 8) -> activation rows
-//   dn_conv_tokens, dn_prep, dn_scan, dn_post   one Gated-DeltaNet layer over a chunk:
+//   dn_conv_tokens, dn_block, dn_scan, dn_post   one Gated-DeltaNet layer over a chunk:
 //       causal conv + silu over the chunk with the carried window; q/k L2 norm, beta, decay;
 //       the recurrence S_t = S_{t-1} e^{g_t} + k_t (v_t - S_{t-1} e^{g_t} k_t) beta_t, o_t = S_t q_t
-//       run sequentially over the chunk with every state row in registers (rows are independent:
-//       8 lanes own a row, 16 dims each; 6144 rows of the full model are 768 warps); gated norm.
+//       run over the chunk in blocks of four tokens with every state row in registers (rows are
+//       independent: 16 lanes own two rows, 8 dims each; 6144 rows of the full model); gated norm.
 // Attention uses attn_prep_tokens_kernel (decode_ops.cu) and attn_prefill_group_kernel
 // (fused_ops.cu).
 #include <cstdio>
@@ -199,24 +199,43 @@ dn_conv_state_kernel(const __half* __restrict__ x, long long ld, __half* __restr
     for (int j = 0; j < 4; j++) conv_state[(size_t)c * 4 + j] = nw[j];
 }
 
-// per (token, key head): L2-normalised q (x 128^-1/2) and k as fp32; per (token, value head):
-// beta = f16(sigmoid(b)), decay e^g with g = -exp(A_log) softplus(a + dt_bias).
-// grid (nk + ceil(nv/32), n); 32 threads.
-__global__ void __launch_bounds__(32)
-dn_prep_kernel(const __half* __restrict__ conv_out, int conv_dim, const __half* __restrict__ x,
-               long long ld, const __half* __restrict__ A_log, const __half* __restrict__ dt_bias,
-               float* __restrict__ qn, float* __restrict__ kn, float2* __restrict__ be, int nk,
-               int nv) {
+// The recurrence is evaluated in blocks of DNB tokens (see dn_scan_kernel); per value head and block
+// dn_block_kernel leaves these coefficients, with P(j..i) = e^g_j ... e^g_i:
+//   c[i][m] = P(m+1..i) k_i . k_m for m < i, 0 above
+//   d[i][j] = P(j+1..i) q_i . k_j for j <= i, 0 above
+//   gam[i]  = P(0..i)       (what is left of the state that enters the block when token i sees it)
+//   tail[i] = P(i+1..DNB-1) (what is left of token i's update when the block ends)
+// Tokens past the end of the chunk count as k = q = 0, beta = 0, e^g = 1: they change nothing.
+#define DNB 4
+struct __align__(16) DnBlock {
+    float c[DNB][4];
+    float d[DNB][4];
+    float gam[DNB];
+    float tail[DNB];
+    float beta[DNB];
+};
+
+// One warp per (key head, block of DNB tokens): L2-normalised q (x 128^-1/2) and k as fp32, their
+// products inside the block, and for each value head of the key head beta = f16(sigmoid(b)), the
+// decay e^g with g = -exp(A_log) softplus(a + dt_bias), and the block's coefficients.
+__global__ void __launch_bounds__(128)
+dn_block_kernel(const __half* __restrict__ conv_out, int conv_dim, const __half* __restrict__ x,
+                long long ld, const __half* __restrict__ A_log, const __half* __restrict__ dt_bias,
+                float* __restrict__ qn, float* __restrict__ kn, DnBlock* __restrict__ blocks, int nk,
+                int nv, int n) {
     pdl_prologue();
     PDL_FRESH(conv_out); PDL_FRESH(x); PDL_FRESH(A_log); PDL_FRESH(dt_bias); PDL_FRESH(qn); PDL_FRESH(kn);
-    PDL_FRESH(be);
-    const int t = blockIdx.y, lane = threadIdx.x;
-    const int key_dim = nk * PF_DK;
-    if ((int)blockIdx.x < nk) {
-        const int kh = blockIdx.x;
-        const __half* row = conv_out + (size_t)t * conv_dim;
-        float4 qv, kv;
-        {
+    PDL_FRESH(blocks);
+    const int lane = threadIdx.x & 31, kh = blockIdx.x * 4 + (threadIdx.x >> 5), blk = blockIdx.y;
+    if (kh >= nk) return;
+    const int key_dim = nk * PF_DK, rep = nv / nk;
+    float4 q[DNB], k[DNB];
+#pragma unroll
+    for (int i = 0; i < DNB; i++) {
+        const int t = blk * DNB + i;
+        float4 qv = make_float4(0.0f, 0.0f, 0.0f, 0.0f), kv = qv;
+        if (t < n) {
+            const __half* row = conv_out + (size_t)t * conv_dim;
             const uint2 a = *reinterpret_cast<const uint2*>(row + kh * PF_DK + lane * 4);
             const uint2 b = *reinterpret_cast<const uint2*>(row + key_dim + kh * PF_DK + lane * 4);
             const float2 a0 = __half22float2(*reinterpret_cast<const __half2*>(&a.x));
@@ -230,33 +249,60 @@ dn_prep_kernel(const __half* __restrict__ conv_out, int conv_dim, const __half* 
         const float kss = warp_sum(kv.x * kv.x + kv.y * kv.y + kv.z * kv.z + kv.w * kv.w);
         const float inv_q = rsqrtf(qss + 1e-6f) * 0.08838834764831845f;
         const float inv_k = rsqrtf(kss + 1e-6f);
-        qv.x *= inv_q; qv.y *= inv_q; qv.z *= inv_q; qv.w *= inv_q;
-        kv.x *= inv_k; kv.y *= inv_k; kv.z *= inv_k; kv.w *= inv_k;
+        q[i] = make_float4(qv.x * inv_q, qv.y * inv_q, qv.z * inv_q, qv.w * inv_q);
+        k[i] = make_float4(kv.x * inv_k, kv.y * inv_k, kv.z * inv_k, kv.w * inv_k);
+        // rows up to the end of the block exist in the workspace (zeros past the chunk's end)
         const size_t o = ((size_t)t * nk + kh) * PF_DK + lane * 4;
-        *reinterpret_cast<float4*>(qn + o) = qv;
-        *reinterpret_cast<float4*>(kn + o) = kv;
-    } else {
-        const int h = ((int)blockIdx.x - nk) * 32 + lane;
-        if (h >= nv) return;
-        const __half* row = x + (size_t)t * ld + conv_dim + (size_t)nv * PF_DK;
-        const float beta = round_f16(1.0f / (1.0f + expf(-__half2float(row[h]))));
-        const float g = -expf(__half2float(A_log[h])) *
-                        softplus_pf(__half2float(row[nv + h]) + __half2float(dt_bias[h]));
-        be[(size_t)t * nv + h] = make_float2(beta, expf(g));
+        *reinterpret_cast<float4*>(qn + o) = q[i];
+        *reinterpret_cast<float4*>(kn + o) = k[i];
+    }
+    float kk[DNB][DNB], qk[DNB][DNB];
+#pragma unroll
+    for (int i = 0; i < DNB; i++)
+#pragma unroll
+        for (int j = 0; j <= i; j++) {
+            qk[i][j] = warp_sum(q[i].x * k[j].x + q[i].y * k[j].y + q[i].z * k[j].z + q[i].w * k[j].w);
+            kk[i][j] = j < i ? warp_sum(k[i].x * k[j].x + k[i].y * k[j].y + k[i].z * k[j].z + k[i].w * k[j].w) : 0.0f;
+        }
+    for (int r = lane; r < rep; r += 32) {
+        const int h = kh * rep + r;
+        const float decay = -expf(__half2float(A_log[h])), dt = __half2float(dt_bias[h]);
+        DnBlock w;
+        float eg[DNB];
+#pragma unroll
+        for (int i = 0; i < DNB; i++) {
+            const int t = blk * DNB + i;
+            eg[i] = 1.0f;
+            w.beta[i] = 0.0f;
+            if (t < n) {
+                const __half* row = x + (size_t)t * ld + conv_dim + (size_t)nv * PF_DK;
+                w.beta[i] = round_f16(1.0f / (1.0f + expf(-__half2float(row[h]))));
+                eg[i] = expf(decay * softplus_pf(__half2float(row[nv + h]) + dt));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < DNB; i++) {
+            float p = 1.0f;                       // P(j+1..i) while j counts down
+#pragma unroll
+            for (int j = DNB - 1; j >= 0; j--) {
+                w.c[i][j] = w.d[i][j] = 0.0f;
+                if (j <= i) {
+                    if (j < i) p *= eg[j + 1];
+                    w.c[i][j] = j < i ? p * kk[i][j] : 0.0f;
+                    w.d[i][j] = p * qk[i][j];
+                }
+            }
+            w.gam[i] = p * eg[0];
+        }
+        float p = 1.0f;
+#pragma unroll
+        for (int i = DNB - 1; i >= 0; i--) {
+            w.tail[i] = p;
+            p *= eg[i];
+        }
+        blocks[(size_t)blk * nv + h] = w;
     }
 }
-
-// The recurrence over the chunk.  CTA = 4 warps = 16 state rows of one value head (384 CTAs for
-// the full model: two or three per SM); a warp owns 4 rows, one per 8-lane group gi = lane >> 3;
-// lane sub = lane & 7 owns dims 32 j + 4 sub .. + 3 (j = 0..3) of its row, so the 8 lanes of a
-// group read one contiguous 128-byte piece of a vector at a time.  The operands of SCAN_TB tokens (the head's
-// normalised k and q, this CTA's 32 values of v, beta and decay) are staged in shared memory by
-// cp.async, double buffered, so the sequential chain never waits on global memory.
-// o[t][h*128 + row] = f16(S_t[row] . q_t).
-#define SCAN_WARPS 4
-#define SCAN_RPG 1                          // state rows per 8-lane group
-#define SCAN_ROWS (SCAN_WARPS * 4 * SCAN_RPG)
-#define SCAN_TB 16
 
 // packed fp32 pair arithmetic (two IEEE fp32 operations per instruction)
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
@@ -275,13 +321,6 @@ __device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
     return d;
 }
 
-struct ScanStage {
-    float k[SCAN_TB][PF_DK];
-    float q[SCAN_TB][PF_DK];
-    __half v[SCAN_TB][SCAN_ROWS];
-    float2 be[SCAN_TB];
-};
-
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gsrc) : "memory");
@@ -292,136 +331,216 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
+// The recurrence over the chunk, DNB = 4 tokens at a time.  Token by token,
+//   delta_t = beta_t (v_t - e^g_t S k_t),  S <- e^g_t S + k_t delta_t,  o_t = S q_t,
+// is a chain of two reductions over the lanes per token.  For a block of tokens all dot products can
+// be taken with the state that ENTERS it, because what the block's own tokens add to S k_i and S q_i
+// is known from their keys (coefficients of dn_block_kernel):
+//   delta_i = beta_i (v_i - gam_i S k_i - sum_{m<i} c_im delta_m)
+//   o_i = gam_i S q_i + sum_{j<=i} d_ij delta_j,   S <- gam_3 S + sum_i tail_i delta_i k_i
+// so a block has ONE reduction and the state is scaled once.  Exact algebra, fp32 throughout.
+// Two value rows' 256 state values live in the registers of 16 lanes (lane sub owns dims 64 j + 4 sub
+// .. + 3 of both); a warp holds 4 rows.  The 16 sums of a block (8 per row) are reduced transposed:
+// a lane gives away the half it will not own, four times (15 shuffles), and ends with one sum.  Bound by
+// shared-memory wavefronts (k and q are read by every warp) and the length of the chain: one row in
+// 8 lanes needs twice the reads of k and q (162 us for 512 tokens of 48 heads against 131), two rows in
+// 8 lanes leave half of the warps (slower still); one token at a time took 231.
+// Operands of SCAN_TB tokens are staged in shared memory by cp.async, double buffered, so the chain
+// never waits on global memory.  o[t][h*128 + row] = f16(o_t[row]).
+#define SCAN_WARPS 4
+#define SCAN_ROWS (SCAN_WARPS * 4)
+#define SCAN_TB 16
+#define SCAN_NB (SCAN_TB / DNB)
+
+struct ScanStage {
+    float k[SCAN_TB][PF_DK];
+    float q[SCAN_TB][PF_DK];
+    DnBlock b[SCAN_NB];
+    __half v[SCAN_TB][SCAN_ROWS];
+};
+
 __global__ void __launch_bounds__(SCAN_WARPS * 32)
 dn_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
-               const float2* __restrict__ be, const __half* __restrict__ conv_out, int conv_dim,
+               const DnBlock* __restrict__ blocks, const __half* __restrict__ conv_out, int conv_dim,
                float* __restrict__ state, __half* __restrict__ o_out, int nk, int nv, int n) {
     pdl_prologue();
-    PDL_FRESH(qn); PDL_FRESH(kn); PDL_FRESH(be); PDL_FRESH(conv_out); PDL_FRESH(state); PDL_FRESH(o_out);
+    PDL_FRESH(qn); PDL_FRESH(kn); PDL_FRESH(blocks); PDL_FRESH(conv_out); PDL_FRESH(state); PDL_FRESH(o_out);
     __shared__ __align__(16) ScanStage stage[2];
     const int per_head = PF_DK / SCAN_ROWS;                  // CTAs per value head
     const int h = blockIdx.x / per_head, part = blockIdx.x % per_head;
     const int kh = h / (nv / nk);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int gi = lane >> 3, sub = lane & 7;
-    const int lrow = (warp * 4 + gi) * SCAN_RPG;             // first of this lane's rows, in the CTA
+    const int sub = lane & 15, mine = (lane >> 3) & 1, s8 = lane & 7;
+    const int lrow = warp * 4 + (lane >> 4) * 2;             // first of this lane's two rows, in the CTA
     const int row0 = part * SCAN_ROWS + lrow;
     const int key_dim = nk * PF_DK;
+    const int nb = (n + DNB - 1) / DNB;
 
-    // stage the operands of tokens [t0, t0 + SCAN_TB) (clamped to the chunk) into buffer b
-    auto issue = [&](int t0, int b) {
+    // stage the operands of blocks [b0, b0 + SCAN_NB) into buffer b; blocks past the end are not read
+    auto issue = [&](int b0, int b) {
         ScanStage& s = stage[b];
-        for (int i = tid; i < SCAN_TB * (PF_DK / 4); i += SCAN_WARPS * 32) {   // 16-byte pieces
+        const int nblk = min(SCAN_NB, nb - b0), nt = nblk * DNB, t0 = b0 * DNB;
+        for (int i = tid; i < nt * (PF_DK / 4); i += SCAN_WARPS * 32) {   // 16-byte pieces
             const int tt = i / (PF_DK / 4), c = i % (PF_DK / 4);
-            const int t = min(t0 + tt, n - 1);
-            const size_t o = ((size_t)t * nk + kh) * PF_DK + c * 4;
+            const size_t o = ((size_t)(t0 + tt) * nk + kh) * PF_DK + c * 4;
             cp_async_16(&s.k[tt][c * 4], kn + o);
             cp_async_16(&s.q[tt][c * 4], qn + o);
         }
-        if (tid < SCAN_TB * (SCAN_ROWS / 8)) {
-            const int tt = tid / (SCAN_ROWS / 8), c = tid % (SCAN_ROWS / 8);
+        for (int i = tid; i < nt * (SCAN_ROWS / 8); i += SCAN_WARPS * 32) {
+            const int tt = i / (SCAN_ROWS / 8), c = i % (SCAN_ROWS / 8);
             const int t = min(t0 + tt, n - 1);
             cp_async_16(&s.v[tt][c * 8], conv_out + (size_t)t * conv_dim + 2 * key_dim + h * PF_DK +
                                              part * SCAN_ROWS + c * 8);
         }
-        if (tid >= 64 && tid < 64 + SCAN_TB) {
-            const int tt = tid - 64;
-            s.be[tt] = be[(size_t)min(t0 + tt, n - 1) * nv + h];
-        }
+        constexpr int BP = (int)sizeof(DnBlock) / 16;
+        if (tid < nblk * BP)
+            cp_async_16(reinterpret_cast<uint8_t*>(&s.b[tid / BP]) + (tid % BP) * 16,
+                        reinterpret_cast<const uint8_t*>(blocks + (size_t)(b0 + tid / BP) * nv + h) + (tid % BP) * 16);
         cp_async_commit();
     };
 
-    __align__(8) float S[SCAN_RPG][16];
+    float2 S[2][4];
     float* sp = state + ((size_t)h * PF_DK + row0) * PF_DK + sub * 4;
 #pragma unroll
-    for (int r = 0; r < SCAN_RPG; r++)
+    for (int r = 0; r < 2; r++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float4 v = *reinterpret_cast<const float4*>(sp + (size_t)r * PF_DK + j * 32);
-            S[r][4 * j] = v.x; S[r][4 * j + 1] = v.y; S[r][4 * j + 2] = v.z; S[r][4 * j + 3] = v.w;
+        for (int j = 0; j < 2; j++) {
+            const float4 v = *reinterpret_cast<const float4*>(sp + (size_t)r * PF_DK + j * 64);
+            S[r][2 * j] = make_float2(v.x, v.y);
+            S[r][2 * j + 1] = make_float2(v.z, v.w);
         }
 
-    const int nblk = (n + SCAN_TB - 1) / SCAN_TB;
-    if (nblk > 0) issue(0, 0);
-    for (int blk = 0; blk < nblk; blk++) {
-        const int cur = blk & 1;
-        if (blk + 1 < nblk) {
-            issue((blk + 1) * SCAN_TB, cur ^ 1);
+    const int nst = (nb + SCAN_NB - 1) / SCAN_NB;
+    issue(0, 0);
+    for (int st = 0; st < nst; st++) {
+        const int cur = st & 1;
+        if (st + 1 < nst) {
+            issue((st + 1) * SCAN_NB, cur ^ 1);
             cp_async_wait<1>();
         } else {
             cp_async_wait<0>();
         }
         __syncthreads();
         const ScanStage& s = stage[cur];
-        const int tcount = min(SCAN_TB, n - blk * SCAN_TB);
-        for (int tt = 0; tt < tcount; tt++) {
-            // the row's 16 state values, k and q as 8 fp32 pairs: packed fp32x2 multiply-adds
-            // halve the instruction count of the scan, which is issue-bound
-            float2 kc[8], qc[8];
+        const int bcount = min(SCAN_NB, nb - st * SCAN_NB);
+        for (int bb = 0; bb < bcount; bb++) {
+            float2 k[DNB][4];
+            float dot[2][2 * DNB];                           // S k_i, then S q_i: this lane's part
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const float4 a = *reinterpret_cast<const float4*>(&s.k[tt][j * 32 + sub * 4]);
-                const float4 c = *reinterpret_cast<const float4*>(&s.q[tt][j * 32 + sub * 4]);
-                kc[2 * j] = make_float2(a.x, a.y); kc[2 * j + 1] = make_float2(a.z, a.w);
-                qc[2 * j] = make_float2(c.x, c.y); qc[2 * j + 1] = make_float2(c.z, c.w);
-            }
-            const float2 bd = s.be[tt];
-            const float beta = bd.x;
-            const float2 eg2 = make_float2(bd.y, bd.y);
-            float vr[SCAN_RPG], kvp[SCAN_RPG], od[SCAN_RPG];
+            for (int i = 0; i < DNB; i++) {
+                const float* ks = &s.k[bb * DNB + i][sub * 4];
+                const float* qs = &s.q[bb * DNB + i][sub * 4];
+                const float4 k0 = *reinterpret_cast<const float4*>(ks), k1 = *reinterpret_cast<const float4*>(ks + 64);
+                const float4 q0 = *reinterpret_cast<const float4*>(qs), q1 = *reinterpret_cast<const float4*>(qs + 64);
+                const float2 q[4] = {make_float2(q0.x, q0.y), make_float2(q0.z, q0.w), make_float2(q1.x, q1.y),
+                                     make_float2(q1.z, q1.w)};
+                k[i][0] = make_float2(k0.x, k0.y);
+                k[i][1] = make_float2(k0.z, k0.w);
+                k[i][2] = make_float2(k1.x, k1.y);
+                k[i][3] = make_float2(k1.z, k1.w);
 #pragma unroll
-            for (int r = 0; r < SCAN_RPG; r++) vr[r] = __half2float(s.v[tt][lrow + r]);
+                for (int r = 0; r < 2; r++) {
+                    float2 ak = fmul2(S[r][0], k[i][0]), aq = fmul2(S[r][0], q[0]);
 #pragma unroll
-            for (int r = 0; r < SCAN_RPG; r++) {
-                float2* S2 = reinterpret_cast<float2*>(S[r]);
-                float2 a[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {            // four independent partial sums (pairs)
-                    S2[2 * j] = fmul2(S2[2 * j], eg2);
-                    S2[2 * j + 1] = fmul2(S2[2 * j + 1], eg2);
-                    a[j] = fmul2(S2[2 * j], kc[2 * j]);
-                    a[j] = ffma2(S2[2 * j + 1], kc[2 * j + 1], a[j]);
+                    for (int j = 1; j < 4; j++) {
+                        ak = ffma2(S[r][j], k[i][j], ak);
+                        aq = ffma2(S[r][j], q[j], aq);
+                    }
+                    dot[r][i] = ak.x + ak.y;
+                    dot[r][DNB + i] = aq.x + aq.y;
                 }
-                kvp[r] = ((a[0].x + a[0].y) + (a[1].x + a[1].y)) + ((a[2].x + a[2].y) + (a[3].x + a[3].y));
             }
+            // lane sub ends with sum s8 of row `mine`
+            float own;
+            {
+                float w8[8], w4[4], w2[2];
 #pragma unroll
-            for (int o = 1; o < 8; o <<= 1)
+                for (int a = 0; a < 8; a++)
+                    w8[a] = (mine ? dot[1][a] : dot[0][a]) + __shfl_xor_sync(0xffffffffu, mine ? dot[0][a] : dot[1][a], 8);
 #pragma unroll
-                for (int r = 0; r < SCAN_RPG; r++) kvp[r] += __shfl_xor_sync(0xffffffffu, kvp[r], o);
+                for (int a = 0; a < 4; a++)
+                    w4[a] = ((s8 & 4) ? w8[a + 4] : w8[a]) + __shfl_xor_sync(0xffffffffu, (s8 & 4) ? w8[a] : w8[a + 4], 4);
 #pragma unroll
-            for (int r = 0; r < SCAN_RPG; r++) {
-                float2* S2 = reinterpret_cast<float2*>(S[r]);
-                const float delta = (vr[r] - kvp[r]) * beta;
-                const float2 d2 = make_float2(delta, delta);
-                float2 a[4];
+                for (int a = 0; a < 2; a++)
+                    w2[a] = ((s8 & 2) ? w4[a + 2] : w4[a]) + __shfl_xor_sync(0xffffffffu, (s8 & 2) ? w4[a] : w4[a + 2], 2);
+                own = ((s8 & 1) ? w2[1] : w2[0]) + __shfl_xor_sync(0xffffffffu, (s8 & 1) ? w2[0] : w2[1], 1);
+            }
+            const DnBlock& w = s.b[bb];
+            const float4 gam = *reinterpret_cast<const float4*>(w.gam);
+            const float4 beta = *reinterpret_cast<const float4*>(w.beta);
+            const float4 tail = *reinterpret_cast<const float4*>(w.tail);
+            const float4 c1 = *reinterpret_cast<const float4*>(w.c[1]);
+            const float4 c2 = *reinterpret_cast<const float4*>(w.c[2]);
+            const float4 c3 = *reinterpret_cast<const float4*>(w.c[3]);
+            const float4 d = *reinterpret_cast<const float4*>(w.d[s8 & 3]);
+            const float gq = w.gam[s8 & 3];
+            const int t0 = (st * SCAN_NB + bb) * DNB;
+            float p[DNB], v[DNB];
+#pragma unroll
+            for (int i = 0; i < DNB; i++) {
+                p[i] = __shfl_sync(0xffffffffu, own, (lane & 24) + i);
+                v[i] = t0 + i < n ? __half2float(s.v[bb * DNB + i][lrow + mine]) : 0.0f;
+            }
+            const float e0 = beta.x * (v[0] - gam.x * p[0]);
+            const float e1 = beta.y * ((v[1] - gam.y * p[1]) - c1.x * e0);
+            const float e2 = beta.z * (((v[2] - gam.z * p[2]) - c2.x * e0) - c2.y * e1);
+            const float e3 = beta.w * ((((v[3] - gam.w * p[3]) - c3.x * e0) - c3.y * e1) - c3.z * e2);
+            const float f[DNB] = {e0 * tail.x, e1 * tail.y, e2 * tail.z, e3 * tail.w};
+            float g[DNB];                                    // the other row's
+#pragma unroll
+            for (int i = 0; i < DNB; i++) g[i] = __shfl_xor_sync(0xffffffffu, f[i], 8);
+            const float2 g2 = make_float2(gam.w, gam.w);
+#pragma unroll
+            for (int r = 0; r < 2; r++)
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    S2[2 * j] = ffma2(kc[2 * j], d2, S2[2 * j]);
-                    S2[2 * j + 1] = ffma2(kc[2 * j + 1], d2, S2[2 * j + 1]);
-                    a[j] = fmul2(S2[2 * j], qc[2 * j]);
-                    a[j] = ffma2(S2[2 * j + 1], qc[2 * j + 1], a[j]);
+                    float2 a = fmul2(S[r][j], g2);
+#pragma unroll
+                    for (int i = 0; i < DNB; i++) {
+                        const float fi = mine == r ? f[i] : g[i];
+                        a = ffma2(k[i][j], make_float2(fi, fi), a);
+                    }
+                    S[r][j] = a;
                 }
-                od[r] = ((a[0].x + a[0].y) + (a[1].x + a[1].y)) + ((a[2].x + a[2].y) + (a[3].x + a[3].y));
-            }
-#pragma unroll
-            for (int o = 1; o < 8; o <<= 1)
-#pragma unroll
-                for (int r = 0; r < SCAN_RPG; r++) od[r] += __shfl_xor_sync(0xffffffffu, od[r], o);
-            if (sub == 0) {
-#pragma unroll
-                for (int r = 0; r < SCAN_RPG; r++)
-                    o_out[((size_t)(blk * SCAN_TB + tt) * nv + h) * PF_DK + row0 + r] =
-                        __float2half(od[r]);
+            if (s8 >= 4 && t0 + (s8 & 3) < n) {              // token s8 - 4 of the block
+                // a later token's delta stays out even if it is not finite
+                float o = fmaf(d.x, e0, gq * own);
+                if (s8 >= 5) o = fmaf(d.y, e1, o);
+                if (s8 >= 6) o = fmaf(d.z, e2, o);
+                if (s8 >= 7) o = fmaf(d.w, e3, o);
+                o_out[((size_t)(t0 + (s8 & 3)) * nv + h) * PF_DK + row0 + mine] = __float2half(o);
             }
         }
         __syncthreads();     // everyone is done with this buffer before it is refilled
     }
 #pragma unroll
-    for (int r = 0; r < SCAN_RPG; r++)
+    for (int r = 0; r < 2; r++)
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-            *reinterpret_cast<float4*>(sp + (size_t)r * PF_DK + j * 32) =
-                make_float4(S[r][4 * j], S[r][4 * j + 1], S[r][4 * j + 2], S[r][4 * j + 3]);
+        for (int j = 0; j < 2; j++)
+            *reinterpret_cast<float4*>(sp + (size_t)r * PF_DK + j * 64) =
+                make_float4(S[r][2 * j].x, S[r][2 * j].y, S[r][2 * j + 1].x, S[r][2 * j + 1].y);
+}
+
+// Unused dynamic shared memory that lets no SM take more than its share of the scan's CTAs.  They are
+// launched while the kernel before still holds some SMs (programmatic dependent launch) and would
+// otherwise crowd the free ones, for the whole chunk: a layer of 512 tokens 249 -> 180 us.
+static size_t scan_padding(int ctas) {
+    static int sms[NVFP4_MAX_DEVICES] = {0};
+    static int opted[NVFP4_MAX_DEVICES] = {0};
+    constexpr int SM_BYTES = 227 * 1024, RESERVED = 1024;
+    const int dev = current_device_index();
+    if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    const int per_sm = (ctas + sms[dev] - 1) / sms[dev];
+    const int pad = (SM_BYTES / per_sm - RESERVED - (int)(2 * sizeof(ScanStage))) & ~127;
+    if (pad <= 0) return 0;
+    if (pad > opted[dev]) {
+        if (cudaFuncSetAttribute(dn_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pad) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        opted[dev] = pad;
+    }
+    return (size_t)pad;
 }
 
 // gated norm per (token, value head): out = f16( f32(f16(o rsqrt(mean(o^2) + eps)) * norm_w) * silu(z) )
@@ -500,8 +619,9 @@ long long nvfp4_dn_prefill_work_bytes(int n, int nk, int nv) {
     const long long conv_dim = (2LL * nk + nv) * PF_DK;
     long long b = (long long)n * conv_dim * 2;            // conv output, fp16
     b = (b + 255) & ~255LL;
-    b += 2LL * n * nk * PF_DK * 4;                         // normalised q and k, fp32
-    b += (long long)n * nv * 8;                            // (beta, decay)
+    const long long nb = (n + DNB - 1) / DNB;              // blocks of the recurrence
+    b += 2LL * nb * DNB * nk * PF_DK * 4;                  // normalised q and k, fp32
+    b += nb * nv * (long long)sizeof(nvfp4::DnBlock);      // the blocks' coefficients
     b = (b + 255) & ~255LL;
     b += (long long)n * nv * PF_DK * 2;                    // recurrence output, fp16
     return b + 256;
@@ -525,10 +645,11 @@ int launch_dn_prefill(const void* x, long long ld, const void* conv_w, void* con
     __half* conv_out = (__half*)w;
     long long off = ((long long)n * conv_dim * 2 + 255) & ~255LL;
     float* qn = (float*)(w + off);
-    float* kn = qn + (size_t)n * nk * PF_DK;
-    off += 2LL * n * nk * PF_DK * 4;
-    float2* be = (float2*)(w + off);
-    off = (off + (long long)n * nv * 8 + 255) & ~255LL;
+    const int nb = (n + DNB - 1) / DNB;
+    float* kn = qn + (size_t)nb * DNB * nk * PF_DK;
+    off += 2LL * nb * DNB * nk * PF_DK * 4;
+    nvfp4::DnBlock* blocks = (nvfp4::DnBlock*)(w + off);
+    off = (off + (long long)nb * nv * (long long)sizeof(nvfp4::DnBlock) + 255) & ~255LL;
     __half* o16 = (__half*)(w + off);
     cudaStream_t st = (cudaStream_t)stream;
     const __half* xh = (const __half*)x;
@@ -539,14 +660,15 @@ int launch_dn_prefill(const void* x, long long ld, const void* conv_w, void* con
     ok = ok && nvfp4::launch_pdl(nvfp4::dn_conv_state_kernel, dim3((conv_dim + 255) / 256),
                                  dim3(256), 0, st, xh, ld, (__half*)conv_state, conv_dim,
                                  n) == cudaSuccess;
-    ok = ok && nvfp4::launch_pdl(nvfp4::dn_prep_kernel, dim3(nk + (nv + 31) / 32, n), dim3(32), 0,
+    ok = ok && nvfp4::launch_pdl(nvfp4::dn_block_kernel, dim3((nk + 3) / 4, nb), dim3(128), 0,
                                  st, (const __half*)conv_out, conv_dim, xh, ld,
-                                 (const __half*)A_log, (const __half*)dt_bias, qn, kn, be, nk,
-                                 nv) == cudaSuccess;
+                                 (const __half*)A_log, (const __half*)dt_bias, qn, kn, blocks, nk,
+                                 nv, n) == cudaSuccess;
     ok = ok && nvfp4::launch_pdl(nvfp4::dn_scan_kernel, dim3(nv * (PF_DK / SCAN_ROWS)),
-                                 dim3(SCAN_WARPS * 32), 0, st, (const float*)qn, (const float*)kn,
-                                 (const float2*)be, (const __half*)conv_out, conv_dim,
-                                 (float*)state, o16, nk, nv, n) == cudaSuccess;
+                                 dim3(SCAN_WARPS * 32), nvfp4::scan_padding(nv * (PF_DK / SCAN_ROWS)), st,
+                                 (const float*)qn, (const float*)kn, (const nvfp4::DnBlock*)blocks,
+                                 (const __half*)conv_out, conv_dim, (float*)state, o16, nk, nv,
+                                 n) == cudaSuccess;
     ok = ok && nvfp4::launch_pdl(nvfp4::dn_post_kernel, dim3(nv, n), dim3(32), 0, st,
                                  (const __half*)o16, xh, ld, conv_dim, (const __half*)norm_w,
                                  (__half*)out, nv, rms_eps) == cudaSuccess;
