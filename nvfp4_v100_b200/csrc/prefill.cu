@@ -124,26 +124,37 @@ embed_rows_kernel(const __half* __restrict__ table, const long long* __restrict_
 
 // Token-minor gate/up rows, interleaved in groups of 8 (rows 16j..16j+7 gate, 16j+8..16j+15 up),
 // to activation rows: act[8j + r][t] = f16( f32(f16(silu(g))) * u ), the silu_mul_kernel chain.
+// VEC: eight tokens a thread, 16-byte accesses (N a multiple of 8, 16-byte aligned matrices); otherwise
+// one.  The grid is flat over rows x token groups (17408 rows of 512 tokens 18.6 -> 11.3 us, of 27 tokens
+// 18.6 -> 2.5, against a CTA per row and 4 bytes a thread).
+template <bool VEC>
 __global__ void __launch_bounds__(256)
 silu_mul_rows_kernel(const __half* __restrict__ gu, __half* __restrict__ act, int inter, int N) {
     pdl_prologue();
     PDL_FRESH(gu); PDL_FRESH(act);
-    const int row = blockIdx.y;                       // activation row 0 .. inter-1
-    const int t = (blockIdx.x * 256 + threadIdx.x) * 2;
-    if (t >= N) return;
+    constexpr int W = VEC ? 8 : 1;
+    const int groups = N / W;
+    const long long id = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (id >= (long long)inter * groups) return;
+    const int row = (int)(id / groups), t = (int)(id % groups) * W;   // activation row 0 .. inter-1
     const size_t grow = (size_t)(row >> 3) * 16 + (row & 7);
     const __half* g = gu + grow * N + t;
     const __half* u = gu + (grow + 8) * N + t;
     __half* o = act + (size_t)row * N + t;
-    if (t + 1 < N && (N & 1) == 0) {
-        const float2 gf = __half22float2(*reinterpret_cast<const __half2*>(g));
-        const float2 uf = __half22float2(*reinterpret_cast<const __half2*>(u));
-        *reinterpret_cast<__half2*>(o) =
-            __floats2half2_rn(round_f16(silu_pf(gf.x)) * uf.x, round_f16(silu_pf(gf.y)) * uf.y);
+    if (VEC) {
+        const uint4 gv = *reinterpret_cast<const uint4*>(g), uv = *reinterpret_cast<const uint4*>(u);
+        const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
+        uint32_t ow[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float2 gf = __half22float2(*reinterpret_cast<const __half2*>(&gw[k]));
+            const float2 uf = __half22float2(*reinterpret_cast<const __half2*>(&uw[k]));
+            const __half2 r = __floats2half2_rn(round_f16(silu_pf(gf.x)) * uf.x, round_f16(silu_pf(gf.y)) * uf.y);
+            ow[k] = *reinterpret_cast<const uint32_t*>(&r);
+        }
+        *reinterpret_cast<uint4*>(o) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
     } else {
-        for (int k = t; k < N && k < t + 2; k++)
-            act[(size_t)row * N + k] = __float2half(
-                round_f16(silu_pf(__half2float(gu[grow * N + k]))) * __half2float(gu[(grow + 8) * N + k]));
+        *o = __float2half(round_f16(silu_pf(__half2float(*g))) * __half2float(*u));
     }
 }
 
@@ -153,50 +164,71 @@ silu_mul_rows_kernel(const __half* __restrict__ gu, __half* __restrict__ act, in
 // ---------------------------------------------------------------------------------------------
 #define PF_DK 128
 
-// conv[t][c] = f16(silu(w0 x[t-3] + w1 x[t-2] + w2 x[t-1] + w3 x[t])), inputs before the chunk
-// taken from the carried window state[c][0..3] (state[c][3] is the newest).
-__global__ void __launch_bounds__(256)
-dn_conv_tokens_kernel(const __half* __restrict__ x, long long ld, const __half* __restrict__ conv_w,
-                      const __half* __restrict__ conv_state, __half* __restrict__ conv_out,
-                      int conv_dim) {
-    pdl_prologue();
-    PDL_FRESH(x); PDL_FRESH(conv_w); PDL_FRESH(conv_state); PDL_FRESH(conv_out);
-    const int c = blockIdx.x * 256 + threadIdx.x;
-    const int t = blockIdx.y;
-    if (c >= conv_dim) return;
-    float win[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int tt = t - 3 + j;    // input index of tap j
-        win[j] = (tt >= 0) ? __half2float(x[(size_t)tt * ld + c])
-                           : __half2float(conv_state[(size_t)c * 4 + 4 + tt]);
-    }
-    const __half* w = conv_w + (size_t)c * 4;
-    float acc = __half2float(w[0]) * win[0];
-    acc = fmaf(__half2float(w[1]), win[1], acc);
-    acc = fmaf(__half2float(w[2]), win[2], acc);
-    acc = fmaf(__half2float(w[3]), win[3], acc);
-    conv_out[(size_t)t * conv_dim + c] = __float2half(silu_pf(acc));
+// the four halves of a channel's window or weights: one 8-byte access where the pointer allows it
+__device__ __forceinline__ uint2 ld_half4(const __half* p) {
+    if (((uintptr_t)p & 7) == 0) return *reinterpret_cast<const uint2*>(p);
+    const __half2 lo = __halves2half2(p[0], p[1]), hi = __halves2half2(p[2], p[3]);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
-// carried window after the chunk: the last four inputs
-__global__ void __launch_bounds__(256)
-dn_conv_state_kernel(const __half* __restrict__ x, long long ld, __half* __restrict__ conv_state,
-                     int conv_dim, int n) {
+// conv[t][c] = f16(silu(w0 x[t-3] + w1 x[t-2] + w2 x[t-1] + w3 x[t])), inputs before the chunk
+// taken from the carried window state[c][0..3] (state[c][3] is the newest).  A thread owns four
+// adjacent channels and T tokens, so every input is loaded once (8 bytes at a time) plus the three before
+// its first token.  T = 8 for long chunks (512 tokens of 10240 channels 24.1 -> 11.2 us against a thread
+// per channel and token); short ones would leave most SMs empty and take T = 2.
+template <int T>
+__global__ void __launch_bounds__(128)
+dn_conv_tokens_kernel(const __half* __restrict__ x, long long ld, const __half* __restrict__ conv_w,
+                      const __half* __restrict__ conv_state, __half* __restrict__ conv_out,
+                      int conv_dim, int n) {
     pdl_prologue();
-    PDL_FRESH(x); PDL_FRESH(conv_state);
-    const int c = blockIdx.x * 256 + threadIdx.x;
+    PDL_FRESH(x); PDL_FRESH(conv_w); PDL_FRESH(conv_state); PDL_FRESH(conv_out);
+    const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
+    const int t0 = blockIdx.y * T;
     if (c >= conv_dim) return;
-    __half old[4], nw[4];
+    auto unpack = [](const uint2 u, float (&f)[4]) {
+        const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
+        const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+        f[0] = lo.x; f[1] = lo.y; f[2] = hi.x; f[3] = hi.y;
+    };
+    float w[4][4];                     // channel, tap
 #pragma unroll
-    for (int j = 0; j < 4; j++) old[j] = conv_state[(size_t)c * 4 + j];
+    for (int e = 0; e < 4; e++) unpack(ld_half4(conv_w + (size_t)(c + e) * 4), w[e]);
+    float win[T + 3][4];               // token t0 - 3 + i, channel
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int tt = n - 4 + j;
-        nw[j] = (tt >= 0) ? x[(size_t)tt * ld + c] : old[4 + tt];
+    for (int i = 0; i < T + 3; i++) {
+        const int t = t0 - 3 + i;
+        uint2 u = make_uint2(0u, 0u);
+        if (t >= 0 && t < n) u = *reinterpret_cast<const uint2*>(x + (size_t)t * ld + c);
+        unpack(u, win[i]);
+    }
+    if (t0 < 3) {                      // (T = 2: the second strip still reaches back to the carried window)
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            float old[4];
+            unpack(ld_half4(conv_state + (size_t)(c + e) * 4), old);
+#pragma unroll
+            for (int i = 0; i < 3; i++)          // input t < 0 is old[4 + t]
+                if (t0 == 0) win[i][e] = old[1 + i];
+                else if (t0 == 2 && i == 0) win[i][e] = old[3];
+        }
     }
 #pragma unroll
-    for (int j = 0; j < 4; j++) conv_state[(size_t)c * 4 + j] = nw[j];
+    for (int i = 0; i < T; i++) {
+        if (t0 + i >= n) break;
+        float r[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            float acc = w[e][0] * win[i][e];
+            acc = fmaf(w[e][1], win[i + 1][e], acc);
+            acc = fmaf(w[e][2], win[i + 2][e], acc);
+            acc = fmaf(w[e][3], win[i + 3][e], acc);
+            r[e] = silu_pf(acc);
+        }
+        const __half2 lo = __floats2half2_rn(r[0], r[1]), hi = __floats2half2_rn(r[2], r[3]);
+        *reinterpret_cast<uint2*>(conv_out + (size_t)(t0 + i) * conv_dim + c) =
+            make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
 }
 
 // The recurrence is evaluated in blocks of DNB tokens (see dn_scan_kernel); per value head and block
@@ -544,14 +576,31 @@ static size_t scan_padding(int ctas) {
 }
 
 // gated norm per (token, value head): out = f16( f32(f16(o rsqrt(mean(o^2) + eps)) * norm_w) * silu(z) )
-// grid (nv, n), 32 threads, lane owns 4 of the head's 128 outputs.
-__global__ void __launch_bounds__(32)
+// A warp per (token, head), lane owns 4 of the head's 128 outputs; eight warps a CTA (one-warp
+// CTAs: 27.4 -> 8.7 us for 512 tokens of 48 heads).  The kernel also stores the carried conv window (the
+// last four inputs): the conv kernel, which reads the old one, has finished by then.  The grid covers
+// conv_dim threads.
+__global__ void __launch_bounds__(256)
 dn_post_kernel(const __half* __restrict__ o_in, const __half* __restrict__ x, long long ld,
-               int conv_dim, const __half* __restrict__ norm_w, __half* __restrict__ out, int nv,
-               float rms_eps) {
+               int conv_dim, const __half* __restrict__ norm_w, __half* __restrict__ out,
+               __half* __restrict__ conv_state, int nv, int n, float rms_eps) {
     pdl_prologue();
-    PDL_FRESH(o_in); PDL_FRESH(x); PDL_FRESH(norm_w); PDL_FRESH(out);
-    const int h = blockIdx.x, t = blockIdx.y, lane = threadIdx.x;
+    PDL_FRESH(o_in); PDL_FRESH(x); PDL_FRESH(norm_w); PDL_FRESH(out); PDL_FRESH(conv_state);
+    const int id = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int t = id / nv, h = id % nv;
+    if (const int c = blockIdx.x * 256 + threadIdx.x; c < conv_dim) {
+        __half old[4], nw[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) old[j] = conv_state[(size_t)c * 4 + j];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int tt = n - 4 + j;
+            nw[j] = (tt >= 0) ? x[(size_t)tt * ld + c] : old[4 + tt];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) conv_state[(size_t)c * 4 + j] = nw[j];
+    }
+    if (t >= n) return;
     const uint2 ov = *reinterpret_cast<const uint2*>(o_in + ((size_t)t * nv + h) * PF_DK + lane * 4);
     const __half* oh = reinterpret_cast<const __half*>(&ov);
     float o[4], ss = 0.0f;
@@ -608,8 +657,10 @@ int launch_embed_rows(const void* table, const void* ids, void* out, int n, int 
 // gu: token-minor [2 * inter][N] with gate/up rows interleaved in groups of 8; act: [inter][N].
 int launch_silu_mul_rows(const void* gu, void* act, int inter, int N, void* stream) {
     if (!gu || !act || inter <= 0 || inter % 8 != 0 || inter > 65535 || N <= 0) return -1;
-    const dim3 grid((N + 511) / 512, inter);
-    return nvfp4::launch_pdl(nvfp4::silu_mul_rows_kernel, grid, dim3(256), 0, (cudaStream_t)stream,
+    const bool vec = N % 8 == 0 && (((uintptr_t)gu | (uintptr_t)act) & 15) == 0;
+    const long long items = (long long)inter * (vec ? N / 8 : N);      // fits the grid: inter < 2^16
+    return nvfp4::launch_pdl(vec ? nvfp4::silu_mul_rows_kernel<true> : nvfp4::silu_mul_rows_kernel<false>,
+                             dim3((unsigned)((items + 255) / 256)), dim3(256), 0, (cudaStream_t)stream,
                              (const __half*)gu, (__half*)act, inter, N) == cudaSuccess ? 0 : -1;
 }
 
@@ -630,7 +681,7 @@ long long nvfp4_dn_prefill_work_bytes(int n, int nk, int nv) {
 // One Gated-DeltaNet layer over a chunk of n tokens.  x: token-major in-projection output
 // [n][ld], row = [mixed | z | b | a]; conv_w, conv_state fp16 [conv_dim][4]; A_log, dt_bias fp16
 // [nv]; norm_w fp16 [128]; state fp32 [nv][128][128] (value-row major), updated; out token-major
-// [n][nv * 128].  nv a multiple of nk.  Five launches on `stream`.  0; -1 bad arguments; -2 launch.
+// [n][nv * 128].  nv a multiple of nk.  Four launches on `stream`.  0; -1 bad arguments; -2 launch.
 int launch_dn_prefill(const void* x, long long ld, const void* conv_w, void* conv_state,
                       const void* A_log, const void* dt_bias, const void* norm_w, void* state,
                       void* work, long long work_bytes, void* out, int n, int nk, int nv,
@@ -654,11 +705,10 @@ int launch_dn_prefill(const void* x, long long ld, const void* conv_w, void* con
     cudaStream_t st = (cudaStream_t)stream;
     const __half* xh = (const __half*)x;
     bool ok = true;
-    ok = ok && nvfp4::launch_pdl(nvfp4::dn_conv_tokens_kernel, dim3((conv_dim + 255) / 256, n),
-                                 dim3(256), 0, st, xh, ld, (const __half*)conv_w,
-                                 (const __half*)conv_state, conv_out, conv_dim) == cudaSuccess;
-    ok = ok && nvfp4::launch_pdl(nvfp4::dn_conv_state_kernel, dim3((conv_dim + 255) / 256),
-                                 dim3(256), 0, st, xh, ld, (__half*)conv_state, conv_dim,
+    const int conv_t = n > 128 ? 8 : 2;
+    ok = ok && nvfp4::launch_pdl(conv_t == 8 ? nvfp4::dn_conv_tokens_kernel<8> : nvfp4::dn_conv_tokens_kernel<2>,
+                                 dim3((conv_dim + 511) / 512, (n + conv_t - 1) / conv_t), dim3(128), 0, st, xh, ld,
+                                 (const __half*)conv_w, (const __half*)conv_state, conv_out, conv_dim,
                                  n) == cudaSuccess;
     ok = ok && nvfp4::launch_pdl(nvfp4::dn_block_kernel, dim3((nk + 3) / 4, nb), dim3(128), 0,
                                  st, (const __half*)conv_out, conv_dim, xh, ld,
@@ -669,9 +719,10 @@ int launch_dn_prefill(const void* x, long long ld, const void* conv_w, void* con
                                  (const float*)qn, (const float*)kn, (const nvfp4::DnBlock*)blocks,
                                  (const __half*)conv_out, conv_dim, (float*)state, o16, nk, nv,
                                  n) == cudaSuccess;
-    ok = ok && nvfp4::launch_pdl(nvfp4::dn_post_kernel, dim3(nv, n), dim3(32), 0, st,
+    ok = ok && nvfp4::launch_pdl(nvfp4::dn_post_kernel,
+                                 dim3((unsigned)max((nv * n + 7) / 8, (conv_dim + 255) / 256)), dim3(256), 0, st,
                                  (const __half*)o16, xh, ld, conv_dim, (const __half*)norm_w,
-                                 (__half*)out, nv, rms_eps) == cudaSuccess;
+                                 (__half*)out, (__half*)conv_state, nv, n, rms_eps) == cudaSuccess;
     return ok ? 0 : -2;
 }
 

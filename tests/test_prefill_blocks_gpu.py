@@ -10,7 +10,7 @@ from tests.gpu_util import dev, ptr, stream, ulp_diff_f16
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nk,nv,n", [(1, 1, 2), (1, 2, 4), (2, 6, 5), (3, 3, 16), (1, 2, 17), (5, 5, 19), (1, 3, 67)])
+@pytest.mark.parametrize("nk,nv,n", [(1, 1, 2), (1, 2, 4), (2, 6, 5), (3, 3, 16), (1, 2, 17), (5, 5, 19), (1, 3, 67), (1, 1, 131)])
 @pytest.mark.parametrize("strong", [False, True])
 def test_deltanet_chunk_against_float64(lib, nk, nv, n, strong):
     # strong: decays down to e^-60 a token, which underflow over a block
