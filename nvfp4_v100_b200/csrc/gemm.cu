@@ -34,6 +34,8 @@
 #include "attn_prefill_tc.cuh"
 #include "common.cuh"
 #include "gemm_few.cuh"
+#include "gemm_pair.cuh"
+#include "gemm_tile.cuh"
 #include "ptx.cuh"
 #include "tmap.cuh"
 
@@ -60,84 +62,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int id)
     atomicExch(&g_gemm_status, 1 + id);
     return false;
 }
-// Epilogue store of one 32-token block of a thread's row (v = 32 fp32 accumulator values), in the
-// layout out_mode asks for.  m = this thread's row, mbase = first row of its 128-row tile,
-// nb = first token of the block.  `piece` counts the token-major staging pieces of this column
-// half (chalf); all four warps of a column half call this together.
-__device__ __forceinline__ void gemm_store_block(const uint32_t (&v)[32], __half* out, int out_mode,
-                                                 uint8_t* smem, int chalf, int& piece, int q, int lane,
-                                                 int m, int mbase, int nb, int M, int N, int ld_out,
-                                                 int n_out) {
-    if (out_mode != GEMM_OUT_FM) {
-        // Token-major: a thread holds one row's 32 tokens, memory wants one token's rows
-        // together.  The four warps of this column half (128 rows) turn the 32 x 128 piece
-        // over in shared memory - the operand ring is free once the accumulation has
-        // retired - and then store 16 bytes (8 rows of one token) per thread.  Two staging
-        // pieces alternate, so the one barrier per piece also orders a piece's writes
-        // after the reads of the piece before last.  (Storing 2 bytes per lane straight
-        // from the registers cost 4 us per 512-token GEMM, 23 us with the residual add.)
-        __half* stg = reinterpret_cast<__half*>(smem + (chalf * 2 + (piece & 1)) * 8192);
-        const int rr = q * 32 + lane;
-#pragma unroll
-        for (int j = 0; j < 32; j++) stg[j * 128 + rr] = __float2half(__uint_as_float(v[j]));
-        asm volatile("bar.sync %0, 128;\n" ::"r"(1 + chalf) : "memory");
-        const bool vec = ((ld_out & 7) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int pid = i * 128 + rr, tok = pid >> 4, part = pid & 15;
-            const int tg = nb + tok, mg = mbase + part * 8;
-            if (tg >= n_out || mg >= M) continue;
-            const uint4 val = *reinterpret_cast<const uint4*>(stg + tok * 128 + part * 8);
-            __half* p = out + (size_t)tg * (size_t)ld_out + mg;
-            const __half2* h2 = reinterpret_cast<const __half2*>(&val);
-            if (vec && mg + 8 <= M) {
-                uint4 o = val;
-                if (out_mode == GEMM_OUT_TM_ADD) {
-                    const uint4 old = *reinterpret_cast<const uint4*>(p);
-                    const __half2* r2 = reinterpret_cast<const __half2*>(&old);
-                    __half2* o2 = reinterpret_cast<__half2*>(&o);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const float2 a = __half22float2(h2[e]), b = __half22float2(r2[e]);
-                        o2[e] = __floats2half2_rn(a.x + b.x, a.y + b.y);
-                    }
-                }
-                *reinterpret_cast<uint4*>(p) = o;
-            } else {
-                const __half* h1 = reinterpret_cast<const __half*>(&val);
-                for (int e = 0; e < 8 && mg + e < M; e++) {
-                    __half r = h1[e];
-                    if (out_mode == GEMM_OUT_TM_ADD) r = __float2half(__half2float(r) + __half2float(p[e]));
-                    p[e] = r;
-                }
-            }
-        }
-        piece++;
-    } else if (m < M && nb < N) {
-        __half* orow = out + (size_t)m * (size_t)N + nb;
-        if (nb + 32 <= N) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-                uint4 o;
-                __half2 t;
-                t = __floats2half2_rn(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
-                o.x = *reinterpret_cast<uint32_t*>(&t);
-                t = __floats2half2_rn(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-                o.y = *reinterpret_cast<uint32_t*>(&t);
-                t = __floats2half2_rn(__uint_as_float(v[j + 4]), __uint_as_float(v[j + 5]));
-                o.z = *reinterpret_cast<uint32_t*>(&t);
-                t = __floats2half2_rn(__uint_as_float(v[j + 6]), __uint_as_float(v[j + 7]));
-                o.w = *reinterpret_cast<uint32_t*>(&t);
-                *reinterpret_cast<uint4*>(orow + j) = o;
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 32; j++)
-                if (nb + j < N) orow[j] = __float2half(__uint_as_float(v[j]));
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------------------------
 // The kernel.  BN = tokens per CTA tile (64, 128 or 256).
 // Shared memory (dynamic, 1024-byte aligned): per stage A tile 128 x 128 B = 16 KB, then per stage
@@ -662,7 +586,8 @@ static int gemm_tile_bn(int N) { return N > 128 ? 256 : N > 64 ? 128 : 64; }
 static bool gemm_tile_rows256(int M, int N) {
     return N > 128 && g_gemm_rows256 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= 120;
 }
-// The CTA-pair kernel takes more than 128 tokens and K % 128 == 0.  Measured at 512 tokens against
+// The CTA-pair kernel of this file: more than 128 tokens and K % 128 == 0, where the one of gemm_pair.cu
+// (A in tensor memory; K % 256 == 0 and 16-byte aligned scales) is not taken.  Measured at 512 tokens against
 // the single-CTA kernel's best tile: 5120 x 5120 36.4 us (40.4), 6144 x 5120 38.4 (42.0), 10240 x
 // 5120 69.4 (77.2), 5120 x 17408 105.7 (121.0) - but 17408 x 5120 75.6 (69.3 with 256-row tiles) and
 // 34816 x 5120 149 (140): it replaces the 128-row tiles, not the 256-row ones.
@@ -702,6 +627,12 @@ int launch_nvfp4_gemmtc_v5(const uint8_t* d_weight_packed, const uint8_t* d_weig
         gemm_few_takes(d_weight_packed, d_weight_scales, N, K)) {
         const int rc = gemm_few_launch(d_weight_packed, d_weight_scales, d_activation, N, false, d_output, N,
                                        M, N, N, K, GEMM_OUT_FM, st);
+        if (rc != -3) return rc;
+    }
+    if (N % 8 == 0 && (((uintptr_t)d_activation | (uintptr_t)d_output) & 15) == 0 && g_gemm_pair &&
+        gemm_pair_takes(d_weight_packed, d_weight_scales, N, K)) {
+        const int rc = gemm_pair_launch(d_weight_packed, d_weight_scales, d_activation, N, false, d_output, N,
+                                        M, N, N, K, GEMM_OUT_FM, st);
         if (rc != -3) return rc;
     }
     const bool tc_ok = (K % 64 == 0) && (N % 8 == 0) &&
@@ -766,6 +697,9 @@ int launch_nvfp4_gemm_w4a16_ex(const uint8_t* d_weight_packed, const uint8_t* d_
                                o, (int)ld_out, M, N8, n_tokens, K, mode, st);
     // token count the kernel's bounds use: feature-major sides are padded to 8
     const int N = (in_tm && out_tm) ? n_tokens : N8;
+    if (g_gemm_pair && gemm_pair_takes(d_weight_packed, d_weight_scales, N, K))
+        return gemm_pair_launch(d_weight_packed, d_weight_scales, static_cast<const __half*>(act), ld_act, in_tm,
+                                o, (int)ld_out, M, N, n_tokens, K, mode, st);
     CUtensorMap map;
     const cuuint32_t estr[2] = {1, 1};
     CUresult r;
@@ -839,13 +773,15 @@ int nvfp4_gemm_status(int reset) {
     if (v == 0 && f != 0) v = (f < 0) ? f : 100 + f;
     const int few = nvfp4::gemm_few_status(reset);  // the few-token kernel's: 200 + its own
     if (v == 0 && few != 0) v = (few < 0) ? few : 200 + few;
+    const int pair = nvfp4::gemm_pair_status(reset);  // the pair kernel's with A in tensor memory: 400 + its own
+    if (v == 0 && pair != 0) v = (pair < 0) ? pair : 400 + pair;
     const int atc = nvfp4::attn_prefill_tc_status(reset);   // the chunk attention kernel's: 300 + its own
     if (v == 0 && atc != 0) v = (atc < 0) ? atc : 300 + atc;
     return v;
 }
 
-// Tuning hook.  Bit 0: 256-row CTA tiles (two accumulators) for more than 128 tokens.  Bit 1: the
-// CTA-pair kernel (clusters of two, cta_group::2) for shapes of more than 128 tokens that do not get
+// Tuning hook.  Bit 0: 256-row CTA tiles (two accumulators) for more than 128 tokens.  Bits 1 and 2: the
+// kernel of gemm_pair.cu for every shape it takes; for the others, bit 1: the CTA-pair kernel (clusters of two, cta_group::2) for shapes of more than 128 tokens that do not get
 // 256-row tiles.  Bit 2: the CTA-pair kernel for every shape it can run.  Default 3.
 void nvfp4_b200_gemm_config(int flags) {
     nvfp4::g_gemm_rows256 = (flags & 1) ? 1 : 0;

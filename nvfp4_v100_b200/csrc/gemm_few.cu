@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "gemm_few.cuh"
+#include "gemm_tile.cuh"
 #include "ptx.cuh"
 #include "tmap.cuh"
 
@@ -82,22 +83,6 @@ __device__ __forceinline__ float4 few_ld_cluster(uint32_t addr) {
                  : "r"(addr)
                  : "memory");
     return v;
-}
-
-// 16 packed bytes (32 weights, two scale blocks) -> 16 words of fp16 pairs, scaled in fp16
-__device__ __forceinline__ void few_dequant(const uint4 p, uint32_t sc2, uint32_t (&o)[16]) {
-    const uint32_t w[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const __half2 s2 = __half2half2(__float2half(e8m0_to_f32((sc2 >> (8 * (j >> 1))) & 0xFFu)));
-        uint32_t h[4];
-        e2m1x8_to_half2x4(w[j], h[0], h[1], h[2], h[3]);
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const __half2 t = __hmul2(*reinterpret_cast<const __half2*>(&h[e]), s2);
-            o[4 * j + e] = *reinterpret_cast<const uint32_t*>(&t);
-        }
-    }
 }
 
 template <int BN, bool IN_TM>
@@ -243,7 +228,7 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
 #pragma unroll
             for (int c = 0; c < 4; c++) {
                 uint32_t o[16];
-                few_dequant(p[c], (c < 2 ? sc.x : sc.y) >> (16 * (c & 1)), o);
+                gemm_dequant32(p[c], (c < 2 ? sc.x : sc.y) >> (16 * (c & 1)), o);
                 tcgen05_st_32x32b_x16(a + (uint32_t)(c * 16), o);
             }
             __syncwarp();                                      // every lane's reads of the stage are done

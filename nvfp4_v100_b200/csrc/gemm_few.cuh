@@ -4,13 +4,6 @@
 
 namespace nvfp4 {
 
-// output layouts of the W4A16 GEMM kernels
-enum {
-    GEMM_OUT_FM = 0,       // out[m][token]
-    GEMM_OUT_TM = 1,       // out[token][m]
-    GEMM_OUT_TM_ADD = 2,   // out[token][m] += result
-};
-
 constexpr int GEMM_FEW_MAX_TOKENS = 128;
 
 // Whether the few-token kernel takes this product (sizes and alignment).
