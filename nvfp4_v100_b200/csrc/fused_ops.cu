@@ -114,15 +114,32 @@ rope_qk_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + expf(-x)); }
 
+// W = 8: 16-byte accesses, for 16-byte aligned vectors long enough to fill the GPU that way (2048 x 17408
+// 145 -> 35.7 us, 128 x 17408 9.7 -> 3.5; 21 x 17408 is even, 65536 and less are faster with 2-byte
+// accesses: 1.2 us against 1.6).
+template <int W>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __half* __restrict__ g, const __half* __restrict__ u,
                 __half* __restrict__ out, int n) {
     pdl_prologue();
     PDL_FRESH(g); PDL_FRESH(u); PDL_FRESH(out);
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= n) return;
-    const float gf = __half2float(g[i]), uf = __half2float(u[i]);
-    out[i] = __float2half(round_f16(silu_f(gf)) * uf);
+    const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * W;
+    if (W == 8 && i + 8 <= n) {
+        const uint4 gv = *reinterpret_cast<const uint4*>(g + i), uv = *reinterpret_cast<const uint4*>(u + i);
+        const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
+        uint32_t ow[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float2 gf = __half22float2(*reinterpret_cast<const __half2*>(&gw[k]));
+            const float2 uf = __half22float2(*reinterpret_cast<const __half2*>(&uw[k]));
+            const __half2 r = __floats2half2_rn(round_f16(silu_f(gf.x)) * uf.x, round_f16(silu_f(gf.y)) * uf.y);
+            ow[k] = *reinterpret_cast<const uint32_t*>(&r);
+        }
+        *reinterpret_cast<uint4*>(out + i) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+        return;
+    }
+    for (long long j = i; j < n && j < i + W; j++)
+        out[j] = __float2half(round_f16(silu_f(__half2float(g[j]))) * __half2float(u[j]));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -720,9 +737,12 @@ int launch_rope_qk(const void* q, const void* k, const void* cs, const void* sn,
 
 int launch_silu_mul(const void* g, const void* u, void* out, int n, void* stream) {
     if (n <= 0 || !g || !u || !out) return -1;
+    const bool wide = n >= (1 << 19) && (((uintptr_t)g | (uintptr_t)u | (uintptr_t)out) & 15) == 0;
+    const long long items = wide ? ((long long)n + 7) / 8 : n;
     const cudaError_t e =
-        nvfp4::launch_pdl(nvfp4::silu_mul_kernel, dim3((n + 255) / 256), dim3(256), 0,
-                          (cudaStream_t)stream, (const __half*)g, (const __half*)u, (__half*)out, n);
+        nvfp4::launch_pdl(wide ? nvfp4::silu_mul_kernel<8> : nvfp4::silu_mul_kernel<1>,
+                          dim3((unsigned)((items + 255) / 256)), dim3(256), 0, (cudaStream_t)stream,
+                          (const __half*)g, (const __half*)u, (__half*)out, n);
     return e == cudaSuccess ? 0 : -2;
 }
 

@@ -106,3 +106,18 @@ def test_silu_mul_rows_with_ragged_and_unaligned_rows(lib, inter, N, shift):
     want = fo.silu_mul(g[:, 0].reshape(-1), g[:, 1].reshape(-1))
     got = act.cpu().numpy()
     assert ulp_diff_f16(got[:inter * N], want.reshape(-1)).max() <= 1 and (got[inter * N:] == 7).all()
+
+
+@pytest.mark.parametrize("n,shift", [((1 << 19) - 1, 0), (1 << 19, 0), ((1 << 19) + 5, 0), (1 << 20, 1), (2048 * 300 + 2047, 0)])
+def test_silu_mul_of_long_vectors(lib, n, shift):
+    rng = np.random.default_rng(n)
+    g = (rng.standard_normal(n) * 3).astype(np.float16)
+    u = rng.standard_normal(n).astype(np.float16)
+    d_g = torch.zeros(n + shift, dtype=torch.float16, device="cuda")[shift:]
+    d_g.copy_(torch.from_numpy(g))
+    d_u = dev(u)
+    out = torch.full((n + 8,), 7.0, dtype=torch.float16, device="cuda")
+    assert lib.launch_silu_mul(ptr(d_g), ptr(d_u), ptr(out), n, stream()) == 0
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    assert ulp_diff_f16(got[:n], fo.silu_mul(g, u)).max() <= 1 and (got[n:] == 7).all()
