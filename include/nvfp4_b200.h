@@ -211,9 +211,9 @@ int launch_nvfp4_gemv_fused(const void* weight_packed, const void* weight_scales
                             const void* norm_w1, float eps, int epilogue, const void* residual,
                             void* stream);
 
-/* launch_attn_decode_heads with the keys of every head split over eight CTAs (no counterpart in
- * the reference): each warp requests its key AND value rows at once, partial softmax results are
- * combined in shared memory, then by the last CTA of a head to finish (in split order, so the
+/* launch_attn_decode_heads with the keys split over several CTAs, each serving one to three query heads
+ * of a KV head (no counterpart in the reference): each warp requests its key AND value rows at once,
+ * partial softmax results are combined in shared memory, then by the last CTA to finish (in split order, so the
  * result does not depend on arrival order).  scratch: nvfp4_attn_split_scratch_bytes(hq) bytes,
  * 16-byte aligned, zeroed once before first use; calls sharing it must not overlap.  Results
  * match launch_attn_decode_heads to the last fp32 bit before the fp16 rounding.

@@ -549,6 +549,185 @@ attn_decode_split_kernel(const __half* __restrict__ q, const __half* __restrict_
     out[(size_t)h * ATT_D + t] = __float2half(a * sg);
 }
 
+// The same for HG query heads that share a KV head per CTA: every key and value row is read once for all
+// of them.  With one head per CTA the six heads of a group read the cache six times from L2, which at
+// 3500 keys is 86 MB and most of the kernel's time (24 heads: 21.5 -> 14.8 us; 1500 keys 12.1 -> 10.1, 513
+// 7.8 -> 7.5, 16 4.8 both).  ATG_SPLIT
+// CTAs per head group take alternate blocks of ATS_WARPS keys.
+#define ATG_SPLIT 16
+#define ATG_ROWS 4
+template <int HG>
+__global__ void __launch_bounds__(ATS_WARPS * 32)
+attn_decode_group_kernel(const __half* __restrict__ q, const __half* __restrict__ keys,
+                         const __half* __restrict__ values, const long long* __restrict__ cum_len,
+                         const __half* __restrict__ gate, __half* __restrict__ out,
+                         float* __restrict__ part, unsigned int* __restrict__ counters,
+                         int max_len, int gqa, float scale) {
+    pdl_prologue();
+    PDL_FRESH(q); PDL_FRESH(keys); PDL_FRESH(values); PDL_FRESH(cum_len); PDL_FRESH(gate); PDL_FRESH(out);
+    PDL_FRESH(part); PDL_FRESH(counters);
+    extern __shared__ __align__(16) float s_part[];          // [HG][ATS_WARPS][ATS_PART]
+    __shared__ float s_f[HG][32 + 1];
+    __shared__ unsigned int s_last;
+    const int h0 = blockIdx.x * HG, sp = blockIdx.y, kv = h0 / gqa;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    long long L64 = *cum_len;
+    if (L64 > max_len) L64 = max_len;
+    if (L64 < 0) L64 = 0;
+    const int L = (int)L64;
+    // short contexts: as many CTAs as one batch of rows a warp needs, the others leave
+    const int splits = min((int)gridDim.y, max(1, (L + ATS_WARPS * ATG_ROWS - 1) / (ATS_WARPS * ATG_ROWS)));
+    if (sp >= splits) return;
+
+    float qf[HG][8];
+#pragma unroll
+    for (int g = 0; g < HG; g++) unpack8(*reinterpret_cast<const uint4*>(q + (size_t)(h0 + g) * ATT_D + lane * 8), qf[g]);
+    const __half* kbase = keys + (size_t)kv * (size_t)max_len * ATT_D + lane * 8;
+    const __half* vbase = values + (size_t)kv * (size_t)max_len * ATT_D + lane * 8;
+    float m[HG], l[HG], o[HG][8];
+#pragma unroll
+    for (int g = 0; g < HG; g++) {
+        m[g] = -3.4e38f;
+        l[g] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; j++) o[g][j] = 0.0f;
+    }
+    // key i belongs to split (i / ATS_WARPS) % splits and warp i % ATS_WARPS
+    const int stride = splits * ATS_WARPS;
+    for (int i0 = sp * ATS_WARPS + warp; i0 < L; i0 += stride * ATG_ROWS) {
+        uint4 kr[ATG_ROWS], vr[ATG_ROWS];
+#pragma unroll
+        for (int u = 0; u < ATG_ROWS; u++) {
+            const int i = i0 + u * stride;
+            const bool ok = i < L;
+            kr[u] = ok ? *reinterpret_cast<const uint4*>(kbase + (size_t)i * ATT_D)
+                       : make_uint4(0u, 0u, 0u, 0u);
+            vr[u] = ok ? *reinterpret_cast<const uint4*>(vbase + (size_t)i * ATT_D)
+                       : make_uint4(0u, 0u, 0u, 0u);
+        }
+        float sc[HG][ATG_ROWS], mb[HG];
+#pragma unroll
+        for (int g = 0; g < HG; g++) mb[g] = m[g];
+#pragma unroll
+        for (int u = 0; u < ATG_ROWS; u++) {
+            float kf[8];
+            unpack8(kr[u], kf);
+#pragma unroll
+            for (int g = 0; g < HG; g++) {
+                float acc = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc = fmaf(qf[g][j], kf[j], acc);
+                acc = warp_sum(acc) * scale;
+                sc[g][u] = (i0 + u * stride < L) ? acc : -3.4e38f;
+                mb[g] = fmaxf(mb[g], sc[g][u]);
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < HG; g++) {
+            const float corr = expf(m[g] - mb[g]);    // 0 on the first batch (m = -3.4e38)
+            l[g] *= corr;
+#pragma unroll
+            for (int j = 0; j < 8; j++) o[g][j] *= corr;
+            m[g] = mb[g];
+        }
+#pragma unroll
+        for (int u = 0; u < ATG_ROWS; u++) {
+            float vf[8];
+            unpack8(vr[u], vf);
+#pragma unroll
+            for (int g = 0; g < HG; g++) {
+                const float p = (i0 + u * stride < L) ? expf(sc[g][u] - m[g]) : 0.0f;
+                l[g] += p;
+#pragma unroll
+                for (int j = 0; j < 8; j++) o[g][j] = fmaf(p, vf[j], o[g][j]);
+            }
+        }
+    }
+    // ---- warps -> CTA partials ----
+#pragma unroll
+    for (int g = 0; g < HG; g++) {
+        float* sw = s_part + (g * ATS_WARPS + warp) * ATS_PART;
+        *reinterpret_cast<float4*>(sw + lane * 8) = make_float4(o[g][0], o[g][1], o[g][2], o[g][3]);
+        *reinterpret_cast<float4*>(sw + lane * 8 + 4) = make_float4(o[g][4], o[g][5], o[g][6], o[g][7]);
+        if (lane == 0) {
+            sw[ATT_D] = m[g];
+            sw[ATT_D + 1] = l[g];
+        }
+    }
+    __syncthreads();
+    if (warp < HG) {                                            // a warp per head, a lane per warp's part
+        const float* sw = s_part + (warp * ATS_WARPS + (lane & 15)) * ATS_PART + ATT_D;
+        const float mv = sw[0], M = warp_max(mv);
+        const float f = expf(mv - M);                           // warps without keys: exp(-huge) = 0
+        const float ls = warp_sum(lane < ATS_WARPS ? sw[1] * f : 0.0f);
+        if (lane < ATS_WARPS) s_f[warp][lane] = f;
+        if (lane == 0) {
+            float* mine = part + ((size_t)(h0 + warp) * ATG_SPLIT + sp) * ATS_PART + ATT_D;
+            mine[0] = M;
+            mine[1] = ls;
+            s_f[warp][32] = 1.0f / ls;
+        }
+    }
+    __syncthreads();
+    for (int i = t; i < HG * ATT_D; i += ATS_WARPS * 32) {
+        const int g = i / ATT_D, d = i % ATT_D;
+        float acc = 0.0f;
+#pragma unroll
+        for (int w = 0; w < ATS_WARPS; w++) acc = fmaf(s_part[(g * ATS_WARPS + w) * ATS_PART + d], s_f[g][w], acc);
+        if (splits == 1) {                                      // nobody to meet
+            const size_t at = (size_t)(h0 + g) * ATT_D + d;
+            const float sg = round_f16(1.0f / (1.0f + expf(-__half2float(gate[at]))));
+            out[at] = __float2half(round_f16(acc * s_f[g][32]) * sg);
+        } else {
+            part[((size_t)(h0 + g) * ATG_SPLIT + sp) * ATS_PART + d] = acc;
+        }
+    }
+    if (splits == 1) return;
+    // ---- CTAs -> heads: the last CTA to arrive combines the parts in split order ----
+    __threadfence();
+    __syncthreads();
+    if (t == 0) {
+        const unsigned int prev = atomicAdd(counters + blockIdx.x, 1u);
+        s_last = (prev == (unsigned)splits - 1) ? 1u : 0u;
+        if (s_last) counters[blockIdx.x] = 0u;                  // ready for the next launch
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    // a thread owns two dims of a head; its parts are requested before the factors are known
+    constexpr int HALF = ATT_D / 2;
+    const int g = t / HALF < HG ? t / HALF : 0, d = (t % HALF) * 2;
+    const float* pd = part + (size_t)(h0 + g) * ATG_SPLIT * ATS_PART + d;
+    float2 v[16];
+#pragma unroll
+    for (int s = 0; s < 16; s++)
+        v[s] = s < splits ? __ldcg(reinterpret_cast<const float2*>(pd + s * ATS_PART)) : make_float2(0.0f, 0.0f);
+    if (warp < HG) {                                            // a warp per head, a lane per split
+        const float* ph = part + (size_t)(h0 + warp) * ATG_SPLIT * ATS_PART + ATT_D;
+        const float mv = lane < splits ? __ldcg(ph + lane * ATS_PART) : -3.4e38f;
+        const float lv = lane < splits ? __ldcg(ph + lane * ATS_PART + 1) : 0.0f;
+        const float f = expf(mv - warp_max(mv));
+        const float ls = warp_sum(lv * f);
+        s_f[warp][lane] = f;
+        if (lane == 0) s_f[warp][32] = 1.0f / ls;
+    }
+    __syncthreads();
+    if (t >= HG * HALF) return;
+    float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int s = 0; s < 16; s++)
+        if (s < splits) {
+            acc.x = fmaf(v[s].x, s_f[g][s], acc.x);
+            acc.y = fmaf(v[s].y, s_f[g][s], acc.y);
+        }
+    const size_t at = (size_t)(h0 + g) * ATT_D + d;
+    const float inv = s_f[g][32];
+    const float2 gt = __half22float2(*reinterpret_cast<const __half2*>(gate + at));
+    *reinterpret_cast<__half2*>(out + at) =
+        __floats2half2_rn(round_f16(acc.x * inv) * round_f16(1.0f / (1.0f + expf(-gt.x))),
+                          round_f16(acc.y * inv) * round_f16(1.0f / (1.0f + expf(-gt.y))));
+}
+
 // Prefill attention for ATT_G consecutive tokens of one query head per CTA: the tokens share
 // every key and value row they load (token g of the group sees L0 + g rows).  Per token the
 // arithmetic and its order are those of attn_one_query — same key-to-warp assignment, same
@@ -815,10 +994,10 @@ int launch_attn_prefill(const void* q, const void* keys, const void* values, int
 // head); the counters (the last hq * 4 bytes ... see the launcher) must be zero before first use.
 long long nvfp4_attn_split_scratch_bytes(int hq) {
     if (hq <= 0) return -1;
-    return (long long)hq * ATS_SPLIT * ATS_PART * 4 + (long long)hq * 4;
+    return (long long)hq * ATG_SPLIT * ATS_PART * 4 + (long long)hq * 4;
 }
 
-// launch_attn_decode_heads with the keys split over eight CTAs per head.  scratch: device buffer
+// launch_attn_decode_heads with the keys split over several CTAs.  scratch: device buffer
 // of nvfp4_attn_split_scratch_bytes(hq) bytes, 16-byte aligned, zeroed once by the caller (the
 // kernel leaves its counters at zero).  Calls that share a scratch buffer must not overlap.
 // 0; -2 bad arguments; else the launch error.
@@ -828,12 +1007,26 @@ int launch_attn_decode_split(const void* q, const void* keys, const void* values
     if (max_len <= 0 || !q || !keys || !values || !cum_len || !gate || !out || !scratch) return -2;
     if (hq <= 0 || hkv <= 0 || hq % hkv != 0 || ((uintptr_t)scratch & 15)) return -2;
     float* part = (float*)scratch;
-    unsigned int* counters = (unsigned int*)(part + (size_t)hq * ATS_SPLIT * ATS_PART);
+    unsigned int* counters = (unsigned int*)(part + (size_t)hq * ATG_SPLIT * ATS_PART);
+    const int gqa = hq / hkv;
+    // Sharing pays where the CTAs of single heads fill the GPU; with 12 heads or fewer a head per CTA is
+    // faster at every length (12: 5.1 us against 7.1 at 513 keys, 12.0 against 13.9 at 3500).
+    const int hg = hq * ATS_SPLIT < 148 ? 1 : gqa % 3 == 0 ? 3 : gqa % 2 == 0 ? 2 : 1;
+    const auto kernel = hg == 3   ? nvfp4::attn_decode_group_kernel<3>
+                        : hg == 2 ? nvfp4::attn_decode_group_kernel<2>
+                                  : nvfp4::attn_decode_split_kernel;
+    const int smem = hg == 1 ? 0 : hg * ATS_WARPS * ATS_PART * (int)sizeof(float);
+    static bool opted[nvfp4::NVFP4_MAX_DEVICES][4] = {};
+    const int dev = nvfp4::current_device_index();
+    if (hg > 1 && !opted[dev][hg]) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -2;
+        opted[dev][hg] = true;
+    }
     const cudaError_t e = nvfp4::launch_pdl(
-        nvfp4::attn_decode_split_kernel, dim3(hq, ATS_SPLIT), dim3(ATS_WARPS * 32), 0,
+        kernel, dim3(hq / hg, hg == 1 ? ATS_SPLIT : ATG_SPLIT), dim3(ATS_WARPS * 32), (size_t)smem,
         (cudaStream_t)stream, (const __half*)q, (const __half*)keys, (const __half*)values,
         (const long long*)cum_len, (const __half*)gate, (__half*)out, part, counters, max_len,
-        hq / hkv, scale);
+        gqa, scale);
     return (e == cudaSuccess) ? 0 : (int)e;
 }
 
