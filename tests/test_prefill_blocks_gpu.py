@@ -121,3 +121,27 @@ def test_silu_mul_of_long_vectors(lib, n, shift):
     torch.cuda.synchronize()
     got = out.cpu().numpy()
     assert ulp_diff_f16(got[:n], fo.silu_mul(g, u)).max() <= 1 and (got[n:] == 7).all()
+
+
+@pytest.mark.parametrize("hq,hkv,n", [(1, 1, 1), (5, 1, 3), (24, 4, 9), (9, 3, 2)])
+def test_attn_prep_of_a_chunk_equals_token_by_token(lib, hq, hkv, n):
+    # eight heads a CTA: fewer, exactly and more than fill one
+    rng = np.random.default_rng(hq + n)
+    max_len, p0, ld = 40, 31, hq * 512 + hkv * 512 + 24
+    qkv = dev(rng.standard_normal((n, ld)).astype(np.float16))
+    w = [dev((1 + 0.1 * rng.standard_normal(256)).astype(np.float32)) for _ in range(2)]
+    tab = [dev(rng.uniform(-1, 1, (max_len, 256)).astype(np.float16)) for _ in range(2)]
+    new = lambda *s: torch.full(s, 7.0, dtype=torch.float16, device="cuda")
+    a = [new(n, hq * 256), new(n, hq * 256), new(hkv, max_len, 256), new(hkv, max_len, 256)]
+    b = [t.clone() for t in a]
+    args = [ptr(t) for t in w + tab]
+    assert lib.launch_attn_prep_tokens(ptr(qkv), ld, *args, p0, n, *[ptr(t) for t in a], hq, hkv, max_len, 1e-6,
+                                       stream()) == 0
+    for t in range(n):
+        pos = torch.tensor([p0 + t], dtype=torch.int64, device="cuda")
+        row = qkv[t].contiguous()
+        assert lib.launch_attn_prep(ptr(row), *args, ptr(pos), ptr(b[0][t]), ptr(b[1][t]), ptr(b[2]), ptr(b[3]), hq,
+                                    hkv, max_len, 1e-6, stream()) == 0
+        torch.cuda.synchronize()
+    for x, y in zip(a, b):
+        assert torch.equal(x, y)
