@@ -288,7 +288,8 @@ class QLinear(nn.Module):
         return yt[:, :tokens].t().contiguous()
 
     def forward(self, x):
-        flat = x if x.dim() == 2 and x.shape[1] == self.K else x.reshape(-1, self.K)
+        rows = x.dim() == 2 and x.shape[1] == self.K
+        flat = x if rows else x.reshape(-1, self.K)
         if flat.dtype is not torch.float16:
             flat = flat.half()
         if not flat.is_contiguous():
@@ -303,7 +304,8 @@ class QLinear(nn.Module):
             y = self._many(flat, tokens)
         if self.bias is not None:
             y = y + self.bias
-        return y if x.dim() == 2 else y.view(*x.shape[:-1], self.M)
+        # the view is also the check of the feature width: reshape alone takes any multiple of K
+        return y if rows else y.view(*x.shape[:-1], self.M)
 
 
 def st_name(name):
