@@ -70,7 +70,10 @@ int launch_nvfp4_gemv2i(const void* weight_packed, const void* weight_scales, co
  * (fp16, N = tokens, token-minor as the reference's caller prepares it).  Weight x block scale in
  * fp16, fp16 x fp16 products, fp32 accumulation, as the reference's wmma kernel.  Runs on tcgen05
  * tensor cores when K % 64 == 0, N % 8 == 0 and the pointers are 16-byte aligned (scales 4-byte),
- * otherwise on a CUDA-core kernel.  Returns 0 or the cudaError_t of the launch; -2 for K % 16 != 0,
+ * otherwise on a CUDA-core kernel.  Weights, like activations, are read only after the previous kernel in
+ * the stream has completed, and the next kernel does not start before that either: a GEMM orders what is
+ * in front of it before what follows, also for successors that read ahead (see the GEMVs' contract below).
+ * The same holds for launch_nvfp4_gemm_w4a16_ex.  Returns 0 or the cudaError_t of the launch; -2 for K % 16 != 0,
  * non-positive sizes or NULL pointers.  kernels/nvfp4_cuda_v5.cu:406-422. */
 int launch_nvfp4_gemmtc_v5(const uint8_t* d_weight_packed, const uint8_t* d_weight_scales,
                            const void* d_activation, void* d_output, int M, int N, int K,

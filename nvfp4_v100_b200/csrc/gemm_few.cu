@@ -14,7 +14,7 @@
 //     workspace in global memory, nobody polls).
 // One CTA (384 threads) = 128 weight rows x BN tokens x its share of K, in stages of 256 elements:
 //   warp 0       TMA producer of the weight ring (128 rows x 128 packed bytes, 128-byte swizzle, and
-//                128 x 16 scale bytes per stage); starts before the previous kernel has finished
+//                128 x 16 scale bytes per stage)
 //   warp 1       MMA issuer: units of 128 k = 8 x tcgen05.mma.kind::f16 (M 128, N BN, K 16)
 //   warp 2       TMA producer of the activation units (BN tokens x 128 k, from L2)
 //   warps 4..11  dequantisation: the four warps of a group own one 32-row quarter each and a group
@@ -45,7 +45,7 @@ constexpr int FEW_BK = 256;                        // K elements of a weight sta
 constexpr int FEW_UK = 128;                        // K elements of an MMA unit
 constexpr int FEW_A_BYTES = FEW_BM * 128;          // packed bytes of a stage
 constexpr int FEW_S_BYTES = FEW_BM * 16;           // scale bytes of a stage
-constexpr int FEW_PRE = 2;                         // weight stages requested at kernel entry
+constexpr int FEW_PRE = 2;                         // weight stages requested before the activations
 constexpr int FEW_MAX_SPLIT = 8;
 constexpr uint32_t FEW_SPIN_LIMIT = 100000;
 
@@ -93,7 +93,6 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
     constexpr int NS = few_stages(BN), NU = few_units(BN), B_BYTES = few_b_bytes(BN);
     constexpr uint32_t TMEM_COLS = 256;            // BN accumulator columns + NU x 64 columns of A
     static_assert(BN + NU * 64 <= 256, "two CTAs share the 512 tensor-memory columns");
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                ~(uintptr_t)1023);
@@ -135,7 +134,9 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
         mbar_init(smem_u32(&bar_accum), 1);
         mbar_init(smem_u32(&bar_breq), 1);
         fence_barrier_init();
-        // weights are constants: requested before the previous kernel has finished
+        // Weights too wait for the previous kernel: it may be the one that writes them (requested ahead
+        // of the wait, a launch is 0.3 to 0.9 us shorter and reads what was there before).
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");
         for (int i = 0; i < FEW_PRE && i < nst; i++) request(i, i);
     }
     if (warp == 1) {
@@ -146,6 +147,10 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem = s_tmem, tmem_a = tmem + BN;
+    // The next kernel starts after the wait, not before: it may read weights of its own ahead of its wait
+    // (the GEMVs do), and those may come from a kernel in front of this one.
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 
     if (warp == 0) {
         if (lane == 0) {
@@ -162,7 +167,6 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
         }
     } else if (warp == 2) {
         if (lane == 0) {
-            asm volatile("griddepcontrol.wait;\n" ::: "memory");   // the activations
             int u = 0;
             uint32_t ph = 0;
             for (int i = 0; i < 2 * nst; i++) {
@@ -258,7 +262,6 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
     if (split > 1) cluster_sync_all();
 
     // ---- sum over the cluster and output: a warp takes one token's 128 rows, a lane four of them ----
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");       // the output may be read by the previous kernel
     const uint32_t red0 = smem_u32(smem);
     const int limit = (out_mode == GEMM_OUT_FM ? N : n_out) - n0;
     for (int t = rank + split * warp; t < BN && t < limit; t += split * (FEW_THREADS / 32)) {

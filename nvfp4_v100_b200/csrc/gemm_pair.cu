@@ -11,7 +11,7 @@
 // 128 rows and loads half of the token tile; one tcgen05.mma.cta_group::2 (M 256, N BN, K 16) runs on
 // both SMs.  Roles, in both CTAs unless said otherwise:
 //   warp 0       TMA producer of the weight ring (stages of 256 k: 128 rows x 128 packed bytes and
-//                128 x 16 scale bytes); starts before the previous kernel has finished
+//                128 x 16 scale bytes)
 //   warp 1       first CTA only: MMA issuer, units of 128 k = 8 MMAs
 //   warp 2       TMA producer of the activation units (BN / 2 tokens x 128 k)
 //   warps 4..11  dequantisation: a group of four warps takes every other unit, a warp one 32-row
@@ -118,7 +118,9 @@ gemm_w4a16_pair_tm_kernel(const __grid_constant__ CUtensorMap w_map, const __gri
         }
         mbar_init(smem_u32(&bar_accum), 1);
         fence_barrier_init();
-        for (int i = 0; i < GP_NS && i < nst; i++) request(i, i);    // weights are constants
+        // weights too wait for the previous kernel: it may be the one that writes them
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");
+        for (int i = 0; i < GP_NS && i < nst; i++) request(i, i);
     }
     if (warp == 1) {
         tcgen05_alloc_pair(smem_u32(&s_tmem), 512);
@@ -129,7 +131,9 @@ gemm_w4a16_pair_tm_kernel(const __grid_constant__ CUtensorMap w_map, const __gri
     cluster_sync_all();      // the peer's barriers are initialised before anything arrives on them
     tcgen05_fence_after();
     const uint32_t tmem = s_tmem, tmem_a = tmem + 256;
-    // only now: a CTA of the next kernel must not take tensor memory before this one has all of it
+    // The next kernel starts only now: its CTAs must not take tensor memory before this one has all of it,
+    // and it may read weights ahead of its own wait (the GEMVs do) that a kernel in front of this one writes.
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 
     if (warp == 0) {
@@ -144,7 +148,6 @@ gemm_w4a16_pair_tm_kernel(const __grid_constant__ CUtensorMap w_map, const __gri
         }
     } else if (warp == 2) {
         if (lane == 0) {
-            asm volatile("griddepcontrol.wait;\n" ::: "memory");     // the activations
             int u = 0;
             uint32_t ph = 0;
             for (int i = 0; i < nun; i++) {
@@ -229,7 +232,6 @@ gemm_w4a16_pair_tm_kernel(const __grid_constant__ CUtensorMap w_map, const __gri
         }
         gp_wait(smem_u32(&bar_accum), 0, 5);
         tcgen05_fence_after();
-        asm volatile("griddepcontrol.wait;\n" ::: "memory");   // the output may be read by the previous kernel
         constexpr int CB = BN / 32 / 2;                        // 32-token blocks of a column half
         int piece = 0;
 #pragma unroll 1
