@@ -1011,7 +1011,9 @@ int launch_attn_decode_split(const void* q, const void* keys, const void* values
     const int gqa = hq / hkv;
     // Sharing pays where the CTAs of single heads fill the GPU; with 12 heads or fewer a head per CTA is
     // faster at every length (12: 5.1 us against 7.1 at 513 keys, 12.0 against 13.9 at 3500).
-    const int hg = hq * ATS_SPLIT < 148 ? 1 : gqa % 3 == 0 ? 3 : gqa % 2 == 0 ? 2 : 1;
+    // The shared kernel reads gates and stores results two at a time: 4-byte aligned pointers only.
+    const bool pairs = (((uintptr_t)gate | (uintptr_t)out) & 3) == 0;
+    const int hg = !pairs || hq * ATS_SPLIT < 148 ? 1 : gqa % 3 == 0 ? 3 : gqa % 2 == 0 ? 2 : 1;
     const auto kernel = hg == 3   ? nvfp4::attn_decode_group_kernel<3>
                         : hg == 2 ? nvfp4::attn_decode_group_kernel<2>
                                   : nvfp4::attn_decode_split_kernel;
