@@ -164,7 +164,7 @@ silu_mul_rows_kernel(const __half* __restrict__ gu, __half* __restrict__ act, in
 // ---------------------------------------------------------------------------------------------
 #define PF_DK 128
 
-// the four halves of a channel's window or weights: one 8-byte access where the pointer allows it
+// four halves (inputs, a channel's window or weights): one 8-byte access where the pointer allows it
 __device__ __forceinline__ uint2 ld_half4(const __half* p) {
     if (((uintptr_t)p & 7) == 0) return *reinterpret_cast<const uint2*>(p);
     const __half2 lo = __halves2half2(p[0], p[1]), hi = __halves2half2(p[2], p[3]);
@@ -175,8 +175,9 @@ __device__ __forceinline__ uint2 ld_half4(const __half* p) {
 // taken from the carried window state[c][0..3] (state[c][3] is the newest).  A thread owns four
 // adjacent channels and T tokens, so every input is loaded once (8 bytes at a time) plus the three before
 // its first token.  T = 8 for long chunks (512 tokens of 10240 channels 24.1 -> 11.2 us against a thread
-// per channel and token); short ones would leave most SMs empty and take T = 2.
-template <int T>
+// per channel and token); short ones would leave most SMs empty and take T = 2.  WIDE: x is 8-byte aligned
+// (it may start at any element; deciding per load instead costs a layer of 512 tokens 1 us).
+template <int T, bool WIDE>
 __global__ void __launch_bounds__(128)
 dn_conv_tokens_kernel(const __half* __restrict__ x, long long ld, const __half* __restrict__ conv_w,
                       const __half* __restrict__ conv_state, __half* __restrict__ conv_out,
@@ -199,7 +200,7 @@ dn_conv_tokens_kernel(const __half* __restrict__ x, long long ld, const __half* 
     for (int i = 0; i < T + 3; i++) {
         const int t = t0 - 3 + i;
         uint2 u = make_uint2(0u, 0u);
-        if (t >= 0 && t < n) u = *reinterpret_cast<const uint2*>(x + (size_t)t * ld + c);
+        if (t >= 0 && t < n) u = WIDE ? *reinterpret_cast<const uint2*>(x + (size_t)t * ld + c) : ld_half4(x + (size_t)t * ld + c);
         unpack(u, win[i]);
     }
     if (t0 < 3) {                      // (T = 2: the second strip still reaches back to the carried window)
@@ -720,8 +721,10 @@ int launch_dn_prefill(const void* x, long long ld, const void* conv_w, void* con
     const __half* xh = (const __half*)x;
     bool ok = true;
     const int conv_t = n > 128 ? 8 : 2;
-    ok = ok && nvfp4::launch_pdl(conv_t == 8 ? nvfp4::dn_conv_tokens_kernel<8> : nvfp4::dn_conv_tokens_kernel<2>,
-                                 dim3((conv_dim + 511) / 512, (n + conv_t - 1) / conv_t), dim3(128), 0, st, xh, ld,
+    const bool wide = ((uintptr_t)x & 7) == 0;                  // (ld is a multiple of 4)
+    const auto conv = conv_t == 8 ? (wide ? nvfp4::dn_conv_tokens_kernel<8, true> : nvfp4::dn_conv_tokens_kernel<8, false>)
+                                  : (wide ? nvfp4::dn_conv_tokens_kernel<2, true> : nvfp4::dn_conv_tokens_kernel<2, false>);
+    ok = ok && nvfp4::launch_pdl(conv, dim3((conv_dim + 511) / 512, (n + conv_t - 1) / conv_t), dim3(128), 0, st, xh, ld,
                                  (const __half*)conv_w, (const __half*)conv_state, conv_out, conv_dim,
                                  n) == cudaSuccess;
     ok = ok && nvfp4::launch_pdl(nvfp4::dn_block_kernel, dim3((nk + 3) / 4, nb), dim3(128), 0,

@@ -145,3 +145,32 @@ def test_attn_prep_of_a_chunk_equals_token_by_token(lib, hq, hkv, n):
         torch.cuda.synchronize()
     for x, y in zip(a, b):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("shift", [1, 2, 3])
+@pytest.mark.parametrize("n", [1, 3, 9, 130])
+def test_deltanet_chunk_with_inputs_at_any_element(lib, n, shift):
+    # x a view that starts at an odd element of a wider row (every access to it is legal at 2 bytes):
+    # the same values, the same bits
+    rng = np.random.default_rng(n + shift)
+    nk, nv = 2, 4
+    C = (2 * nk + nv) * 128
+    width = C + nv * 128 + 2 * nv
+    ld = width + 8
+    x = rng.standard_normal((n, width)).astype(np.float16)
+    results = []
+    for at in (0, shift):
+        room = torch.zeros(n * ld + 8, dtype=torch.float16, device="cuda")
+        rows = room[at:at + n * ld].view(n, ld)
+        rows[:, :width] = dev(x)
+        args = [dev(np.random.default_rng(1).standard_normal(s).astype(np.float16)) for s in ((C, 4), (C, 4), nv, nv, 128)]
+        state = dev(np.random.default_rng(2).standard_normal((nv, 128, 128)).astype(np.float32))
+        nbytes = lib.nvfp4_dn_prefill_work_bytes(n, nk, nv)
+        work = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+        out = torch.zeros((n, nv * 128), dtype=torch.float16, device="cuda")
+        assert lib.launch_dn_prefill(ptr(rows), ld, *[ptr(a) for a in args], ptr(state), ptr(work), nbytes, ptr(out), n,
+                                     nk, nv, 1e-6, stream()) == 0
+        torch.cuda.synchronize()
+        results.append((out, state, args[1]))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
