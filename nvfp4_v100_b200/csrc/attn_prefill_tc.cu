@@ -225,7 +225,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             auto piece = [&]() {
                 if (ok) ok = atc_wait(smem_u32(&bar_full[s]), ph, 2);
                 tcgen05_fence_after();
-                return ok;
             };
             auto done = [&]() {
                 tcgen05_commit(smem_u32(&bar_empty[s]));
@@ -233,7 +232,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             };
             auto scores = [&](int i) {
                 const uint32_t d = tmem + (uint32_t)((i & 1) * 128);
-                for (int h = 0; h < 2 && piece(); h++) {
+                for (int h = 0; h < 2; h++) {
+                    piece();
                     const uint32_t a = smem_u32(smem + 2 * h * ATC_Q_GROUP), b = smem_u32(smem_ring + s * ATC_PIECE);
 #pragma unroll
                     for (int kk = 0; kk < 8; kk++)           // 128 dims, 16 at a time
@@ -244,12 +244,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 }
                 tcgen05_commit(smem_u32(&bar_s[i & 1]));
             };
-            if (ok) scores(0);
-            for (int i = 0; i < steps && ok; i++) {
+            scores(0);
+            for (int i = 0; i < steps; i++) {
                 if (i + 1 < steps) scores(i + 1);
                 if (ok) ok = atc_wait(smem_u32(&bar_p[i & 1]), (uint32_t)(i >> 1) & 1u, 3);
                 tcgen05_fence_after();
-                for (int h = 0; h < 2 && piece(); h++) {
+                for (int h = 0; h < 2; h++) {
+                    piece();
                     const uint32_t a = tmem + (uint32_t)((i & 1) * 128 + h * 64), b = smem_u32(smem_ring + s * ATC_PIECE);
 #pragma unroll
                     for (int kk = 0; kk < 8; kk++)           // four 16-key steps of hi, then of lo
@@ -272,6 +273,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         for (int i = 0; i < steps; i++) {
             const int b = i & 1;
             if (ok) ok = atc_wait(smem_u32(&bar_s[b]), (uint32_t)(i >> 1) & 1u, 4);
+            __syncwarp();                                    // the accesses below are .aligned
             tcgen05_fence_after();
             const uint32_t at = tmem + lane_base + (uint32_t)(b * 128 + half * 64);
             uint32_t sv[2][32];
@@ -306,6 +308,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 if (mt > m + ATC_RESCALE) m = mt;
                 l *= f;
                 if (ok) ok = atc_wait(smem_u32(&bar_o[b ^ 1]), (uint32_t)((i - 1) >> 1) & 1u, 5);
+                __syncwarp();
                 tcgen05_fence_after();
 #pragma unroll 1
                 for (int c = 0; c < 128; c += 16) {
@@ -348,6 +351,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         float* tile = reinterpret_cast<float*>(smem);
         if (steps > 0) {
             atc_wait(smem_u32(&bar_o[(steps - 1) & 1]), (uint32_t)((steps - 1) >> 1) & 1u, 6);
+            __syncwarp();
             tcgen05_fence_after();
         }
 #pragma unroll

@@ -151,13 +151,14 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap act_map,
         const uint32_t idesc = (1u << 4) | (IN_TM ? 0u : (1u << 16)) | ((uint32_t)(BN >> 3) << 17) |
                                ((uint32_t)(GEMM_BM >> 4) << 24);
         // stage index, phase and operand addresses are kept by increment (no division, no
-        // address arithmetic from scratch in this one-thread loop)
+        // address arithmetic from scratch in this loop)
         int s = 0;
         uint32_t ph = 0;
+        bool ok = true;
         uint32_t a_base = smem_u32(smem_a), b_base = smem_u32(smem_b);
         uint32_t bar_f = smem_u32(&bar_full[0]), bar_e = smem_u32(&bar_empty[0]);
         for (int it = 0; it < ksteps; it++) {
-            if (!mbar_wait(bar_f, ph, 1)) break;
+            if (ok) ok = mbar_wait(bar_f, ph, 1);
             tcgen05_fence_after();
 #pragma unroll
             for (int kk = 0; kk < GEMM_BK / 16; kk++) {

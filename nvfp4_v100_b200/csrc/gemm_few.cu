@@ -195,8 +195,9 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
                                ((uint32_t)(FEW_BM >> 4) << 24);
         int u = 0;
         uint32_t ph = 0;
+        bool ok = true;
         for (int i = 0; i < 2 * nst; i++) {
-            if (!few_wait(smem_u32(&bar_ready[u]), ph, 2)) break;
+            if (ok) ok = few_wait(smem_u32(&bar_ready[u]), ph, 2);
             tcgen05_fence_after();
             const uint32_t b = smem_u32(smem_b + u * B_BYTES);
             const uint32_t a = tmem_a + (uint32_t)(u * 64);
@@ -227,6 +228,8 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
                 p[c] = *reinterpret_cast<const uint4*>(row + (((grp * 4 + c) ^ (r & 7)) << 4));
             const uint2 sc = *reinterpret_cast<const uint2*>(smem_s + s * FEW_S_BYTES + r * 16 + grp * 8);
             if (ok) ok = few_wait(smem_u32(&bar_free[u]), uph ^ 1u, 4);
+            __syncwarp();                                      // every lane's reads of the stage are done, and the
+            if (lane == 0) mbar_arrive(smem_u32(&bar_empty[s]));   // stores below are .aligned
             tcgen05_fence_after();
             const uint32_t a = tmem_a + lane_base + (uint32_t)(u * 64);
 #pragma unroll
@@ -235,8 +238,6 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
                 gemm_dequant32(p[c], (c < 2 ? sc.x : sc.y) >> (16 * (c & 1)), o);
                 tcgen05_st_32x32b_x16(a + (uint32_t)(c * 16), o);
             }
-            __syncwarp();                                      // every lane's reads of the stage are done
-            if (lane == 0) mbar_arrive(smem_u32(&bar_empty[s]));
             tcgen05_wait_st();
             tcgen05_fence_before();
             __syncwarp();
@@ -247,6 +248,7 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
         }
         // accumulator -> shared memory [token][row] (the rings are idle: every copy has been consumed)
         few_wait(smem_u32(&bar_accum), 0, 5);
+        __syncwarp();
         tcgen05_fence_after();
         float* red = reinterpret_cast<float*>(smem);
         constexpr int CW = BN / 2;                             // token columns per group

@@ -195,13 +195,13 @@ gemm_fp4_block_scaled_kernel(const __grid_constant__ CUtensorMap w_map,
         int s = 0, ti = 0;
         uint32_t ph = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ti++) {
+        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ti++) {
             // the epilogue of the tile before must have read the accumulator
-            if (ti > 0 && !f4_wait(smem_u32(&bar_acc_free), (uint32_t)(ti - 1) & 1u, 5)) break;
+            if (ok && ti > 0) ok = f4_wait(smem_u32(&bar_acc_free), (uint32_t)(ti - 1) & 1u, 5);
             tcgen05_fence_after();
             for (int it = 0; it < ksteps; it++) {
                 // (the scale writers arrive only after they saw the stage's copies land)
-                if (!f4_wait(smem_u32(&bar_sf[s]), ph, 1)) { ok = false; break; }
+                if (ok) ok = f4_wait(smem_u32(&bar_sf[s]), ph, 1);
                 tcgen05_fence_after();
                 const uint32_t a_base = smem_u32(smem_a + s * A_BYTES);
                 const uint32_t b_base = smem_u32(smem_b + s * B_BYTES);

@@ -407,15 +407,14 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             const uint64_t b_desc0 = make_desc_sw128(smem_u32(smem_b), 16, 1024);
             int s = 0, ks = ks0, seg = 0, bs = 0;
             uint32_t ph = 0;
-            bool first = true;
+            bool first = true, ok = true;
             for (int i = 0; i < nst; i++) {
                 const int buf = seg & 1;
-                if (first &&  // the flush warps must have drained this accumulator's previous use
-                    !tc_wait_poll(smem_u32(&bar_acc_empty[buf]), (((uint32_t)seg >> 1) & 1u) ^ 1u, 1))
-                    break;
+                if (ok && first)  // the flush warps must have drained this accumulator's previous use
+                    ok = tc_wait_poll(smem_u32(&bar_acc_empty[buf]), (((uint32_t)seg >> 1) & 1u) ^ 1u, 1);
                 // the scale writers arrive here only after they saw the stage's copies land and
                 // its digit planes written
-                if (!tc_wait_poll(smem_u32(&bar_ready[s]), ph, 3)) break;
+                if (ok) ok = tc_wait_poll(smem_u32(&bar_ready[s]), ph, 3);
                 tcgen05_fence_after();
                 if (rec && i == 0 && lane == 0) atomicMax(dbg + 5, tc_now());
                 const uint64_t adesc = a_desc0 + (uint64_t)(s * (TC_A_BYTES >> 4));
@@ -807,18 +806,15 @@ gemv_tc_mlp_kernel(const __grid_constant__ CUtensorMap w_map0, const __grid_cons
             int s = 0, seg = 0, bs = 0;
             uint32_t ph = 0;
             bool ok = true;
-            for (int p = 0; p < 2 && ok; p++) {
+            for (int p = 0; p < 2; p++) {
                 const int nst = p ? R1.nst : R0.nst, nk = p ? R1.nk : R0.nk;
                 int ks = p ? R1.ks0 : R0.ks0;
                 bool first = true;
                 for (int i = 0; i < nst; i++) {
                     const int buf = seg & 1;
-                    if (first &&
-                        !tc_wait_poll(smem_u32(&bar_acc_empty[buf]), (((uint32_t)seg >> 1) & 1u) ^ 1u, 1)) {
-                        ok = false;
-                        break;
-                    }
-                    if (!tc_wait_poll(smem_u32(&bar_ready[s]), ph, 3)) { ok = false; break; }
+                    if (ok && first)
+                        ok = tc_wait_poll(smem_u32(&bar_acc_empty[buf]), (((uint32_t)seg >> 1) & 1u) ^ 1u, 1);
+                    if (ok) ok = tc_wait_poll(smem_u32(&bar_ready[s]), ph, 3);
                     tcgen05_fence_after();
                     const uint64_t adesc = a_desc0 + (uint64_t)(s * (TC_A_BYTES >> 4));
                     const uint64_t bdesc = b_desc0 + (uint64_t)(bs * (TC_B_BYTES >> 4));

@@ -82,7 +82,10 @@ __device__ __forceinline__ void tcgen05_fence_before() {
 __device__ __forceinline__ void tcgen05_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 }
-// MMA and commit instructions are called by a whole converged warp and executed by one elected lane.
+// MMA and commit instructions are called by a whole converged warp and executed by one elected lane.  A
+// bounded wait answers lane by lane, and where it runs out may do so on some lanes only, so a role that
+// issues them never leaves its loop on that answer: it writes `if (ok) ok = wait(..)` and goes on, on every
+// lane (elect.sync itself waits for all 32), to numbers that the status word says are wrong.
 // With `if (lane == 0)` around the issuing loop instead, the loop's control flow is not uniform for
 // the compiler, which then moves every operand from general to uniform registers before each MMA:
 // measured 78 cycles per MMA and 85 per commit, more than a narrow MMA takes.  (The CTA-pair forms
