@@ -57,11 +57,12 @@ static_assert(ATC_ROWS * ATC_LD * 4 <= ATC_SMEM - 1024, "the output tile takes t
 
 __device__ int g_atc_status = 0;
 
-// Bounded wait (about 2 s), parked by the hardware.
-__device__ __forceinline__ bool atc_wait(uint32_t bar, uint32_t parity, int id) {
+// Bounded wait (about 2 s), parked by the hardware.  One that runs out is noted for the host and the CTA.
+__device__ __forceinline__ bool atc_wait(uint32_t bar, uint32_t parity, int id, volatile int& ran_out) {
     for (uint32_t i = 0; i < ATC_SPIN_LIMIT; i++)
         if (mbar_try_wait_hint(bar, parity, 20000)) return true;
     atomicExch(&g_atc_status, 1 + id);
+    ran_out = 1;
     return false;
 }
 __device__ __forceinline__ float atc_ld_cluster(uint32_t addr) {
@@ -135,6 +136,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     __shared__ __align__(8) uint64_t bar_p[2];               // weights of a step ready
     __shared__ __align__(8) uint64_t bar_o[2];               // O holds a step
     __shared__ uint32_t s_tmem;
+    __shared__ volatile int s_ran_out;                       // a wait of this CTA has
+    __shared__ int s_next[2];                                // the ring slot after the last piece, and its lap
     __shared__ float s_mx[2][2][ATC_ROWS];                   // step parity, key half, row
     __shared__ float s_m[ATC_ROWS], s_l[2][ATC_ROWS];
 
@@ -162,6 +165,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             mbar_init(smem_u32(&bar_p[b]), 8);
             mbar_init(smem_u32(&bar_o[b]), 1);
         }
+        s_ran_out = 0;
         fence_barrier_init();
     }
     if (warp == 1) {
@@ -186,7 +190,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             uint32_t ph = 0;
             bool ok = true;
             auto slot = [&]() {                              // the next free piece of the ring
-                if (ok) ok = atc_wait(smem_u32(&bar_empty[s]), ph ^ 1u, 0);
+                if (ok) ok = atc_wait(smem_u32(&bar_empty[s]), ph ^ 1u, 0, s_ran_out);
                 return ok;
             };
             auto next = [&]() { if (++s == ATC_SLOTS) { s = 0; ph ^= 1u; } };
@@ -213,6 +217,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 if (i + 1 < steps) load_k(i + 1);
                 load_v(i);
             }
+            s_next[0] = s;
+            s_next[1] = (int)ph;
         }
     } else if (warp == 1) {
         if (steps > 0) {
@@ -221,9 +227,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             const uint32_t idesc_o = (1u << 4) | (1u << 16) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
             int s = 0;
             uint32_t ph = 0;
-            bool ok = atc_wait(smem_u32(&bar_q), 0, 1);
+            bool ok = atc_wait(smem_u32(&bar_q), 0, 1, s_ran_out);
             auto piece = [&]() {
-                if (ok) ok = atc_wait(smem_u32(&bar_full[s]), ph, 2);
+                if (ok) ok = atc_wait(smem_u32(&bar_full[s]), ph, 2, s_ran_out);
                 tcgen05_fence_after();
             };
             auto done = [&]() {
@@ -247,7 +253,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             scores(0);
             for (int i = 0; i < steps; i++) {
                 if (i + 1 < steps) scores(i + 1);
-                if (ok) ok = atc_wait(smem_u32(&bar_p[i & 1]), (uint32_t)(i >> 1) & 1u, 3);
+                if (ok) ok = atc_wait(smem_u32(&bar_p[i & 1]), (uint32_t)(i >> 1) & 1u, 3, s_ran_out);
                 tcgen05_fence_after();
                 for (int h = 0; h < 2; h++) {
                     piece();
@@ -272,7 +278,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         bool ok = true;
         for (int i = 0; i < steps; i++) {
             const int b = i & 1;
-            if (ok) ok = atc_wait(smem_u32(&bar_s[b]), (uint32_t)(i >> 1) & 1u, 4);
+            if (ok) ok = atc_wait(smem_u32(&bar_s[b]), (uint32_t)(i >> 1) & 1u, 4, s_ran_out);
             __syncwarp();                                    // the accesses below are .aligned
             tcgen05_fence_after();
             const uint32_t at = tmem + lane_base + (uint32_t)(b * 128 + half * 64);
@@ -307,7 +313,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 const float f = (mt > m + ATC_RESCALE) ? expf(m - mt) : 1.0f;
                 if (mt > m + ATC_RESCALE) m = mt;
                 l *= f;
-                if (ok) ok = atc_wait(smem_u32(&bar_o[b ^ 1]), (uint32_t)((i - 1) >> 1) & 1u, 5);
+                if (ok) ok = atc_wait(smem_u32(&bar_o[b ^ 1]), (uint32_t)((i - 1) >> 1) & 1u, 5, s_ran_out);
                 __syncwarp();
                 tcgen05_fence_after();
 #pragma unroll 1
@@ -350,7 +356,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         // O -> shared memory (Q and the ring are idle: the last MMA has retired, every copy was consumed)
         float* tile = reinterpret_cast<float*>(smem);
         if (steps > 0) {
-            atc_wait(smem_u32(&bar_o[(steps - 1) & 1]), (uint32_t)((steps - 1) >> 1) & 1u, 6);
+            atc_wait(smem_u32(&bar_o[(steps - 1) & 1]), (uint32_t)((steps - 1) >> 1) & 1u, 6, s_ran_out);
             __syncwarp();
             tcgen05_fence_after();
         }
@@ -372,6 +378,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     }
     tcgen05_fence_before();
     __syncthreads();
+    // No copy may be in flight when the CTA leaves.  Where no wait has run out, all have been consumed by now
+    // (waiting for them all the same costs 0.6 to 1 us); a slot that was never filled answers at once.
+    if (threadIdx.x == 0 && s_ran_out) {
+        if (steps > 0) atc_wait(smem_u32(&bar_q), 0, 7, s_ran_out);
+        for (int j = 0; j < ATC_SLOTS && steps > 0; j++)
+            atc_wait(smem_u32(&bar_full[j]), (uint32_t)s_next[1] ^ (j < s_next[0] ? 0u : 1u), 7, s_ran_out);
+    }
     if (split > 1) cluster_sync_all();
 
     // ---- weighted sum over the cluster, gate, output: a warp takes a row, a lane 4 + 4 dims ----

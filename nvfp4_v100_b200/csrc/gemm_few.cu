@@ -157,19 +157,22 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
             // the other stages follow the first activation units, which would queue behind them in
             // the SM's request path
             few_wait(smem_u32(&bar_breq), 0, 6);
-            int s = FEW_PRE;
+            int s = FEW_PRE, issued = min(FEW_PRE, nst);
             uint32_t ph = 0;
-            for (int i = FEW_PRE; i < nst; i++) {
+            for (int i = FEW_PRE; i < nst; i++, issued++) {
                 if (s == NS) { s = 0; ph ^= 1u; }
                 if (!few_wait(smem_u32(&bar_empty[s]), ph ^ 1u, 0)) break;
                 request(i, s++);
             }
+            // no copy may be in flight when the CTA leaves, also where a wait has run out
+            for (int i = max(issued - NS, 0); i < issued; i++)
+                few_wait(smem_u32(&bar_full[i % NS]), (uint32_t)(i / NS) & 1u, 7);
         }
     } else if (warp == 2) {
         if (lane == 0) {
-            int u = 0;
+            int u = 0, issued = 0;
             uint32_t ph = 0;
-            for (int i = 0; i < 2 * nst; i++) {
+            for (int i = 0; i < 2 * nst; i++, issued++) {
                 if (!few_wait(smem_u32(&bar_free[u]), ph ^ 1u, 1)) break;
                 const uint32_t bar = smem_u32(&bar_ready[u]);
                 const uint32_t dst = smem_u32(smem_b + u * B_BYTES);
@@ -188,6 +191,8 @@ gemm_w4a16_few_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
                 if (i == (NU < 2 * nst ? NU : 2 * nst) - 1) mbar_arrive(smem_u32(&bar_breq));
                 if (++u == NU) { u = 0; ph ^= 1u; }
             }
+            for (int i = max(issued - NU, 0); i < issued; i++)
+                few_wait(smem_u32(&bar_ready[i % NU]), (uint32_t)(i / NU) & 1u, 8);
         }
     } else if (warp == 1) {
         // D fp32, A fp16 (tensor memory), B fp16 (K-major, or MN-major if token-minor), N = BN, M = 128

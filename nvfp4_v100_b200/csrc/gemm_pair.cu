@@ -138,19 +138,22 @@ gemm_w4a16_pair_tm_kernel(const __grid_constant__ CUtensorMap w_map, const __gri
 
     if (warp == 0) {
         if (lane == 0) {
-            int s = 0;
+            int s = 0, issued = min(GP_NS, nst);
             uint32_t ph = 0;
-            for (int i = GP_NS; i < nst; i++) {
+            for (int i = GP_NS; i < nst; i++, issued++) {
                 if (!gp_wait(smem_u32(&bar_empty[s]), ph, 0)) break;
                 request(i, s);
                 if (++s == GP_NS) { s = 0; ph ^= 1u; }
             }
+            // no copy may be in flight when the CTA leaves, also where a wait has run out
+            for (int i = max(issued - GP_NS, 0); i < issued; i++)
+                gp_wait(smem_u32(&bar_full[i % GP_NS]), (uint32_t)(i / GP_NS) & 1u, 6);
         }
     } else if (warp == 2) {
         if (lane == 0) {
-            int u = 0;
+            int u = 0, issued = 0;
             uint32_t ph = 0;
-            for (int i = 0; i < nun; i++) {
+            for (int i = 0; i < nun; i++, issued++) {
                 if (!gp_wait(smem_u32(&bar_free[u]), ph ^ 1u, 1)) break;
                 const uint32_t bar = cluster_map_shared(smem_u32(&bar_ready[u]), 0);
                 mbar_arrive_expect_tx_cluster(bar, TX);
@@ -167,6 +170,10 @@ gemm_w4a16_pair_tm_kernel(const __grid_constant__ CUtensorMap w_map, const __gri
                 }
                 if (++u == GP_NU) { u = 0; ph ^= 1u; }
             }
+            // (ready is the first CTA's and counts both CTAs' copies; the second stays until the first has synced)
+            if (rank == 0)
+                for (int i = max(issued - GP_NU, 0); i < issued; i++)
+                    gp_wait(smem_u32(&bar_ready[i % GP_NU]), (uint32_t)(i / GP_NU) & 1u, 7);
         }
     } else if (warp == 1) {
         if (rank == 0) {

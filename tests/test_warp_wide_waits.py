@@ -26,12 +26,12 @@ def _block(text, start):
     raise AssertionError("unbalanced braces")
 
 
-def _roles(name, pattern):
+def _roles(name, pattern, one_thread=False):
     text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
     for m in re.finditer(r"if \(warp (?:==|>=) \d+\)", text):
         body = _block(text, m.end())
-        one_thread = re.match(r"\{\s*if \(lane == 0\)", body)    # nothing to agree on
-        if not one_thread and re.search(pattern, body):
+        one = re.match(r"\{\s*if \(lane == 0", body)              # one thread's loop: nothing to agree on
+        if bool(one) == one_thread and re.search(pattern, body):
             yield m.group(0), body
 
 
@@ -64,3 +64,21 @@ def test_aligned_accesses_stand_behind_a_syncwarp(name):
             seen += kind == "access"
             parted = kind == "wait" or (parted and kind != "sync")
     assert seen, "no such role found: the pattern no longer fits the source"
+
+
+@pytest.mark.parametrize("name,rings", [("gemm_few.cu", {"bar_full", "bar_ready"}), ("gemm_pair.cu", {"bar_full", "bar_ready"}),
+                                        ("attn_prefill_tc.cu", {"bar_full", "bar_q"})])
+def test_copies_are_waited_for_before_the_cta_leaves(name, rings):
+    # a thread that stops copying early (its own wait ran out) has copies in flight: behind the last
+    # copy, that thread (thread 0, or the first of its role) waits for every barrier that copies complete
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+    kernel = _block(text, text.index("__global__"))
+    roles = [b for _, b in _roles(name, r"\b(?:tma_load_\w+|request)\(", one_thread=True)]
+    assert roles
+    waited = set()
+    for body in roles:
+        last = max(m.start() for m in re.finditer(r"\b(?:tma_load_\w+|request)\(|\bbreak;", body))
+        waited |= set(re.findall(r"_wait\(smem_u32\(&(\w+)", body[last:]))
+    for m in re.finditer(r"if \(threadIdx\.x == 0 && s_ran_out\)", kernel):
+        waited |= set(re.findall(r"_wait\(smem_u32\(&(\w+)", _block(kernel, m.end())))
+    assert rings <= waited
