@@ -526,13 +526,18 @@ dn_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
 #pragma unroll
             for (int i = 0; i < DNB; i++) {
                 p[i] = __shfl_sync(0xffffffffu, own, (lane & 24) + i);
-                v[i] = t0 + i < n ? __half2float(s.v[bb * DNB + i][lrow + mine]) : 0.0f;
+                v[i] = __half2float(s.v[bb * DNB + i][lrow + mine]);
             }
             const float e0 = beta.x * (v[0] - gam.x * p[0]);
             const float e1 = beta.y * ((v[1] - gam.y * p[1]) - c1.x * e0);
             const float e2 = beta.z * (((v[2] - gam.z * p[2]) - c2.x * e0) - c2.y * e1);
             const float e3 = beta.w * ((((v[3] - gam.w * p[3]) - c3.x * e0) - c3.y * e1) - c3.z * e2);
-            const float f[DNB] = {e0 * tail.x, e1 * tail.y, e2 * tail.z, e3 * tail.w};
+            float f[DNB] = {e0 * tail.x, e1 * tail.y, e2 * tail.z, e3 * tail.w};
+            if (t0 + DNB > n) {                              // a place past the end adds nothing, also where zero
+#pragma unroll                                               // times what the block holds is not zero
+                for (int i = 1; i < DNB; i++)
+                    if (t0 + i >= n) f[i] = 0.0f;
+            }
             float g[DNB];                                    // the other row's
 #pragma unroll
             for (int i = 0; i < DNB; i++) g[i] = __shfl_xor_sync(0xffffffffu, f[i], 8);

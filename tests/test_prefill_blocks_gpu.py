@@ -174,3 +174,24 @@ def test_deltanet_chunk_with_inputs_at_any_element(lib, n, shift):
         results.append((out, state, args[1]))
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 6, 7, 17])
+def test_deltanet_state_after_an_infinite_last_value(lib, n):
+    # The last token of a chunk that ends inside a block of four: S = S e^g + k delta with delta infinite
+    # leaves infinities of k's sign, whatever the block's empty places hold.
+    rng = np.random.default_rng(n)
+    C, ld = 384, 384 + 128 + 4
+    x = rng.standard_normal((n, ld)).astype(np.float16)
+    x[n - 1, 256:384] = np.inf
+    d = [dev(a) for a in (x, np.full((C, 4), 0.5, np.float16), np.zeros((C, 4), np.float16), np.zeros(1, np.float16),
+                          np.zeros(1, np.float16), np.ones(128, np.float16), np.zeros((1, 128, 128), np.float32))]
+    nbytes = lib.nvfp4_dn_prefill_work_bytes(n, 1, 1)
+    work = torch.full((nbytes,), 0xFF, dtype=torch.uint8, device="cuda")
+    out = torch.zeros((n, 128), dtype=torch.float16, device="cuda")
+    assert lib.launch_dn_prefill(ptr(d[0]), ld, ptr(d[1]), ptr(d[2]), ptr(d[3]), ptr(d[4]), ptr(d[5]), ptr(d[6]), ptr(work),
+                                 nbytes, ptr(out), n, 1, 1, 1e-6, stream()) == 0
+    torch.cuda.synchronize()
+    acc = (x[max(0, n - 4):, 128:256].astype(np.float64) * 0.5).sum(0)          # k before its (positive) silu and norm
+    state = d[6].cpu().numpy()[0]
+    assert np.isinf(state).all() and (np.sign(state) == np.sign(acc)).all()
