@@ -578,21 +578,22 @@ dn_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
 // otherwise crowd the free ones, for the whole chunk: a layer of 512 tokens 249 -> 180 us.
 static size_t scan_padding(int ctas) {
     static int sms[NVFP4_MAX_DEVICES] = {0};
-    static int opted[NVFP4_MAX_DEVICES] = {0};
+    static bool opted[NVFP4_MAX_DEVICES] = {false};
     constexpr int SM_BYTES = 227 * 1024, RESERVED = 1024;
+    constexpr int MOST = (SM_BYTES - RESERVED - (int)(2 * sizeof(ScanStage))) & ~127;
     const int dev = current_device_index();
     if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    const int per_sm = (ctas + sms[dev] - 1) / sms[dev];
-    const int pad = (SM_BYTES / per_sm - RESERVED - (int)(2 * sizeof(ScanStage))) & ~127;
-    if (pad <= 0) return 0;
-    if (pad > opted[dev]) {
-        if (cudaFuncSetAttribute(dn_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pad) != cudaSuccess) {
+    // the opt-in is the same whatever this call needs: another thread's first call cannot lower it
+    if (!opted[dev]) {
+        if (cudaFuncSetAttribute(dn_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST) != cudaSuccess) {
             cudaGetLastError();
             return 0;
         }
-        opted[dev] = pad;
+        opted[dev] = true;
     }
-    return (size_t)pad;
+    const int per_sm = (ctas + sms[dev] - 1) / sms[dev];
+    const int pad = (SM_BYTES / per_sm - RESERVED - (int)(2 * sizeof(ScanStage))) & ~127;
+    return pad > 0 ? (size_t)pad : 0;
 }
 
 // gated norm per (token, value head): out = f16( f32(f16(o rsqrt(mean(o^2) + eps)) * norm_w) * silu(z) )

@@ -1,0 +1,49 @@
+"""First calls of one entry point from several threads at once, in a process of its own."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+PROGRAM = """
+import threading
+import torch
+from nvfp4_v100_b200 import _lib
+from tests.gpu_util import ptr
+
+lib = _lib.load()
+HEADS = [1, 19, 37, 56, 74, 100, 148, 2]      # the scan's padding differs from head count to head count
+n = 5
+start, codes = threading.Barrier(len(HEADS)), {}
+
+def call(nv):
+    C = (2 + nv) * 128
+    ld = C + nv * 128 + 2 * nv
+    ld += -ld % 4
+    z = lambda *s: torch.zeros(s, dtype=torch.float16, device="cuda")
+    x, cw, cs, al, dt, nw, out = z(n, ld), z(C, 4), z(C, 4), z(nv), z(nv), z(128), z(n, nv * 128)
+    state = torch.zeros((nv, 128, 128), device="cuda")
+    nbytes = lib.nvfp4_dn_prefill_work_bytes(n, 1, nv)
+    work = torch.zeros(nbytes, dtype=torch.uint8, device="cuda")
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    start.wait()
+    codes[nv] = [lib.launch_dn_prefill(ptr(x), ld, ptr(cw), ptr(cs), ptr(al), ptr(dt), ptr(nw), ptr(state), ptr(work),
+                                       nbytes, ptr(out), n, 1, nv, 1e-6, side.cuda_stream) for _ in range(20)]
+    side.synchronize()
+
+threads = [threading.Thread(target=call, args=(nv,)) for nv in HEADS]
+for t in threads:
+    t.start()
+for t in threads:
+    t.join()
+assert codes == {nv: [0] * 20 for nv in HEADS}, codes
+"""
+
+
+def test_deltanet_chunk():
+    for _ in range(4):
+        subprocess.run([sys.executable, "-c", PROGRAM], cwd=ROOT, check=True, timeout=120)
