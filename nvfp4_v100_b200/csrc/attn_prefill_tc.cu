@@ -14,8 +14,9 @@
 //                O += P(i) . V(i) (M 128, N 256, P from tensor memory)
 //   warps 4..11  softmax: a thread owns 64 of the 128 scores of its row
 // Tensor memory: two S/P buffers of 128 columns and the 256 columns of O.  P takes the place of its
-// own scores.  It stays at fp32 weight precision: p = hi + lo, two fp16 numbers (22 significant bits,
-// p scaled by 2^12 so that small weights keep them too), and O accumulates hi . V and lo . V.
+// own scores and is carried as p = hi + lo, two fp16 numbers whose sum is within 2^-23 of p's power of two
+// (the kernel before held it in fp32: 2^-24) and, p being scaled by 2^12, within 2^-37 for small weights;
+// O accumulates hi . V and lo . V.
 // O is rescaled only when a row's maximum has grown by more than 2 since the last time (so p stays
 // below 2^15); otherwise the old reference point stays and nothing waits on the MMAs.
 // Few tokens leave SMs idle: then the keys are split over the CTAs of a cluster, whose (max, sum, O)
@@ -29,7 +30,8 @@
 //   512 after 0      27.1 (386)     512 after 3488  123 (3596)     26 after 511   16.2 (58.9)
 //   512 after 512    41.1 (859)     512 after 9000  253 (8670)    100 after 0    17.6 (45.7)
 // i.e. 20 us fixed and 26 us per 1024 keys of 512 tokens: 100 CTAs, 3072 cycles of MMAs per step.
-// Relative error against float64 unchanged (3.5e-4: the fp16 rounding of the output).
+// Relative error against float64 as before (3.5e-4, the fp16 rounding of the output; see ATC_CHAIN).  Of the
+// outputs 0.2 to 0.8 % are not the correctly rounded ones, against 0.1 % before.
 #include <cuda.h>
 
 #include "attn_prefill_tc.cuh"
@@ -49,6 +51,12 @@ constexpr int ATC_Q_GROUP = ATC_ROWS * 128;         // bytes of 64 dims of all r
 constexpr int ATC_SMEM = 4 * ATC_Q_GROUP + ATC_SLOTS * ATC_PIECE + 1024;
 constexpr int ATC_LD = ATC_D + 4;                   // floats per row of the output tile in shared memory
 constexpr int ATC_MAX_SPLIT = 8;
+// Key steps of one CTA's accumulation.  An MMA truncates the fp32 sum that it adds to (a bias towards
+// zero, twice per 16 keys), where the kernel before rounded to nearest: with all 32 steps of 4000 keys in
+// one CTA the outputs' relative error against float64 was 3.1e-4 of itself above that kernel's (24 seeds,
+// standard error 4e-5), with 16 steps 9e-5, with 8 steps 2e-5, which is none.  The partial results of a
+// cluster are added by ordinary fp32 instructions.
+constexpr int ATC_CHAIN = 8;
 constexpr float ATC_P_SCALE = 4096.0f;
 constexpr float ATC_RESCALE = 2.0f;                 // e^2 * 4096 < 65504
 constexpr float ATC_NO_MAX = -3.4e38f;
@@ -548,10 +556,12 @@ int attn_prefill_tc_launch(const __half* q, const __half* keys, const __half* va
         !encode(vm, values, (cuuint64_t)lcap, (cuuint64_t)hkv, head, 64, 1))
         return -3;
     const int tiles = (n_tokens + bt - 1) / bt, steps = (lcap + ATC_KEYS - 1) / ATC_KEYS;
-    // key split: the fewest steps per CTA among the splits whose clusters all run at once
+    // key split: the fewest steps per CTA among the splits whose clusters all run at once, and more where
+    // the accumulation would get too long (512 tokens after 3488: 115 -> 125 us, after 2048 79 -> 95)
     int split = 1;
     for (int s = 2; s <= ATC_MAX_SPLIT && s <= steps; s++)
         if (tiles * hkv <= atc_clusters(dev, s) && (steps + s - 1) / s < (steps + split - 1) / split) split = s;
+    split = max(split, min(ATC_MAX_SPLIT, (steps + ATC_CHAIN - 1) / ATC_CHAIN));
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[2];
     atc_config(cfg, at, dim3((unsigned)(tiles * split), (unsigned)hkv), split);
