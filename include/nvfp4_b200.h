@@ -96,12 +96,14 @@ int get_kernel_shared_mem_bytes(void);                          /* kernels/nvfp4
 /* 0 if no bounded wait inside the tensor-core GEMM ever ran out; 1 + wait id otherwise.  reset != 0
  * clears it.  Synchronous.  No counterpart in the reference. */
 int nvfp4_gemm_status(int reset);
-/* Tuning hook of the W4A16 GEMM entry points.  Bit 0: 256-row CTA tiles (two accumulators in tensor
- * memory, the activation tile fetched once for twice the rows) for more than 128 tokens when they
- * still give every SM a CTA.  Bit 1: the CTA-pair kernel (clusters of two CTAs, tcgen05
- * cta_group::2: each CTA dequantises 128 rows and loads half of a 256-token tile) for shapes of more
- * than 128 tokens that do not get 256-row tiles.  Bit 2: the CTA-pair kernel wherever it can run
- * (more than 128 tokens, K % 128 == 0).  Default 3.  All kernels give bit-identical results. */
+/* Tuning hook of the W4A16 GEMM entry points for more than 128 tokens.  Bit 0: 256-row CTA tiles (two
+ * accumulators in tensor memory, the activation tile fetched once for twice the rows) when they still
+ * give every SM a CTA.  Bit 1: CTA-pair kernels (clusters of two CTAs, tcgen05 cta_group::2: each CTA
+ * dequantises 128 rows and loads half of a token tile): the one with the weights in tensor memory
+ * (K % 256 == 0, 16-byte aligned scales) except where 256-row tiles are faster (K below some 1000 to
+ * 4000, depending on the output layout), the other (K % 128 == 0) where 256-row tiles are not used.
+ * Bit 2: CTA-pair kernels wherever they can run.  Default 3.  All of them give bit-identical results;
+ * at most 128 tokens have a kernel of their own, which splits K and adds in another order. */
 void nvfp4_b200_gemm_config(int flags);
 
 /* Tuning hook; no counterpart in the reference.  warps per CTA (0 = auto, 2, 4 or 8), resident

@@ -596,6 +596,12 @@ static bool gemm_use_pair(int M, int N, int K) {
     if (!g_gemm_pair || N <= 128 || K % (GEMM_BK * PAIR_KS) != 0) return false;
     return g_gemm_pair == 2 || !gemm_tile_rows256(M, N);
 }
+// The kernel of gemm_pair.cu: wherever it can run, except where 256-row tiles are faster (short K).
+static bool gemm_use_pair_tm(const uint8_t* packed, const uint8_t* scales, int M, int N, int K, int out_mode) {
+    if (!g_gemm_pair || !gemm_pair_takes(packed, scales, N, K)) return false;
+    return g_gemm_pair == 2 || !gemm_tile_rows256(M, N) || gemm_pair_beats_tiles(M, N, K, out_mode);
+}
+// Those tiles are then what the shape gets, not the pair kernel of this file.
 template <bool IN_TM>
 static cudaError_t launch_tc_any(const CUtensorMap& map, const uint8_t* packed, const uint8_t* scales,
                                  __half* out, int M, int N, int K, int ld_out, int out_mode, int n_out,
@@ -630,8 +636,8 @@ int launch_nvfp4_gemmtc_v5(const uint8_t* d_weight_packed, const uint8_t* d_weig
                                        M, N, N, K, GEMM_OUT_FM, st);
         if (rc != -3) return rc;
     }
-    if (N % 8 == 0 && (((uintptr_t)d_activation | (uintptr_t)d_output) & 15) == 0 && g_gemm_pair &&
-        gemm_pair_takes(d_weight_packed, d_weight_scales, N, K)) {
+    if (N % 8 == 0 && (((uintptr_t)d_activation | (uintptr_t)d_output) & 15) == 0 &&
+        gemm_use_pair_tm(d_weight_packed, d_weight_scales, M, N, K, GEMM_OUT_FM)) {
         const int rc = gemm_pair_launch(d_weight_packed, d_weight_scales, d_activation, N, false, d_output, N,
                                         M, N, N, K, GEMM_OUT_FM, st);
         if (rc != -3) return rc;
@@ -698,7 +704,7 @@ int launch_nvfp4_gemm_w4a16_ex(const uint8_t* d_weight_packed, const uint8_t* d_
                                o, (int)ld_out, M, N8, n_tokens, K, mode, st);
     // token count the kernel's bounds use: feature-major sides are padded to 8
     const int N = (in_tm && out_tm) ? n_tokens : N8;
-    if (g_gemm_pair && gemm_pair_takes(d_weight_packed, d_weight_scales, N, K))
+    if (gemm_use_pair_tm(d_weight_packed, d_weight_scales, M, N, K, mode))
         return gemm_pair_launch(d_weight_packed, d_weight_scales, static_cast<const __half*>(act), ld_act, in_tm,
                                 o, (int)ld_out, M, N, n_tokens, K, mode, st);
     CUtensorMap map;
@@ -781,9 +787,10 @@ int nvfp4_gemm_status(int reset) {
     return v;
 }
 
-// Tuning hook.  Bit 0: 256-row CTA tiles (two accumulators) for more than 128 tokens.  Bits 1 and 2: the
-// kernel of gemm_pair.cu for every shape it takes; for the others, bit 1: the CTA-pair kernel (clusters of two, cta_group::2) for shapes of more than 128 tokens that do not get
-// 256-row tiles.  Bit 2: the CTA-pair kernel for every shape it can run.  Default 3.
+// Tuning hook, more than 128 tokens.  Bit 0: 256-row CTA tiles (two accumulators).  Bit 1: CTA-pair kernels
+// (clusters of two, cta_group::2) - the one of gemm_pair.cu where it is the faster one, the one of this file
+// for shapes that neither it nor 256-row tiles take.  Bit 2: CTA-pair kernels for every shape they can run.
+// Default 3.
 void nvfp4_b200_gemm_config(int flags) {
     nvfp4::g_gemm_rows256 = (flags & 1) ? 1 : 0;
     nvfp4::g_gemm_pair = (flags & 4) ? 2 : (flags & 2) ? 1 : 0;

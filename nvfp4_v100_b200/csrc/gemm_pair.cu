@@ -279,6 +279,23 @@ static int gp_tile_tokens(int dev, int M, int N) {
     return cost(192) < cost(256) ? 192 : 256;
 }
 
+// Against the 256-row tiles of gemm.cu (one CTA per 256 rows x 256 tokens), which overlap less but have
+// twice the tensor memory to themselves: both run in rounds, a round costs a fixed part (set-up, first
+// bytes, epilogue) and a part per k, in ns.  The fixed part counts twice here, two rounds of pairs doing the
+// work of one of tiles.  17408 x K at 2048 tokens, token-major / added into the output / feature-major, us:
+//   K =  512   tiles 64 / 103 / 57, pairs 70 / 124 / 74       K = 3072   tiles 191 / 249 / 183, pairs 169 / 243 / 180
+bool gemm_pair_beats_tiles(int M, int N, int K, int out_mode) {
+    const int dev = current_device_index();
+    const long long slots = gp_slots(dev), rows = (M + 255) / 256, bn = gp_tile_tokens(dev, M, N);
+    static const int tile_fixed[3] = {8700, 9700, 17000};                // by out_mode
+    static const int pair_fixed[2][3] = {{6800, 6300, 10500}, {7100, 6100, 11700}};   // 192, 256 tokens
+    const long long tile_rounds = (rows * ((N + 255) / 256) + 2 * slots - 1) / (2 * slots);
+    const long long pair_rounds = (rows * ((N + bn - 1) / bn) + slots - 1) / slots;
+    const long long tiles = tile_rounds * (tile_fixed[out_mode] + 119LL * K / 10);
+    const long long pairs = pair_rounds * (pair_fixed[bn == 256][out_mode] + 5LL * K * bn / 256);
+    return pairs < tiles;
+}
+
 template <int BN, bool IN_TM>
 static cudaError_t gp_launch(const CUtensorMap& wm, const CUtensorMap& sm, const CUtensorMap& am, __half* out, int M,
                              int N, int K, int ld_out, int out_mode, int n_out, cudaStream_t st) {

@@ -7,6 +7,13 @@ from tests.gpu_util import ptr, stream
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def pairs_for_every_shape(lib):
+    lib.nvfp4_b200_gemm_config(7)            # by default short K goes to 256-row tiles where those fill the GPU
+    yield
+    lib.nvfp4_b200_gemm_config(3)
+
+
 @pytest.mark.parametrize("M,n,K", [
     (256, 129, 256),        # one pair, one weight stage, one token past the few-token kernel
     (257, 192, 512),        # a pair with one row in its first CTA only; exactly one 192-token tile
@@ -52,3 +59,29 @@ def test_against_float64(lib, M, n, K, flags):
         want = want + old.double()
         bound = bound + want.abs() * 2 ** -11
     assert ((got - want).abs() <= bound * 1.001).all(), ((got - want).abs() / bound).max().item()
+
+
+@pytest.mark.parametrize("M,n,K", [
+    (20000, 520, 512), (20000, 520, 2560), (20000, 520, 5120),      # tiles, tiles or pairs by output layout, pairs
+    (10240, 1000, 256), (4096, 2048, 1024),                         # last rounds nearly empty and full
+])
+@pytest.mark.parametrize("flags", [0, 1, 2, 3, 6, 7])
+def test_the_choice_does_not_show(lib, M, n, K, flags):
+    # whichever kernel the shape and the output layout get: the same bits
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + K)
+    p = torch.randint(0, 256, (M, K // 2), dtype=torch.uint8, device="cuda", generator=g)
+    s = torch.randint(118, 123, (M, K // 16), dtype=torch.uint8, device="cuda", generator=g)
+    n8 = (n + 7) // 8 * 8
+    act = torch.randn((n, K) if flags & 1 else (K, n8), device="cuda", generator=g).half()
+    shape = (n, M) if flags & 2 else (M, n8)
+    old = torch.randn(shape, device="cuda", generator=g).half()
+    outs = []
+    for config in (7, 3, 1):
+        lib.nvfp4_b200_gemm_config(config)
+        outs.append(old.clone())
+        assert lib.launch_nvfp4_gemm_w4a16_ex(ptr(p), ptr(s), ptr(act), act.shape[1], ptr(outs[-1]), shape[1], M, n, K,
+                                              flags, stream()) == 0
+    torch.cuda.synchronize()
+    assert lib.nvfp4_gemm_status(0) == 0
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
