@@ -520,7 +520,15 @@ bool attn_prefill_tc_takes(const void* q, const void* keys, const void* values, 
                            int len0, int n_tokens, int hq, int hkv) {
     if (hq / hkv > ATC_ROWS) return false;
     if (((uintptr_t)q | (uintptr_t)keys | (uintptr_t)values | (uintptr_t)gate | (uintptr_t)out) & 15) return false;
-    return (long long)n_tokens * (len0 + n_tokens - 1) >= ATTN_TC_MIN_PAIRS;
+    const int L = len0 + n_tokens - 1, gqa = hq / hkv;
+    if ((long long)n_tokens * L < ATTN_TC_MIN_PAIRS) return false;
+    // Few heads: while the other kernel's CTAs (a head's eight tokens) fit on half of the SMs they all run
+    // at once and take a time that only the keys decide; this kernel's first 256 keys cost by its rows.  In
+    // ns, measured for 1 to 32 heads, e.g. 64 tokens of 6 heads 9.7 us against 18.3, 32 of 12 heads after 98
+    // 13.9 against 19.1, 24 of 24 heads after 150 15.6 against 19.2; 16 of 24 heads after 242 19.6 against 15.1.
+    if (2LL * hq * ((n_tokens + 7) / 8) <= device_sms(current_device_index()))
+        return 6700 + 47LL * L >= 9500 + 75 * gqa * min(n_tokens, ATC_ROWS / gqa);
+    return true;
 }
 
 int attn_prefill_tc_launch(const __half* q, const __half* keys, const __half* values, int len0, int n_tokens,

@@ -90,6 +90,16 @@ static inline int current_device_index() {
     return dev;
 }
 
+// Streaming multiprocessors of the device (148 where the driver does not say).
+static inline int device_sms(int dev) {
+    static int cached[NVFP4_MAX_DEVICES] = {};
+    if (cached[dev] == 0) {
+        int n = 0;
+        cached[dev] = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+    }
+    return cached[dev];
+}
+
 // Programmatic dependent launch.  A kernel that starts with pdl_prologue() may be launched with
 // the programmatic-stream-serialization attribute: it becomes resident while the previous kernel
 // in the stream is still draining, lets ITS successor do the same, and then waits for the

@@ -41,6 +41,8 @@ def _run(lib, q, keys, vals, p0, n, gate, hq, hkv, scale):
     (43, 1000, 9, 3, 1100, 1.0),        # 42 tokens a tile; weights on very few keys
     (512, 3488, 24, 4, 4100, 1 / 16),   # the last chunk of a long document
     (1024, 0, 6, 1, 1024, 1 / 16),
+    (64, 0, 12, 6, 64, 1 / 16),         # (the first two shapes with enough heads for this kernel)
+    (65, 63, 12, 6, 200, 1 / 16),
 ])
 def test_against_float64(lib, n, p0, hq, hkv, max_len, scale):
     q, gate, keys, vals = _inputs(n, p0, hq, hkv, max_len, n + p0)
@@ -62,9 +64,10 @@ def test_against_float64(lib, n, p0, hq, hkv, max_len, scale):
         assert ((got - want).abs() <= bound).all(), (h, ((got - want).abs() / bound).max().item())
 
 
-def test_infinities_and_nan_as_the_decode_kernel(lib):
+@pytest.mark.parametrize("hq,hkv", [(6, 2), (12, 4)])           # one query at a time; tensor cores
+def test_infinities_and_nan_as_the_decode_kernel(lib, hq, hkv):
     # a later token's value never reaches an earlier one, an unmasked one does as in fp32
-    n, p0, hq, hkv, scale = 70, 130, 6, 2, 1 / 16
+    n, p0, scale = 70, 130, 1 / 16
     q, gate, keys, vals = _inputs(n, p0, hq, hkv, 256, 3)
     vals[0, 150, 3] = float("inf")
     vals[0, 170, 5] = -float("inf")
@@ -102,3 +105,24 @@ def test_accumulation_stays_short(lib, n, p0):
         o = torch.softmax((q[:, sl].double() @ k.T * scale).masked_fill(mask, -float("inf")), -1) @ v
         other += (out[:, sl] != (o.half().double() * torch.sigmoid(gate[:, sl].double()).half().double()).half()).sum().item()
     assert other <= 0.011 * out.numel(), other / out.numel()
+
+
+@pytest.mark.parametrize("n,p0,hq,hkv,same", [
+    (64, 0, 6, 1, True), (46, 46, 12, 2, True), (24, 150, 24, 4, True), (128, 0, 1, 1, True),
+    (64, 0, 24, 4, False), (32, 98, 24, 4, False), (16, 300, 6, 1, False),
+])
+def test_few_heads_keep_the_decode_kernels_bits(lib, n, p0, hq, hkv, same):
+    # both sides of the line below which a chunk goes through the kernel with the decode kernel's arithmetic
+    q, gate, keys, vals = _inputs(n, p0, hq, hkv, p0 + n, n)
+    out = _run(lib, q, keys, vals, p0, n, gate, hq, hkv, 1 / 16)
+    want = torch.empty_like(out)
+    for t in range(n):
+        ln = torch.tensor([p0 + t + 1], dtype=torch.int64, device="cuda")
+        qt, gt = q[t].contiguous(), gate[t].contiguous()
+        assert lib.launch_attn_decode_heads(ptr(qt), ptr(keys), ptr(vals), ptr(ln), ptr(gt), ptr(want[t]), p0 + n,
+                                            hq, hkv, 1 / 16, stream()) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(out, want) == same
+    # one fp16 step in the rounded sum and one in the product, sums in another order (see above; scores below 8)
+    bound = want.double().abs() * 2 ** -9 + 2 * vals.double().abs().max() * (2 ** -20 + 8 * 2 ** -21)
+    assert ((out.double() - want.double()).abs() <= bound).all()
