@@ -552,8 +552,10 @@ attn_decode_split_kernel(const __half* __restrict__ q, const __half* __restrict_
 // The same for HG query heads that share a KV head per CTA: every key and value row is read once for all
 // of them.  With one head per CTA the six heads of a group read the cache six times from L2, which at
 // 3500 keys is 86 MB and most of the kernel's time (24 heads: 21.5 -> 14.8 us; 1500 keys 12.1 -> 10.1, 513
-// 7.8 -> 7.5, 16 4.8 both).  ATG_SPLIT
-// CTAs per head group take alternate blocks of ATS_WARPS keys.
+// 7.8 -> 7.5, 16 4.8 both).  Up to ATG_SPLIT CTAs per head group take alternate blocks of ATS_WARPS keys, no
+// more than run at once (one per SM): with 16 for every group, two heads a CTA were slower than one between
+// 1000 and 3500 keys.  Two heads a CTA, 32 heads at 513 / 1500 / 3500 keys: 6.8 / 9.9 / 17.6 us against 8.5 /
+// 11.8 / 21.8 with one (16 CTAs a group 6.8 / 14.1 / 22.0); 64 heads 8.9 / 14.3 / 30.0 against 14.6 / 21.1 / 40.1.
 #define ATG_SPLIT 16
 #define ATG_ROWS 4
 template <int HG>
@@ -1008,24 +1010,24 @@ int launch_attn_decode_split(const void* q, const void* keys, const void* values
     if (hq <= 0 || hkv <= 0 || hq % hkv != 0 || ((uintptr_t)scratch & 15)) return -2;
     float* part = (float*)scratch;
     unsigned int* counters = (unsigned int*)(part + (size_t)hq * ATG_SPLIT * ATS_PART);
-    const int gqa = hq / hkv;
+    const int gqa = hq / hkv, dev = nvfp4::current_device_index();
     // Sharing pays where the CTAs of single heads fill the GPU; with 12 heads or fewer a head per CTA is
     // faster at every length (12: 5.1 us against 7.1 at 513 keys, 12.0 against 13.9 at 3500).
     // The shared kernel reads gates and stores results two at a time: 4-byte aligned pointers only.
     const bool pairs = (((uintptr_t)gate | (uintptr_t)out) & 3) == 0;
-    const int hg = !pairs || hq * ATS_SPLIT < 148 ? 1 : gqa % 3 == 0 ? 3 : gqa % 2 == 0 ? 2 : 1;
+    const int hg = !pairs || hq * ATS_SPLIT < nvfp4::device_sms(dev) ? 1 : gqa % 3 == 0 ? 3 : gqa % 2 == 0 ? 2 : 1;
     const auto kernel = hg == 3   ? nvfp4::attn_decode_group_kernel<3>
                         : hg == 2 ? nvfp4::attn_decode_group_kernel<2>
                                   : nvfp4::attn_decode_split_kernel;
+    const int splits = max(1, min(ATG_SPLIT, nvfp4::device_sms(dev) / (hq / hg)));
     const int smem = hg == 1 ? 0 : hg * ATS_WARPS * ATS_PART * (int)sizeof(float);
     static bool opted[nvfp4::NVFP4_MAX_DEVICES][4] = {};
-    const int dev = nvfp4::current_device_index();
     if (hg > 1 && !opted[dev][hg]) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -2;
         opted[dev][hg] = true;
     }
     const cudaError_t e = nvfp4::launch_pdl(
-        kernel, dim3(hq / hg, hg == 1 ? ATS_SPLIT : ATG_SPLIT), dim3(ATS_WARPS * 32), (size_t)smem,
+        kernel, dim3(hq / hg, hg == 1 ? ATS_SPLIT : splits), dim3(ATS_WARPS * 32), (size_t)smem,
         (cudaStream_t)stream, (const __half*)q, (const __half*)keys, (const __half*)values,
         (const long long*)cum_len, (const __half*)gate, (__half*)out, part, counters, max_len,
         gqa, scale);

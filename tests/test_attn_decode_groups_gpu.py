@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 D = 256
 
 
-@pytest.mark.parametrize("hq,hkv,max_len", [(24, 4, 4100), (3, 1, 600), (20, 4, 600), (32, 2, 600), (64, 1, 600), (19, 19, 300)])
+@pytest.mark.parametrize("hq,hkv,max_len", [(24, 4, 4100), (3, 1, 600), (20, 4, 600), (32, 2, 600), (64, 1, 600), (19, 19, 300),
+                                           (96, 8, 600), (320, 8, 300)])   # 32 and 160 head groups: 4 CTAs and 1 a group
 def test_against_float64(lib, hq, hkv, max_len):
     g = torch.Generator(device="cuda")
     g.manual_seed(hq * 100 + hkv)
