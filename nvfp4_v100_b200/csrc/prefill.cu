@@ -124,24 +124,23 @@ embed_rows_kernel(const __half* __restrict__ table, const long long* __restrict_
 
 // Token-minor gate/up rows, interleaved in groups of 8 (rows 16j..16j+7 gate, 16j+8..16j+15 up),
 // to activation rows: act[8j + r][t] = f16( f32(f16(silu(g))) * u ), the silu_mul_kernel chain.
-// VEC: eight tokens a thread, 16-byte accesses (N a multiple of 8, 16-byte aligned matrices); otherwise
-// one.  The grid is flat over rows x token groups (17408 rows of 512 tokens 18.6 -> 11.3 us, of 27 tokens
-// 18.6 -> 2.5, against a CTA per row and 4 bytes a thread).
-template <bool VEC>
+// W tokens a thread: eight with 16-byte accesses (N a multiple of 8, 16-byte aligned matrices), two with
+// 4-byte ones (N even), or two with single ones (ODD).  flat: rows and token groups share the grid's x, so
+// many short rows leave no CTA nearly empty (17408 rows of 27 tokens 18.3 -> 3.1 us against a CTA per row);
+// otherwise a row is blockIdx.y, which saves the division where the rows' CTAs run at once anyway.
+template <int W, bool ODD>
 __global__ void __launch_bounds__(256)
-silu_mul_rows_kernel(const __half* __restrict__ gu, __half* __restrict__ act, int inter, int N) {
+silu_mul_rows_kernel(const __half* __restrict__ gu, __half* __restrict__ act, int inter, int N, bool flat) {
     pdl_prologue();
     PDL_FRESH(gu); PDL_FRESH(act);
-    constexpr int W = VEC ? 8 : 1;
-    const int groups = N / W;
-    const long long id = (long long)blockIdx.x * 256 + threadIdx.x;
-    if (id >= (long long)inter * groups) return;
-    const int row = (int)(id / groups), t = (int)(id % groups) * W;   // activation row 0 .. inter-1
-    const size_t grow = (size_t)(row >> 3) * 16 + (row & 7);
+    const unsigned groups = ((unsigned)N + W - 1) / W, id = blockIdx.x * 256 + threadIdx.x;
+    const unsigned row = flat ? id / groups : blockIdx.y, group = flat ? id % groups : id;
+    if (row >= (unsigned)inter || group >= groups) return;
+    const size_t t = (size_t)group * W, grow = (size_t)(row >> 3) * 16 + (row & 7);
     const __half* g = gu + grow * N + t;
     const __half* u = gu + (grow + 8) * N + t;
     __half* o = act + (size_t)row * N + t;
-    if (VEC) {
+    if constexpr (W == 8) {
         const uint4 gv = *reinterpret_cast<const uint4*>(g), uv = *reinterpret_cast<const uint4*>(u);
         const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
         uint32_t ow[4];
@@ -153,8 +152,17 @@ silu_mul_rows_kernel(const __half* __restrict__ gu, __half* __restrict__ act, in
             ow[k] = *reinterpret_cast<const uint32_t*>(&r);
         }
         *reinterpret_cast<uint4*>(o) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+    } else if constexpr (!ODD) {
+        const float2 gf = __half22float2(*reinterpret_cast<const __half2*>(g));
+        const float2 uf = __half22float2(*reinterpret_cast<const __half2*>(u));
+        *reinterpret_cast<__half2*>(o) =
+            __floats2half2_rn(round_f16(silu_pf(gf.x)) * uf.x, round_f16(silu_pf(gf.y)) * uf.y);
     } else {
-        *o = __float2half(round_f16(silu_pf(__half2float(*g))) * __half2float(*u));
+        const bool two = t + 1 < (size_t)N;
+        const float g0 = __half2float(g[0]), u0 = __half2float(u[0]);
+        const float g1 = two ? __half2float(g[1]) : 0.0f, u1 = two ? __half2float(u[1]) : 0.0f;
+        o[0] = __float2half(round_f16(silu_pf(g0)) * u0);
+        if (two) o[1] = __float2half(round_f16(silu_pf(g1)) * u1);
     }
 }
 
@@ -678,11 +686,19 @@ int launch_embed_rows(const void* table, const void* ids, void* out, int n, int 
 // gu: token-minor [2 * inter][N] with gate/up rows interleaved in groups of 8; act: [inter][N].
 int launch_silu_mul_rows(const void* gu, void* act, int inter, int N, void* stream) {
     if (!gu || !act || inter <= 0 || inter % 8 != 0 || inter > 65535 || N <= 0) return -1;
-    const bool vec = N % 8 == 0 && (((uintptr_t)gu | (uintptr_t)act) & 15) == 0;
-    const long long items = (long long)inter * (vec ? N / 8 : N);      // fits the grid: inter < 2^16
-    return nvfp4::launch_pdl(vec ? nvfp4::silu_mul_rows_kernel<true> : nvfp4::silu_mul_rows_kernel<false>,
-                             dim3((unsigned)((items + 255) / 256)), dim3(256), 0, (cudaStream_t)stream,
-                             (const __half*)gu, (__half*)act, inter, N) == cudaSuccess ? 0 : -1;
+    const uintptr_t at = (uintptr_t)gu | (uintptr_t)act;
+    // eight tokens a thread once that fills the GPU (1024 rows of 512 tokens 1.9 us with two, 2.5 with eight;
+    // of 2048 5.7 and 4.2)
+    const bool wide = N % 8 == 0 && (at & 15) == 0 && (long long)inter * N >= (1LL << 20);
+    const bool even = N % 2 == 0 && (at & 3) == 0;
+    const auto kernel = wide   ? nvfp4::silu_mul_rows_kernel<8, false>
+                        : even ? nvfp4::silu_mul_rows_kernel<2, false>
+                               : nvfp4::silu_mul_rows_kernel<2, true>;
+    const long long groups = wide ? N / 8 : ((long long)N + 1) / 2, items = (long long)inter * groups;
+    const bool flat = inter > 8 * nvfp4::device_sms(nvfp4::current_device_index()) && items < 0x7fffff00LL;
+    const dim3 grid = flat ? dim3((unsigned)((items + 255) / 256)) : dim3((unsigned)((groups + 255) / 256), (unsigned)inter);
+    return nvfp4::launch_pdl(kernel, grid, dim3(256), 0, (cudaStream_t)stream, (const __half*)gu, (__half*)act, inter, N,
+                             flat) == cudaSuccess ? 0 : -1;
 }
 
 // Bytes of workspace launch_dn_prefill needs for n tokens.

@@ -93,7 +93,9 @@ def test_deltanet_chunk_keeps_a_bad_token_from_earlier_ones(lib):
     assert not np.isfinite(outs[1][6:]).any()
 
 
-@pytest.mark.parametrize("inter,N,shift", [(8, 1, 0), (24, 13, 0), (8, 8, 0), (64, 264, 0), (16, 16, 2)])
+@pytest.mark.parametrize("inter,N,shift", [(8, 1, 0), (24, 13, 0), (8, 8, 0), (64, 264, 0), (16, 16, 2), (16, 18, 0), (16, 18, 1),
+                                           (2048, 7, 0), (2048, 10, 0), (2048, 512, 0), (2048, 512, 1), (512, 2048, 0),
+                                           (1192, 515, 0)])    # many short rows, long rows, in each width
 def test_silu_mul_rows_with_ragged_and_unaligned_rows(lib, inter, N, shift):
     rng = np.random.default_rng(inter + N)
     gu = (rng.standard_normal((2 * inter, N)) * 3).astype(np.float16)
