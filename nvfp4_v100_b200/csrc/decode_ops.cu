@@ -96,12 +96,29 @@ attn_prep_kernel(const __half* __restrict__ qkv, const float* __restrict__ q_w1,
                         hq, hkv, max_len, eps);
 }
 
-// Prefill: token blockIdx.y of a chunk starting at position pos0; qkv is token-major with `ld`
-// halves between token rows, q_out / gate_out token-major [tokens][hq * 256].  A warp per head, lane l
-// holding dims l, l + 32, ..: each group of 32 dims is summed over the lanes and the eight sums in order, as
-// attn_prep_one_token's eight warps do (the same bits), but nothing meets in shared memory, and the eight
-// heads of a CTA share their token's cos and sin: 512 tokens of 24 + 8 heads 19.3 -> 9.2 us against a CTA
-// per head and token (8 tokens 1.9 -> 2.1).
+// Prefill: token blockIdx.y of a chunk starting at position pos0; qkv is token-major with `ld` halves between
+// token rows, q_out / gate_out token-major [tokens][hq * 256].  Two forms with the same bits.
+// A CTA per head, as in the decode step, while two CTAs an SM hold the chunk (8 tokens of 24 + 8 heads 1.9 us
+// against 2.1):
+__global__ void __launch_bounds__(256)
+attn_prep_few_tokens_kernel(const __half* __restrict__ qkv, long long ld,
+                            const float* __restrict__ q_w1, const float* __restrict__ k_w1,
+                            const __half* __restrict__ cos_tab, const __half* __restrict__ sin_tab,
+                            int pos0, __half* __restrict__ q_out, __half* __restrict__ gate_out,
+                            __half* __restrict__ keys, __half* __restrict__ values, int hq, int hkv,
+                            int max_len, float eps) {
+    pdl_prologue();
+    PDL_FRESH(qkv); PDL_FRESH(q_w1); PDL_FRESH(k_w1); PDL_FRESH(cos_tab); PDL_FRESH(sin_tab); PDL_FRESH(q_out);
+    PDL_FRESH(gate_out); PDL_FRESH(keys); PDL_FRESH(values);
+    const size_t t = blockIdx.y;
+    attn_prep_one_token(qkv + t * (size_t)ld, q_w1, k_w1, cos_tab, sin_tab, (long long)pos0 + (long long)t,
+                        q_out + t * (size_t)hq * 256, gate_out + t * (size_t)hq * 256, keys, values, hq, hkv,
+                        max_len, eps);
+}
+
+// A warp per head, lane l holding dims l, l + 32, ..: each group of 32 dims is summed over the lanes and the
+// eight sums in order, as attn_prep_one_token's eight warps do, but nothing meets in shared memory, and the
+// eight heads of a CTA share their token's cos and sin (512 tokens of 24 + 8 heads 19.3 -> 9.2 us):
 __global__ void __launch_bounds__(256)
 attn_prep_tokens_kernel(const __half* __restrict__ qkv, long long ld,
                         const float* __restrict__ q_w1, const float* __restrict__ k_w1,
@@ -390,8 +407,10 @@ int launch_attn_prep_tokens(const void* qkv, long long ld, const void* q_w1, con
         hq <= 0 || hkv <= 0 || max_len <= 0 || n_tokens <= 0 || n_tokens > 65535 || pos0 < 0 ||
         pos0 + n_tokens > max_len || ld < (long long)hq * 512 + 2LL * hkv * 256)
         return -1;
-    return nvfp4::launch_pdl(nvfp4::attn_prep_tokens_kernel, dim3((hq + 2 * hkv + 7) / 8, n_tokens),
-                             dim3(256), 0, (cudaStream_t)stream, (const __half*)qkv, ld,
+    const int heads = hq + 2 * hkv;
+    const bool few = (long long)heads * n_tokens <= 2 * nvfp4::device_sms(nvfp4::current_device_index());
+    return nvfp4::launch_pdl(few ? nvfp4::attn_prep_few_tokens_kernel : nvfp4::attn_prep_tokens_kernel,
+                             dim3(few ? heads : (heads + 7) / 8, n_tokens), dim3(256), 0, (cudaStream_t)stream, (const __half*)qkv, ld,
                              (const float*)q_w1, (const float*)k_w1, (const __half*)cos_tab,
                              (const __half*)sin_tab, pos0, (__half*)q_out, (__half*)gate_out,
                              (__half*)keys, (__half*)values, hq, hkv, max_len, eps) == cudaSuccess

@@ -125,11 +125,12 @@ def test_silu_mul_of_long_vectors(lib, n, shift):
     assert ulp_diff_f16(got[:n], fo.silu_mul(g, u)).max() <= 1 and (got[n:] == 7).all()
 
 
-@pytest.mark.parametrize("hq,hkv,n", [(1, 1, 1), (5, 1, 3), (24, 4, 9), (9, 3, 2)])
+@pytest.mark.parametrize("hq,hkv,n", [(1, 1, 1), (5, 1, 3), (24, 4, 9), (9, 3, 2),
+                                      (24, 4, 10), (1, 1, 100), (5, 1, 60), (9, 3, 30)])
 def test_attn_prep_of_a_chunk_equals_token_by_token(lib, hq, hkv, n):
-    # eight heads a CTA: fewer, exactly and more than fill one
+    # a CTA a head; then, with more tokens, eight heads a CTA: fewer, exactly and more than fill one
     rng = np.random.default_rng(hq + n)
-    max_len, p0, ld = 40, 31, hq * 512 + hkv * 512 + 24
+    max_len, p0, ld = 140, 31, hq * 512 + hkv * 512 + 24
     qkv = dev(rng.standard_normal((n, ld)).astype(np.float16))
     w = [dev((1 + 0.1 * rng.standard_normal(256)).astype(np.float32)) for _ in range(2)]
     tab = [dev(rng.uniform(-1, 1, (max_len, 256)).astype(np.float16)) for _ in range(2)]
