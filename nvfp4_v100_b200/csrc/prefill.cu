@@ -305,43 +305,51 @@ dn_block_kernel(const __half* __restrict__ conv_out, int conv_dim, const __half*
             qk[i][j] = warp_sum(q[i].x * k[j].x + q[i].y * k[j].y + q[i].z * k[j].z + q[i].w * k[j].w);
             kk[i][j] = j < i ? warp_sum(k[i].x * k[j].x + k[i].y * k[j].y + k[i].z * k[j].z + k[i].w * k[j].w) : 0.0f;
         }
-    for (int r = lane; r < rep; r += 32) {
-        const int h = kh * rep + r;
-        const float decay = -expf(__half2float(A_log[h])), dt = __half2float(dt_bias[h]);
-        DnBlock w;
+    // A lane per (value head, token of the block): its beta and decay, then its row of the coefficients.  (With one
+    // lane for a head's four tokens a chunk waits for it: a layer of 5 tokens 14.1 -> 12.7 us, of 512 143.5 -> 142.7.)
+    const int i = lane & 3, t = blk * DNB + i;
+    float ki[4], qi[4];                            // row i of the products
+#pragma unroll
+    for (int j = 0; j < DNB; j++) {
+        ki[j] = qi[j] = 0.0f;
+#pragma unroll
+        for (int m = j; m < DNB; m++)
+            if (m == i) {
+                ki[j] = kk[m][j];
+                qi[j] = qk[m][j];
+            }
+    }
+    for (int r0 = 0; r0 < rep; r0 += 8) {
+        const int r = r0 + (lane >> 2), h = kh * rep + min(r, rep - 1);
+        float e = 1.0f, beta = 0.0f;
+        if (t < n) {
+            const float decay = -expf(__half2float(A_log[h])), dt = __half2float(dt_bias[h]);
+            const __half* row = x + (size_t)t * ld + conv_dim + (size_t)nv * PF_DK;
+            beta = round_f16(1.0f / (1.0f + expf(-__half2float(row[h]))));
+            e = expf(decay * softplus_pf(__half2float(row[nv + h]) + dt));
+        }
         float eg[DNB];
 #pragma unroll
-        for (int i = 0; i < DNB; i++) {
-            const int t = blk * DNB + i;
-            eg[i] = 1.0f;
-            w.beta[i] = 0.0f;
-            if (t < n) {
-                const __half* row = x + (size_t)t * ld + conv_dim + (size_t)nv * PF_DK;
-                w.beta[i] = round_f16(1.0f / (1.0f + expf(-__half2float(row[h]))));
-                eg[i] = expf(decay * softplus_pf(__half2float(row[nv + h]) + dt));
-            }
+        for (int j = 0; j < DNB; j++) eg[j] = __shfl_sync(0xffffffffu, e, (lane & 28) + j);
+        float c[4], d[4], p = 1.0f;                // p = P(j+1..i) while j counts down
+#pragma unroll
+        for (int j = DNB - 1; j >= 0; j--) {
+            if (j + 1 < DNB && j < i) p *= eg[j + 1 < DNB ? j + 1 : j];
+            c[j] = j < i ? p * ki[j] : 0.0f;
+            d[j] = j <= i ? p * qi[j] : 0.0f;
         }
+        float tail = 1.0f;
 #pragma unroll
-        for (int i = 0; i < DNB; i++) {
-            float p = 1.0f;                       // P(j+1..i) while j counts down
-#pragma unroll
-            for (int j = DNB - 1; j >= 0; j--) {
-                w.c[i][j] = w.d[i][j] = 0.0f;
-                if (j <= i) {
-                    if (j < i) p *= eg[j + 1];
-                    w.c[i][j] = j < i ? p * kk[i][j] : 0.0f;
-                    w.d[i][j] = p * qk[i][j];
-                }
-            }
+        for (int j = DNB - 1; j > 0; j--)
+            if (j > i) tail *= eg[j];
+        if (r < rep) {
+            DnBlock& w = blocks[(size_t)h * gridDim.y + blk];
+            *reinterpret_cast<float4*>(w.c[i]) = make_float4(c[0], c[1], c[2], c[3]);
+            *reinterpret_cast<float4*>(w.d[i]) = make_float4(d[0], d[1], d[2], d[3]);
             w.gam[i] = p * eg[0];
+            w.tail[i] = tail;
+            w.beta[i] = beta;
         }
-        float p = 1.0f;
-#pragma unroll
-        for (int i = DNB - 1; i >= 0; i--) {
-            w.tail[i] = p;
-            p *= eg[i];
-        }
-        blocks[(size_t)h * gridDim.y + blk] = w;
     }
 }
 
