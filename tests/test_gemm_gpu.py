@@ -522,3 +522,57 @@ def test_few_token_kernel_against_the_oracle(lib, M, n, K):
     assert np.array_equal(fm, tm)
     assert np.array_equal(add, (resid.T.astype(np.float32) + tm.astype(np.float32)).astype(np.float16))
     assert oc.rel_error_floored(tm[rows], ref).max() <= 2e-3 * max(1.0, (K / 4096) ** 0.5)
+
+
+@pytest.mark.parametrize("M,n,K,shift", [
+    (300, 136, 384, 0), (640, 200, 1152, 0), (5120, 509, 640, 0),      # pairs with both operands in shared memory
+    (20000, 300, 384, 0),                                              # 256-row tiles
+    (640, 100, 320, 0), (1000, 13, 448, 0), (129, 65, 64, 0),          # 128 and 64 tokens a tile
+    (300, 200, 512, 4), (640, 100, 512, 4), (1000, 13, 1024, 8),       # scales aligned to 4 or 8 bytes only
+])
+def test_kernels_for_what_the_tensor_memory_ones_do_not_take(lib, M, n, K, shift):
+    # K % 256 != 0 or scales that no TMA copy can start at: every layout against float64, and the pair
+    # kernel with the same bits as the single-CTA tiles
+    rng = np.random.default_rng(M + n + K + shift)
+    p = rng.integers(0, 256, size=(M, K // 2), dtype=np.uint8)
+    s = rng.integers(118, 123, size=(M, K // 16), dtype=np.uint8)
+    act = rng.standard_normal((n, K)).astype(np.float16)
+    N8 = (n + 7) // 8 * 8
+    d_p, d_a = dev(p), dev(act)
+    d_s = torch.zeros(s.size + 16, dtype=torch.uint8, device="cuda")[shift:shift + s.size]
+    d_s.copy_(torch.from_numpy(s.reshape(-1)))
+    a_fm = torch.zeros((K, N8), dtype=torch.float16, device="cuda")
+    a_fm[:, :n] = d_a.t()
+    resid = torch.from_numpy(rng.standard_normal((n, M)).astype(np.float16)).cuda()
+    rows = np.arange(M) if M <= 1024 else np.unique(np.r_[0, M - 1, rng.integers(0, M, 500)])
+    ref = oc.decode(p[rows], s[rows]).astype(np.float64) @ act.T.astype(np.float64)
+
+    def run(flags):
+        a, ld_a = (d_a, K) if flags & 1 else (a_fm, N8)
+        shape = (n, M) if flags & 2 else (M, N8)
+        out = torch.full((shape[0] * shape[1] + 16,), float("nan"), dtype=torch.float16, device="cuda")
+        if flags & 4:
+            out[:n * M] = resid.view(-1)
+        assert lib.launch_nvfp4_gemm_w4a16_ex(ptr(d_p), ptr(d_s), ptr(a), ld_a, ptr(out), shape[1], M, n, K, flags,
+                                              stream()) == 0
+        torch.cuda.synchronize()
+        assert torch.isnan(out[-16:]).all(), "wrote past the output"
+        return out[:-16].view(shape)
+
+    lib.nvfp4_gemm_status(1)
+    try:
+        for flags in (0, 1, 2, 3, 6, 7):
+            got = run(flags)
+            lib.nvfp4_b200_gemm_config(1)                              # single-CTA tiles only
+            assert torch.equal(got, run(flags)), flags
+            lib.nvfp4_b200_gemm_config(3)
+            y = (got.t() if flags & 2 else got[:, :n])[torch.from_numpy(rows).cuda()].cpu().numpy()
+            if flags & 4:
+                r = resid.t()[torch.from_numpy(rows).cuda()].cpu().numpy()
+                assert np.array_equal(y, (r.astype(np.float32) + plain.astype(np.float32)).astype(np.float16)), flags
+            else:
+                plain = y
+                assert oc.rel_error_floored(y, ref).max() <= 2e-3 * max(1.0, (K / 4096) ** 0.5), flags
+    finally:
+        lib.nvfp4_b200_gemm_config(3)
+    assert lib.nvfp4_gemm_status(0) == 0, "a bounded wait inside the kernel ran out"
