@@ -796,10 +796,12 @@ void nvfp4_b200_gemm_config(int flags) {
     nvfp4::g_gemm_pair = (flags & 4) ? 2 : (flags & 2) ? 1 : 0;
 }
 
-// Shared memory of the tensor-core GEMM's widest tile, for callers that size their launches the
-// way the reference's get_kernel_shared_mem_bytes does (kernels/nvfp4_cuda_v5.cu:460-464).
+// The most shared memory that a launch of the tensor-core GEMM asks for, for callers that size their launches
+// the way the reference's get_kernel_shared_mem_bytes does (kernels/nvfp4_cuda_v5.cu:460-464).
 int get_kernel_shared_mem_bytes() {
-    return 3 * (2 * nvfp4::GEMM_BM * 128 + 4 * nvfp4::GEMM_BK * 128) + 1024;
+    const int widest_tile = 3 * (2 * nvfp4::GEMM_BM * 128 + 4 * nvfp4::GEMM_BK * 128) + 1024;
+    const int pair = nvfp4::gemm_pair_shared_bytes();
+    return pair > widest_tile ? pair : widest_tile;
 }
 
 }  // extern "C"

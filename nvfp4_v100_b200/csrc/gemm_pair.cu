@@ -361,6 +361,8 @@ int gemm_pair_launch(const uint8_t* packed, const uint8_t* scales, const __half*
     return (int)e;
 }
 
+int gemm_pair_shared_bytes() { return GP_SMEM; }
+
 int gemm_pair_status(int reset) {
     int v = 0;
     if (cudaMemcpyFromSymbol(&v, g_pair_status, sizeof(int)) != cudaSuccess) return -1;

@@ -16,6 +16,9 @@ int gemm_pair_launch(const uint8_t* packed, const uint8_t* scales, const __half*
                      bool in_tm, __half* out, int ld_out, int M, int N, int n_tokens, int K, int out_mode,
                      cudaStream_t st);
 
+// Dynamic shared memory of a launch, the most that any kernel behind the GEMM entry points asks for.
+int gemm_pair_shared_bytes();
+
 // 0 or 1 + the id of the first bounded wait that ran out.  Synchronises the device.
 int gemm_pair_status(int reset);
 

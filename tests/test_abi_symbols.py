@@ -91,3 +91,9 @@ def test_fused_op_argument_validation(lib):
     assert lib.launch_dn_fused(*args, 1e-6, None) == -1
     assert lib.nvfp4_b200_gemv_config(3, 0, 0) == -2
     assert lib.nvfp4_b200_gemv_config(0, 0, 0) == 0
+
+
+def test_reported_shared_memory_covers_every_gemm_kernel(lib):
+    # the widest launch is the CTA-pair kernel with its weights in tensor memory: four units of activations
+    # (128 tokens x 128 k fp16), four weight stages (128 rows x (128 packed + 16 scale bytes)), alignment
+    assert lib.get_kernel_shared_mem_bytes() == 4 * 32768 + 4 * 128 * 144 + 1024
