@@ -970,7 +970,8 @@ static int attn_decode_launch(const void* q, const void* keys, const void* value
 int launch_attn_prefill(const void* q, const void* keys, const void* values, int len0,
                         int n_tokens, const void* gate, void* out, int max_len, int hq, int hkv,
                         float scale, void* stream) {
-    static int smem_set[nvfp4::NVFP4_MAX_DEVICES] = {0};
+    static bool opted[nvfp4::NVFP4_MAX_DEVICES] = {false};
+    constexpr int SMEM_MOST = 150 * 1024;
     const int dev = nvfp4::current_device_index();
     if (max_len <= 0 || max_len > 47104 || n_tokens <= 0 || n_tokens > 65535) return -2;
     if (len0 < 1 || len0 + n_tokens - 1 > max_len) return -2;
@@ -978,18 +979,19 @@ int launch_attn_prefill(const void* q, const void* keys, const void* values, int
     if (hq <= 0 || hkv <= 0 || hq % hkv != 0) return -2;
     const int lcap = len0 + n_tokens - 1;
     const int smem = ATT_G * lcap * (int)sizeof(float);
-    if (smem > 150 * 1024) return -2;
+    if (smem > SMEM_MOST) return -2;
     if (nvfp4::attn_prefill_tc_takes(q, keys, values, gate, out, len0, n_tokens, hq, hkv)) {
         const int rc = nvfp4::attn_prefill_tc_launch((const __half*)q, (const __half*)keys, (const __half*)values, len0,
                                                      n_tokens, (const __half*)gate, (__half*)out, max_len, hq, hkv,
                                                      scale, (cudaStream_t)stream);
         if (rc != -3) return rc;     // -3: no tensor maps from this driver
     }
-    if (smem > 8 * 1024 && smem > smem_set[dev]) {
-        if (cudaFuncSetAttribute(nvfp4::attn_prefill_group_kernel,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    // the opt-in is the same whatever this call needs: another thread's first call cannot lower it
+    if (!opted[dev]) {
+        if (cudaFuncSetAttribute(nvfp4::attn_prefill_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 SMEM_MOST) != cudaSuccess)
             return -2;
-        smem_set[dev] = smem;
+        opted[dev] = true;
     }
     const cudaError_t e = nvfp4::launch_pdl(
         nvfp4::attn_prefill_group_kernel, dim3(hq, (n_tokens + ATT_G - 1) / ATT_G),

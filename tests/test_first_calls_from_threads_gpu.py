@@ -8,7 +8,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
-PROGRAM = """
+DELTANET = """
 import threading
 import torch
 from nvfp4_v100_b200 import _lib
@@ -44,6 +44,36 @@ assert codes == {nv: [0] * 20 for nv in HEADS}, codes
 """
 
 
-def test_deltanet_chunk():
+ATTENTION = """
+import threading
+import torch
+from nvfp4_v100_b200 import _lib
+from tests.gpu_util import ptr
+
+lib = _lib.load()
+CONTEXTS = [3000, 300, 2000, 600, 3900, 1200, 900, 2500]      # one query: scores of its keys in shared memory
+start, codes = threading.Barrier(len(CONTEXTS)), {}
+
+def call(keys):
+    z = lambda *s: torch.zeros(s, dtype=torch.float16, device="cuda")
+    q, gate, k, v, out = z(256), z(256), z(keys, 256), z(keys, 256), z(256)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    start.wait()
+    codes[keys] = [lib.launch_attn_prefill(ptr(q), ptr(k), ptr(v), keys, 1, ptr(gate), ptr(out), keys, 1, 1, 0.0625,
+                                           side.cuda_stream) for _ in range(20)]
+    side.synchronize()
+
+threads = [threading.Thread(target=call, args=(keys,)) for keys in CONTEXTS]
+for t in threads:
+    t.start()
+for t in threads:
+    t.join()
+assert codes == {keys: [0] * 20 for keys in CONTEXTS}, codes
+"""
+
+
+@pytest.mark.parametrize("program", [DELTANET, ATTENTION], ids=["deltanet", "attention"])
+def test_no_call_fails(program):
     for _ in range(4):
-        subprocess.run([sys.executable, "-c", PROGRAM], cwd=ROOT, check=True, timeout=120)
+        subprocess.run([sys.executable, "-c", program], cwd=ROOT, check=True, timeout=120)
