@@ -527,7 +527,7 @@ bool attn_prefill_tc_takes(const void* q, const void* keys, const void* values, 
     // ns, measured for 1 to 32 heads, e.g. 64 tokens of 6 heads 9.7 us against 18.3, 32 of 12 heads after 98
     // 13.9 against 19.1, 24 of 24 heads after 150 15.6 against 19.2; 16 of 24 heads after 242 19.6 against 15.1.
     if (2LL * hq * ((n_tokens + 7) / 8) <= device_sms(current_device_index()))
-        return 6700 + 47LL * L >= 9500 + 75 * gqa * min(n_tokens, ATC_ROWS / gqa);
+        return 6700 + 48LL * L >= 9500 + 75 * gqa * min(n_tokens, ATC_ROWS / gqa);
     return true;
 }
 
