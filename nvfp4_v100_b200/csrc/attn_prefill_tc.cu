@@ -26,10 +26,10 @@
 // a later token is not, and hi . inf + lo . inf need not be inf.
 // Every wait is bounded and reported through nvfp4_gemm_status.
 //
-// Measured, 24 query / 4 KV heads, us (before: attn_prefill_group_kernel), tokens after context:
-//   512 after 0      27.1 (386)     512 after 3488  123 (3596)     26 after 511   16.2 (58.9)
-//   512 after 512    41.1 (859)     512 after 9000  253 (8670)    100 after 0    17.6 (45.7)
-// i.e. 20 us fixed and 26 us per 1024 keys of 512 tokens: 100 CTAs, 3072 cycles of MMAs per step.
+// Measured, 24 query / 4 KV heads, us (in brackets attn_prefill_group_kernel), tokens after context:
+//   512 after 0      27.7 (395)     512 after 3488  127 (3598)     26 after 511   16.4 (59.3)
+//   512 after 512    40.8 (859)     512 after 9000  300 (8681)    100 after 0    18.0 (46.0)
+// i.e. some 20 us fixed and 28 us per 1024 keys of 512 tokens: 3072 cycles of MMAs per step and tile.
 // Relative error against float64 as before (3.5e-4, the fp16 rounding of the output; see ATC_CHAIN).  Of the
 // outputs 0.2 to 0.8 % are not the correctly rounded ones, against 0.1 % before.
 #include <cuda.h>

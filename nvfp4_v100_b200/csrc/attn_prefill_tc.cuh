@@ -5,7 +5,7 @@
 namespace nvfp4 {
 
 // (token, key) pairs of a chunk from which the tensor-core kernel is the faster one: 64 tokens of an
-// empty cache 25.4 -> 17.6 us, 8 tokens after 511 30.7 -> 11.8; below it the one-query-at-a-time kernel
+// empty cache 25.7 -> 18.2 us, 8 tokens after 511 30.9 -> 12.3; below it the one-query-at-a-time kernel
 // takes 8 to 20 us (16 after 64: 11.2, 26 after 64: 20.4) except for a handful of tokens deep in a context.
 // (24 heads; with few heads the line lies higher, see attn_prefill_tc_takes.)
 constexpr long long ATTN_TC_MIN_PAIRS = 4096;

@@ -10,9 +10,10 @@
 //   warp 0        : TMA producer.  One elected thread issues cp.async.bulk.tensor.2d loads of the
 //                   activation tile ([64 k] x [64 tokens] boxes, 128-byte swizzle) into a 4-stage
 //                   shared-memory ring, completion on an mbarrier (transaction bytes).
-//   warp 1        : MMA issuer.  One elected thread issues tcgen05.mma.kind::f16 (M = 128, N = BN,
-//                   K = 16, four per stage) with shared-memory descriptors; the fp32 accumulator
-//                   lives in tensor memory (BN columns).  tcgen05.commit releases each stage.
+//   warp 1        : MMA issuer.  The whole warp runs the loop, an elected lane issues
+//                   tcgen05.mma.kind::f16 (M = 128, N = BN, K = 16, four per stage) with
+//                   shared-memory descriptors; the fp32 accumulator lives in tensor memory (BN
+//                   columns).  tcgen05.commit releases each stage.
 //   warps 2..9    : weight producers, two threads per weight row: 16 packed bytes + 2 scale bytes
 //                   each per K step from global memory, nibbles -> fp16 (cvt.rn.f16x2.e2m1x2) x
 //                   scale, written as a K-major, 128-byte-swizzled A tile; then the epilogue:

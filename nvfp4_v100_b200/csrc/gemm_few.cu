@@ -4,7 +4,7 @@
 //
 // The tile kernel of gemm.cu keeps 16 KB of weight bytes in flight per SM (registers of the
 // dequantising warps) and runs one CTA of K / 64 dependent steps per 128 rows: at 32 tokens it took
-// 61 us for 17408 x 5120 (0.8 TB/s) and 138 us for 5120 x 17408 (40 CTAs on 148 SMs).  Here:
+// 42 us for 17408 x 5120 (1.2 TB/s) and 129 us for 5120 x 17408 (40 CTAs on 148 SMs).  Here:
 //   * raw weight and scale bytes come by TMA into a shared-memory ring (54 to 90 KB in flight per
 //     CTA, two CTAs per SM), so the stream does not depend on the dequantising warps' registers;
 //   * the dequantised fp16 tile goes to TENSOR MEMORY (tcgen05.st) and is the MMA's A operand from
@@ -23,10 +23,10 @@
 // then all warps: accumulator -> shared memory -> sum over the cluster -> output.
 // Every wait is bounded and reported through nvfp4_gemm_status.
 //
-// Measured (weights cold, graph replay, us; before: the tile kernel of gemm.cu), 3 / 32 / 128 tokens:
-//   5120 x 6144     8.3 /  9.5 / 14.4   (50 /  49 /  43)      17408 x 5120   15.3 / 16.1 / 21.4   (45 / 39 / 36)
-//   5120 x 17408   16.9 / 17.5 / 24.2  (131 / 127 / 108)      34816 x 5120   24.7 / 25.3 / 40.6   (89 / 68 / 69)
-// i.e. about 6 us fixed (launch, first bytes, cluster sum) plus 5.3 TB/s.  The stream alone, without
+// Measured (weights cold, graph replay, us; in brackets the tile kernel of gemm.cu), 3 / 32 / 128 tokens:
+//   5120 x 6144     9.4 / 10.5 / 15.6   (51 /  50 /  44)      17408 x 5120   17.4 / 18.1 / 22.9   (47 / 42 / 39)
+//   5120 x 17408   19.0 / 20.2 / 27.0  (132 / 129 / 111)      34816 x 5120   34.7 / 36.2 / 48.4  (112 / 87 / 89)
+// i.e. some 6 us fixed (launch, first bytes, cluster sum) plus 3.5 to 4.5 TB/s.  The stream alone, without
 // conversion and MMAs, runs at 6.3 TB/s; the conversions (2 instructions per pair of weights) take
 // most of the rest.  128 tokens are bound by the activation units from L2 (32 KB for 9 KB of weights).
 #include <cuda.h>

@@ -4,6 +4,10 @@
 
 namespace nvfp4 {
 
+// One token tile.  Above it the CTA-pair kernel, which needs enough rows to fill the GPU: 136 tokens 16480 x
+// 5120 25.4 us against 35.8 with two token tiles here, 34816 x 5120 51.3 / 71.4.  Narrow matrices lie the other
+// way up to 256 tokens (5120 x 17408 63.2 / 40.2, 5120 x 6144 26.2 / 19.4, 1024 x 5120 22.6 / 9.7; 128 tokens
+// 26.3, 15.4 and 8.5): a rule by rows as well is not built.
 constexpr int GEMM_FEW_MAX_TOKENS = 128;
 
 // Whether the few-token kernel takes this product (sizes and alignment).

@@ -21,10 +21,10 @@
 // columns and four units of 64 columns of A (all 512 for BN = 256).
 // Every wait is bounded and reported through nvfp4_gemm_status.
 //
-// Measured, us (before: the better of the two kernels of gemm.cu), 136 / 2048 tokens:
-//   5120 x 6144    25.3 (43.5) /  89 (156)     16480 x 5120   24.4 (36.6) / 285 (326)
-//   5120 x 17408   62.9 (106)  / 236 (410)     34816 x 5120   50.1 (64.6) / 584 (640)
-// i.e. 1.2 to 1.55 PFLOP/s at 2048 tokens.
+// Measured, us (in brackets the better of the two kernels of gemm.cu), 136 / 2048 tokens:
+//   5120 x 6144    26.4 (44.7) /  88 (154)     16480 x 5120   27.1 (41.4) / 251 (289)
+//   5120 x 17408   63.5 (110)  / 231 (410)     34816 x 5120   64.1 (83.4) / 506 (617)
+// i.e. 1.4 to 1.6 PFLOP/s at 2048 tokens.
 #include <cuda.h>
 
 #include "common.cuh"

@@ -715,9 +715,10 @@ class DecodeEngine:
         total = len(tokens)
         if start + total > c.max_len:
             raise ValueError("prompt longer than the cache")
-        # the chunk attention kernel keeps a group's scores in shared memory (150 KB): checked
-        # here, before the first launch, because a failure in the middle of a prompt would leave
-        # the caches and states of earlier chunks and layers already advanced
+        # launch_attn_prefill takes contexts whose scores for a group of tokens fit in shared memory
+        # (150 KB; small chunks need that): checked here, before the first launch, because a failure
+        # in the middle of a prompt would leave the caches and states of earlier chunks and layers
+        # already advanced
         if start + total > PREFILL_MAX_CONTEXT:
             raise ValueError(f"chunked prefill handles contexts up to {PREFILL_MAX_CONTEXT} tokens "
                              f"(got {start + total}); feed the rest through step()")

@@ -409,6 +409,7 @@ def test_cta_pair_kernel_equals_the_single_cta_kernel(lib, M, n, K):
     # the CTA-pair kernel (clusters of two, one M = 256 MMA on both SMs' tensor cores, each CTA
     # holding half of the token tile) adds the same products in the same K order: every layout
     # combination is bit-identical to the single-CTA kernel, which the tests above pin to the oracle
+    # (K % 256 == 0 throughout: the pair kernel with its weights in tensor memory; the other one below)
     rng = np.random.default_rng(M * 3 + n + K)
     p = rng.integers(0, 256, size=(M, K // 2), dtype=np.uint8)
     s = rng.integers(118, 123, size=(M, K // 16), dtype=np.uint8)

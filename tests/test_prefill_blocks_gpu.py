@@ -1,5 +1,5 @@
 """The chunk kernels of the Gated DeltaNet and the row-wise silu-mul at the sizes where their tiles
-end: blocks of 4 tokens, operand stages of 16, conv strips of 16 tokens, 8-token accesses."""
+end: blocks of 4 tokens, operand stages of 16, conv strips of 2 or 8 tokens, 2- or 8-token accesses."""
 import numpy as np
 import pytest
 import torch
