@@ -28,7 +28,7 @@
 // out, the result of that tile is wrong and nvfp4_gemv_tc_status says so; nothing hangs.
 //
 // One CTA (320 threads; 111 KB of shared memory: a 5-stage weight ring of 18 KB stages, an 8-slot
-// ring of 2 KB digit-plane tiles, a 1 KB digit table; 256 columns of tensor memory; two CTAs per SM):
+// ring of 2 KB digit-plane tiles; 256 columns of tensor memory; two CTAs per SM):
 //   thread 0    TMA producer: per stage 128 rows x 128 packed bytes (128-byte swizzle) and the
 //               128 x 16 scale bytes.  Two stages are requested at kernel entry, BEFORE the previous
 //               kernel in the stream has finished (programmatic dependent launch: weights are
@@ -63,10 +63,10 @@ constexpr int TC_B_BYTES = 16 * 128;           // activation digit planes of a s
 constexpr int TC_S_BYTES = TC_BM * 16;         // weight scale bytes of a stage
 constexpr int TC_SF_COLS = 32;                 // tensor-memory columns of a stage's scale bytes
 constexpr uint32_t TC_EMPTY = 0xFFFFFFFFu;      // an empty partial-sum slot
-// dynamic shared memory: weight ring of st stages, digit-plane ring, digit table, exponent bytes,
+// dynamic shared memory: weight ring of st stages, digit-plane ring, exponent bytes,
 // scratch; tensor memory: 2 x 16 accumulator columns + st x 32 scale columns
 __host__ __device__ constexpr int tc_smem_bytes(int st) {
-    return st * (TC_A_BYTES + TC_S_BYTES) + TC_NB * (TC_B_BYTES + 16) + 1024 + 128 + 1024 /*alignment*/;
+    return st * (TC_A_BYTES + TC_S_BYTES) + TC_NB * (TC_B_BYTES + 16) + 128 + 1024 /*alignment*/;
 }
 __host__ __device__ constexpr int tc_tmem_cols(int st) { return 32 + st * TC_SF_COLS <= 128 ? 128 : 256; }
 
@@ -137,20 +137,12 @@ __device__ __forceinline__ int tc_cta_of(unsigned g, unsigned total, unsigned G)
     return (int)(((g + 1u) * G - 1u) / total);
 }
 
-// The 32-bit fraction |x| / 2^L of an fp16 bit pattern (sign stripped), L = the block's exponent.
-__device__ __forceinline__ uint32_t tc_fraction(uint32_t h15, int L) {
-    const uint32_t e = h15 >> 10, m = h15 & 0x3FFu;
-    const uint32_t m11 = e ? (m | 0x400u) : m;
-    const int sh = (int)(e ? e : 1u) + 7 - L;       // |x| = m11 * 2^(max(e,1) - 25)
-    return sh >= 0 ? (m11 << sh) : (sh > -32 ? (m11 >> (-sh)) : 0u);
-}
-
 // Digit planes of 8 consecutive activations (one 16-byte vector; lane o of a warp holds elements
 // 8o .. 8o+7 of a 256-element stage) -> 16 words, one per plane row of the B tile, and the block's
-// exponent byte.  lut[b] holds the E2M1 codes of the four base-4 digits of byte b, one per byte
-// (first digit = most significant = lowest byte).
-__device__ __forceinline__ void tc_digit_planes(const uint4 xv, const uint32_t* lut, uint8_t* btile,
-                                                uint8_t* lbytes, int lane) {
+// exponent byte.  All by bit operations on whole words: a transpose of the eight 32-bit fractions by nibbles puts
+// two digits of every element into one word, and a digit with bits h, l is the E2M1 code (h, l & ~h, h & l).  (A table of
+// codes per byte in shared memory took 32 scattered reads a lane, which the SM's other CTA waited for as well.)
+__device__ __forceinline__ void tc_digit_planes(const uint4 xv, uint8_t* btile, uint8_t* lbytes, int lane) {
     const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
     uint32_t hmax = 0;
 #pragma unroll
@@ -161,31 +153,49 @@ __device__ __forceinline__ void tc_digit_planes(const uint4 xv, const uint32_t* 
     hmax = max(hmax, __shfl_xor_sync(0xffffffffu, hmax, 1));   // lanes 2b, 2b+1 share block b
     const uint32_t em = hmax >> 10;
     const uint32_t m11 = em ? ((hmax & 0x3FFu) | 0x400u) : (hmax & 0x3FFu);
-    const int L = (32 - __clz(m11)) + (int)(em ? em : 1u) - 25;
+    const int bits = 32 - __clz(m11);
+    const int L = bits + (int)(em ? em : 1u) - 25;
+    // the fraction |x| / 2^L: significand m (|x| = m 2^(e - 25), e at least 1) with the block's largest at bit 31
+    const uint32_t left = em ? 21u : (uint32_t)min(32 - bits, 31);
+    const int right = em ? (int)em : 1;
     uint32_t u[8], sgn = 0;
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-        const uint32_t h = (xw[e >> 1] >> (16 * (e & 1))) & 0xFFFFu;
-        u[e] = tc_fraction(h & 0x7FFFu, L);
-        sgn |= ((h >> 12) & 8u) << (4 * e);
+    for (int k = 0; k < 8; k++) {
+        const uint32_t h = (xw[k >> 1] >> (16 * (k & 1))) & 0x7FFFu;
+        const uint32_t e = max(h >> 10, 1u);
+        u[k] = __funnelshift_rc((h + 1024u - e * 1024u) << left, 0u, (uint32_t)(right - (int)e));   // (32 and more: 0)
     }
 #pragma unroll
-    for (int q = 0; q < 4; q++) {                  // planes 4q .. 4q+3 = byte 3-q of the fraction
-        uint32_t pr[4];
+    for (int w = 0; w < 4; w++) sgn |= (((xw[w] >> 12) & 0x8u) | ((xw[w] >> 24) & 0x80u)) << (8 * w);
+    // nibbles of elements 2 i and 2 i + 1 side by side: byte k of ev[i] = their nibbles 2 k, of od[i] = 2 k + 1
+    uint32_t ev[4], od[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++)               // elements 2i (low nibble) and 2i+1 (high)
-            pr[i] = lut[(u[2 * i] >> (24 - 8 * q)) & 0xFFu] | (lut[(u[2 * i + 1] >> (24 - 8 * q)) & 0xFFu] << 4);
-        // 4x4 byte transpose: pr[i] byte p -> plane p byte i
-        const uint32_t t0 = tc_prmt(pr[0], pr[1], 0x5140u), t1 = tc_prmt(pr[2], pr[3], 0x5140u);
-        const uint32_t t2 = tc_prmt(pr[0], pr[1], 0x7362u), t3 = tc_prmt(pr[2], pr[3], 0x7362u);
-        const uint32_t o[4] = {tc_prmt(t0, t1, 0x5410u), tc_prmt(t0, t1, 0x7632u),
-                               tc_prmt(t2, t3, 0x5410u), tc_prmt(t2, t3, 0x7632u)};
+    for (int i = 0; i < 4; i++) {
+        const uint32_t a = u[2 * i], c = u[2 * i + 1];
+        ev[i] = (a & 0x0F0F0F0Fu) | ((c << 4) & 0xF0F0F0F0u);
+        od[i] = ((a >> 4) & 0x0F0F0F0Fu) | (c & 0xF0F0F0F0u);
+    }
+    // 4 x 4 byte transposes: word n = nibble n of all eight elements
+    auto transpose = [](const uint32_t (&v)[4], uint32_t (&o)[4]) {
+        const uint32_t t0 = tc_prmt(v[0], v[1], 0x5140u), t1 = tc_prmt(v[2], v[3], 0x5140u);
+        const uint32_t t2 = tc_prmt(v[0], v[1], 0x7362u), t3 = tc_prmt(v[2], v[3], 0x7362u);
+        o[0] = tc_prmt(t0, t1, 0x5410u);
+        o[1] = tc_prmt(t0, t1, 0x7632u);
+        o[2] = tc_prmt(t2, t3, 0x5410u);
+        o[3] = tc_prmt(t2, t3, 0x7632u);
+    };
+    uint32_t te[4], to[4];
+    transpose(ev, te);
+    transpose(od, to);
+    auto put = [&](int row, uint32_t word) {
+        const int chunk = (lane >> 2) ^ (row & 7);              // 128-byte swizzle
+        *reinterpret_cast<uint32_t*>(btile + row * 128 + chunk * 16 + (lane & 3) * 4) = word | sgn;
+    };
 #pragma unroll
-        for (int p = 0; p < 4; p++) {
-            const int row = 4 * q + p;
-            const int chunk = (lane >> 2) ^ (row & 7);      // 128-byte swizzle
-            *reinterpret_cast<uint32_t*>(btile + row * 128 + chunk * 16 + (lane & 3) * 4) = o[p] | sgn;
-        }
+    for (int n = 0; n < 8; n++) {                              // nibble 7 - n: planes 2 n and 2 n + 1
+        const uint32_t t = ((7 - n) & 1) ? to[(7 - n) >> 1] : te[(7 - n) >> 1];
+        put(2 * n, ((t >> 1) & 0x44444444u) | ((t >> 1) & ~(t >> 2) & 0x22222222u) | ((t >> 3) & (t >> 2) & 0x11111111u));
+        put(2 * n + 1, ((t << 1) & 0x44444444u) | ((t << 1) & ~t & 0x22222222u) | ((t >> 1) & t & 0x11111111u));
     }
     if ((lane & 1) == 0) lbytes[lane >> 1] = (uint8_t)(L + 125);
 }
@@ -253,8 +263,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     uint8_t* smem_a = smem;                                   // ST x 16 KB packed weights
     uint8_t* smem_b = smem_a + ST * TC_A_BYTES;               // NB x 2 KB digit planes
     uint8_t* smem_s = smem_b + NB * TC_B_BYTES;               // ST x 2 KB weight scale bytes
-    uint32_t* lut = reinterpret_cast<uint32_t*>(smem_s + ST * TC_S_BYTES);   // 256 words
-    uint8_t* smem_l = reinterpret_cast<uint8_t*>(lut + 256);  // NB x 16 exponent bytes
+    uint8_t* smem_l = smem_s + ST * TC_S_BYTES;  // NB x 16 exponent bytes
     float* s_part = reinterpret_cast<float*>(smem_l + NB * 16);              // 9 partial sums
     __shared__ __align__(8) uint64_t bar_full[ST];            // TMA bytes landed
     __shared__ __align__(8) uint64_t bar_ready[ST];           // scale bytes written to tensor memory
@@ -279,7 +288,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     const int tile0 = (int)(g0 / nk), ks0 = (int)(g0 % nk);
 
     // The copy-issuing thread starts the first ST stages at once: it needs only the barriers, which
-    // it initialises itself; tensor memory, the digit table and the other warps come later.
+    // it initialises itself; tensor memory and the other warps come later.
     int p_s = 0, p_tile = tile0, p_ks = ks0, p_i = 0;       // producer state (thread 0)
     uint32_t p_ph = 0;
     if (threadIdx.x == 0) {
@@ -312,13 +321,6 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     if (warp == 1) {
         tcgen05_alloc(smem_u32(&s_tmem), TC_TMEM_COLS);
         tcgen05_relinquish();
-    }
-    if (threadIdx.x >= 64) {                                  // digit-code table, one entry each
-        const uint32_t v = threadIdx.x - 64;
-        uint32_t w = 0;
-#pragma unroll
-        for (int p = 0; p < 4; p++) w |= ((0x5420u >> (4 * ((v >> (6 - 2 * p)) & 3u))) & 0xFu) << (8 * p);
-        lut[v] = w;
     }
     tcgen05_fence_before();
     __syncthreads();
@@ -508,7 +510,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                     }
                     // the slot's previous planes (stage cv - 8) must have been consumed
                     tc_wait(smem_u32(&bar_bempty[slot]), (((uint32_t)cv >> 3) & 1u) ^ 1u, 7);
-                    tc_digit_planes(xv, lut, smem_b + slot * TC_B_BYTES, smem_l + slot * 16, lane);
+                    tc_digit_planes(xv, smem_b + slot * TC_B_BYTES, smem_l + slot * 16, lane);
                     fence_proxy_async_smem();        // the tensor core reads the planes (async proxy)
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&bar_bfull[slot]));
@@ -645,8 +647,7 @@ gemv_tc_mlp_kernel(const __grid_constant__ CUtensorMap w_map0, const __grid_cons
     uint8_t* smem_a = smem;
     uint8_t* smem_b = smem_a + ST * TC_A_BYTES;
     uint8_t* smem_s = smem_b + NB * TC_B_BYTES;
-    uint32_t* lut = reinterpret_cast<uint32_t*>(smem_s + ST * TC_S_BYTES);
-    uint8_t* smem_l = reinterpret_cast<uint8_t*>(lut + 256);
+    uint8_t* smem_l = smem_s + ST * TC_S_BYTES;
     float* s_part = reinterpret_cast<float*>(smem_l + NB * 16);
     __shared__ __align__(8) uint64_t bar_full[ST];
     __shared__ __align__(8) uint64_t bar_ready[ST];
@@ -697,13 +698,6 @@ gemv_tc_mlp_kernel(const __grid_constant__ CUtensorMap w_map0, const __grid_cons
     if (warp == 1) {
         tcgen05_alloc(smem_u32(&s_tmem), TC_TMEM_COLS);
         tcgen05_relinquish();
-    }
-    if (threadIdx.x >= 64) {
-        const uint32_t v = threadIdx.x - 64;
-        uint32_t w = 0;
-#pragma unroll
-        for (int p = 0; p < 4; p++) w |= ((0x5420u >> (4 * ((v >> (6 - 2 * p)) & 3u))) & 0xFu) << (8 * p);
-        lut[v] = w;
     }
     tcgen05_fence_before();
     __syncthreads();
@@ -942,7 +936,7 @@ gemv_tc_mlp_kernel(const __grid_constant__ CUtensorMap w_map0, const __grid_cons
                             }
                         }
                         tc_wait(smem_u32(&bar_bempty[slot]), (((uint32_t)cv >> 3) & 1u) ^ 1u, 7);
-                        tc_digit_planes(xv, lut, smem_b + slot * TC_B_BYTES, smem_l + slot * 16, lane);
+                        tc_digit_planes(xv, smem_b + slot * TC_B_BYTES, smem_l + slot * 16, lane);
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(smem_u32(&bar_bfull[slot]));
