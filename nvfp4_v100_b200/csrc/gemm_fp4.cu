@@ -38,7 +38,7 @@ namespace nvfp4 {
 constexpr int F4_BM = 128;
 constexpr int F4_BK = 256;                 // elements of K per stage = 128 bytes per row
 constexpr int F4_THREADS = 192;
-constexpr int F4_PAIR_THREADS = 320;       // the CTA-pair kernel: two sets of scale-writing warps
+constexpr int F4_PAIR_THREADS = 352;       // the CTA-pair kernel
 constexpr uint32_t F4_SPIN_LIMIT = 1u << 24;
 
 __device__ int g_fp4_status = 0;           // 0 ok; otherwise 1 + id of the wait that ran out
@@ -58,23 +58,6 @@ __device__ __forceinline__ void tcgen05_mma_fp4_block16(uint32_t taddr, uint64_t
         "elect.sync _|e, 0xffffffff;\n"
         "setp.ne.u32 p, %4, 0;\n"
         "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::
-            "r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
-        : "memory");
-}
-// Non-suspending poll: for barriers that the peer CTA of a pair, or a commit issued there, arrives on.
-__device__ __forceinline__ bool f4_wait_poll(uint32_t bar, uint32_t parity, int id) {
-    for (uint32_t i = 0; i < F4_SPIN_LIMIT; i++)
-        if (mbar_test_wait_cluster(bar, parity)) return true;
-    atomicExch(&g_fp4_status, 1 + id);
-    return false;
-}
-__device__ __forceinline__ void tcgen05_mma_fp4_block16_pair(uint32_t taddr, uint64_t adesc, uint64_t bdesc,
-                                                             uint32_t idesc, uint32_t sfa, uint32_t sfb,
-                                                             uint32_t accumulate) {
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "setp.ne.u32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::
             "r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
         : "memory");
 }
@@ -360,47 +343,108 @@ gemm_fp4_block_scaled_kernel(const __grid_constant__ CUtensorMap w_map,
 }
 
 // ---------------------------------------------------------------------------------------------
-// CTA-pair kernel (cluster of two, tcgen05 cta_group::2) for more than 128 tokens: a pair computes
-// 256 weight rows x 256 tokens.  Each CTA loads its own 128 weight rows and HALF of the token tile
-// (plus its rows' scale bytes and the scale bytes of all 256 tokens, which every tensor core needs);
-// one thread of the pair's first CTA issues M = 256 MMAs for both SMs.  Per SM and stage that is 38
-// KB from L2 instead of 54 KB - the single-CTA kernel stops at the SM's ingest rate (about 41 bytes
-// per clock), not at the tensor pipe.
-// Barriers (same offsets in both CTAs): full[s] local (this CTA's copies landed; its scale
-// writers wait on it), sf[s] in the first CTA only (one arrival per scale-writing warp of either
-// CTA once its columns are in tensor memory - which also says that CTA's operands have landed),
-// empty[s] / accum committed to in each CTA.
+// CTA-pair kernel (cluster of two, tcgen05 cta_group::2): a pair walks tiles of 256 weight rows x BN = 192 or 256
+// tokens.  Each CTA loads its own 128 weight rows, HALF of the token tile, its rows' scale bytes and the
+// scale bytes of all BN tokens (every tensor core needs them); the pair's first CTA issues M = 256 MMAs for both SMs.
+//
+// What bounds it is the warp that issues the MMAs: a wait takes it 170 cycles, an MMA 60, a copy of scale bytes 20, and a
+// stage's MMAs run 440.  So there is one barrier a stage, which the copies of the operands complete themselves, and it is
+// asked a stage ahead.  The scale bytes go their own way ahead of the operands: copied 64 bytes a row (four stages) at a
+// time, rearranged by four warps into a ring as deep as the operands', and moved to tensor memory by tcgen05.cp,
+// issued with the MMAs that read them.  (Warps that store them there have to wait for the MMAs of two stages before.)
+// That copy wants a K block's bytes as 32 pieces of 16, piece l = 4 bytes of each of rows l, l + 32, l + 64, l + 96.
+// 192 tokens leave room in tensor memory for two accumulators, so that a tile's epilogue (four warps of its own, through
+// shared memory and TMA stores) runs under the next tile's MMAs; 256 tokens have one, and 10 % more work per stage.
+// 17408 x 5120 at 8192 tokens 383 -> 338 us (4.3 PFLOP/s; with the K loop's copies alone 233, its MMAs alone 292).
+//
+// Roles per CTA (352 threads): warp 0 operand copies, warp 1 MMAs (first CTA), warps 2..5 scale bytes, every fourth
+// stage each, warps 6..9 epilogue, warp 10 scale copies.
+// Barriers (same offsets in both CTAs): full[s] in the first CTA (both CTAs' operands of a stage landed, both CTAs' scale
+// bytes rearranged), sfull[u] local (scale bytes of four stages landed), sempty[u] local (rearranged), empty[s] and
+// acc_full[a] committed to in each CTA, acc_free[a] in the first CTA (the epilogue warps of both have read the
+// accumulator).
 // ---------------------------------------------------------------------------------------------
-template <int ST>
-__global__ void __launch_bounds__(F4_PAIR_THREADS)
+constexpr int F4P_SK = 4;                            // stages per box of scale bytes
+constexpr int F4P_SF = 3 * 2048;                     // rearranged scale bytes of a stage: weights, two groups of 128 tokens
+constexpr int F4P_OUT = 32 * 64;                     // an epilogue warp's 32 rows x 32 tokens of fp16
+template <int BN>
+struct F4Pair {
+    static constexpr int ACCS = BN == 256 ? 1 : 2;                       // accumulators
+    static constexpr int ST = BN == 256 ? 4 : 5;                         // ring of stages
+    static constexpr int A = F4_BM * 128, B = BN / 2 * 128;              // operand bytes of a stage
+    static constexpr int SA = F4_BM * 16 * F4P_SK, SB = BN * 16 * F4P_SK;    // scale bytes of a box
+    static constexpr int SMEM = ST * (A + B + F4P_SF) + 2 * (SA + SB) + 4 * F4P_OUT + 1024;
+};
+
+// called by a whole converged warp; one elected lane issues (see tcgen05_mma_f16)
+__device__ __forceinline__ void f4p_mma(uint32_t taddr, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa,
+                                        uint32_t sfb, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p, e;\n"
+        "elect.sync _|e, 0xffffffff;\n"
+        "setp.ne.u32 p, %4, 0;\n"
+        "@e tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n}\n" ::
+            "r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
+        : "memory");
+}
+// 512 bytes of shared memory (32 pieces of 16) -> 4 columns of tensor memory, all four lane quarters, in both CTAs
+__device__ __forceinline__ void f4p_copy(uint32_t taddr, uint64_t desc) {
+    asm volatile(
+        "{\n.reg .pred e;\n"
+        "elect.sync _|e, 0xffffffff;\n"
+        "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;\n}\n" ::"r"(taddr), "l"(desc)
+        : "memory");
+}
+// arrives on the barrier at this offset in both CTAs once the MMAs issued so far have retired
+__device__ __forceinline__ void f4p_commit(uint32_t bar) {
+    asm volatile(
+        "{\n.reg .pred e;\n.reg .b16 m;\n"
+        "mov.b16 m, 3;\n"
+        "elect.sync _|e, 0xffffffff;\n"
+        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n}\n" ::"r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void f4p_store(const CUtensorMap* map, uint32_t src, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];\n" ::"l"(map), "r"(src),
+                 "r"(c0), "r"(c1)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+}
+__device__ __forceinline__ uint32_t f4p_half2(uint32_t a, uint32_t b) {
+    const __half2 t = __floats2half2_rn(__uint_as_float(a), __uint_as_float(b));
+    return *reinterpret_cast<const uint32_t*>(&t);
+}
+
+// o_map: the output as boxes of 32 rows x 32 tokens; only used where `tma_out` (16-byte row pitch)
+template <int BN>
+__global__ void __launch_bounds__(F4_PAIR_THREADS, 1)
 gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap a_map,
                      const __grid_constant__ CUtensorMap ws_map, const __grid_constant__ CUtensorMap as_map,
-                     __half* __restrict__ out, int M, int n_tokens, int K, int ld_out) {
-    constexpr int BN = 256, HALF = 128;
-    constexpr int A_BYTES = F4_BM * 128;             // this CTA's weight rows of a stage
-    constexpr int B_BYTES = HALF * 128;              // this CTA's half of the token tile
-    constexpr int SA_BYTES = F4_BM * 16, SB_BYTES = BN * 16;
-    constexpr int NB = BN / 32;                      // token rows per lane = scale columns per MMA
-    constexpr int SFA_COLS = 16, SFB_COLS = 4 * NB, SF_COLS = SFA_COLS + SFB_COLS;
-    constexpr int TCOLS = f4_tmem_cols(BN + ST * SF_COLS);
-    static_assert(BN + ST * SF_COLS <= 512, "tensor memory");
+                     const __grid_constant__ CUtensorMap o_map, int tma_out, __half* __restrict__ out, int M,
+                     int n_tokens, int K, int ld_out) {
+    using T = F4Pair<BN>;
+    constexpr int HALF = BN / 2, ST = T::ST, SK = F4P_SK, ACCS = T::ACCS;
+    constexpr int NB = BN / 32;                      // groups of 32 tokens
+    constexpr int SFB = 8;                           // token-scale columns per MMA (a multiple of 4)
+    constexpr int SF_STRIDE = 64;                    // columns of a stage (two take turns): 16 for the weights, 4 x SFB
+    static_assert(NB <= SFB && ACCS * BN + 2 * SF_STRIDE <= 512 && 16 + 4 * SFB <= SF_STRIDE, "tensor memory");
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                ~(uintptr_t)1023);
     uint8_t* smem_a = smem;
-    uint8_t* smem_b = smem + ST * A_BYTES;
-    uint8_t* smem_sa = smem_b + ST * B_BYTES;
-    uint8_t* smem_sb = smem_sa + ST * SA_BYTES;
-    __shared__ __align__(8) uint64_t bar_full[ST];
-    __shared__ __align__(8) uint64_t bar_sf[ST];
-    __shared__ __align__(8) uint64_t bar_empty[ST];
-    __shared__ __align__(8) uint64_t bar_accum;
-    __shared__ __align__(8) uint64_t bar_acc_free;    // first CTA's: both epilogues have read the accumulators
+    uint8_t* smem_b = smem_a + ST * T::A;
+    uint8_t* smem_sa = smem_b + ST * T::B;
+    uint8_t* smem_sb = smem_sa + 2 * T::SA;
+    uint8_t* smem_sf = smem_sb + 2 * T::SB;
+    uint8_t* smem_o = smem_sf + ST * F4P_SF;
+    __shared__ __align__(8) uint64_t bar_full[ST], bar_empty[ST];
+    __shared__ __align__(8) uint64_t bar_sfull[2], bar_sempty[2];
+    __shared__ __align__(8) uint64_t bar_acc_full[2], bar_acc_free[2];
     __shared__ uint32_t s_tmem;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_cta_rank();
-    // a pair walks the pair tiles pair, pair + pairs, ... (256 rows x 256 tokens each, row pair fastest)
+    // a pair walks the pair tiles pair, pair + pairs, ... (row pair fastest)
     const int pairs = (int)(gridDim.x >> 1), pair0 = (int)(blockIdx.x >> 1);
     const int tiles_m = (M + 2 * F4_BM - 1) / (2 * F4_BM);
     const int ntiles = tiles_m * ((n_tokens + BN - 1) / BN);
@@ -408,16 +452,19 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < ST; s++) {
-            mbar_init(smem_u32(&bar_full[s]), 1);
-            mbar_init(smem_u32(&bar_sf[s]), 8);       // 4 scale-writing warps of each CTA
+            mbar_init(smem_u32(&bar_full[s]), 4);        // a copy-issuing thread and a scale warp of each CTA
             mbar_init(smem_u32(&bar_empty[s]), 1);
         }
-        mbar_init(smem_u32(&bar_accum), 1);
-        mbar_init(smem_u32(&bar_acc_free), 16);   // 8 epilogue warps of each CTA
+        for (int u = 0; u < 2; u++) {
+            mbar_init(smem_u32(&bar_sfull[u]), 1);
+            mbar_init(smem_u32(&bar_sempty[u]), 4);      // the scale warps of this CTA
+            mbar_init(smem_u32(&bar_acc_full[u]), 1);
+            mbar_init(smem_u32(&bar_acc_free[u]), 8);    // four epilogue warps of each CTA
+        }
         fence_barrier_init();
     }
     if (warp == 0) {
-        tcgen05_alloc_pair(smem_u32(&s_tmem), TCOLS);
+        tcgen05_alloc_pair(smem_u32(&s_tmem), 512);
         tcgen05_relinquish_pair();
     }
     tcgen05_fence_before();
@@ -425,149 +472,206 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
     cluster_sync_all();
     tcgen05_fence_after();
     const uint32_t tmem = s_tmem;
-    const uint32_t tmem_sf = tmem + BN;
+    const uint32_t tmem_sf = tmem + ACCS * BN;
 
     if (warp == 0) {
         if (lane == 0) {
-            int s = 0;
+            int s = 0, issued = 0;
             uint32_t ph = 0;
             bool ok = true;
             for (int tile = pair0; tile < ntiles && ok; tile += pairs) {
-                const int m0 = ((tile % tiles_m) * 2 + (int)rank) * F4_BM, n0 = (tile / tiles_m) * BN;
-                const int nh = n0 + (int)rank * HALF;
-                for (int it = 0; it < ksteps; it++) {
-                    if (!f4_wait_poll(smem_u32(&bar_empty[s]), ph ^ 1u, 0)) { ok = false; break; }
-                    const uint32_t bar = smem_u32(&bar_full[s]);
-                    mbar_arrive_expect_tx(bar, A_BYTES + B_BYTES + SA_BYTES + SB_BYTES);
-                    tma_load_2d(smem_u32(smem_a + s * A_BYTES), &w_map, it * 128, m0, bar);
-                    tma_load_2d(smem_u32(smem_b + s * B_BYTES), &a_map, it * 128, nh, bar);
-                    tma_load_2d(smem_u32(smem_sa + s * SA_BYTES), &ws_map, it * 16, m0, bar);
-                    tma_load_2d(smem_u32(smem_sb + s * SB_BYTES), &as_map, it * 16, n0, bar);
+                const int m0 = ((tile % tiles_m) * 2 + (int)rank) * F4_BM, nh = (tile / tiles_m) * BN + (int)rank * HALF;
+                for (int it = 0; it < ksteps; it++, issued++) {
+                    ok = f4_wait(smem_u32(&bar_empty[s]), ph ^ 1u, 0);
+                    if (!ok) break;
+                    const uint32_t bar = cluster_map_shared(smem_u32(&bar_full[s]), 0);
+                    mbar_arrive_expect_tx_cluster(bar, T::A + T::B);
+                    tma_load_2d_pair(smem_u32(smem_a + s * T::A), &w_map, it * 128, m0, bar);
+                    tma_load_2d_pair(smem_u32(smem_b + s * T::B), &a_map, it * 128, nh, bar);
                     if (++s == ST) { s = 0; ph ^= 1u; }
                 }
             }
+            // No copy may be in flight when the CTA leaves, also where a wait has run out.  (full is the first CTA's and
+            // counts both CTAs' copies; the second stays until the first has synced.)
+            if (rank == 0)
+                for (int i = max(issued - ST, 0); i < issued; i++)
+                    f4_wait(smem_u32(&bar_full[i % ST]), (uint32_t)(i / ST) & 1u, 7);
+        }
+    } else if (warp == 10) {
+        if (lane == 0) {
+            int boxes = 0;
+            bool ok = true;
+            for (int tile = pair0; tile < ntiles && ok; tile += pairs) {
+                const int m0 = ((tile % tiles_m) * 2 + (int)rank) * F4_BM, n0 = (tile / tiles_m) * BN;
+                for (int it = 0; it < ksteps; it += SK, boxes++) {
+                    const int u = boxes & 1;
+                    ok = f4_wait(smem_u32(&bar_sempty[u]), ((uint32_t)(boxes >> 1) & 1u) ^ 1u, 6);
+                    if (!ok) break;
+                    const uint32_t bar = smem_u32(&bar_sfull[u]);
+                    mbar_arrive_expect_tx(bar, T::SA + T::SB);
+                    // x = byte along K / 16 (a multiple of 64); what lies past the end of a row or of the matrix is
+                    // filled with zero bytes
+                    tma_load_2d(smem_u32(smem_sa + u * T::SA), &ws_map, it * 16, m0, bar);
+                    tma_load_2d(smem_u32(smem_sb + u * T::SB), &as_map, it * 16, n0, bar);
+                }
+            }
+            for (int i = max(boxes - 2, 0); i < boxes; i++)
+                f4_wait(smem_u32(&bar_sfull[i & 1]), (uint32_t)(i >> 1) & 1u, 7);
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | (1u << 23) |
                                    ((uint32_t)((2 * F4_BM) >> 4) << 24);
-            int s = 0, ti = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int tile = pair0; tile < ntiles && ok; tile += pairs, ti++) {
-                // both CTAs' epilogues of the tile before must have read their accumulators
-                if (ti > 0 && !f4_wait_poll(smem_u32(&bar_acc_free), (uint32_t)(ti - 1) & 1u, 5)) break;
-                tcgen05_fence_after();
+            // descriptors: +1 in the low word = 16 bytes further in shared memory
+            const uint64_t a_desc = make_desc_sw128(smem_u32(smem_a), 16, 1024);
+            const uint64_t b_desc = make_desc_sw128(smem_u32(smem_b), 16, 1024);
+            // scale bytes: 32 rows of 16 bytes, 128 bytes from one eight to the next, no swizzle
+            const uint64_t s_desc = (uint64_t)((smem_u32(smem_sf) >> 4) & 0x3FFF) | ((uint64_t)8 << 32) | ((uint64_t)1 << 46);
+            int s = 0, set = 0, acc = 0;
+            uint32_t ph = 0, aph = 0;
+            bool ok = true, ready = false;
+            for (int tile = pair0; tile < ntiles; tile += pairs) {
+                // both CTAs' epilogues must have read what this accumulator held
+                if (ok) ok = f4_wait(smem_u32(&bar_acc_free[acc]), aph ^ 1u, 5);
+                const uint32_t d = tmem + (uint32_t)(acc * BN);
                 for (int it = 0; it < ksteps; it++) {
-                    if (!f4_wait_poll(smem_u32(&bar_sf[s]), ph, 1)) { ok = false; break; }
+                    if (ok && !ready) ok = f4_wait(smem_u32(&bar_full[s]), ph, 1);
+                    __syncwarp();
                     tcgen05_fence_after();
-                    const uint32_t a_base = smem_u32(smem_a + s * A_BYTES);
-                    const uint32_t b_base = smem_u32(smem_b + s * B_BYTES);
-                    const uint32_t sf = tmem_sf + (uint32_t)(s * SF_COLS);
+                    // the next stage's barrier is asked before this stage's instructions are issued, which hide the
+                    // answer's 170 cycles (16 instructions a stage are what this warp can issue in time)
+                    const bool wrap = s + 1 == ST;
+                    const bool next = mbar_test_wait_cluster(smem_u32(&bar_full[wrap ? 0 : s + 1]), wrap ? ph ^ 1u : ph);
+                    const uint64_t ad = a_desc + (uint64_t)(s * (T::A >> 4)), bd = b_desc + (uint64_t)(s * (T::B >> 4));
+                    const uint64_t sd = s_desc + (uint64_t)(s * (F4P_SF >> 4));
+                    const uint32_t sf = tmem_sf + (uint32_t)(set * SF_STRIDE);
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++) {
-                        const uint64_t adesc = make_desc_sw128(a_base + kk * 32, 16, 1024);
-                        const uint64_t bdesc = make_desc_sw128(b_base + kk * 32, 16, 1024);
-                        tcgen05_mma_fp4_block16_pair(tmem, adesc, bdesc, idesc, sf + (uint32_t)(kk * 4),
-                                                     sf + (uint32_t)(SFA_COLS + kk * NB), (it | kk) != 0 ? 1u : 0u);
+                        f4p_copy(sf + (uint32_t)(kk * 4), sd + 32 * kk);
+                        f4p_copy(sf + (uint32_t)(16 + kk * SFB), sd + 128 + 32 * kk);
+                        f4p_copy(sf + (uint32_t)(16 + kk * SFB + 4), sd + 256 + 32 * kk);
                     }
-                    const uint32_t be = smem_u32(&bar_empty[s]);
-                    tcgen05_commit_pair(cluster_map_shared(be, 0));
-                    tcgen05_commit_pair(cluster_map_shared(be, 1));
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++)   // 64 elements of K = 32 bytes further along the swizzled row
+                        f4p_mma(d, ad + 2 * kk, bd + 2 * kk, idesc, sf + (uint32_t)(kk * 4), sf + (uint32_t)(16 + kk * SFB),
+                                (it | kk) != 0 ? 1u : 0u);
+                    f4p_commit(smem_u32(&bar_empty[s]));
+                    ready = __all_sync(0xffffffffu, next);
+                    set ^= 1;
                     if (++s == ST) { s = 0; ph ^= 1u; }
                 }
-                const uint32_t ba = smem_u32(&bar_accum);
-                tcgen05_commit_pair(cluster_map_shared(ba, 0));
-                tcgen05_commit_pair(cluster_map_shared(ba, 1));
+                f4p_commit(smem_u32(&bar_acc_full[acc]));
+                if (++acc == ACCS) acc = 0;
+                if (acc == 0) aph ^= 1u;
             }
+        }
+    } else if (warp < 6) {
+        // ---------------- scale bytes, rows -> pieces ----------------
+        // Every warp goes through every box, in order, and arrives for it, with or without a stage of its own in it: a
+        // barrier's parity tells a phase only from the one before, so nobody may be two boxes of a slot ahead or behind.
+        const int mine = warp - 2;                         // of the stages i: those with i % 4 == mine
+        bool ok = true;
+        int g = 0, box = 0;                                // stages and boxes before this tile
+        for (int tile = pair0; tile < ntiles; tile += pairs) {
+            for (int it0 = 0; it0 < ksteps; it0 += SK, box++) {
+                const int u = box & 1, j = (mine - g - it0) & 3;       // own stage of this box: it0 + j
+                if (ok) ok = f4_wait(smem_u32(&bar_sfull[u]), (uint32_t)(box >> 1) & 1u, 3);
+                __syncwarp();
+                if (j < SK && it0 + j < ksteps) {
+                    // the slot's pieces have been read: the MMAs of stage i - ST have retired
+                    const int i = g + it0 + j, s = i % ST;
+                    if (ok) ok = f4_wait(smem_u32(&bar_empty[s]), ((uint32_t)(i / ST) & 1u) ^ 1u, 9);
+                    __syncwarp();
+                    // 16 bytes of a row: piece j of its 64, in the 64-byte swizzle
+                    const int c16 = lane * 64 + (j ^ ((lane >> 1) & 3)) * 16;
+                    uint8_t* dst = smem_sf + s * F4P_SF + lane * 16;
+#pragma unroll
+                    for (int part = 0; part < 3; part++) { // weights, tokens 0..127, the others
+                        const uint8_t* src = part == 0 ? smem_sa + u * T::SA + c16
+                                                       : smem_sb + u * T::SB + (part - 1) * 8192 + c16;
+                        uint4 v[4];
+#pragma unroll
+                        for (int c = 0; c < 4; c++)
+                            v[c] = c < 2 || part < 2 || BN == 256 ? *reinterpret_cast<const uint4*>(src + c * 2048) : make_uint4(0u, 0u, 0u, 0u);
+                        *reinterpret_cast<uint4*>(dst + part * 2048) = make_uint4(v[0].x, v[1].x, v[2].x, v[3].x);
+                        *reinterpret_cast<uint4*>(dst + part * 2048 + 512) = make_uint4(v[0].y, v[1].y, v[2].y, v[3].y);
+                        *reinterpret_cast<uint4*>(dst + part * 2048 + 1024) = make_uint4(v[0].z, v[1].z, v[2].z, v[3].z);
+                        *reinterpret_cast<uint4*>(dst + part * 2048 + 1536) = make_uint4(v[0].w, v[1].w, v[2].w, v[3].w);
+                    }
+                    fence_proxy_async_smem();              // the tensor core reads them (async proxy)
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(cluster_map_shared(smem_u32(&bar_full[s]), 0));
+                }
+                if (lane == 0) mbar_arrive(smem_u32(&bar_sempty[u]));
+            }
+            g += ksteps;
         }
     } else {
-        // ---------------- scale-factor writers (this CTA's tensor memory) ----------------
-        // Two sets of four warps (a warp reaches the 32 lanes of tensor memory given by its index
-        // modulo 4) take alternate stages: from the landing of a stage's bytes to the arrival on
-        // sf[s] a set needs longer than the tensor core needs for the stage's MMAs.
+        // ---------------- epilogue: this CTA's 128 rows x BN tokens ----------------
         const int q = warp & 3;
-        const int set = (warp - 2) >> 2;
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
+        uint8_t* o = smem_o + (warp - 6) * F4P_OUT;
         bool ok = true;
-        int ti = 0;
-        for (int tile = pair0; tile < ntiles; tile += pairs, ti++) {
-        const int m0 = ((tile % tiles_m) * 2 + (int)rank) * F4_BM, n0 = (tile / tiles_m) * BN;
-        for (int it = set; it < ksteps; it += 2) {
-            const int g = ti * ksteps + it;              // stages since the kernel began
-            const int s = g % ST;
-            const uint32_t ph = (uint32_t)(g / ST) & 1u;
-            if (ok) ok = f4_wait(smem_u32(&bar_full[s]), ph, 3);
-            tcgen05_fence_after();
-            const uint8_t* sa = smem_sa + s * SA_BYTES;
-            const uint8_t* sb = smem_sb + s * SB_BYTES;
-            uint4 wv[4], av[NB];
-#pragma unroll
-            for (int c = 0; c < 4; c++) wv[c] = *reinterpret_cast<const uint4*>(sa + (c * 32 + lane) * 16);
-#pragma unroll
-            for (int c = 0; c < NB; c++) av[c] = *reinterpret_cast<const uint4*>(sb + (c * 32 + lane) * 16);
-            uint32_t wa[4][4], wb[4][NB];
-#pragma unroll
-            for (int c = 0; c < 4; c++) { wa[0][c] = wv[c].x; wa[1][c] = wv[c].y; wa[2][c] = wv[c].z; wa[3][c] = wv[c].w; }
-#pragma unroll
-            for (int c = 0; c < NB; c++) { wb[0][c] = av[c].x; wb[1][c] = av[c].y; wb[2][c] = av[c].z; wb[3][c] = av[c].w; }
-            const uint32_t sf = tmem_sf + (uint32_t)(s * SF_COLS) + lane_base;
-#pragma unroll
-            for (int kk = 0; kk < 4; kk++) {
-                tcgen05_st_32x32b<4>(sf + (uint32_t)(kk * 4), wa[kk]);
-                tcgen05_st_32x32b<NB>(sf + (uint32_t)(SFA_COLS + kk * NB), wb[kk]);
-            }
-            tcgen05_wait_st();
-            tcgen05_fence_before();
+        int acc = 0;
+        uint32_t aph = 0;
+        for (int tile = pair0; tile < ntiles; tile += pairs) {
+            const int m0 = ((tile % tiles_m) * 2 + (int)rank) * F4_BM + q * 32, n0 = (tile / tiles_m) * BN;
+            if (ok) ok = f4_wait(smem_u32(&bar_acc_full[acc]), aph, 4);
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(cluster_map_shared(smem_u32(&bar_sf[s]), 0));
-        }
-
-        // ---------------- epilogue: this CTA's 128 rows x 256 tokens ----------------
-        if (ok) ok = f4_wait_poll(smem_u32(&bar_accum), (uint32_t)ti & 1u, 4);
-        tcgen05_fence_after();
-        const int m = m0 + q * 32 + lane;
+            tcgen05_fence_after();
 #pragma unroll 1
-        for (int cb = set * (BN / 64); cb < (set + 1) * (BN / 64); cb++) {    // each set half of the tokens
-            uint32_t v[32];
-            tcgen05_ld_32x32b_x32(tmem + lane_base + (uint32_t)(cb * 32), v);
-            tcgen05_wait_ld();
-            const int nb = n0 + cb * 32;
-            if (m < M && nb < n_tokens) {
-                __half* orow = out + (size_t)m * (size_t)ld_out + nb;
-                if (nb + 32 <= n_tokens && (ld_out & 7) == 0) {
-#pragma unroll
-                    for (int j = 0; j < 32; j += 8) {
-                        uint4 o;
-                        __half2 t;
-                        t = __floats2half2_rn(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
-                        o.x = *reinterpret_cast<uint32_t*>(&t);
-                        t = __floats2half2_rn(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-                        o.y = *reinterpret_cast<uint32_t*>(&t);
-                        t = __floats2half2_rn(__uint_as_float(v[j + 4]), __uint_as_float(v[j + 5]));
-                        o.z = *reinterpret_cast<uint32_t*>(&t);
-                        t = __floats2half2_rn(__uint_as_float(v[j + 6]), __uint_as_float(v[j + 7]));
-                        o.w = *reinterpret_cast<uint32_t*>(&t);
-                        *reinterpret_cast<uint4*>(orow + j) = o;
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (nb + j < n_tokens) orow[j] = __float2half(__uint_as_float(v[j]));
+            for (int cb = 0; cb < BN / 32; cb++) {
+                uint32_t v[32];
+                tcgen05_ld_32x32b_x32(tmem + lane_base + (uint32_t)(acc * BN + cb * 32), v);
+                tcgen05_wait_ld();
+                if (cb == BN / 32 - 1) {       // the accumulator is read: the MMAs of the tile after the next may start
+                    tcgen05_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(cluster_map_shared(smem_u32(&bar_acc_free[acc]), 0));
                 }
+                const int nb = n0 + cb * 32;
+                if (nb >= n_tokens || m0 >= M) continue;
+                // (a TMA store that ends inside 16 bytes writes them all: the last tokens of a ragged count go by hand)
+                if (tma_out && (nb + 32 <= n_tokens || (n_tokens & 7) == 0)) {
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+                    __syncwarp();
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        const uint32_t* x = &v[c * 8];
+                        *reinterpret_cast<uint4*>(o + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) =
+                            make_uint4(f4p_half2(x[0], x[1]), f4p_half2(x[2], x[3]), f4p_half2(x[4], x[5]), f4p_half2(x[6], x[7]));
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) f4p_store(&o_map, smem_u32(o), nb, m0);
+                } else if (m0 + lane < M) {
+                    __half* orow = out + (size_t)(m0 + lane) * (size_t)ld_out + nb;
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        const uint32_t* x = &v[c * 8];
+                        if (tma_out && nb + c * 8 + 8 <= n_tokens) {
+                            *reinterpret_cast<uint4*>(orow + c * 8) =
+                                make_uint4(f4p_half2(x[0], x[1]), f4p_half2(x[2], x[3]), f4p_half2(x[4], x[5]), f4p_half2(x[6], x[7]));
+                        } else if (nb + c * 8 < n_tokens) {
+#pragma unroll
+                            for (int j = 0; j < 8; j++)
+                                if (nb + c * 8 + j < n_tokens) orow[c * 8 + j] = __float2half(__uint_as_float(x[j]));
+                        }
+                    }
+                }
+                __syncwarp();
             }
+            if (++acc == ACCS) acc = 0;
+            if (acc == 0) aph ^= 1u;
         }
-        // this warp's part of the accumulator is read: tell the thread that issues the next tile's MMAs
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(cluster_map_shared(smem_u32(&bar_acc_free), 0));
-        }   // tiles
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
     }
 
+    __syncwarp();
     tcgen05_fence_before();
     __syncthreads();
     cluster_sync_all();
-    if (warp == 0) tcgen05_dealloc_pair(tmem, TCOLS);
+    if (warp == 0) tcgen05_dealloc_pair(tmem, 512);
 }
 
 // Workspace of the K split, one per device: fp32 partial tiles (at most F4_SPLIT_CTAS CTAs of 128 x
@@ -650,29 +754,57 @@ static cudaError_t launch_fp4(const CUtensorMap& wm, const CUtensorMap& am, cons
 }
 
 static int g_f4_pairs_override = 0;  // pairs of the tile-walking pair kernel (0: one per two SMs)
-static int g_f4_pair = 1;           // the CTA-pair kernel: 1 = more than 128 tokens and K >= 10240, 2 = more than 128 tokens, 0 = never
+static int g_f4_pair_bn = 0;        // token tile of the CTA-pair kernel: 192, 256, or 0 = by fp4_pair_tokens
+static int g_f4_pair = 1;           // the CTA-pair kernel: 1 = where fp4_pair_tokens says so, 2 = more than 128 tokens, 0 = never
+
+// Token tile of the CTA-pair kernel for this problem, 0 where the single-CTA kernel takes it.  GEMM alone, us, single-CTA
+// kernel (as it was chosen before) / pairs of 192 / pairs of 256 tokens:
+//   17408 x 5120: 192 tokens 18.2 / 16.5 / 17.4, 256 tokens 17.6 / 23.4 / 18.0, 1000: 57 / 56 / 51, 2048: 106 / 95 / 92,
+//   8192: 438 / 373 / 376 (a long run; 383 / 338 apart); 6144 x 5120, 8192: 143 / 121 / 117; 5120 x 17408, 8192: 326 /
+//   336 / 306; 4096 x 1024, 8192: 42 / 30 / 34, but 129 tokens 10.6 / 11.4 / 11.8, 800: 12.5 / 13.4 / 13.0.
+// Few deep tiles used to be split over K.  The partial tiles of 128 and more tokens are what that waits for: 5120 x 17408,
+// 65 tokens 34.2 / 31.4 / 35, 129 tokens 59.6 / 32.2 / 35.7; 1024 x 17408, 129 tokens 110 / 31; at 64 tokens 21.4 / 31.1.
+// Both widths run in rounds of pairs, a round costs a part per stage and a fixed part (ns, fitted to the above).
+static int fp4_pair_tokens(int M, int n, int K) {
+    const int st = K / F4_BK, sms = f4_sm_count(current_device_index());
+    const int tiles1 = ((M + F4_BM - 1) / F4_BM) * ((n + 255) / 256);
+    if (g_f4_pair == 0) return 0;
+    if (g_f4_pair == 1) {
+        const bool few_deep = g_f4_split && tiles1 * 2 <= sms && st >= 40;
+        if (few_deep ? n <= 64 : n <= 128 || M <= F4_BM) return 0;
+        if (st <= 4 && tiles1 <= sms) return 0;
+    } else if (n <= 128) {
+        return 0;
+    }
+    if (g_f4_pair_bn) return g_f4_pair_bn;
+    const long long rows = (M + 255) / 256, pairs = std::max(1, sms / 2);
+    const long long r192 = (rows * ((n + 191) / 192) + pairs - 1) / pairs, r256 = (rows * ((n + 255) / 256) + pairs - 1) / pairs;
+    const int bn = r256 * (454LL * st + 2900) < r192 * (407LL * st + 1100) ? 256 : 192;
+    // one round of single CTAs on the whole GPU is as fast as one of 256-token pairs, and is there sooner
+    return g_f4_pair == 1 && bn == 256 && tiles1 <= sms && st < 40 ? 0 : bn;
+}
+
+template <int BN>
 static cudaError_t launch_fp4_pair(const CUtensorMap& wm, const CUtensorMap& am, const CUtensorMap& ws,
-                                   const CUtensorMap& as, __half* out, int M, int n, int K, int ld,
-                                   cudaStream_t st) {
-    constexpr int ST = 5;
-    constexpr int SMEM = ST * (F4_BM * 128 + 128 * 128 + F4_BM * 16 + 256 * 16) + 1024;
+                                   const CUtensorMap& as, const CUtensorMap& om, bool tma_out, __half* out, int M, int n,
+                                   int K, int ld, cudaStream_t st) {
     static bool attr[NVFP4_MAX_DEVICES] = {false};
     const int dev = current_device_index();
     if (!attr[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_fp4_pair_kernel<ST>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        const cudaError_t e = cudaFuncSetAttribute(gemm_fp4_pair_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   F4Pair<BN>::SMEM);
         if (e != cudaSuccess) return e;
         attr[dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    // a pair of CTAs per pair of SMs walks the 256 x 256 tiles (one pair per tile with bit 3 of the config)
-    const int ptiles = ((M + 255) / 256) * ((n + 255) / 256);
+    // a pair of CTAs per pair of SMs walks the 256 x BN tiles (one pair per tile with bit 3 of the config)
+    const int ptiles = ((M + 255) / 256) * ((n + BN - 1) / BN);
     const int pairs = g_f4_persistent ? std::min(ptiles, g_f4_pairs_override > 0 ? g_f4_pairs_override
                                                                                : f4_sm_count(dev) / 2)
                                       : ptiles;
     cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
     cfg.blockDim = dim3(F4_PAIR_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = SMEM;
+    cfg.dynamicSmemBytes = F4Pair<BN>::SMEM;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -681,7 +813,7 @@ static cudaError_t launch_fp4_pair(const CUtensorMap& wm, const CUtensorMap& am,
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemm_fp4_pair_kernel<ST>, wm, am, ws, as, out, M, n, K, ld);
+    return cudaLaunchKernelEx(&cfg, gemm_fp4_pair_kernel<BN>, wm, am, ws, as, om, tma_out ? 1 : 0, out, M, n, K, ld);
 }
 
 static bool byte_matrix_map(EncodeTiledFn enc, CUtensorMap* map, const void* base, int rows, int K,
@@ -695,16 +827,27 @@ static bool byte_matrix_map(EncodeTiledFn enc, CUtensorMap* map, const void* bas
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// scale bytes [rows][K/16]: boxes of 16 bytes (one 256-element stage) x box_rows rows, unswizzled
+// scale bytes [rows][K/16]: boxes of 16 bytes (one 256-element stage, unswizzled) or 64 bytes (four of them, 64-byte
+// swizzle) x box_rows rows
 static bool scale_matrix_map(EncodeTiledFn enc, CUtensorMap* map, const void* base, int rows, int K,
-                             int box_rows) {
+                             int box_rows, int box_bytes) {
     const cuuint64_t dims[2] = {(cuuint64_t)(K / 16), (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)(K / 16)};
-    const cuuint32_t box[2] = {16, (cuuint32_t)box_rows};
+    const cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+               CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// the output [M][ld] as boxes of 32 rows x 32 tokens (what lies past row M or token n is not written)
+static bool out_matrix_map(EncodeTiledFn enc, CUtensorMap* map, void* base, int M, int n, int ld) {
+    const cuuint64_t dims[2] = {(cuuint64_t)n, (cuuint64_t)M};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(__half)};
+    const cuuint32_t box[2] = {32, 32};
+    const cuuint32_t estr[2] = {1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace nvfp4
@@ -728,24 +871,22 @@ int launch_nvfp4_gemm_fp4(const uint8_t* w_packed, const uint8_t* w_scales, cons
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return -3;
     const int BN = n_tokens > 128 ? 256 : n_tokens > 64 ? 128 : n_tokens > 32 ? 64 : 32;
-    // The pair kernel takes more than 128 tokens.  Measured at 8192 tokens: a stage costs it 790
-    // cycles against 950, a tile's fixed part (prologue, cluster barriers, epilogue) 7.9 us against
-    // 5.5: it wins from about 40 stages on (5120 x 17408: 310 us against 342; 6144 x 5120, 20
-    // stages: 168 against 161).  Few deep-K tiles are better served by the K split.
-    const int tiles1 = ((M + F4_BM - 1) / F4_BM) * ((n_tokens + 255) / 256);
-    const bool few_deep = g_f4_split && tiles1 * 2 <= f4_sm_count(current_device_index()) && K / F4_BK >= 40;
-    const bool pair = n_tokens > 128 && M > F4_BM && !few_deep &&
-                      (g_f4_pair == 2 || (g_f4_pair == 1 && K / F4_BK >= 40));
-    CUtensorMap wm, am, wsm, asm_;
+    const int pbn = fp4_pair_tokens(M, n_tokens, K);
+    const bool pair = pbn != 0;
+    CUtensorMap wm, am, wsm, asm_, om;
+    const bool tma_out = pair && (ld_out & 7) == 0;
     if (!byte_matrix_map(enc, &wm, w_packed, M, K, F4_BM) ||
-        !byte_matrix_map(enc, &am, a_packed, n_tokens, K, pair ? 128 : BN) ||
-        !scale_matrix_map(enc, &wsm, w_scales, M, K, F4_BM) ||
-        !scale_matrix_map(enc, &asm_, a_scales, n_tokens, K, BN))
+        !byte_matrix_map(enc, &am, a_packed, n_tokens, K, pair ? pbn / 2 : BN) ||
+        !scale_matrix_map(enc, &wsm, w_scales, M, K, F4_BM, pair ? 64 : 16) ||
+        !scale_matrix_map(enc, &asm_, a_scales, n_tokens, K, pair ? pbn : BN, pair ? 64 : 16) ||
+        (tma_out && !out_matrix_map(enc, &om, out, M, n_tokens, ld_out)))
         return -3;
+    if (!tma_out) om = am;                           // not used by the kernel
     cudaStream_t st = (cudaStream_t)stream;
     __half* o = static_cast<__half*>(out);
     const cudaError_t e =
-        pair      ? launch_fp4_pair(wm, am, wsm, asm_, o, M, n_tokens, K, ld_out, st)
+        pbn == 256 ? launch_fp4_pair<256>(wm, am, wsm, asm_, om, tma_out, o, M, n_tokens, K, ld_out, st)
+      : pbn == 192 ? launch_fp4_pair<192>(wm, am, wsm, asm_, om, tma_out, o, M, n_tokens, K, ld_out, st)
       : BN == 256 ? launch_fp4<256, 4>(wm, am, wsm, asm_, o, M, n_tokens, K, ld_out, st)
       : BN == 128 ? launch_fp4<128, 6>(wm, am, wsm, asm_, o, M, n_tokens, K, ld_out, st)
       : BN == 64  ? launch_fp4<64, 6>(wm, am, wsm, asm_, o, M, n_tokens, K, ld_out, st)
@@ -768,13 +909,14 @@ int nvfp4_gemm_fp4_status(int reset) {
     return v;
 }
 
-// Bit 0: K split of the FP4 GEMM for shapes with few output tiles.  Bit 1: the CTA-pair kernel for
-// more than 128 tokens and K >= 10240.  Bit 2: the CTA-pair kernel for every K.  Bit 3: one CTA (pair)
-// per output tile instead of one per SM (two SMs) walking the tiles.  Bits 8..15: number of pairs of
-// the walking pair kernel (0 = half the SM count).  Default 3.
+// Bit 0: K split of the FP4 GEMM for shapes with few output tiles.  Bit 1: the CTA-pair kernel where it is
+// faster.  Bit 2: the CTA-pair kernel for more than 128 tokens.  Bit 3: one CTA (pair) per output tile instead of one
+// per SM (two SMs) walking the tiles.  Bits 4, 5: its token tile always 256, always 192.  Bits 8..15: number of pairs of the
+// walking pair kernel (0 = half the SM count).  Default 3.
 void nvfp4_b200_gemm_fp4_config(int flags) {
     nvfp4::g_f4_split = (flags & 1) ? 1 : 0;
     nvfp4::g_f4_pair = (flags & 4) ? 2 : (flags & 2) ? 1 : 0;
+    nvfp4::g_f4_pair_bn = (flags & 16) ? 256 : (flags & 32) ? 192 : 0;
     nvfp4::g_f4_persistent = (flags & 8) ? 0 : 1;
     nvfp4::g_f4_pairs_override = (flags >> 8) & 0xFF;     // bits 8..15: CTA pairs of the tile-walking pair kernel
 }
