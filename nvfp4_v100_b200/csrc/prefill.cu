@@ -22,6 +22,7 @@
 #include <cstdio>
 
 #include "common.cuh"
+#include "dn_chunk.cuh"
 
 namespace nvfp4 {
 
@@ -716,10 +717,14 @@ long long nvfp4_dn_prefill_work_bytes(int n, int nk, int nv) {
     const long long conv_dim = (2LL * nk + nv) * PF_DK;
     long long b = (long long)n * conv_dim * 2;            // conv output, fp16
     b = (b + 255) & ~255LL;
-    const long long nb = (n + DNB - 1) / DNB;              // blocks of the recurrence
-    b += 2LL * nb * DNB * nk * PF_DK * 4;                  // normalised q and k, fp32
-    b += nb * nv * (long long)sizeof(nvfp4::DnBlock);      // the blocks' coefficients
-    b = (b + 255) & ~255LL;
+    if (nvfp4::dn_chunk_takes(n, nv)) {
+        b += nvfp4::dn_chunk_work_bytes(n, nk, nv);
+    } else {
+        const long long nb = (n + DNB - 1) / DNB;          // blocks of the recurrence
+        b += 2LL * nb * DNB * nk * PF_DK * 4;              // normalised q and k, fp32
+        b += nb * nv * (long long)sizeof(nvfp4::DnBlock);  // the blocks' coefficients
+        b = (b + 255) & ~255LL;
+    }
     b += (long long)n * nv * PF_DK * 2;                    // recurrence output, fp16
     return b + 256;
 }
@@ -741,13 +746,6 @@ int launch_dn_prefill(const void* x, long long ld, const void* conv_w, void* con
     unsigned char* w = (unsigned char*)work;
     __half* conv_out = (__half*)w;
     long long off = ((long long)n * conv_dim * 2 + 255) & ~255LL;
-    float* qn = (float*)(w + off);
-    const int nb = (n + DNB - 1) / DNB;
-    float* kn = qn + (size_t)nb * DNB * nk * PF_DK;
-    off += 2LL * nb * DNB * nk * PF_DK * 4;
-    nvfp4::DnBlock* blocks = (nvfp4::DnBlock*)(w + off);
-    off = (off + (long long)nb * nv * (long long)sizeof(nvfp4::DnBlock) + 255) & ~255LL;
-    __half* o16 = (__half*)(w + off);
     cudaStream_t st = (cudaStream_t)stream;
     const __half* xh = (const __half*)x;
     bool ok = true;
@@ -758,15 +756,30 @@ int launch_dn_prefill(const void* x, long long ld, const void* conv_w, void* con
     ok = ok && nvfp4::launch_pdl(conv, dim3((conv_dim + 511) / 512, (n + conv_t - 1) / conv_t), dim3(128), 0, st, xh, ld,
                                  (const __half*)conv_w, (const __half*)conv_state, conv_out, conv_dim,
                                  n) == cudaSuccess;
-    ok = ok && nvfp4::launch_pdl(nvfp4::dn_block_kernel, dim3((nk + 3) / 4, nb), dim3(128), 0,
-                                 st, (const __half*)conv_out, conv_dim, xh, ld,
-                                 (const __half*)A_log, (const __half*)dt_bias, qn, kn, blocks, nk,
-                                 nv, n) == cudaSuccess;
-    ok = ok && nvfp4::launch_pdl(nvfp4::dn_scan_kernel, dim3(nv * (PF_DK / SCAN_ROWS)),
-                                 dim3(SCAN_WARPS * 32), nvfp4::scan_padding(nv * (PF_DK / SCAN_ROWS)), st,
-                                 (const float*)qn, (const float*)kn, (const nvfp4::DnBlock*)blocks,
-                                 (const __half*)conv_out, conv_dim, (float*)state, o16, nk, nv,
-                                 n) == cudaSuccess;
+    __half* o16;
+    if (nvfp4::dn_chunk_takes(n, nv)) {
+        void* blocks = w + off;
+        o16 = (__half*)(w + off + nvfp4::dn_chunk_work_bytes(n, nk, nv));
+        ok = ok && nvfp4::dn_chunk_launch(conv_out, conv_dim, xh, ld, (const __half*)A_log, (const __half*)dt_bias,
+                                          (float*)state, blocks, o16, n, nk, nv, st) == cudaSuccess;
+    } else {
+        float* qn = (float*)(w + off);
+        const int nb = (n + DNB - 1) / DNB;
+        float* kn = qn + (size_t)nb * DNB * nk * PF_DK;
+        off += 2LL * nb * DNB * nk * PF_DK * 4;
+        nvfp4::DnBlock* blocks = (nvfp4::DnBlock*)(w + off);
+        off = (off + (long long)nb * nv * (long long)sizeof(nvfp4::DnBlock) + 255) & ~255LL;
+        o16 = (__half*)(w + off);
+        ok = ok && nvfp4::launch_pdl(nvfp4::dn_block_kernel, dim3((nk + 3) / 4, nb), dim3(128), 0,
+                                     st, (const __half*)conv_out, conv_dim, xh, ld,
+                                     (const __half*)A_log, (const __half*)dt_bias, qn, kn, blocks, nk,
+                                     nv, n) == cudaSuccess;
+        ok = ok && nvfp4::launch_pdl(nvfp4::dn_scan_kernel, dim3(nv * (PF_DK / SCAN_ROWS)),
+                                     dim3(SCAN_WARPS * 32), nvfp4::scan_padding(nv * (PF_DK / SCAN_ROWS)), st,
+                                     (const float*)qn, (const float*)kn, (const nvfp4::DnBlock*)blocks,
+                                     (const __half*)conv_out, conv_dim, (float*)state, o16, nk, nv,
+                                     n) == cudaSuccess;
+    }
     ok = ok && nvfp4::launch_pdl(nvfp4::dn_post_kernel,
                                  dim3((unsigned)max((nv * n + 7) / 8, (conv_dim + 255) / 256)), dim3(256), 0, st,
                                  (const __half*)o16, xh, ld, conv_dim, (const __half*)norm_w,
