@@ -20,6 +20,7 @@
 // block's update is summed on its own before it meets the state, so the state is rounded once per block.
 #include <cstddef>
 
+#include "common.cuh"
 #include "dn_chunk.cuh"
 
 #define DC 128              // dims of a head (keys and values)
