@@ -368,7 +368,8 @@ int launch_nvfp4_decode_rows(const void* packed, const void* scales, const void*
  * rule with fp32 accumulation.  K % 256 == 0; weight pointers and activation 16-byte aligned.  The
  * first call on a device allocates a workspace (do it outside stream capture).  0; -2 shape or
  * pointer not taken; -3 no tensor-map encoder / no memory; else the launch's cudaError_t.
- * nvfp4_gemv_tc_status: 0, or 1 + id of the first bounded wait in that kernel that ran out. */
+ * nvfp4_gemv_tc_status: 0, or 1 + id of the first bounded wait in that kernel that ran out (20 + for the
+ *   kernel of two activations, which launch_nvfp4_gemv2 and gemv2i hand matrices of 10 M elements to). */
 int launch_nvfp4_gemv_tc(const uint8_t* weight_packed, const uint8_t* weight_scales,
                          const void* activation, void* output, int M, int K, void* stream);
 /* The same with the neighbours of launch_nvfp4_gemv_fused: prologue 1 = RMSNorm of the activation

@@ -395,6 +395,7 @@ static int few_clusters(int dev, int split) {
     const int wider = few_clusters_one_per_sm(dev, (split + 1) / 2);
     return twice > wider ? twice : wider;
 }
+int gemm_few_clusters(int dev, int split) { return few_clusters(dev, split); }
 
 template <int BN, bool IN_TM>
 static cudaError_t few_launch(const CUtensorMap& wm, const CUtensorMap& sm, const CUtensorMap& am, __half* out,

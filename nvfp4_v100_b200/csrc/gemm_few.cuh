@@ -22,4 +22,7 @@ int gemm_few_launch(const uint8_t* packed, const uint8_t* scales, const __half* 
 // 0 or 1 + the id of the first bounded wait that ran out.  Synchronises the device.
 int gemm_few_status(int reset);
 
+// Clusters of `split` CTAs (1 to 8) that run at once with two CTAs per SM.
+int gemm_few_clusters(int dev, int split);
+
 }  // namespace nvfp4

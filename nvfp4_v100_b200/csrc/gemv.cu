@@ -24,6 +24,7 @@
 #include "common.cuh"
 #include "comm_layout.cuh"
 #include "gemv_stream.cuh"
+#include "gemv_tc2.cuh"
 
 namespace nvfp4 {
 
@@ -895,6 +896,14 @@ int gemv_dispatch(const void* packed, const void* scales, const void* a0, const 
             return NVFP4_ERR_LAUNCH;
         }
     }
+    if (fast && nact == 2 && !old_kernel_tuned() && aligned(scales, 16)) {
+        const int rc = gemv_tc2_launch((const uint8_t*)packed, (const uint8_t*)scales, a0, a1, false, out, M, K, st);
+        if (rc == 0) return NVFP4_OK;
+        if (rc != NVFP4_ERR_SHAPE && rc != -3) {
+            fprintf(stderr, "%s (tensor-core kernel): error %d\n", who, rc);
+            return NVFP4_ERR_LAUNCH;
+        }
+    }
     if (fast && nact == 1 && !old_kernel_tuned() && aligned(scales, 16) &&
         plan_stream(M, K, GS_PRO_NONE, GS_EPI_STORE, &sp)) {
         e = launch_stream(packed, scales, a0, out, M, K, GS_PRO_NONE, nullptr, 0.0f, GS_EPI_STORE,
@@ -942,6 +951,14 @@ int gemv2i_dispatch(const void* packed, const void* scales, const void* act_i, v
     cudaError_t e;
     const bool fast = !g_cfg.force_generic && (K % 128 == 0) && aligned(packed, 32) &&
                       aligned(scales, 8) && K * 4 <= 200 * 1024;
+    if (fast && !old_kernel_tuned() && aligned(scales, 16)) {
+        const int rc = gemv_tc2_launch((const uint8_t*)packed, (const uint8_t*)scales, act_i, act_i, true, out, M, K, st);
+        if (rc == 0) return NVFP4_OK;
+        if (rc != NVFP4_ERR_SHAPE && rc != -3) {
+            fprintf(stderr, "launch_nvfp4_gemv2i (tensor-core kernel): error %d\n", rc);
+            return NVFP4_ERR_LAUNCH;
+        }
+    }
     if (fast) {
         GemvPlan plan = plan_gemv(M, K);
         GemvExtra none = {};
