@@ -27,6 +27,32 @@ __device__ __forceinline__ void gemm_dequant32(const uint4 p, uint32_t sc2, uint
     }
 }
 
+// Eight rows of one token to (or into) memory; `rows` of them exist, `vec`: p is 16-byte aligned.
+__device__ __forceinline__ void gemm_store_rows8(const uint4 val, __half* p, bool vec, int rows, bool add) {
+    const __half2* h2 = reinterpret_cast<const __half2*>(&val);
+    if (vec && rows >= 8) {
+        uint4 o = val;
+        if (add) {
+            const uint4 old = *reinterpret_cast<const uint4*>(p);
+            const __half2* r2 = reinterpret_cast<const __half2*>(&old);
+            __half2* o2 = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const float2 a = __half22float2(h2[e]), b = __half22float2(r2[e]);
+                o2[e] = __floats2half2_rn(a.x + b.x, a.y + b.y);
+            }
+        }
+        *reinterpret_cast<uint4*>(p) = o;
+    } else {
+        const __half* h1 = reinterpret_cast<const __half*>(&val);
+        for (int e = 0; e < 8 && e < rows; e++) {
+            __half r = h1[e];
+            if (add) r = __float2half(__half2float(r) + __half2float(p[e]));
+            p[e] = r;
+        }
+    }
+}
+
 // Epilogue store of one 32-token block of a thread's row (v = 32 fp32 accumulator values), in the
 // layout out_mode asks for.  m = this thread's row, mbase = first row of its 128-row tile,
 // nb = first token of the block.  `piece` counts the token-major staging pieces of this column
@@ -56,28 +82,7 @@ __device__ __forceinline__ void gemm_store_block(const uint32_t (&v)[32], __half
             if (tg >= n_out || mg >= M) continue;
             const uint4 val = *reinterpret_cast<const uint4*>(stg + tok * 128 + part * 8);
             __half* p = out + (size_t)tg * (size_t)ld_out + mg;
-            const __half2* h2 = reinterpret_cast<const __half2*>(&val);
-            if (vec && mg + 8 <= M) {
-                uint4 o = val;
-                if (out_mode == GEMM_OUT_TM_ADD) {
-                    const uint4 old = *reinterpret_cast<const uint4*>(p);
-                    const __half2* r2 = reinterpret_cast<const __half2*>(&old);
-                    __half2* o2 = reinterpret_cast<__half2*>(&o);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const float2 a = __half22float2(h2[e]), b = __half22float2(r2[e]);
-                        o2[e] = __floats2half2_rn(a.x + b.x, a.y + b.y);
-                    }
-                }
-                *reinterpret_cast<uint4*>(p) = o;
-            } else {
-                const __half* h1 = reinterpret_cast<const __half*>(&val);
-                for (int e = 0; e < 8 && mg + e < M; e++) {
-                    __half r = h1[e];
-                    if (out_mode == GEMM_OUT_TM_ADD) r = __float2half(__half2float(r) + __half2float(p[e]));
-                    p[e] = r;
-                }
-            }
+            gemm_store_rows8(val, p, vec, M - mg, out_mode == GEMM_OUT_TM_ADD);
         }
         piece++;
     } else if (m < M && nb < N) {
