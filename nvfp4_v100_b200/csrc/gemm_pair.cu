@@ -54,8 +54,7 @@ constexpr int GP_NS = 4, GP_NU = 4;
 constexpr int GP_B_HALF = 16384;                   // room for 128 tokens x 64 k
 constexpr int GP_B_BYTES = 2 * GP_B_HALF;
 constexpr int GP_E_BYTES = 16 * GP_BM * 2;         // staging of an output piece: 16 tokens x 128 rows
-constexpr int GP_SMEM = GP_NU * GP_B_BYTES + GP_NS * (GP_W_BYTES + GP_S_BYTES) + 4 * GP_E_BYTES + 1024;
-constexpr int GP_SMEM_ONE = GP_SMEM - 4 * GP_E_BYTES;
+constexpr int GP_SMEM = GP_NU * GP_B_BYTES + GP_NS * (GP_W_BYTES + GP_S_BYTES) + 1024;
 constexpr int GP_COLS = 8;                         // column tiles that take turns over the same weight rows
 constexpr uint32_t GP_SPIN_LIMIT = 1u << 24;
 constexpr uint32_t GP_PARKED_LIMIT = 100000;       // x 20 us
@@ -154,7 +153,7 @@ gemm_w4a16_pair_tm_kernel(const __grid_constant__ CUtensorMap w_map, const __gri
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gp_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* smem_w = smem + GP_NU * GP_B_BYTES;
     uint8_t* smem_s = smem_w + GP_NS * GP_W_BYTES;
-    uint8_t* smem_e = smem_s + GP_NS * GP_S_BYTES;
+    __shared__ __align__(16) uint8_t smem_e[ONE ? 16 : 4 * GP_E_BYTES];
     __shared__ __align__(8) uint64_t bar_full[GP_NS];    // weight stage landed
     __shared__ __align__(8) uint64_t bar_empty[GP_NS];   // all 8 dequantising warps have read it
     __shared__ __align__(8) uint64_t bar_ready[GP_NU];   // first CTA: both CTAs' A in tensor memory, both halves of B
@@ -443,19 +442,18 @@ bool gemm_pair_beats_tiles(int M, int N, int K, int out_mode) {
 template <bool IN_TM, bool ONE>
 static cudaError_t gp_launch(const CUtensorMap& wm, const CUtensorMap& sm, const CUtensorMap& am, __half* out, int M,
                              int N, int K, int ld_out, int out_mode, int n_out, int bn, int pairs, cudaStream_t st) {
-    constexpr int SMEM = ONE ? GP_SMEM_ONE : GP_SMEM;
     static bool opted[NVFP4_MAX_DEVICES] = {false};
     const int dev = current_device_index();
     if (!opted[dev]) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_w4a16_pair_tm_kernel<IN_TM, ONE>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM);
         if (e != cudaSuccess) return e;
         opted[dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
     cfg.blockDim = dim3(ONE ? GP_THREADS_ONE : GP_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = SMEM;
+    cfg.dynamicSmemBytes = GP_SMEM;
     cfg.stream = st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
