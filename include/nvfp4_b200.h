@@ -92,6 +92,13 @@ int launch_nvfp4_gemmtc_v5(const uint8_t* d_weight_packed, const uint8_t* d_weig
 int launch_nvfp4_gemm_w4a16_ex(const uint8_t* d_weight_packed, const uint8_t* d_weight_scales,
                                const void* act, long long ld_act, void* out, long long ld_out, int M,
                                int n_tokens, int K, int flags, void* stream);
+/* Gate and up projection of a chunk with the activation between them and the down projection: W [M][K] with gate and
+ * up rows interleaved in groups of 8 (M % 16 == 0), act token-major [n_tokens][ld_act], out [M / 2][N], N = n_tokens
+ * rounded up to 8: what launch_nvfp4_gemm_w4a16_ex (flags 1) into gu [M][N] and launch_silu_mul_rows give, bit for
+ * bit, in one launch where the shape allows it (gu is then left as it is).  gu and out must not overlap.  Return
+ * values of those two. */
+int launch_nvfp4_gemm_silu(const uint8_t* d_weight_packed, const uint8_t* d_weight_scales, const void* act,
+                           long long ld_act, void* gu, void* out, int M, int n_tokens, int K, void* stream);
 int get_kernel_shared_mem_bytes(void);                          /* kernels/nvfp4_cuda_v5.cu:460-464 */
 /* 0 if no bounded wait inside the tensor-core GEMM ever ran out; 1 + wait id otherwise.  reset != 0
  * clears it.  Synchronous.  No counterpart in the reference. */

@@ -69,6 +69,7 @@ __device__ __forceinline__ uint4 ld_stream_u4(const void* p) {
 }
 
 __device__ __forceinline__ float round_f16(float x) { return __half2float(__float2half(x)); }
+__device__ __forceinline__ float silu_pf(float x) { return x / (1.0f + expf(-x)); }
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

@@ -128,6 +128,28 @@ __device__ __forceinline__ void gp_store_piece(const uint32_t (&h)[8], __half* o
         }
         return;
     }
+    if (out_mode == GEMM_OUT_FM_SILU) {
+        // Rows in groups of eight gate rows and their eight up rows: the lane with a gate row takes tokens 0..7
+        // and the one eight lanes on tokens 8..15.  The fp16 values and roundings are those of a separate pass
+        // (silu_mul_rows_kernel), which took 15 us for 34816 rows of 512 tokens; here they run under the next
+        // tile's MMAs.
+        const bool up = rr & 8;
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? h[j] : h[4 + j], 8);
+            const uint32_t gw = up ? got : h[j], uw = up ? h[4 + j] : got;
+            const float2 gf = __half22float2(*reinterpret_cast<const __half2*>(&gw));
+            const float2 uf = __half22float2(*reinterpret_cast<const __half2*>(&uw));
+            const __half2 r = __floats2half2_rn(round_f16(silu_pf(gf.x)) * uf.x, round_f16(silu_pf(gf.y)) * uf.y);
+            o[j] = *reinterpret_cast<const uint32_t*>(&r);
+        }
+        const int m = m0 + rr, t = nb + (up ? 8 : 0);
+        if (m < M && t < N)
+            *reinterpret_cast<uint4*>(out + (size_t)(m / 16 * 8 + (m & 7)) * (size_t)N + t) =
+                make_uint4(o[0], o[1], o[2], o[3]);
+        return;
+    }
     // A thread holds one row's tokens, memory wants one token's rows together: turned over in shared memory.  Two
     // pieces alternate, so the one barrier per piece also orders its writes after the reads of the last but one.
 #pragma unroll
@@ -466,6 +488,19 @@ static cudaError_t gp_launch(const CUtensorMap& wm, const CUtensorMap& sm, const
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, gemm_w4a16_pair_tm_kernel<IN_TM, ONE>, wm, sm, am, out, M, N, K, ld_out, out_mode,
                               n_out, bn, (M + 2 * GP_BM - 1) / (2 * GP_BM), (N + bn - 1) / bn);
+}
+
+// The activation in the epilogue makes a tile's stores longer (9.5 us per 256 tokens against 3.7), which costs nothing
+// while they run under the next tile's MMAs and pays for itself against a pass of its own.  34816 x K, GEMM and pass /
+// fused, us: K = 5120 at 136 / 512 / 2048 tokens 53 / 126 / 475 and 53 / 117 / 427; K = 1024 at 512 42 and 45.
+bool gemm_pair_fuses_silu(int M, int N, int K) {
+    const int dev = current_device_index();
+    const long long bn = gp_tile_tokens(dev, M, N), tiles = (long long)((M + 255) / 256) * ((N + bn - 1) / bn);
+    const long long per_pair = (tiles + gp_slots(dev) - 1) / gp_slots(dev);
+    if (per_pair < 2) return false;                          // (no output warps)
+    const long long mma = 5LL * K * bn / 256, plain = 3700 * bn / 256, silu = 9500 * bn / 256;   // ns
+    const long long pass = 500 + (long long)M * N * 3 / 4400;
+    return (per_pair - 1) * (mma > silu ? mma : silu) + silu < (per_pair - 1) * (mma > plain ? mma : plain) + plain + pass;
 }
 
 bool gemm_pair_takes(const uint8_t* packed, const uint8_t* scales, int N, int K) {

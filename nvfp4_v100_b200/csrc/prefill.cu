@@ -26,7 +26,6 @@
 
 namespace nvfp4 {
 
-__device__ __forceinline__ float silu_pf(float x) { return x / (1.0f + expf(-x)); }
 __device__ __forceinline__ float softplus_pf(float x) { return (x > 20.0f) ? x : log1pf(expf(x)); }
 
 // dst[c][r] = src[r][c] for r < R, c < C; dst rows are ld_dst long and columns R .. ld_dst-1 are

@@ -804,17 +804,17 @@ class DecodeEngine:
                     ok(lib.launch_add_transposed(ptr(B["h"]), ptr(B["dT"]), Np, n, H, st), "add")
                 rmsnorm(L.post_w1, n)
                 if self.prefill_token_major:
-                    # gate/up leaves [2 inter][tokens] for the row-wise silu-mul; the down
-                    # projection reads that layout and adds into the token-major residual
-                    gemm_ex(L.w_gu, B["xn"], H, B["yT"], Np, n, 1)
+                    # silu(gate) * up leaves as [inter][tokens]; the down projection reads that
+                    # layout and adds into the token-major residual
+                    ok(lib.launch_nvfp4_gemm_silu(
+                        ptr(L.w_gu.packed), ptr(L.w_gu.scales), ptr(B["xn"]), H, ptr(B["yT"]),
+                        ptr(B["actT"]), L.w_gu.M, n, L.w_gu.K, st), "launch_nvfp4_gemm_silu")
+                    residual_gemm(L.w_down, B["actT"], Np, 0, n)
                 else:
                     to_gemm(B["xn"], n, H, Np)
                     gemm(L.w_gu, B["xT"], B["yT"], Np)
-                ok(lib.launch_silu_mul_rows(ptr(B["yT"]), ptr(B["actT"]), self.inter_l, Np, st),
-                   "launch_silu_mul_rows")
-                if self.prefill_token_major:
-                    residual_gemm(L.w_down, B["actT"], Np, 0, n)
-                else:
+                    ok(lib.launch_silu_mul_rows(ptr(B["yT"]), ptr(B["actT"]), self.inter_l, Np, st),
+                       "launch_silu_mul_rows")
                     gemm(L.w_down, B["actT"], B["dT"], Np)
                     if self.world > 1:
                         dist.all_reduce(B["dT"][:H * Np])
