@@ -156,13 +156,22 @@ __device__ __forceinline__ void gp_store_piece(const uint32_t (&h)[8], __half* o
     for (int j = 0; j < 16; j++) stg[j * GP_BM + rr] = __ushort_as_half((unsigned short)(h[j >> 1] >> (16 * (j & 1))));
     asm volatile("bar.sync %0, 128;\n" ::"r"(bar) : "memory");
     const bool vec = ((ld_out & 7) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
+    uint4 old[2] = {};
+    if (out_mode == GEMM_OUT_TM_ADD && vec) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int tg = nb + ((i * 128 + rr) >> 4), mg = m0 + (rr & 15) * 8;
+            if (tg < n_out && mg + 8 <= M)
+                old[i] = *reinterpret_cast<const uint4*>(out + (size_t)tg * (size_t)ld_out + mg);
+        }
+    }
 #pragma unroll
     for (int i = 0; i < 2; i++) {
         const int pid = i * 128 + rr, tok = pid >> 4, part = pid & 15;
         const int tg = nb + tok, mg = m0 + part * 8;
         if (tg < n_out && mg < M)
             gemm_store_rows8(*reinterpret_cast<const uint4*>(stg + tok * GP_BM + part * 8),
-                             out + (size_t)tg * (size_t)ld_out + mg, vec, M - mg, out_mode == GEMM_OUT_TM_ADD);
+                             out + (size_t)tg * (size_t)ld_out + mg, vec, M - mg, out_mode == GEMM_OUT_TM_ADD, old[i]);
     }
 }
 
@@ -446,13 +455,13 @@ static int gp_tile_tokens(int dev, int M, int N) {
 // MMAs of the next, so what is left for the tiles is K so short that the stores take longer than the MMAs and
 // there are too few tiles a pair to spread them.  4096 x K at 2048 tokens, token-major / added into the output /
 // feature-major, us:
-//   K =  256   tiles 14.5 / 19.6 / 12.2, pairs 14.6 / 26.2 / 12.6
-//   K = 1024   tiles 22.7 / 28.2 / 20.3, pairs 20.1 / 31.5 / 19.1
-//   K = 2048   tiles 34.1 / 39.5 / 32.4, pairs 29.5 / 37.4 / 28.6
+//   K =  256   tiles 14.6 / 15.9 / 12.2, pairs 15.0 / 21.3 / 13.1
+//   K = 1024   tiles 23.4 / 24.3 / 20.6, pairs 20.9 / 26.7 / 19.6
+//   K = 2048   tiles 34.6 / 36.1 / 32.7, pairs 30.1 / 33.6 / 29.2
 bool gemm_pair_beats_tiles(int M, int N, int K, int out_mode) {
     const int dev = current_device_index();
     const long long slots = gp_slots(dev), rows = (M + 255) / 256, bn = gp_tile_tokens(dev, M, N);
-    static const int tile_fixed[3] = {9500, 11800, 17000}, store[3] = {3700, 4600, 10800};   // by out_mode; 256 tokens
+    static const int tile_fixed[3] = {9500, 11800, 13000}, store[3] = {3900, 4800, 8500};   // by out_mode; 256 tokens
     const long long tile_rounds = (rows * ((N + 255) / 256) + 2 * slots - 1) / (2 * slots);
     const long long per_pair = (rows * ((N + bn - 1) / bn) + slots - 1) / slots;
     const long long mma = 5LL * K * bn / 256, out = store[out_mode] * bn / 256;
@@ -490,7 +499,7 @@ static cudaError_t gp_launch(const CUtensorMap& wm, const CUtensorMap& sm, const
                               n_out, bn, (M + 2 * GP_BM - 1) / (2 * GP_BM), (N + bn - 1) / bn);
 }
 
-// The activation in the epilogue makes a tile's stores longer (9.5 us per 256 tokens against 3.7), which costs nothing
+// The activation in the epilogue makes a tile's stores longer (9.5 us per 256 tokens against 3.9), which costs nothing
 // while they run under the next tile's MMAs and pays for itself against a pass of its own.  34816 x K, GEMM and pass /
 // fused, us: K = 5120 at 136 / 512 / 2048 tokens 53 / 126 / 475 and 53 / 117 / 427; K = 1024 at 512 42 and 45.
 bool gemm_pair_fuses_silu(int M, int N, int K) {
@@ -498,7 +507,7 @@ bool gemm_pair_fuses_silu(int M, int N, int K) {
     const long long bn = gp_tile_tokens(dev, M, N), tiles = (long long)((M + 255) / 256) * ((N + bn - 1) / bn);
     const long long per_pair = (tiles + gp_slots(dev) - 1) / gp_slots(dev);
     if (per_pair < 2) return false;                          // (no output warps)
-    const long long mma = 5LL * K * bn / 256, plain = 3700 * bn / 256, silu = 9500 * bn / 256;   // ns
+    const long long mma = 5LL * K * bn / 256, plain = 3900 * bn / 256, silu = 9500 * bn / 256;   // ns
     const long long pass = 500 + (long long)M * N * 3 / 4400;
     return (per_pair - 1) * (mma > silu ? mma : silu) + silu < (per_pair - 1) * (mma > plain ? mma : plain) + plain + pass;
 }

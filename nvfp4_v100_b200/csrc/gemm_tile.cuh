@@ -28,13 +28,14 @@ __device__ __forceinline__ void gemm_dequant32(const uint4 p, uint32_t sc2, uint
     }
 }
 
-// Eight rows of one token to (or into) memory; `rows` of them exist, `vec`: p is 16-byte aligned.
-__device__ __forceinline__ void gemm_store_rows8(const uint4 val, __half* p, bool vec, int rows, bool add) {
+// Eight rows of one token to (or into) memory; `rows` of them exist, `vec`: p is 16-byte aligned.  `old`: what is
+// there, if vec and all eight rows.  The caller reads it for all its pieces at once: read here, each read waited
+// for the store before it (5120 x 6144 at 512 tokens added into the output 33.0 us, now 30.6; stored 29.4).
+__device__ __forceinline__ void gemm_store_rows8(const uint4 val, __half* p, bool vec, int rows, bool add, const uint4 old) {
     const __half2* h2 = reinterpret_cast<const __half2*>(&val);
     if (vec && rows >= 8) {
         uint4 o = val;
         if (add) {
-            const uint4 old = *reinterpret_cast<const uint4*>(p);
             const __half2* r2 = reinterpret_cast<const __half2*>(&old);
             __half2* o2 = reinterpret_cast<__half2*>(&o);
 #pragma unroll
@@ -76,6 +77,15 @@ __device__ __forceinline__ void gemm_store_block(const uint32_t (&v)[32], __half
         for (int j = 0; j < 32; j++) stg[j * 128 + rr] = __float2half(__uint_as_float(v[j]));
         asm volatile("bar.sync %0, 128;\n" ::"r"(1 + chalf) : "memory");
         const bool vec = ((ld_out & 7) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
+        uint4 old[4] = {};
+        if (out_mode == GEMM_OUT_TM_ADD && vec) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int tg = nb + ((i * 128 + rr) >> 4), mg = mbase + (rr & 15) * 8;
+                if (tg < n_out && mg + 8 <= M)
+                    old[i] = *reinterpret_cast<const uint4*>(out + (size_t)tg * (size_t)ld_out + mg);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int pid = i * 128 + rr, tok = pid >> 4, part = pid & 15;
@@ -83,7 +93,7 @@ __device__ __forceinline__ void gemm_store_block(const uint32_t (&v)[32], __half
             if (tg >= n_out || mg >= M) continue;
             const uint4 val = *reinterpret_cast<const uint4*>(stg + tok * 128 + part * 8);
             __half* p = out + (size_t)tg * (size_t)ld_out + mg;
-            gemm_store_rows8(val, p, vec, M - mg, out_mode == GEMM_OUT_TM_ADD);
+            gemm_store_rows8(val, p, vec, M - mg, out_mode == GEMM_OUT_TM_ADD, old[i]);
         }
         piece++;
     } else if (m < M && nb < N) {
