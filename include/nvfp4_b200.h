@@ -92,11 +92,11 @@ int launch_nvfp4_gemmtc_v5(const uint8_t* d_weight_packed, const uint8_t* d_weig
 int launch_nvfp4_gemm_w4a16_ex(const uint8_t* d_weight_packed, const uint8_t* d_weight_scales,
                                const void* act, long long ld_act, void* out, long long ld_out, int M,
                                int n_tokens, int K, int flags, void* stream);
-/* Gate and up projection of a chunk with the activation between them and the down projection: W [M][K] with gate and
- * up rows interleaved in groups of 8 (M % 16 == 0), act token-major [n_tokens][ld_act], out [M / 2][N], N = n_tokens
- * rounded up to 8: what launch_nvfp4_gemm_w4a16_ex (flags 1) into gu [M][N] and launch_silu_mul_rows give, bit for
- * bit, in one launch where the shape allows it (gu is then left as it is).  gu and out must not overlap.  Return
- * values of those two. */
+/* Gate and up projection of a chunk with the activation between them and the down projection, all token-major: W
+ * [M][K] with gate and up rows interleaved in groups of 8 (M % 16 == 0), act [n_tokens][ld_act], out
+ * [n_tokens][M / 2]: what launch_nvfp4_gemm_w4a16_ex (flags 3) into gu [n_tokens][M] and launch_silu_mul_tokens give,
+ * bit for bit, in one launch where that is faster (gu is then left as it is).  gu and out 16-byte aligned, not
+ * overlapping.  Return values of those two. */
 int launch_nvfp4_gemm_silu(const uint8_t* d_weight_packed, const uint8_t* d_weight_scales, const void* act,
                            long long ld_act, void* gu, void* out, int M, int n_tokens, int K, void* stream);
 int get_kernel_shared_mem_bytes(void);                          /* kernels/nvfp4_cuda_v5.cu:460-464 */
@@ -318,6 +318,7 @@ int launch_allreduce_residual(void* h, const void* const* bufs, int rank, int wo
  *   launch_add_transposed  h[t][c] += dT[c][t] (fp32 add, one rounding): residual add from a GEMM output
  *   launch_embed_rows      out[t][:] = table[ids[t]], ids device int64 [n]
  *   launch_silu_mul_rows   gu token-minor [2*inter][N], gate/up rows interleaved by 8 -> act [inter][N]
+ *   launch_silu_mul_tokens the same token-major: gu [n][2*inter] -> act [n][inter], 16-byte aligned
  *   launch_attn_prep_tokens  launch_attn_prep for the n_tokens rows of a chunk starting at position
  *                          pos0 (host int); qkv token-major, ld halves per row; q_out/gate_out
  *                          token-major [n_tokens][hq*256]; token i writes cache row pos0 + i
@@ -336,6 +337,7 @@ int launch_add_transposed(void* h, const void* dT, long long ldT, int n, int C, 
 int launch_embed_rows(const void* table, const void* ids, void* out, int n, int hidden,
                       long long vocab, void* stream);
 int launch_silu_mul_rows(const void* gu, void* act, int inter, int N, void* stream);
+int launch_silu_mul_tokens(const void* gu, void* act, int inter, int n, void* stream);
 int launch_attn_prep_tokens(const void* qkv, long long ld, const void* q_w1, const void* k_w1,
                             const void* cos_tab, const void* sin_tab, int pos0, int n_tokens,
                             void* q_out, void* gate_out, void* keys, void* values, int hq, int hkv,

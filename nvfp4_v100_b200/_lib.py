@@ -78,6 +78,7 @@ SIGNATURES = {
     "launch_add_transposed": ([_vp, _vp, _ll, _i, _i, _vp], _i),
     "launch_embed_rows": ([_vp, _vp, _vp, _i, _i, _ll, _vp], _i),
     "launch_silu_mul_rows": ([_vp, _vp, _i, _i, _vp], _i),
+    "launch_silu_mul_tokens": ([_vp, _vp, _i, _i, _vp], _i),
     "launch_attn_prep_tokens": ([_vp, _ll] + [_vp] * 4 + [_i, _i] + [_vp] * 4 + [_i, _i, _i, _f, _vp], _i),
     "launch_attn_prefill": ([_vp, _vp, _vp, _i, _i, _vp, _vp, _i, _i, _i, _f, _vp], _i),
     "nvfp4_dn_prefill_work_bytes": ([_i, _i, _i], _ll),

@@ -735,23 +735,24 @@ int launch_nvfp4_gemm_w4a16_ex(const uint8_t* d_weight_packed, const uint8_t* d_
     return (e == cudaSuccess) ? 0 : (int)e;
 }
 
-// Gate and up projection with silu(gate) * up: W rows interleaved by 8 as launch_silu_mul_rows takes them, token-major
-// activations, out[M / 2][N8] feature-major.  Fused where the pair GEMM goes from tile to tile and its output warps
-// have the time (gemm_pair_fuses_silu); elsewhere the GEMM into `gu` and a pass over it, with the same bits.
+// Gate and up projection with silu(gate) * up: W rows interleaved by 8 (launch_silu_mul_tokens), everything
+// token-major.  Fused where the pair GEMM goes from tile to tile and its output warps have the time
+// (gemm_pair_fuses_silu); elsewhere the GEMM into `gu` and a pass over it, with the same bits.
 int launch_nvfp4_gemm_silu(const uint8_t* d_weight_packed, const uint8_t* d_weight_scales, const void* act,
                            long long ld_act, void* gu, void* out, int M, int n_tokens, int K, void* stream) {
     using namespace nvfp4;
-    if (M <= 0 || M % 16 != 0 || n_tokens <= 0 || K <= 0 || !d_weight_packed || !d_weight_scales || !act || !gu || !out)
+    if (M <= 0 || M % 16 != 0 || n_tokens <= 0 || K <= 0 || !d_weight_packed || !d_weight_scales || !act || !gu ||
+        !out || (((uintptr_t)gu | (uintptr_t)out) & 15) != 0)
         return NVFP4_ERR_SHAPE;
-    const int N8 = (n_tokens + 7) / 8 * 8;
-    if (ld_act % 8 == 0 && ld_act >= K && ld_act <= 0x7fffffffLL && (((uintptr_t)act | (uintptr_t)out) & 15) == 0 &&
-        gemm_use_pair_tm(d_weight_packed, d_weight_scales, M, N8, K, GEMM_OUT_FM) && gemm_pair_fuses_silu(M, N8, K))
+    if (ld_act % 8 == 0 && ld_act >= K && ld_act <= 0x7fffffffLL && ((uintptr_t)act & 15) == 0 &&
+        gemm_use_pair_tm(d_weight_packed, d_weight_scales, M, n_tokens, K, GEMM_OUT_TM) &&
+        gemm_pair_fuses_silu(M, n_tokens, K))
         return gemm_pair_launch(d_weight_packed, d_weight_scales, static_cast<const __half*>(act), ld_act, true,
-                                static_cast<__half*>(out), N8, M, N8, n_tokens, K, GEMM_OUT_FM_SILU,
+                                static_cast<__half*>(out), M / 2, M, n_tokens, n_tokens, K, GEMM_OUT_TM_SILU,
                                 (cudaStream_t)stream);
-    const int rc = launch_nvfp4_gemm_w4a16_ex(d_weight_packed, d_weight_scales, act, ld_act, gu, N8, M, n_tokens, K, 1,
+    const int rc = launch_nvfp4_gemm_w4a16_ex(d_weight_packed, d_weight_scales, act, ld_act, gu, M, M, n_tokens, K, 3,
                                               stream);
-    return rc != 0 ? rc : launch_silu_mul_rows(gu, out, M / 2, N8, stream);
+    return rc != 0 ? rc : launch_silu_mul_tokens(gu, out, M / 2, n_tokens, stream);
 }
 
 // W4A4 product with the reference format on both sides: out[M, N] = dequant(W) .

@@ -128,26 +128,27 @@ __device__ __forceinline__ void gp_store_piece(const uint32_t (&h)[8], __half* o
         }
         return;
     }
-    if (out_mode == GEMM_OUT_FM_SILU) {
-        // Rows in groups of eight gate rows and their eight up rows: the lane with a gate row takes tokens 0..7
-        // and the one eight lanes on tokens 8..15.  The fp16 values and roundings are those of a separate pass
-        // (silu_mul_rows_kernel), which took 15 us for 34816 rows of 512 tokens; here they run under the next
-        // tile's MMAs.
-        const bool up = rr & 8;
-        uint32_t o[4];
+    if (out_mode == GEMM_OUT_TM_SILU) {
+        // Rows in groups of eight gate rows and their eight up rows: the lane with a gate row takes the even pairs
+        // of tokens and the one eight lanes on the odd ones.  The fp16 values and roundings are those of a pass of
+        // its own (silu_mul_tokens_kernel), which took 13 us for 34816 rows of 512 tokens; here they run under
+        // the next tile's MMAs.  64 results a token, in rows of 72 halves (no bank conflicts).
+        const int up = (rr >> 3) & 1, row = rr / 16 * 8 + (rr & 7);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? h[j] : h[4 + j], 8);
-            const uint32_t gw = up ? got : h[j], uw = up ? h[4 + j] : got;
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? h[2 * j] : h[2 * j + 1], 8);
+            const uint32_t gw = up ? got : h[2 * j], uw = up ? h[2 * j + 1] : got;
             const float2 gf = __half22float2(*reinterpret_cast<const __half2*>(&gw));
             const float2 uf = __half22float2(*reinterpret_cast<const __half2*>(&uw));
-            const __half2 r = __floats2half2_rn(round_f16(silu_pf(gf.x)) * uf.x, round_f16(silu_pf(gf.y)) * uf.y);
-            o[j] = *reinterpret_cast<const uint32_t*>(&r);
+            __half* o = stg + (2 * (2 * j + up)) * 72 + row;
+            o[0] = __float2half(round_f16(silu_pf(gf.x)) * uf.x);
+            o[72] = __float2half(round_f16(silu_pf(gf.y)) * uf.y);
         }
-        const int m = m0 + rr, t = nb + (up ? 8 : 0);
-        if (m < M && t < N)
-            *reinterpret_cast<uint4*>(out + (size_t)(m / 16 * 8 + (m & 7)) * (size_t)N + t) =
-                make_uint4(o[0], o[1], o[2], o[3]);
+        asm volatile("bar.sync %0, 128;\n" ::"r"(bar) : "memory");
+        const int tg = nb + (rr >> 3), mg = m0 / 2 + (rr & 7) * 8;
+        if (tg < n_out && mg < M / 2)
+            *reinterpret_cast<uint4*>(out + (size_t)tg * (size_t)ld_out + mg) =
+                *reinterpret_cast<const uint4*>(stg + (rr >> 3) * 72 + (rr & 7) * 8);
         return;
     }
     // A thread holds one row's tokens, memory wants one token's rows together: turned over in shared memory.  Two

@@ -10,7 +10,7 @@ bool gemm_pair_takes(const uint8_t* packed, const uint8_t* scales, int N, int K)
 // Whether it is the faster one where gemm.cu has 256-row tiles for the shape (both give the same bits).
 bool gemm_pair_beats_tiles(int M, int N, int K, int out_mode);
 
-// Whether GEMM_OUT_FM_SILU is possible (more tiles than pairs of SMs) and faster than GEMM_OUT_FM and a pass after it.
+// Whether GEMM_OUT_TM_SILU is possible (more tiles than pairs of SMs) and faster than GEMM_OUT_TM and a pass after it.
 bool gemm_pair_fuses_silu(int M, int N, int K);
 
 // act: token-major [n_tokens][ld_act] (in_tm) or token-minor [K][ld_act]; N = tokens the output holds in

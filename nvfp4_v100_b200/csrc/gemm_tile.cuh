@@ -9,7 +9,7 @@ enum {
     GEMM_OUT_FM = 0,       // out[m][token]
     GEMM_OUT_TM = 1,       // out[token][m]
     GEMM_OUT_TM_ADD = 2,   // out[token][m] += result
-    GEMM_OUT_FM_SILU = 3,  // out[m / 16 * 8 + m % 8][token] = silu(row m) * row m + 8, m % 16 < 8 (gemm_pair.cu only)
+    GEMM_OUT_TM_SILU = 3,  // out[token][m / 16 * 8 + m % 8] = silu(row m) * row m + 8, m % 16 < 8 (gemm_pair.cu only)
 };
 
 // 16 packed bytes (32 weights, two scale blocks) -> 16 words of fp16 pairs, scaled in fp16

@@ -167,6 +167,26 @@ silu_mul_rows_kernel(const __half* __restrict__ gu, __half* __restrict__ act, in
     }
 }
 
+// The same for token-major rows: sixteen neighbours (eight gates, their eight ups) make eight results.
+__global__ void __launch_bounds__(256)
+silu_mul_tokens_kernel(const __half* __restrict__ gu, __half* __restrict__ act, long long pieces) {
+    pdl_prologue();
+    PDL_FRESH(gu); PDL_FRESH(act);
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= pieces) return;
+    const uint4 gv = reinterpret_cast<const uint4*>(gu)[2 * i], uv = reinterpret_cast<const uint4*>(gu)[2 * i + 1];
+    const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
+    uint32_t ow[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 gf = __half22float2(*reinterpret_cast<const __half2*>(&gw[k]));
+        const float2 uf = __half22float2(*reinterpret_cast<const __half2*>(&uw[k]));
+        const __half2 r = __floats2half2_rn(round_f16(silu_pf(gf.x)) * uf.x, round_f16(silu_pf(gf.y)) * uf.y);
+        ow[k] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+    reinterpret_cast<uint4*>(act)[i] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Gated DeltaNet over a chunk.  x: token-major in-projection output, row t =
 // [ mixed (conv_dim = 2 key_dim + nv*128) | z (nv*128) | b (nv) | a (nv) ], ld halves per row.
@@ -708,6 +728,15 @@ int launch_silu_mul_rows(const void* gu, void* act, int inter, int N, void* stre
     const dim3 grid = flat ? dim3((unsigned)((items + 255) / 256)) : dim3((unsigned)((groups + 255) / 256), (unsigned)inter);
     return nvfp4::launch_pdl(kernel, grid, dim3(256), 0, (cudaStream_t)stream, (const __half*)gu, (__half*)act, inter, N,
                              flat) == cudaSuccess ? 0 : -1;
+}
+
+// gu: token-major [n][2 * inter] with gate/up columns interleaved in groups of 8; act: [n][inter].
+int launch_silu_mul_tokens(const void* gu, void* act, int inter, int n, void* stream) {
+    if (!gu || !act || inter <= 0 || inter % 8 != 0 || n <= 0 || (((uintptr_t)gu | (uintptr_t)act) & 15) != 0) return -1;
+    const long long pieces = (long long)inter / 8 * n, blocks = (pieces + 255) / 256;
+    if (blocks > 0x7fffffffLL) return -1;
+    return nvfp4::launch_pdl(nvfp4::silu_mul_tokens_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream,
+                             (const __half*)gu, (__half*)act, pieces) == cudaSuccess ? 0 : -1;
 }
 
 // Bytes of workspace launch_dn_prefill needs for n tokens.

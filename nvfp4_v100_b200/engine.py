@@ -804,12 +804,10 @@ class DecodeEngine:
                     ok(lib.launch_add_transposed(ptr(B["h"]), ptr(B["dT"]), Np, n, H, st), "add")
                 rmsnorm(L.post_w1, n)
                 if self.prefill_token_major:
-                    # silu(gate) * up leaves as [inter][tokens]; the down projection reads that
-                    # layout and adds into the token-major residual
                     ok(lib.launch_nvfp4_gemm_silu(
                         ptr(L.w_gu.packed), ptr(L.w_gu.scales), ptr(B["xn"]), H, ptr(B["yT"]),
                         ptr(B["actT"]), L.w_gu.M, n, L.w_gu.K, st), "launch_nvfp4_gemm_silu")
-                    residual_gemm(L.w_down, B["actT"], Np, 0, n)
+                    residual_gemm(L.w_down, B["actT"], L.w_down.K, 1, n)
                 else:
                     to_gemm(B["xn"], n, H, Np)
                     gemm(L.w_gu, B["xT"], B["yT"], Np)

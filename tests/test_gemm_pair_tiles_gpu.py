@@ -70,7 +70,7 @@ def test_launches_side_by_side(lib):
         assert all(torch.equal(job[-1][0], o) for o in job[-1][1:])
 
 
-# fused: 192, 256 (groups of columns), 160 and 224 tokens a tile, the last rows of a tile missing, padded tokens; in two
+# fused: 192, 256 (groups of columns), 160 and 224 tokens a tile, the last rows of a tile missing; in two
 # launches: short K, one tile a pair, few tokens, K of 64
 @pytest.mark.parametrize("M,n,K", [
     (30000, 190, 4096), (4096, 4400, 2560), (18960, 257, 5120), (2064, 4999, 5120),
@@ -85,15 +85,17 @@ def test_gate_up_with_the_activation(lib, M, n, K, wide):
     s = torch.randint(108, 134 if wide else 122, (M, K // 16), dtype=torch.uint8, device="cuda", generator=g)
     n8 = (n + 7) // 8 * 8
     x = torch.randn((n, K), device="cuda", generator=g).half()
-    gu, spare = (torch.zeros((M, n8), dtype=torch.float16, device="cuda") for _ in range(2))
-    want, got = (torch.full((M // 2 * n8 + 64,), 7.0, dtype=torch.float16, device="cuda") for _ in range(2))
+    gu, rows, spare = (torch.zeros(d, dtype=torch.float16, device="cuda") for d in ((M, n8), (M // 2, n8), (n, M)))
+    got = torch.full((n * M // 2 + 64,), 7.0, dtype=torch.float16, device="cuda")
     lib.nvfp4_b200_gemm_config(1)
     assert lib.launch_nvfp4_gemm_w4a16_ex(ptr(p), ptr(s), ptr(x), K, ptr(gu), n8, M, n, K, 1, stream()) == 0
-    assert lib.launch_silu_mul_rows(ptr(gu), ptr(want), M // 2, n8, stream()) == 0
+    assert lib.launch_silu_mul_rows(ptr(gu), ptr(rows), M // 2, n8, stream()) == 0
     lib.nvfp4_b200_gemm_config(3)
     assert lib.launch_nvfp4_gemm_silu(ptr(p), ptr(s), ptr(x), K, ptr(spare), ptr(got), M, n, K, stream()) == 0
     torch.cuda.synchronize()
     assert lib.nvfp4_gemm_status(0) == 0
     assert (got[-64:] == 7).all()
-    a, b = got[:-64], want[:-64]
+    a, b = got[:-64].view(n, M // 2), rows[:, :n].t()
     assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a[~a.isnan()], b[~b.isnan()])
+    fused = (n, K) in ((190, 4096), (4400, 2560), (257, 5120), (4999, 5120))
+    assert (spare == 0).all().item() == fused
