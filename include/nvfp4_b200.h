@@ -222,6 +222,13 @@ int launch_nvfp4_gemv_fused(const void* weight_packed, const void* weight_scales
                             const void* activation, void* output, int M, int K, int prologue,
                             const void* norm_w1, float eps, int epilogue, const void* residual,
                             void* stream);
+/* The same for calls that follow one another on one stream, like those of a decode step: the tensor-core kernel, whose
+ * workspace belongs to the device, takes matrices from 30 instead of 35 * 2^20 elements
+ * (nvfp4_gemv_tc_wanted_step). */
+int launch_nvfp4_gemv_step(const void* weight_packed, const void* weight_scales,
+                           const void* activation, void* output, int M, int K, int prologue,
+                           const void* norm_w1, float eps, int epilogue, const void* residual,
+                           void* stream);
 
 /* launch_attn_decode_heads with the keys split over several CTAs, each serving one to three query heads
  * of a KV head (no counterpart in the reference): each warp requests its key AND value rows at once,
@@ -414,6 +421,7 @@ void nvfp4_b200_gemv_tc_prefetch(int stages_at_entry);
 void nvfp4_b200_gemv_tc_ctas(int per_sm);
 int nvfp4_gemv_tc_wanted(int M, int K);
 int nvfp4_gemv_tc_wanted_plain(int M, int K);
+int nvfp4_gemv_tc_wanted_step(int M, int K);
 void nvfp4_b200_gemv_tc_config_plain(int min_mega_elements);
 int nvfp4_gemv_tc_prepare(void);
 /* Timing probe of launch_nvfp4_gemv_tc: while a device buffer of 128 int64 words is set, launch n

@@ -49,6 +49,7 @@ SIGNATURES = {
     "launch_silu_mul": ([_vp, _vp, _vp, _i, _vp], _i),
     "launch_attn_decode": ([_vp] * 6 + [_i, _f, _vp], _i),
     "launch_attn_decode_heads": ([_vp] * 6 + [_i, _i, _i, _f, _vp], _i),
+    "launch_nvfp4_gemv_step": ([_vp, _vp, _vp, _vp, _i, _i, _i, _vp, _f, _i, _vp, _vp], _i),
     "launch_nvfp4_gemv_fused": ([_vp, _vp, _vp, _vp, _i, _i, _i, _vp, _f, _i, _vp, _vp], _i),
     "nvfp4_attn_split_scratch_bytes": ([_i], _ll),
     "launch_attn_decode_split": ([_vp] * 7 + [_i, _i, _i, _f, _vp], _i),
@@ -101,6 +102,7 @@ SIGNATURES = {
     "launch_nvfp4_mlp_tc": ([_vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _i, _i, _vp], _i),
     "nvfp4_gemv_tc_wanted": ([_i, _i], _i),
     "nvfp4_gemv_tc_wanted_plain": ([_i, _i], _i),
+    "nvfp4_gemv_tc_wanted_step": ([_i, _i], _i),
     "nvfp4_b200_gemv_tc_config_plain": ([_i], None),
     "nvfp4_gemv_tc_prepare": ([], _i),
     "nvfp4_gemv_tc_probe": ([_vp], None),

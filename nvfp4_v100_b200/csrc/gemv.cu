@@ -982,7 +982,7 @@ int gemv2i_dispatch(const void* packed, const void* scales, const void* act_i, v
 // shape and alignment rules of that kernel are requirements here.
 int gemv_ex_dispatch(const void* packed, const void* scales, const void* act, void* out, int M,
                      int K, int prologue, const void* norm_w1, float eps, int epilogue,
-                     const void* residual, void* stream) {
+                     const void* residual, void* stream, bool step) {
     if (K <= 0 || K % 128 != 0 || M <= 0) return NVFP4_ERR_SHAPE;
     if (!packed || !scales || !act || !out) return NVFP4_ERR_SHAPE;
     if (!aligned(packed, 32) || !aligned(scales, 8) || !aligned(act, 16) || !aligned(out, 2))
@@ -994,7 +994,8 @@ int gemv_ex_dispatch(const void* packed, const void* scales, const void* act, vo
     if (epilogue == EPI_RESIDUAL && !residual) return NVFP4_ERR_SHAPE;
     if (epilogue == EPI_SILU_MUL && M % 16 != 0) return NVFP4_ERR_SHAPE;
     // large matrices: the FP4 tensor-core kernel (TMA ring, no weight byte through a register)
-    if (!old_kernel_tuned() && nvfp4_gemv_tc_wanted(M, K) && aligned(scales, 16)) {
+    if (!old_kernel_tuned() && (step ? nvfp4_gemv_tc_wanted_step(M, K) : nvfp4_gemv_tc_wanted(M, K)) &&
+        aligned(scales, 16)) {
         const int rc = launch_nvfp4_gemv_tc_fused((const uint8_t*)packed, (const uint8_t*)scales, act, out,
                                                   M, K, prologue, norm_w1, eps, epilogue, residual, stream);
         if (rc == 0) return NVFP4_OK;
@@ -1177,7 +1178,17 @@ int launch_nvfp4_gemv_fused(const void* weight_packed, const void* weight_scales
                             const void* norm_w1, float eps, int epilogue, const void* residual,
                             void* stream) {
     return nvfp4::gemv_ex_dispatch(weight_packed, weight_scales, activation, output, M, K,
-                                   prologue, norm_w1, eps, epilogue, residual, stream);
+                                   prologue, norm_w1, eps, epilogue, residual, stream, false);
+}
+
+// The same for a caller whose other projections use the tensor-core GEMV's workspace anyway (a decode step): matrices
+// of 30 M elements go there too.  Not for everybody: the register-streaming kernel that they otherwise get has no
+// workspace, so calls on several streams may run side by side.
+int launch_nvfp4_gemv_step(const void* weight_packed, const void* weight_scales, const void* activation, void* output,
+                           int M, int K, int prologue, const void* norm_w1, float eps, int epilogue,
+                           const void* residual, void* stream) {
+    return nvfp4::gemv_ex_dispatch(weight_packed, weight_scales, activation, output, M, K,
+                                   prologue, norm_w1, eps, epilogue, residual, stream, true);
 }
 
 // Every single-activation GEMV generation of the reference library resolves to the same kernel;

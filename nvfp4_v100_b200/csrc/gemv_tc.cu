@@ -1137,10 +1137,9 @@ int launch_nvfp4_gemv_tc_fused(const uint8_t* weight_packed, const uint8_t* weig
 // register-streaming kernel, whose fixed cost per launch is lower.  0 = never route.
 //   fused entry (launch_nvfp4_gemv_fused: the decode engine's calls, activation hot in L2, other
 //   kernels in between): default 35 = the MLP projections, the fused input projections and the
-//   vocabulary head of the 27B decoder, and on two GPUs their shards.  A decode step measured
-//   258 tok/s with 40 or 60, 251 with 25, 199 with routing off on one GPU (the 31 M-element output
-//   projections stay on the register-streaming kernel); on two GPUs 281 tok/s with 30, 273 with
-//   40, 244 with 60 (the 37 M-element shard of the fused q/k/v projection).
+//   vocabulary head of the 27B decoder, and on two GPUs their shards.  On two GPUs a decode step
+//   measured 281 tok/s with 30, 273 with 40, 244 with 60 (the 37 M-element shard of the fused q/k/v
+//   projection).
 //   plain entry (launch_nvfp4_gemv_v8, timed back to back on cold activations): default 40; at
 //   89 M elements this kernel takes 11.4 us against 14.7 us, at 52 M 8.2 against 8.6 us, at 44.5 M
 //   (the two-GPU shards of the MLP projections) 7.4 / 7.6 against 8.4 / 8.1 us, at 31 M the
@@ -1155,6 +1154,12 @@ void nvfp4_b200_gemv_tc_config_plain(int min_mega_elements) {
 }
 int nvfp4_gemv_tc_wanted(int M, int K) {
     return g_tc_route_min > 0 && (long long)M * K >= g_tc_route_min && K % nvfp4::TC_BK == 0;
+}
+// launch_nvfp4_gemv_step: 30 by default.  The output projections of the 27B decoder (5120 x 6144, residual added) take
+// 6.0 us on the register-streaming kernel and 6.3 here, back to back; in a decode step, between other launches of
+// this kernel, they are the faster ones here: 3597 -> 3558 us a step (3546 to 3578 with 25, 20, 15 and 10).
+int nvfp4_gemv_tc_wanted_step(int M, int K) {
+    return g_tc_route_min > 0 && (long long)M * K >= g_tc_route_min / 7 * 6 && K % nvfp4::TC_BK == 0;
 }
 int nvfp4_gemv_tc_wanted_plain(int M, int K) {
     return g_tc_route_min_plain > 0 && (long long)M * K >= g_tc_route_min_plain && K % nvfp4::TC_BK == 0;

@@ -443,7 +443,10 @@ class DecodeEngine:
             self.n_launch += 1
             self.n_collective += 1
             return
-        rc = self.lib.launch_nvfp4_gemv_fused(
+        # where gate/up uses the tensor-core GEMV's workspace, the projections a little smaller may too
+        gu = self.layers[0].w_gu
+        step = self.lib.nvfp4_gemv_tc_wanted(gu.M, gu.K)
+        rc = (self.lib.launch_nvfp4_gemv_step if step else self.lib.launch_nvfp4_gemv_fused)(
             vp(m.packed.data_ptr()), vp(m.scales.data_ptr()), vp(x.data_ptr()), vp(out_ptr),
             m.M, m.K, 0 if pro_w1 is None else 1,
             vp(0 if pro_w1 is None else pro_w1.data_ptr()), float(self.cfg.rms_eps), epi,

@@ -241,3 +241,32 @@ def test_mlp_block_rejects_bad_arguments(lib):
     assert f(one, one, one, one, one, one, one, 1e-6, 500, 256, None) == -2      # inter % 256
     assert f(one, one, one, one, one, one, None, 1e-6, 512, 256, None) == -2     # norm weights missing
     assert f(one, one, one, one, one, one, one, 1e-6, 512, 12288, None) == -2    # hidden > 11520
+
+
+def test_routing_of_a_decode_step(lib):
+    # 30 M elements: the output projections; the public entry leaves them to the kernel without a workspace
+    assert lib.nvfp4_gemv_tc_wanted_step(5120, 6144) == 1 and lib.nvfp4_gemv_tc_wanted_step(5119, 6144) == 0
+    assert lib.nvfp4_gemv_tc_wanted(5120, 6144) == 0
+    lib.nvfp4_b200_gemv_tc_config(0)
+    assert lib.nvfp4_gemv_tc_wanted_step(34816, 5120) == 0
+    lib.nvfp4_b200_gemv_tc_config(35)
+
+
+@pytest.mark.parametrize("M,K", [(5120, 6144), (8192, 3840), (5121, 6144), (2560, 2560)])
+def test_step_entry_against_the_two_kernels(lib, M, K):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    p = torch.randint(0, 256, (M, K // 2), dtype=torch.uint8, device="cuda", generator=g)
+    s = torch.randint(118, 123, (M, K // 16), dtype=torch.uint8, device="cuda", generator=g)
+    x, h = torch.randn(K, device="cuda", generator=g).half(), torch.randn(M, device="cuda", generator=g).half()
+    w1 = torch.rand(K, device="cuda", generator=g) + 0.5
+    tc = lib.nvfp4_gemv_tc_wanted_step(M, K)
+    for pro in (0, 1):
+        outs = []
+        for entry in (lib.launch_nvfp4_gemv_step, lib.launch_nvfp4_gemv_tc_fused if tc else lib.launch_nvfp4_gemv_fused):
+            out = torch.zeros(M, dtype=torch.float16, device="cuda")
+            assert entry(ptr(p), ptr(s), ptr(x), ptr(out), M, K, pro, ptr(w1), 1e-6, 1, ptr(h), stream()) == 0
+            outs.append(out)
+        torch.cuda.synchronize()
+        assert torch.equal(*outs)
+    assert lib.nvfp4_gemv_tc_status(0) == 0
