@@ -6,17 +6,17 @@
 // The reference prefills through the third-party model code (pipeline/_qwen38_infer.py:796-809:
 // 512-token chunks, every Linear running launch_nvfp4_gemmtc_v5, attention and the gated delta
 // rule in PyTorch).  Here the chunk's activations are token-major [tokens][features] between the
-// operators and at the GEMMs (launch_nvfp4_gemm_w4a16_ex); only gate/up -> silu-mul -> down stays
-// [features][tokens]:
+// operators and at the GEMMs (launch_nvfp4_gemm_w4a16_ex, launch_nvfp4_gemm_silu):
 //   transpose_f16 / add_transposed   layout changes around launch_nvfp4_gemmtc_v5 (the second fused with
 //                                    the residual add), for a caller that keeps to that entry point
 //   embed_rows                       token ids -> embedding rows
-//   silu_mul_rows                    gate/up rows (interleaved by 8) -> activation rows
+//   silu_mul_tokens, silu_mul_rows   gate/up (interleaved by 8) -> activations, token-major and token-minor
 //   dn_conv_tokens, dn_block, dn_scan, dn_post   one Gated-DeltaNet layer over a chunk:
 //       causal conv + silu over the chunk with the carried window; q/k L2 norm, beta, decay;
 //       the recurrence S_t = S_{t-1} e^{g_t} + k_t (v_t - S_{t-1} e^{g_t} k_t) beta_t, o_t = S_t q_t
 //       run over the chunk in blocks of four tokens with every state row in registers (rows are
-//       independent: 16 lanes own two rows, 8 dims each; 6144 rows of the full model); gated norm.
+//       independent: 16 lanes own two rows, 8 dims each; 6144 rows of the full model), longer chunks in
+//       blocks of 64 on the tensor cores (dn_chunk.cu); gated norm.
 // Attention uses the chunk forms of attn_prep (decode_ops.cu) and launch_attn_prefill: the tensor-core
 // kernel (attn_prefill_tc.cu) or, for small chunks, attn_prefill_group_kernel (fused_ops.cu).
 #include <cstdio>
