@@ -597,6 +597,10 @@ static bool gemm_use_pair(int M, int N, int K) {
     if (!g_gemm_pair || N <= 128 || K % (GEMM_BK * PAIR_KS) != 0) return false;
     return g_gemm_pair == 2 || !gemm_tile_rows256(M, N);
 }
+// The kernel of gemm_few.cu: up to 128 tokens, and up to 256 of narrow matrices (not where a policy is forced).
+static bool gemm_use_few(const uint8_t* packed, const uint8_t* scales, int M, int N, int K) {
+    return gemm_few_takes(packed, scales, N, K) || (g_gemm_pair == 1 && gemm_few_takes_two(packed, scales, M, N, K));
+}
 // The kernel of gemm_pair.cu: wherever it can run, except where 256-row tiles are faster (short K).
 static bool gemm_use_pair_tm(const uint8_t* packed, const uint8_t* scales, int M, int N, int K, int out_mode) {
     if (!g_gemm_pair || !gemm_pair_takes(packed, scales, N, K)) return false;
@@ -632,7 +636,7 @@ int launch_nvfp4_gemmtc_v5(const uint8_t* d_weight_packed, const uint8_t* d_weig
     if (!d_weight_packed || !d_weight_scales || !d_activation || !d_output) return NVFP4_ERR_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
     if (N % 8 == 0 && (((uintptr_t)d_activation | (uintptr_t)d_output) & 15) == 0 &&
-        gemm_few_takes(d_weight_packed, d_weight_scales, N, K)) {
+        gemm_use_few(d_weight_packed, d_weight_scales, M, N, K)) {
         const int rc = gemm_few_launch(d_weight_packed, d_weight_scales, d_activation, N, false, d_output, N,
                                        M, N, N, K, GEMM_OUT_FM, st);
         if (rc != -3) return rc;
@@ -700,7 +704,7 @@ int launch_nvfp4_gemm_w4a16_ex(const uint8_t* d_weight_packed, const uint8_t* d_
     const int mode = !out_tm ? GEMM_OUT_FM : add ? GEMM_OUT_TM_ADD : GEMM_OUT_TM;
     __half* o = static_cast<__half*>(out);
     cudaStream_t st = (cudaStream_t)stream;
-    if (gemm_few_takes(d_weight_packed, d_weight_scales, N8, K))
+    if (gemm_use_few(d_weight_packed, d_weight_scales, M, N8, K))
         return gemm_few_launch(d_weight_packed, d_weight_scales, static_cast<const __half*>(act), ld_act, in_tm,
                                o, (int)ld_out, M, N8, n_tokens, K, mode, st);
     // token count the kernel's bounds use: feature-major sides are padded to 8

@@ -1,4 +1,4 @@
-// Dense W4A16 GEMM for at most 128 tokens (batched decode, short prompts, ragged prompt ends):
+// Dense W4A16 GEMM for at most 128 tokens, 256 on narrow matrices (batched decode, short prompts, ragged prompt ends):
 // out = dequant(W)[M, K] . act, the arithmetic of gemm.cu (weight x block scale in fp16, fp16
 // products, fp32 accumulation), bound by reading the weights from HBM (0.5625 bytes each).
 //
@@ -428,6 +428,19 @@ static cudaError_t few_launch(const CUtensorMap& wm, const CUtensorMap& sm, cons
 
 bool gemm_few_takes(const uint8_t* packed, const uint8_t* scales, int N, int K) {
     return N <= GEMM_FEW_MAX_TOKENS && K % FEW_BK == 0 && (((uintptr_t)packed | (uintptr_t)scales) & 15) == 0;
+}
+
+// 129 to 256 tokens are two column tiles of 128.  For narrow matrices the CTA pairs of gemm_pair.cu leave most of the GPU
+// idle, while here K is split until the SMs are full: pairs / this kernel at 129 and 256 tokens, us: 1024 x 5120 19.3
+// / 9.9 and 19.7 / 11.8, 5120 x 6144 23.7 / 19.3 and 24.8 / 19.5, 5120 x 17408 53.7 / 39.3 and 56.1 / 41.6, 1024 x 17408
+// 51.4 / 18.2 and 51.4 / 20.5.  Wider ones are split less and read their weights twice (6144 x 5120 21.0 / 20.0,
+// feature-major 22.7 / 24.8; 10240 x 5120 23.3 / 31.4), and a short K leaves a CTA too little
+// (5120 x 1024 9.2 / 9.7 at 256, feature-major 9.3 / 10.4; 2048 x 1024 8.7 / 7.0).
+bool gemm_few_takes_two(const uint8_t* packed, const uint8_t* scales, int M, int N, int K) {
+    const int rows = (M + FEW_BM - 1) / FEW_BM;
+    return N > GEMM_FEW_MAX_TOKENS && N <= 2 * GEMM_FEW_MAX_TOKENS && K % FEW_BK == 0 &&
+           (((uintptr_t)packed | (uintptr_t)scales) & 15) == 0 && (K >= 12 * FEW_BK || rows <= 20) &&
+           2LL * rows * 7 <= 4LL * device_sms(current_device_index());
 }
 
 int gemm_few_launch(const uint8_t* packed, const uint8_t* scales, const __half* act, long long ld_act,

@@ -6,12 +6,15 @@ namespace nvfp4 {
 
 // One token tile.  Above it the CTA-pair kernel, which needs enough rows to fill the GPU: 136 tokens 16480 x
 // 5120 25.4 us against 35.8 with two token tiles here, 34816 x 5120 51.3 / 71.4.  Narrow matrices lie the other
-// way up to 256 tokens (5120 x 17408 63.2 / 40.2, 5120 x 6144 26.2 / 19.4, 1024 x 5120 22.6 / 9.7; 128 tokens
-// 26.3, 15.4 and 8.5): a rule by rows as well is not built.
+// way up to 256 tokens: gemm_few_takes_two.
 constexpr int GEMM_FEW_MAX_TOKENS = 128;
 
 // Whether the few-token kernel takes this product (sizes and alignment).
 bool gemm_few_takes(const uint8_t* packed, const uint8_t* scales, int N, int K);
+
+// Whether the kernel is the faster one for this product of 129 to 256 tokens (its sums over K are in another order than
+// those of the kernels it then replaces).
+bool gemm_few_takes_two(const uint8_t* packed, const uint8_t* scales, int M, int N, int K);
 
 // act: token-major [N][ld_act] (in_tm) or token-minor [K][ld_act]; N = tokens the output holds in
 // feature-major mode, n_out = tokens written in token-major mode.  0, -3, or a cudaError_t.
