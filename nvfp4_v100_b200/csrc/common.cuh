@@ -118,10 +118,10 @@ __device__ __forceinline__ void pdl_prologue() {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 
-// Launch with the attribute (kernels that call pdl_prologue() first thing).
+// Launch with the attribute if `programmatic`, else ordered after everything in front of it in the stream.
 template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                     cudaStream_t st, Args... args) {
+static inline cudaError_t launch_pdl_if(bool programmatic, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                        cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -131,8 +131,14 @@ static inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 b
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = programmatic ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+// Launch with the attribute (kernels that call pdl_prologue() first thing).
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                     cudaStream_t st, Args... args) {
+    return launch_pdl_if(true, kernel, grid, block, smem, st, args...);
 }
 
 }  // namespace nvfp4

@@ -761,6 +761,8 @@ static int num_sms() {
 }
 
 // A caller that sets one of the register-streaming kernel's tuning values wants that kernel.
+bool gemv_reads_ahead() { return !g_cfg.no_pdl; }
+
 static bool old_kernel_tuned() {
     return g_cfg.warps || g_cfg.ctas_per_sm || g_cfg.max_split || g_cfg.force_split;
 }

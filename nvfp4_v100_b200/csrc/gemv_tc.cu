@@ -958,7 +958,7 @@ static cudaError_t tc_launch_st(int dev, int G, cudaStream_t st, const CUtensorM
         if (e != cudaSuccess) return e;
         attr[dev] = true;
     }
-    return launch_pdl(gemv_tc_kernel<ST, PRO, EPI, DBG>, dim3((unsigned)G), dim3(TC_THREADS),
+    return launch_pdl_if(gemv_reads_ahead(), gemv_tc_kernel<ST, PRO, EPI, DBG>, dim3((unsigned)G), dim3(TC_THREADS),
                       (size_t)tc_smem_bytes(ST), st, wm, sm, x, y, ws->part, ws->counters, M, K, fz, dbg);
 }
 static int g_tc_ring = 5;      // weight-ring depth: 5 (110 KB per CTA) or 3 (74 KB)
@@ -1116,8 +1116,8 @@ int launch_nvfp4_mlp_tc(const uint8_t* gu_packed, const uint8_t* gu_scales, cons
     a.part = ws->part;
     a.gbar = ws->counters;
     a.pre = g_tc_pre;
-    const cudaError_t e = launch_pdl(gemv_tc_mlp_kernel<5>, dim3((unsigned)G), dim3(TC_THREADS),
-                                     (size_t)tc_smem_bytes(5), (cudaStream_t)stream, m[0], m[1], m[2], m[3], a);
+    const cudaError_t e = launch_pdl_if(gemv_reads_ahead(), gemv_tc_mlp_kernel<5>, dim3((unsigned)G), dim3(TC_THREADS),
+                                        (size_t)tc_smem_bytes(5), (cudaStream_t)stream, m[0], m[1], m[2], m[3], a);
     return (e == cudaSuccess) ? 0 : (int)e;
 }
 

@@ -312,7 +312,7 @@ static cudaError_t t2_launch(const CUtensorMap& wm, const CUtensorMap& sm, const
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = gemv_reads_ahead() ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, gemv_tc2_kernel<IL>, wm, sm, packed, scales, x0, x1, y, M, K, split);
 }
 
