@@ -12,7 +12,9 @@
 // carrying the block scale 2^(L - 2j - 2) (an exact E8M0 byte).  Then sum_j (W . column_j) = W . x
 // with every product exact; only the fp32 accumulation rounds.  The 16 columns are the minimum N
 // of a 128-row MMA, so the digits cost no extra tensor-core time.  (Bits of an element more than
-// 2^21 below its block's largest are dropped: a relative 2^-31 of that block's contribution.)
+// 2^21 below its block's largest are dropped: a relative 2^-31 of that block's contribution.)  Infinities and NaN
+// have no digits: they make the sums NaN, and rows that are NaN are formed again in plain fp32 (tc_plain_row), so that
+// they come out as IEEE arithmetic gives them.
 //
 // Work: row tiles of 128 x K stages of 256 elements, numbered tile-major (a CTA reads consecutive
 // K of the same rows: DRAM pages stay open; a K-chunk-major order measured 25 % slower); the stages
@@ -117,6 +119,26 @@ struct TcFuse {
     float eps;
     const __half* residual;
     int pre;       // weight stages requested at kernel entry; the others follow the activation request
+    const uint8_t *packed, *scales;       // the weights, for rows whose sum is NaN
+};
+
+// Eight activations as they are multiplied, for tc_plain_row (from L2: another CTA may have written them just now).
+template <int PRO>
+struct TcLoad {
+    const __half* x;
+    const float* norm_w1;
+    float inv;
+    __device__ __forceinline__ uint4 operator()(int k) const {
+        uint4 v = __ldcg(reinterpret_cast<const uint4*>(x + k));
+        if (PRO == TPRO_RMSNORM) {
+            __half2* h = reinterpret_cast<__half2*>(&v);
+            for (int e = 0; e < 4; e++) {
+                const float2 f = __half22float2(h[e]);
+                h[e] = __halves2half2(__float2half(f.x * inv * norm_w1[k + 2 * e]), __float2half(f.y * inv * norm_w1[k + 2 * e + 1]));
+            }
+        }
+        return v;
+    }
 };
 
 // Final value of row `row` (this lane's; the warp's 32 rows are consecutive and start at a
@@ -420,6 +442,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                     if (lane == 0) mbar_arrive(smem_u32(&bar_bfull[slot]));
                 }
             };
+            int redo = 0x7fffffff;       // first tile with a NaN among this warp's rows: it and the later ones are not stored
             int seg = 0, tile = tile0, left = nst, seg_len = nk - ks0, done = 0;
             while (left > 0) {
                 if (seg_len > left) seg_len = left;
@@ -442,7 +465,8 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 const int c_first = tc_cta_of((unsigned)tile * nk, total, G);
                 const int c_last = tc_cta_of((unsigned)(tile + 1) * nk - 1u, total, G);
                 if (c_first == c_last) {
-                    tc_store<EPI>(sum, row, lane, M, y, fz);
+                    if (__any_sync(0xffffffffu, sum != sum)) redo = min(redo, tile);
+                    if (tile < redo) tc_store<EPI>(sum, row, lane, M, y, fz);
                 } else if (b != c_first) {
                     // a contributor: one store into slot (tile + CTA) - unique, because a CTA
                     // boundary inside a tile adds one slot - and done.  An empty slot holds the
@@ -483,7 +507,8 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                                        TC_EMPTY);
                             }
                     }
-                    tc_store<EPI>(tot, row, lane, M, y, fz);
+                    if (__any_sync(0xffffffffu, tot != tot)) redo = min(redo, tile);
+                    if (tile < redo) tc_store<EPI>(tot, row, lane, M, y, fz);
                 }
                 left -= seg_len;
                 done += seg_len;
@@ -492,6 +517,15 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 seg++;
             }
             if (rec && lane == 0) atomicMax(dbg + 7, tc_now());
+            // The tiles whose result is this CTA's, from `redo` on: in plain fp32.  (Down here, where it is not in the way of
+            // the code above: a call inside that loop cost every launch 0.13 us.)
+            for (; redo < tile; redo++) {
+                if (tc_cta_of((unsigned)redo * nk, total, G) != b) continue;
+                const int row = redo * TC_BM + q * 32 + lane;
+                const float tot = tc_plain_row(fz.packed, fz.scales, TcLoad<PRO>{x, fz.norm_w1, inv}, min(row, M - 1), K);
+                __syncwarp();
+                tc_store<EPI>(tot, row, lane, M, y, fz);
+            }
         }
     }
 
@@ -524,6 +558,7 @@ struct TcMlpArgs {
     float* part;               // partial-sum slots: (ntiles0 + G) for phase 0, then those of phase 1
     unsigned int* gbar;        // {arrival count, generation}
     int pre;                   // weight stages requested at kernel entry
+    const uint8_t *gu_packed, *gu_scales, *down_packed, *down_scales;   // for rows whose sum is NaN
 };
 struct TcRange { int ntiles, nk, nst, tile0, ks0; unsigned total; };
 __device__ __forceinline__ TcRange tc_range(int M, int K, unsigned G, unsigned b) {
@@ -846,6 +881,7 @@ gemv_tc_mlp_kernel(const __grid_constant__ CUtensorMap w_map0, const __grid_cons
                         if (lane == 0) mbar_arrive(smem_u32(&bar_bfull[slot]));
                     }
                 };
+                int redo = 0x7fffffff;                   // as in gemv_tc_kernel
                 int tile = R.tile0, left = R.nst, seg_len = R.nk - R.ks0, done = 0;
                 while (left > 0) {
                     if (seg_len > left) seg_len = left;
@@ -899,7 +935,8 @@ gemv_tc_mlp_kernel(const __grid_constant__ CUtensorMap w_map0, const __grid_cons
                         }
                     }
                     // (both calls contain warp shuffles or none: `store` is uniform over the warp)
-                    if (store) {
+                    if (store && __any_sync(0xffffffffu, tot != tot)) redo = min(redo, tile);
+                    if (store && tile < redo) {
                         if (p == 0) tc_store<TEPI_SILU_MUL>(tot, row, lane, M, act, fz);
                         else tc_store<TEPI_RESIDUAL>(tot, row, lane, M, h, fz);
                     }
@@ -908,6 +945,16 @@ gemv_tc_mlp_kernel(const __grid_constant__ CUtensorMap w_map0, const __grid_cons
                     seg_len = R.nk;
                     tile++;
                     seg++;
+                }
+                for (; redo < tile; redo++) {
+                    if (tc_cta_of((unsigned)redo * R.nk, R.total, G) != (int)b) continue;
+                    const int row = redo * TC_BM + q * 32 + lane, r = min(row, M - 1);
+                    const float tot =
+                        p == 0 ? tc_plain_row(a.gu_packed, a.gu_scales, TcLoad<TPRO_RMSNORM>{x, a.norm_w1, inv}, r, K0)
+                               : tc_plain_row(a.down_packed, a.down_scales, TcLoad<TPRO_NONE>{x, nullptr, 1.0f}, r, K1);
+                    __syncwarp();
+                    if (p == 0) tc_store<TEPI_SILU_MUL>(tot, row, lane, M, act, fz);
+                    else tc_store<TEPI_RESIDUAL>(tot, row, lane, M, h, fz);
                 }
             }
         }
@@ -1020,7 +1067,7 @@ static int tc_launch(const uint8_t* weight_packed, const uint8_t* weight_scales,
                 CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return -3;
     }
-    const TcFuse fz = {norm_w1, eps, static_cast<const __half*>(residual), g_tc_pre};
+    const TcFuse fz = {norm_w1, eps, static_cast<const __half*>(residual), g_tc_pre, weight_packed, weight_scales};
     const __half* x = static_cast<const __half*>(activation);
     __half* y = static_cast<__half*>(output);
     cudaStream_t st = (cudaStream_t)stream;
@@ -1116,6 +1163,10 @@ int launch_nvfp4_mlp_tc(const uint8_t* gu_packed, const uint8_t* gu_scales, cons
     a.part = ws->part;
     a.gbar = ws->counters;
     a.pre = g_tc_pre;
+    a.gu_packed = gu_packed;
+    a.gu_scales = gu_scales;
+    a.down_packed = down_packed;
+    a.down_scales = down_scales;
     const cudaError_t e = launch_pdl_if(gemv_reads_ahead(), gemv_tc_mlp_kernel<5>, dim3((unsigned)G), dim3(TC_THREADS),
                                         (size_t)tc_smem_bytes(5), (cudaStream_t)stream, m[0], m[1], m[2], m[3], a);
     return (e == cudaSuccess) ? 0 : (int)e;

@@ -43,6 +43,8 @@ __device__ __forceinline__ uint32_t tc_prmt(uint32_t a, uint32_t b, uint32_t sel
 // exponent byte.  All by bit operations on whole words: a transpose of the eight 32-bit fractions by nibbles puts
 // two digits of every element into one word, and a digit with bits h, l is the E2M1 code (h, l & ~h, h & l).  (A table of
 // codes per byte in shared memory took 32 scattered reads a lane, which the SM's other CTA waited for as well.)
+// A block with a value that is not finite has no digits: its exponent byte is 255, a NaN scale, so that every sum it
+// enters is NaN and the rows are formed by tc_plain_row instead.
 __device__ __forceinline__ void tc_digit_planes(const uint4 xv, uint8_t* btile, uint8_t* lbytes, int lane) {
     const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
     uint32_t hmax = 0;
@@ -98,7 +100,34 @@ __device__ __forceinline__ void tc_digit_planes(const uint4 xv, uint8_t* btile, 
         put(2 * n, ((t >> 1) & 0x44444444u) | ((t >> 1) & ~(t >> 2) & 0x22222222u) | ((t >> 3) & (t >> 2) & 0x11111111u));
         put(2 * n + 1, ((t << 1) & 0x44444444u) | ((t << 1) & ~t & 0x22222222u) | ((t >> 1) & t & 0x11111111u));
     }
-    if ((lane & 1) == 0) lbytes[lane >> 1] = (uint8_t)(L + 125);
+    if ((lane & 1) == 0) lbytes[lane >> 1] = (uint8_t)(em == 31u ? 255 : L + 125);
+}
+
+// A row's sum in plain fp32, block by block, as the register-streaming kernels form it: for sums that came out as NaN (an
+// activation that is not finite).  load(k): the activations k .. k + 7.
+template <typename LOAD>
+__device__ __noinline__ float tc_plain_row(const uint8_t* packed, const uint8_t* scales, const LOAD load, int row, int K) {
+    const uint8_t* w = packed + (size_t)row * (K / 2);
+    const uint8_t* sc = scales + (size_t)row * (K / 16);
+    float sum = 0.0f;
+    for (int b = 0; b < K / 16; b++) {
+        const uint2 p = *reinterpret_cast<const uint2*>(w + b * 8);
+        float acc = 0.0f;
+        for (int half = 0; half < 2; half++) {
+            uint32_t h[4];
+            e2m1x8_to_half2x4(half ? p.y : p.x, h[0], h[1], h[2], h[3]);
+            const uint4 xv = load(b * 16 + half * 8);
+            const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
+            for (int e = 0; e < 4; e++) {
+                const float2 wf = __half22float2(*reinterpret_cast<const __half2*>(&h[e]));
+                const float2 xf = __half22float2(*reinterpret_cast<const __half2*>(&xw[e]));
+                acc = fmaf(wf.x, xf.x, acc);
+                acc = fmaf(wf.y, xf.y, acc);
+            }
+        }
+        sum = fmaf(acc, e8m0_to_f32(sc[b]), sum);
+    }
+    return sum;
 }
 
 }  // namespace nvfp4

@@ -14,7 +14,8 @@
 //   warp 1      MMA issuer: four MMAs M128 N32 K64 a stage
 //   warps 2..5  scale bytes of the weights and of the digit columns -> tensor memory
 //   warps 6..9  digit conversion, a warp one activation of every other stage; then the sums of their rows
-// An activation with a value that is not finite has no digits: its rows are then summed in plain fp32 from global memory.
+// An activation with a value that is not finite has no digits: its sums are NaN, and its rows are then summed in plain fp32
+// from global memory.
 // Every wait is bounded and reported through nvfp4_gemv_tc_status (20 + id).
 //
 // Measured: at gemv_tc2_takes.
@@ -56,32 +57,12 @@ __device__ __forceinline__ uint4 t2_load(const __half* x0, const __half* x1, int
     return make_uint4(tc_prmt(p.x, p.y, sel), tc_prmt(p.z, p.w, sel), tc_prmt(q.x, q.y, sel), tc_prmt(q.z, q.w, sel));
 }
 
-// A row's sum over stages [st0, st1) in plain fp32, block by block, as the register-streaming kernels form it.
 template <bool IL>
-__device__ __noinline__ float t2_plain_row(const uint8_t* packed, const uint8_t* scales, const __half* x0, const __half* x1,
-                                           int a, int row, int K, int st0, int st1) {
-    const uint8_t* w = packed + (size_t)row * (K / 2);
-    const uint8_t* sc = scales + (size_t)row * (K / 16);
-    float sum = 0.0f;
-    for (int b = st0 * (TC_BK / 16); b < st1 * (TC_BK / 16); b++) {
-        const uint2 p = *reinterpret_cast<const uint2*>(w + b * 8);
-        float acc = 0.0f;
-        for (int half = 0; half < 2; half++) {
-            uint32_t h[4];
-            e2m1x8_to_half2x4(half ? p.y : p.x, h[0], h[1], h[2], h[3]);
-            const uint4 xv = t2_load<IL>(x0, x1, a, b * 16 + half * 8);
-            const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
-            for (int e = 0; e < 4; e++) {
-                const float2 wf = __half22float2(*reinterpret_cast<const __half2*>(&h[e]));
-                const float2 xf = __half22float2(*reinterpret_cast<const __half2*>(&xw[e]));
-                acc = fmaf(wf.x, xf.x, acc);
-                acc = fmaf(wf.y, xf.y, acc);
-            }
-        }
-        sum = fmaf(acc, e8m0_to_f32(sc[b]), sum);
-    }
-    return sum;
-}
+struct T2Load {
+    const __half *x0, *x1;
+    int a;
+    __device__ __forceinline__ uint4 operator()(int k) const { return t2_load<IL>(x0, x1, a, k); }
+};
 
 template <bool IL>
 __global__ void __launch_bounds__(T2_THREADS)
@@ -103,7 +84,6 @@ gemv_tc2_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     __shared__ __align__(8) uint64_t bar_acc;
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_xreq;                           // the activation loads have been issued
-    __shared__ int s_bad[2];                                  // the activation is not finite
     __shared__ float s_red[T2_MAX_SPLIT][2][TC_BM];           // (first CTA) every CTA's sums
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -131,7 +111,6 @@ gemv_tc2_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         }
         mbar_init(smem_u32(&bar_acc), 1);
         s_xreq = 0;
-        s_bad[0] = s_bad[1] = 0;
         fence_barrier_init();
         for (int i = 0; i < T2_PRE && i < nst; i++) request(i, i);
     }
@@ -226,15 +205,10 @@ gemv_tc2_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
             uint4 next = make_uint4(0u, 0u, 0u, 0u);
             if (i < nst) next = t2_load<IL>(x0, x1, a, (st0 + i) * TC_BK + lane * 8);
             if (threadIdx.x == 192) s_xreq = 1;
-            uint32_t bad = 0;
             for (; i < nst; i += 2) {
                 const int slot = i % NB;
                 const uint4 xv = next;
                 if (i + 2 < nst) next = t2_load<IL>(x0, x1, a, (st0 + i + 2) * TC_BK + lane * 8);
-                const uint32_t w[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-                for (int e = 0; e < 4; e++)
-                    bad |= (uint32_t)((w[e] & 0x7C00u) == 0x7C00u) | (uint32_t)((w[e] & 0x7C000000u) == 0x7C000000u);
                 t2_wait(smem_u32(&bar_bempty[slot]), ((uint32_t)(i / NB) & 1u) ^ 1u, 5);
                 __syncwarp();
                 tc_digit_planes(xv, smem_b + slot * T2_B_BYTES + a * 2048, smem_l + slot * 32 + a * 16, lane);
@@ -242,7 +216,6 @@ gemv_tc2_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&bar_bfull[slot]));
             }
-            if (__any_sync(0xffffffffu, bad != 0u) && lane == 0) atomicOr(&s_bad[a], 1);
             t2_wait(smem_u32(&bar_acc), 0, 6);
             __syncwarp();
             tcgen05_fence_after();
@@ -254,13 +227,6 @@ gemv_tc2_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 sum[0] += __uint_as_float(v[j]);
                 sum[1] += __uint_as_float(v[16 + j]);
             }
-            asm volatile("bar.sync 1, 128;\n" ::: "memory");     // s_bad is complete
-            const int row = tile * TC_BM + q * 32 + lane;
-            if (row < M)
-#pragma unroll
-                for (int t = 0; t < 2; t++)
-                    if (s_bad[t]) sum[t] = t2_plain_row<IL>(packed, scales, x0, x1, t, row, K, st0, st0 + nst);
-            __syncwarp();
         }
     }
     asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");                 // the first CTA runs
@@ -282,6 +248,7 @@ gemv_tc2_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         for (int t = 0; t < 2; t++) {
             float tot = s_red[0][t][r];
             for (int c = 1; c < split; c++) tot += s_red[c][t][r];
+            if (tot != tot) tot = tc_plain_row(packed, scales, T2Load<IL>{x0, x1, t}, row, K);
             y[(size_t)t * M + row] = __float2half(tot);
         }
 }
