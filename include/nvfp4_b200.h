@@ -381,11 +381,11 @@ int launch_nvfp4_decode_rows(const void* packed, const void* scales, const void*
  * semantics of launch_nvfp4_gemv_v8 (kernels/nvfp4_gemv.cu:88-100).  Weight and scale bytes go
  * HBM -> shared memory (TMA) -> tcgen05.mma kind::mxf4nvf4 without passing through registers; the
  * fp16 activation enters as 16 exact base-4 digit columns, so the products are those of the W4A16
- * rule with fp32 accumulation (a row whose sum is NaN, as with an infinity or a NaN in the activation, is summed
- * again in plain fp32, so that it is what the other GEMVs give).  K % 256 == 0; weight pointers and activation
- * 16-byte aligned.  The
- * first call on a device allocates a workspace (do it outside stream capture).  0; -2 shape or
- * pointer not taken; -3 no tensor-map encoder / no memory; else the launch's cudaError_t.
+ * rule with fp32 accumulation (a row whose sum is not finite is formed again in plain fp32, so that
+ * infinities and NaN in the activation and scale bytes of 255 give what the other GEMVs give).
+ * K % 256 == 0; weight pointers and activation 16-byte aligned.  The first call on a device
+ * allocates a workspace (do it outside stream capture).  0; -2 shape or pointer not taken; -3 no
+ * tensor-map encoder / no memory; else the launch's cudaError_t.
  * nvfp4_gemv_tc_status: 0, or 1 + id of the first bounded wait in that kernel that ran out (20 + for the
  *   kernel of two activations, which launch_nvfp4_gemv2 and gemv2i hand matrices of 10 M elements to). */
 int launch_nvfp4_gemv_tc(const uint8_t* weight_packed, const uint8_t* weight_scales,

@@ -13,8 +13,8 @@
 // with every product exact; only the fp32 accumulation rounds.  The 16 columns are the minimum N
 // of a 128-row MMA, so the digits cost no extra tensor-core time.  (Bits of an element more than
 // 2^21 below its block's largest are dropped: a relative 2^-31 of that block's contribution.)  Infinities and NaN
-// have no digits: they make the sums NaN, and rows that are NaN are formed again in plain fp32 (tc_plain_row), so that
-// they come out as IEEE arithmetic gives them.
+// have no digits: they make the sums NaN, and rows that are not finite are formed again in plain fp32 (tc_plain_row), so
+// that they come out as IEEE arithmetic gives them.
 //
 // Work: row tiles of 128 x K stages of 256 elements, numbered tile-major (a CTA reads consecutive
 // K of the same rows: DRAM pages stay open; a K-chunk-major order measured 25 % slower); the stages
@@ -119,7 +119,7 @@ struct TcFuse {
     float eps;
     const __half* residual;
     int pre;       // weight stages requested at kernel entry; the others follow the activation request
-    const uint8_t *packed, *scales;       // the weights, for rows whose sum is NaN
+    const uint8_t *packed, *scales;       // the weights, for rows whose sum is not finite
 };
 
 // Eight activations as they are multiplied, for tc_plain_row (from L2: another CTA may have written them just now).
@@ -442,7 +442,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                     if (lane == 0) mbar_arrive(smem_u32(&bar_bfull[slot]));
                 }
             };
-            int redo = 0x7fffffff;       // first tile with a NaN among this warp's rows: it and the later ones are not stored
+            int redo = 0x7fffffff;       // first tile with a sum of this warp's that is not finite: it and the later ones are not stored
             int seg = 0, tile = tile0, left = nst, seg_len = nk - ks0, done = 0;
             while (left > 0) {
                 if (seg_len > left) seg_len = left;
@@ -465,7 +465,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 const int c_first = tc_cta_of((unsigned)tile * nk, total, G);
                 const int c_last = tc_cta_of((unsigned)(tile + 1) * nk - 1u, total, G);
                 if (c_first == c_last) {
-                    if (__any_sync(0xffffffffu, sum != sum)) redo = min(redo, tile);
+                    if (__any_sync(0xffffffffu, tc_not_finite(sum))) redo = min(redo, tile);
                     if (tile < redo) tc_store<EPI>(sum, row, lane, M, y, fz);
                 } else if (b != c_first) {
                     // a contributor: one store into slot (tile + CTA) - unique, because a CTA
@@ -507,7 +507,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                                        TC_EMPTY);
                             }
                     }
-                    if (__any_sync(0xffffffffu, tot != tot)) redo = min(redo, tile);
+                    if (__any_sync(0xffffffffu, tc_not_finite(tot))) redo = min(redo, tile);
                     if (tile < redo) tc_store<EPI>(tot, row, lane, M, y, fz);
                 }
                 left -= seg_len;
@@ -558,7 +558,7 @@ struct TcMlpArgs {
     float* part;               // partial-sum slots: (ntiles0 + G) for phase 0, then those of phase 1
     unsigned int* gbar;        // {arrival count, generation}
     int pre;                   // weight stages requested at kernel entry
-    const uint8_t *gu_packed, *gu_scales, *down_packed, *down_scales;   // for rows whose sum is NaN
+    const uint8_t *gu_packed, *gu_scales, *down_packed, *down_scales;   // for rows whose sum is not finite
 };
 struct TcRange { int ntiles, nk, nst, tile0, ks0; unsigned total; };
 __device__ __forceinline__ TcRange tc_range(int M, int K, unsigned G, unsigned b) {
@@ -935,7 +935,7 @@ gemv_tc_mlp_kernel(const __grid_constant__ CUtensorMap w_map0, const __grid_cons
                         }
                     }
                     // (both calls contain warp shuffles or none: `store` is uniform over the warp)
-                    if (store && __any_sync(0xffffffffu, tot != tot)) redo = min(redo, tile);
+                    if (store && __any_sync(0xffffffffu, tc_not_finite(tot))) redo = min(redo, tile);
                     if (store && tile < redo) {
                         if (p == 0) tc_store<TEPI_SILU_MUL>(tot, row, lane, M, act, fz);
                         else tc_store<TEPI_RESIDUAL>(tot, row, lane, M, h, fz);

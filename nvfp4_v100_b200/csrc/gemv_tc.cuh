@@ -103,8 +103,12 @@ __device__ __forceinline__ void tc_digit_planes(const uint4 xv, uint8_t* btile, 
     if ((lane & 1) == 0) lbytes[lane >> 1] = (uint8_t)(em == 31u ? 255 : L + 125);
 }
 
-// A row's sum in plain fp32, block by block, as the register-streaming kernels form it: for sums that came out as NaN (an
-// activation that is not finite).  load(k): the activations k .. k + 7.
+// Whether a row has to be formed by tc_plain_row.  An infinity too: a digit column's part of a sum can overflow where the
+// sum does not (scale bytes near 254).
+__device__ __forceinline__ bool tc_not_finite(float sum) { return !(fabsf(sum) <= 3.402823466e38f); }
+// A row's sum in plain fp32, block by block, as the register-streaming kernels form it: for sums that are not finite (an
+// activation that is not; a scale byte of 255, which is infinity here and NaN to the tensor core).  load(k): the
+// activations k .. k + 7.
 template <typename LOAD>
 __device__ __noinline__ float tc_plain_row(const uint8_t* packed, const uint8_t* scales, const LOAD load, int row, int K) {
     const uint8_t* w = packed + (size_t)row * (K / 2);

@@ -14,8 +14,8 @@
 //   warp 1      MMA issuer: four MMAs M128 N32 K64 a stage
 //   warps 2..5  scale bytes of the weights and of the digit columns -> tensor memory
 //   warps 6..9  digit conversion, a warp one activation of every other stage; then the sums of their rows
-// An activation with a value that is not finite has no digits: its sums are NaN, and its rows are then summed in plain fp32
-// from global memory.
+// An activation with a value that is not finite has no digits: its sums are NaN, and rows that are not finite are summed in
+// plain fp32 from global memory.
 // Every wait is bounded and reported through nvfp4_gemv_tc_status (20 + id).
 //
 // Measured: at gemv_tc2_takes.
@@ -248,7 +248,7 @@ gemv_tc2_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         for (int t = 0; t < 2; t++) {
             float tot = s_red[0][t][r];
             for (int c = 1; c < split; c++) tot += s_red[c][t][r];
-            if (tot != tot) tot = tc_plain_row(packed, scales, T2Load<IL>{x0, x1, t}, row, K);
+            if (tc_not_finite(tot)) tot = tc_plain_row(packed, scales, T2Load<IL>{x0, x1, t}, row, K);
             y[(size_t)t * M + row] = __float2half(tot);
         }
 }
