@@ -3,21 +3,32 @@
 // Token by token (a value head's state S is 128 rows of 128; e^g decay, beta update strength, q and k L2-normalised)
 //   delta_t = beta_t (v_t - e^g_t S k_t),  S <- e^g_t S + delta_t k_t^T,  o_t = S q_t.
 // For a block of C = 64 tokens that meets the state S, with P(j..i) = e^g_j ... e^g_i and G_i = P(0..i):
-//   R_i  = v_i - G_i S k_i                                      all products with the state that enters
-//   (I + A) delta = beta R,   A[i][m] = beta_i P(m+1..i) k_i.k_m  (m < i)
-//   delta = T R,              T = (I + A)^-1 diag(beta)           one 64 x 64 matrix per head and block
+//   R_i  = beta_i (v_i - G_i S k_i)                             all products with the state that enters
+//   (I + A) delta = R,        A[i][m] = beta_i P(m+1..i) k_i.k_m  (m < i)
+//   delta = X R,              X = (I + A)^-1                      one 64 x 64 matrix per head and block
 //   o_i  = G_i S q_i + sum_{j<=i} D[i][j] delta_j,  D[i][j] = P(j+1..i) q_i.k_j
 //   S   <- G_63 S + sum_i P(i+1..63) delta_i k_i^T
-// which is the same algebra with five contractions in the place of a chain of 64 steps.  T and D depend on q, k,
+// which is the same algebra with five contractions in the place of a chain of 64 steps.  X and D depend on q, k,
 // beta and g only: dn_chunk_prep_kernel makes them for all heads and blocks at once, and the chain that is left
 // (dn_chunk_scan_kernel) runs over n / 64 blocks.
 //
 // Precision: q and k are fp16 numbers times an fp32 norm, so the raw fp16 numbers are EXACT tensor-core operands and
-// the norms scale the results.  The fp32 operands (S, R, delta, T, D) enter as two fp16 numbers whose sum is within
-// 2^-24 of the value, an fp32 rounding: a row is scaled by a power of two that puts its largest element at
-// 2^14..2^15, so that elements down to 2^-29 of the row's largest keep that relative error and smaller ones are within
-// 2^-40 of the largest.  Products of two split operands leave out low x low (2^-24 of the product).  Sums are fp32, and a
-// block's update is summed on its own before it meets the state, so the state is rounded once per block.
+// the norms scale the results.  The fp32 operands (S, R, delta, X, D) enter as two fp16 numbers: a row is scaled by a
+// power of two that puts its largest element at 2^14..2^15, the first number is the element rounded to fp16 and the second
+// 2^11 times what that leaves, with an accumulator of its own.  Together they hold 23 bits: within 2^-23 of the element
+// down to 2^-28 of the row's largest, and within 2^-51 of the largest below.  (Without the 2^11 the second number goes
+// subnormal from 2^-16 of the largest on: a token beside one 2^20 times as large kept 9 bits.)  fp32 has 24, so what is
+// not a sum of many such products is kept out of them: X's unit diagonal and D's diagonal are applied in fp32, and delta
+// times its factor meets the state as three numbers, which hold more than fp32 does.  Products of two split operands leave
+// out low x low (2^-24 of the product).  Sums are fp32, and a block's update is summed on its own before it meets the
+// state, so the state is rounded once per block.
+// Measured against float64 from the same fp16 q, k, v (16 / 48 heads), four tokens at a time / this.  Error of the state, and
+// share of the outputs that are not the correctly rounded fp16:
+//   usual decays        512 tokens 6.9e-8 / 5.5e-8, 6.8e-5 / 5.2e-5       100 tokens 8.8e-8 / 6.3e-8, 7.3e-5 / 6.0e-5
+//   hardly any decay    512 tokens 5.1e-6 / 3.1e-7, 7.5e-3 / 1.3e-3       100 tokens 1.4e-6 / 2.3e-7, 1.7e-3 / 9.6e-4
+//   that and keys alike 512 tokens 4.4e-6 / 9.3e-7, 9.0e-3 / 3.5e-3       100 tokens 1.2e-6 / 5.3e-7, 2.1e-3 / 2.4e-3
+//   large tokens first  512 tokens 7.7e-7 / 1.7e-7, 1.8e-4 / 1.0e-4       100 tokens 4.8e-7 / 1.2e-7, 1.8e-4 / 1.0e-4
+// (With two numbers everywhere the first line is 1.0e-7, 1.4e-4, and without the 2^11 the last one 2.0e-5, 3.3e-2.)
 #include <cstddef>
 
 #include "common.cuh"
@@ -37,15 +48,17 @@ struct __align__(16) DcKQ {
 };
 // per value head and block
 struct __align__(16) DcHead {
-    __half t_hi[CH][TLD], t_lo[CH][TLD];            // T, row i times a power of two (its inverse in t_inv[i])
-    __half d_hi[CH][TLD], d_lo[CH][TLD];            // D, the same
-    float t_inv[CH], d_inv[CH];
+    __half x_hi[CH][TLD], x_lo[CH][TLD];            // X below its diagonal, row i times a power of two (inverse in x_inv[i])
+    __half d_hi[CH][TLD], d_lo[CH][TLD];            // D below its diagonal, the same
+    float x_inv[CH], d_inv[CH];
+    float beta[CH];
+    float d_diag[CH];                               // D's diagonal: q_i.k_i
     float ksc[CH];                                  // G_i / |k_i|
     float qsc[CH];                                  // G_i / |q_i| / sqrt(128)
-    float usc[CH];                                  // P(i+1..63) / |k_i|
+    float usc[CH], usl[CH];                         // P(i+1..63) / |k_i| and what its rounding to fp32 leaves
     float glast[4];                                 // G_63
     // for the token-by-token form (non-finite values only)
-    float eg[CH], beta[CH], ik[CH], iq[CH];
+    float eg[CH], ik[CH], iq[CH];
 };
 static_assert(sizeof(DcKQ) % 16 == 0 && sizeof(DcHead) % 16 == 0, "copied in 16-byte pieces");
 constexpr int DC_HEAD_COPY = (int)offsetof(DcHead, eg);      // bytes the scan stages
@@ -78,13 +91,31 @@ __device__ __forceinline__ void dc_scale(float mx, float& s, float& inv) {
     s = __uint_as_float((uint32_t)(268 - ex) << 23);
     inv = __uint_as_float((uint32_t)(ex - 14) << 23);
 }
+constexpr float DC_LO = 2048.0f, DC_LO_INV = 1.0f / 2048.0f;     // what a low half is scaled by
 // Two fp32 numbers -> hi and lo fp16 pairs.
 __device__ __forceinline__ void dc_split(float x, float y, uint32_t& hi, uint32_t& lo) {
     const __half2 h = __floats2half2_rn(x, y);
     const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+    const __half2 l = __floats2half2_rn((x - f.x) * DC_LO, (y - f.y) * DC_LO);
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+// The products x (u.x + ul.x) and y (u.y + ul.y), times s, as three fp16 pairs, the last on the scale of lo: what rounding
+// the product to fp32 leaves goes into them as well.  (s, a power of two, only ever meets the product: it can be as large
+// as that is small.)
+__device__ __forceinline__ void dc_split3(float x, float y, const float2 u, const float2 ul, float s, uint32_t& hi,
+                                          uint32_t& lo, uint32_t& rest) {
+    const float px = x * u.x, py = y * u.y;
+    const float ex = fmaf(x, ul.x, fmaf(x, u.x, -px)), ey = fmaf(y, ul.y, fmaf(y, u.y, -py));
+    const __half2 h = __floats2half2_rn(px * s, py * s);
+    const float2 f = __half22float2(h);
+    const float rx = fmaf(ex, s, fmaf(px, s, -f.x)) * DC_LO, ry = fmaf(ey, s, fmaf(py, s, -f.y)) * DC_LO;
+    const __half2 l = __floats2half2_rn(rx, ry);
+    const float2 g = __half22float2(l);
+    const __half2 r = __floats2half2_rn(rx - g.x, ry - g.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+    rest = *reinterpret_cast<const uint32_t*>(&r);
 }
 __device__ __forceinline__ float dc_quad_max(float v) {
     v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
@@ -108,7 +139,7 @@ __device__ __forceinline__ double dc_rsqrt(double s) {
 }
 __device__ __forceinline__ float dc_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
-// One CTA per (value head, block): T and D with their scales, the scales of the other products, and (first value
+// One CTA per (value head, block): X and D with their scales, the scales of the other products, and (first value
 // head of a key head) the block's keys and queries.  k.k and q.k are tensor-core products of the raw fp16 numbers.  The
 // inverse of I + A (unit lower triangular) goes by blocks: 16 x 16 by substitution, a thread per column, then twice
 // [X1 0; -X2 A21 X1, X2].  Sums run over the lower triangle only, so that a token with a non-finite value does
@@ -251,8 +282,15 @@ dn_chunk_prep_kernel(const __half* __restrict__ conv_out, int conv_dim, const __
                 if (p <= mt) {
                     uint32_t b[4];
                     dc_ldsm(b, &s.kq.k[p * 16 + (lane >> 4) * 8 + (lane & 7)][kk * 16 + ((lane >> 3) & 1) * 8]);
-                    dc_mma(acc[2 * p], a, b[0], b[1]);
-                    dc_mma(acc[2 * p + 1], a, b[2], b[3]);
+                    // (sixteen products at a time: the tensor core truncates the sum it adds to, the addition here rounds)
+                    float c0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, c1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                    dc_mma(c0, a, b[0], b[1]);
+                    dc_mma(c1, a, b[2], b[3]);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        acc[2 * p][e] += c0[e];
+                        acc[2 * p + 1][e] += c1[e];
+                    }
                 }
         }
         const int r = mt * 16 + (lane >> 2), c = (lane & 3) * 2;
@@ -300,7 +338,9 @@ dn_chunk_prep_kernel(const __half* __restrict__ conv_out, int conv_dim, const __
                 for (int e = 0; e < 4; e++) {
                     const int j = j0 + e;
                     const float p = dc_exp(gi, s.g2[j]) * kk[e];
-                    dv[e4 * 4 + e] = j <= i ? p * (iqi * dd[e]) : 0.0f;    // (selected, not multiplied: above the
+                    const float d = p * (iqi * dd[e]);
+                    if (j == i) out.d_diag[i] = d;
+                    dv[e4 * 4 + e] = j < i ? d : 0.0f;                     // (selected, not multiplied: above the
                     av[e] = j < i ? p * (bk * aa[e]) : 0.0f;               // diagonal there is nothing to trust)
                 }
             }
@@ -311,7 +351,9 @@ dn_chunk_prep_kernel(const __half* __restrict__ conv_out, int conv_dim, const __
             const double gam = exp(s.g[i]), tail = exp(s.g[CH - 1] - s.g[i]);
             out.ksc[i] = (float)(gam * s.ikd[i]);
             out.qsc[i] = (float)(gam * s.iqd[i]);
-            out.usc[i] = (float)(tail * s.ikd[i]);
+            const double us = tail * s.ikd[i];
+            out.usc[i] = (float)us;
+            out.usl[i] = (float)(us - (double)(float)us);
             out.eg[i] = s.eg[i];
             out.beta[i] = s.beta[i];
             out.ik[i] = s.ik[i];
@@ -393,22 +435,21 @@ dn_chunk_prep_kernel(const __half* __restrict__ conv_out, int conv_dim, const __
     }
     __syncthreads();
     {
-        float tv[16];
+        float xv[16];
 #pragma unroll
         for (int e4 = 0; e4 < 4; e4++) {
             const int m0 = part * 16 + e4 * 4;
             const float4 x4 = *reinterpret_cast<const float4*>(&s.inv.x[i][m0]);
-            const float4 b4 = *reinterpret_cast<const float4*>(&s.beta[m0]);
-            const float xx[4] = {x4.x, x4.y, x4.z, x4.w}, bb[4] = {b4.x, b4.y, b4.z, b4.w};
+            const float xx[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
-            for (int e = 0; e < 4; e++) tv[e4 * 4 + e] = m0 + e <= i ? xx[e] * bb[e] : 0.0f;
+            for (int e = 0; e < 4; e++) xv[e4 * 4 + e] = m0 + e < i ? xx[e] : 0.0f;
         }
-        store_row(tv, &out.t_hi[i][part * 16], &out.t_lo[i][part * 16], &out.t_inv[i]);
+        store_row(xv, &out.x_hi[i][part * 16], &out.x_lo[i][part * 16], &out.x_inv[i]);
     }
 }
 
 // The tokens of one block for a warp's 16 rows, one after the other: for blocks in which something is not finite,
-// where a product with a zero of T or D would spread it to earlier tokens.  The state rows are in global memory.
+// where a product with a zero of X or D would spread it to earlier tokens.  The state rows are in global memory.
 __device__ __noinline__ void dn_chunk_plain(float* state, const DcHead* head, const DcKQ* kq, const __half* v,
                                             int conv_dim, __half* o, int ldo, int count, int lane) {
     for (int r = 0; r < 16; r++) {
@@ -434,7 +475,7 @@ __device__ __noinline__ void dn_chunk_plain(float* state, const DcHead* head, co
 // The chain.  A pair of warps owns 16 rows of a head's state.  The first one, the chain warp, holds them as the
 // accumulators of sixteen m16n8 tiles (dims 8 j .. 8 j + 7 in tile j) and goes from block to block: R, delta, next state.
 // The second one, the output warp, makes o from the operands the first one leaves in shared memory (the split state that
-// enters the block, the split delta), and requests the next block's k, q, T, D and v.  Two accumulator tiles packed
+// enters the block, delta), and requests the next block's k, q, X, D and v.  Two accumulator tiles packed
 // to fp16 are the A operand of the next product, so what all rows share is all that has to pass through shared memory.
 // The products of the small halves have accumulators of their own: the tensor core truncates the sum it adds to,
 // and those of the large halves are then 8 (S k, S q) or up to 4 (the others) additions long.
@@ -447,8 +488,8 @@ struct DcScanSmem {
         __half v[CH][VLD];
     } stage[2];
     uint4 s_hi[W][8][32], s_lo[W][8][32];           // A operands: the state that enters the block, 16 dims each
-    uint4 d_hi[W][4][32], d_lo[W][4][32];           // delta, 16 tokens each
-    float2 s_inv[W][32], d_inv[W][32];              // what the rows g and g + 8 were scaled by
+    float4 delta[W][8][32];                         // delta, 8 tokens each
+    float2 s_inv[W][32];                            // what the rows g and g + 8 were scaled by
     int plain[W];
 };
 
@@ -580,24 +621,33 @@ dn_chunk_scan_kernel(const DcKQ* __restrict__ kq, const DcHead* __restrict__ hea
 #pragma unroll
             for (int nt = 0; nt < 8; nt++) {
                 const float2 qs = *reinterpret_cast<const float2*>(&hd.qsc[nt * 8 + t4 * 2]);
-                qh[nt][0] = (qh[nt][0] + ql[nt][0]) * si.x * qs.x;
-                qh[nt][1] = (qh[nt][1] + ql[nt][1]) * si.x * qs.y;
-                qh[nt][2] = (qh[nt][2] + ql[nt][2]) * si.y * qs.x;
-                qh[nt][3] = (qh[nt][3] + ql[nt][3]) * si.y * qs.y;
+                qh[nt][0] = fmaf(ql[nt][0], DC_LO_INV, qh[nt][0]) * si.x * qs.x;
+                qh[nt][1] = fmaf(ql[nt][1], DC_LO_INV, qh[nt][1]) * si.x * qs.y;
+                qh[nt][2] = fmaf(ql[nt][2], DC_LO_INV, qh[nt][2]) * si.y * qs.x;
+                qh[nt][3] = fmaf(ql[nt][3], DC_LO_INV, qh[nt][3]) * si.y * qs.y;
             }
             dc_pair_sync(1 + w);                             // delta is there; the entering state has been read
             if (sm.plain[w]) continue;                       // (the chain warp writes this block's outputs)
-            float oh[8][4], ol[8][4];
+            float oh[8][4], ol[8][4], dl[8][4], s0, s1, i0, i1;
+#pragma unroll
+            for (int nt = 0; nt < 8; nt++) {
+                const float4 d4 = sm.delta[w][nt][lane];
+                const float2 dd = *reinterpret_cast<const float2*>(&hd.d_diag[nt * 8 + t4 * 2]);
+                dl[nt][0] = d4.x; dl[nt][1] = d4.y; dl[nt][2] = d4.z; dl[nt][3] = d4.w;
+                qh[nt][0] = fmaf(d4.x, dd.x, qh[nt][0]);
+                qh[nt][1] = fmaf(d4.y, dd.y, qh[nt][1]);
+                qh[nt][2] = fmaf(d4.z, dd.x, qh[nt][2]);
+                qh[nt][3] = fmaf(d4.w, dd.y, qh[nt][3]);
+            }
+            dc_row_scales(dl, s0, s1, i0, i1);
             dc_zero(oh);
             dc_zero(ol);
 #pragma unroll
             for (int m = 0; m < 4; m++) {
                 uint32_t hi[4], lo[4];
-                dc_from(sm.d_hi[w][m][lane], hi);
-                dc_from(sm.d_lo[w][m][lane], lo);
+                dc_operand(dl[2 * m], dl[2 * m + 1], s0, s1, hi, lo);
                 dc_triangle(oh, ol, hi, lo, m, hd.d_hi, hd.d_lo, lr, lc);
             }
-            const float2 dv = sm.d_inv[w][lane];
             __half* op = o_out + ((size_t)(c * CH + t4 * 2) * nv + h) * DC + row0 + g;
 #pragma unroll
             for (int nt = 0; nt < 8; nt++) {
@@ -607,8 +657,8 @@ dn_chunk_scan_kernel(const DcKQ* __restrict__ kq, const DcHead* __restrict__ hea
                     if (nt * 8 + t4 * 2 + u < count) {
                         const float dt = u ? di.y : di.x;
                         __half* o = op + (size_t)(nt * 8 + u) * nv * DC;
-                        o[0] = __float2half(fmaf((oh[nt][u] + ol[nt][u]) * dv.x, dt, qh[nt][u]));
-                        o[8] = __float2half(fmaf((oh[nt][2 + u] + ol[nt][2 + u]) * dv.y, dt, qh[nt][2 + u]));
+                        o[0] = __float2half(fmaf(fmaf(ol[nt][u], DC_LO_INV, oh[nt][u]) * i0, dt, qh[nt][u]));
+                        o[8] = __float2half(fmaf(fmaf(ol[nt][2 + u], DC_LO_INV, oh[nt][2 + u]) * i1, dt, qh[nt][2 + u]));
                     }
             }
         }
@@ -654,7 +704,7 @@ dn_chunk_scan_kernel(const DcKQ* __restrict__ kq, const DcHead* __restrict__ hea
         if (!active) continue;
         const typename DcScanSmem<W>::Stage& s = sm.stage[c & 1];
         const DcHead& hd = *reinterpret_cast<const DcHead*>(s.head);
-        // ---- S k, raw; R = v - G S k ----
+        // ---- S k, raw; R = beta (v - G S k) ----
         float r[8][4], rl[8][4];
         dc_zero(r);
         dc_zero(rl);
@@ -683,13 +733,14 @@ dn_chunk_scan_kernel(const DcKQ* __restrict__ kq, const DcHead* __restrict__ hea
                 const float2 v0 = __half22float2(*reinterpret_cast<const __half2*>(&v[2 * u]));
                 const float2 v1 = __half22float2(*reinterpret_cast<const __half2*>(&v[2 * u + 1]));
                 const float2 ks = *reinterpret_cast<const float2*>(&hd.ksc[nt * 8 + t4 * 2]);
-                r[nt][0] = fmaf(-(r[nt][0] + rl[nt][0]) * inv0, ks.x, v0.x);
-                r[nt][1] = fmaf(-(r[nt][1] + rl[nt][1]) * inv0, ks.y, v0.y);
-                r[nt][2] = fmaf(-(r[nt][2] + rl[nt][2]) * inv1, ks.x, v1.x);
-                r[nt][3] = fmaf(-(r[nt][3] + rl[nt][3]) * inv1, ks.y, v1.y);
+                const float2 bt = *reinterpret_cast<const float2*>(&hd.beta[nt * 8 + t4 * 2]);
+                r[nt][0] = fmaf(-fmaf(rl[nt][0], DC_LO_INV, r[nt][0]) * inv0, ks.x, v0.x) * bt.x;
+                r[nt][1] = fmaf(-fmaf(rl[nt][1], DC_LO_INV, r[nt][1]) * inv0, ks.y, v0.y) * bt.y;
+                r[nt][2] = fmaf(-fmaf(rl[nt][2], DC_LO_INV, r[nt][2]) * inv1, ks.x, v1.x) * bt.x;
+                r[nt][3] = fmaf(-fmaf(rl[nt][3], DC_LO_INV, r[nt][3]) * inv1, ks.y, v1.y) * bt.y;
             }
         }
-        // ---- delta = T R ----
+        // ---- delta = X R ----
         float i0, i1, dh[8][4], dl[8][4];
         dc_row_scales(r, s0, s1, i0, i1);
         dc_zero(dh);
@@ -698,30 +749,23 @@ dn_chunk_scan_kernel(const DcKQ* __restrict__ kq, const DcHead* __restrict__ hea
         for (int m = 0; m < 4; m++) {
             uint32_t hi[4], lo[4];
             dc_operand(r[2 * m], r[2 * m + 1], s0, s1, hi, lo);
-            dc_triangle(dh, dl, hi, lo, m, hd.t_hi, hd.t_lo, lr, lc);
+            dc_triangle(dh, dl, hi, lo, m, hd.x_hi, hd.x_lo, lr, lc);
         }
         float bad = 0.0f;
 #pragma unroll
         for (int nt = 0; nt < 8; nt++) {
-            const float2 ti = *reinterpret_cast<const float2*>(&hd.t_inv[nt * 8 + t4 * 2]);
-            dh[nt][0] = (dh[nt][0] + dl[nt][0]) * i0 * ti.x;
-            dh[nt][1] = (dh[nt][1] + dl[nt][1]) * i0 * ti.y;
-            dh[nt][2] = (dh[nt][2] + dl[nt][2]) * i1 * ti.x;
-            dh[nt][3] = (dh[nt][3] + dl[nt][3]) * i1 * ti.y;
+            const float2 xi = *reinterpret_cast<const float2*>(&hd.x_inv[nt * 8 + t4 * 2]);
+            dh[nt][0] = fmaf(fmaf(dl[nt][0], DC_LO_INV, dh[nt][0]) * i0, xi.x, r[nt][0]);
+            dh[nt][1] = fmaf(fmaf(dl[nt][1], DC_LO_INV, dh[nt][1]) * i0, xi.y, r[nt][1]);
+            dh[nt][2] = fmaf(fmaf(dl[nt][2], DC_LO_INV, dh[nt][2]) * i1, xi.x, r[nt][2]);
+            dh[nt][3] = fmaf(fmaf(dl[nt][3], DC_LO_INV, dh[nt][3]) * i1, xi.y, r[nt][3]);
 #pragma unroll
             for (int e = 0; e < 4; e++) bad = fmaf(dh[nt][e], 0.0f, bad);       // NaN if one of them is not finite
         }
         const bool plain = __any_sync(0xffffffffu, bad != 0.0f);                // (NaN != 0)
         if (!plain) {
-            dc_row_scales(dh, s0, s1, i0, i1);
-            sm.d_inv[w][lane] = make_float2(i0, i1);
 #pragma unroll
-            for (int m = 0; m < 4; m++) {
-                uint32_t hi[4], lo[4];
-                dc_operand(dh[2 * m], dh[2 * m + 1], s0, s1, hi, lo);
-                sm.d_hi[w][m][lane] = dc_u4(hi);
-                sm.d_lo[w][m][lane] = dc_u4(lo);
-            }
+            for (int nt = 0; nt < 8; nt++) sm.delta[w][nt][lane] = make_float4(dh[nt][0], dh[nt][1], dh[nt][2], dh[nt][3]);
         }
         if (lane == 0) sm.plain[w] = plain;
         dc_pair_sync(1 + w);
@@ -735,15 +779,27 @@ dn_chunk_scan_kernel(const DcKQ* __restrict__ kq, const DcHead* __restrict__ hea
             load_state();
         } else {
             // ---- S <- G_63 S + sum_i P(i+1..63) delta_i k_i^T ----
+            {
+                float u[8][4];
 #pragma unroll
-            for (int nt = 0; nt < 8; nt++) {
-                const float2 us = *reinterpret_cast<const float2*>(&hd.usc[nt * 8 + t4 * 2]);
-                dh[nt][0] *= us.x; dh[nt][1] *= us.y; dh[nt][2] *= us.x; dh[nt][3] *= us.y;
+                for (int nt = 0; nt < 8; nt++) {
+                    const float2 us = *reinterpret_cast<const float2*>(&hd.usc[nt * 8 + t4 * 2]);
+                    u[nt][0] = dh[nt][0] * us.x; u[nt][1] = dh[nt][1] * us.y;
+                    u[nt][2] = dh[nt][2] * us.x; u[nt][3] = dh[nt][3] * us.y;
+                }
+                dc_row_scales(u, s0, s1, i0, i1);
             }
-            dc_row_scales(dh, s0, s1, i0, i1);
-            uint32_t hi[4][4], lo[4][4];
+            uint32_t hi[4][4], lo[4][4], rest[4][4];
 #pragma unroll
-            for (int m = 0; m < 4; m++) dc_operand(dh[2 * m], dh[2 * m + 1], s0, s1, hi[m], lo[m]);
+            for (int m = 0; m < 4; m++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {        // (dc_operand's order)
+                    const int nt = 2 * m + (e >> 1);
+                    dc_split3(dh[nt][(e & 1) * 2], dh[nt][(e & 1) * 2 + 1],
+                              *reinterpret_cast<const float2*>(&hd.usc[nt * 8 + t4 * 2]),
+                              *reinterpret_cast<const float2*>(&hd.usl[nt * 8 + t4 * 2]), (e & 1) ? s1 : s0, hi[m][e],
+                              lo[m][e], rest[m][e]);
+                }
             const float gl = hd.glast[0];
 #pragma unroll
             for (int jj = 0; jj < 4; jj++) {
@@ -763,14 +819,18 @@ dn_chunk_scan_kernel(const DcKQ* __restrict__ kq, const DcHead* __restrict__ hea
                     dc_mma(ul[1], lo[m], b0[2], b0[3]);
                     dc_mma(ul[2], lo[m], b1[0], b1[1]);
                     dc_mma(ul[3], lo[m], b1[2], b1[3]);
+                    dc_mma(ul[0], rest[m], b0[0], b0[1]);
+                    dc_mma(ul[1], rest[m], b0[2], b0[3]);
+                    dc_mma(ul[2], rest[m], b1[0], b1[1]);
+                    dc_mma(ul[3], rest[m], b1[2], b1[3]);
                 }
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const int j = jj * 4 + i;
-                    S[j][0] = fmaf(S[j][0], gl, (uh[i][0] + ul[i][0]) * i0);
-                    S[j][1] = fmaf(S[j][1], gl, (uh[i][1] + ul[i][1]) * i0);
-                    S[j][2] = fmaf(S[j][2], gl, (uh[i][2] + ul[i][2]) * i1);
-                    S[j][3] = fmaf(S[j][3], gl, (uh[i][3] + ul[i][3]) * i1);
+                    S[j][0] = fmaf(S[j][0], gl, fmaf(ul[i][0], DC_LO_INV, uh[i][0]) * i0);
+                    S[j][1] = fmaf(S[j][1], gl, fmaf(ul[i][1], DC_LO_INV, uh[i][1]) * i0);
+                    S[j][2] = fmaf(S[j][2], gl, fmaf(ul[i][2], DC_LO_INV, uh[i][2]) * i1);
+                    S[j][3] = fmaf(S[j][3], gl, fmaf(ul[i][3], DC_LO_INV, uh[i][3]) * i1);
                 }
             }
         }
@@ -779,12 +839,24 @@ dn_chunk_scan_kernel(const DcKQ* __restrict__ kq, const DcHead* __restrict__ hea
     if (active) store_state();
 }
 
-// A layer of 16 key heads, us, four tokens at a time / blocks of 64 (conv, gated norm and launches included):
-//   48 value heads: 80 tokens 31.7 / 35.9, 100: 37.7 / 36.0, 128: 45.9 / 36.5, 512: 142 / 71, 1024: 279 / 137
-//   64: 64 tokens 33.5 / 31.7, 512: 183 / 88      24: 129 tokens 39.2 / 42.7, 160: 43.9 / 39.8, 512: 109 / 64
-//   12: 200 tokens 39.8 / 46.0, 256: 48.6 / 45.3, 512: 83 / 60      1: 100 tokens 22.4 / 22.2, 512: 79 / 47
-// A block costs 4 us of chain however few heads there are; four tokens cost less the fewer there are.
-bool dn_chunk_takes(int n, int nv) { return n >= (nv >= 56 ? 64 : nv >= 40 ? 100 : nv >= 20 ? 160 : 256); }
+// us of a layer, four tokens at a time / blocks of 64 (conv, gated norm and launches included):
+//   64 value heads: 64 tokens 31.6 / 29.6, 72: 34.8 / 37.4, 512: 178 / 90     56: 64 tokens 31.4 / 29.3, 80: 36.7 / 37.2
+//   48: 100 tokens 37.4 / 37.3, 128: 45.5 / 38.2, 512: 142 / 76, 1024: 279 / 146       40: 100 tokens 36.0 / 36.9, 112: 38.9 / 36.6
+//   24: 160 tokens 43.7 / 44.4, 176: 46.4 / 45.0, 512: 109 / 69               20: 160 tokens 42.5 / 40.5
+//   18: 256 tokens 47.5 / 51.0    12: 256 tokens 48.5 / 49.7, 288: 52.7 / 54.5, 320: 56.9 / 54.5, 512: 83 / 70
+//   1: 256 tokens 44.4 / 36.5
+// The one takes a time per token, more with more heads; the other one per block, the last block's empty places included.
+// Both lines in ns, as fitted to the above; chunks shorter than those were not tried.
+bool dn_chunk_takes(int n, int nv) {
+    if (n < (nv < 20 ? 256 : 64)) return false;
+    const int blocks = (n + CH - 1) / CH;
+    const long long four = 10500 + (long long)n * (nv < 20 ? 140 : 130 + 3LL * nv);
+    const long long b64 = nv >= 56   ? 22000 + 7500LL * blocks
+                          : nv >= 40 ? 25000 + 6300LL * blocks
+                          : nv >= 20 ? 25500 + 1000LL * (nv < 24 ? nv - 20 : 4) + 5000LL * blocks
+                                     : 17000 + 1000LL * (nv < 13 ? nv : 13) + 5000LL * blocks;
+    return b64 < four;
+}
 
 long long dn_chunk_work_bytes(int n, int nk, int nv) {
     const long long nblk = (n + CH - 1) / CH;

@@ -19,6 +19,7 @@
 //       blocks of 64 on the tensor cores (dn_chunk.cu); gated norm.
 // Attention uses the chunk forms of attn_prep (decode_ops.cu) and launch_attn_prefill: the tensor-core
 // kernel (attn_prefill_tc.cu) or, for small chunks, attn_prefill_group_kernel (fused_ops.cu).
+#include <algorithm>
 #include <cstdio>
 
 #include "common.cuh"
@@ -745,14 +746,14 @@ long long nvfp4_dn_prefill_work_bytes(int n, int nk, int nv) {
     const long long conv_dim = (2LL * nk + nv) * PF_DK;
     long long b = (long long)n * conv_dim * 2;            // conv output, fp16
     b = (b + 255) & ~255LL;
-    if (nvfp4::dn_chunk_takes(n, nv)) {
-        b += nvfp4::dn_chunk_work_bytes(n, nk, nv);
-    } else {
-        const long long nb = (n + DNB - 1) / DNB;          // blocks of the recurrence
-        b += 2LL * nb * DNB * nk * PF_DK * 4;              // normalised q and k, fp32
-        b += nb * nv * (long long)sizeof(nvfp4::DnBlock);  // the blocks' coefficients
-        b = (b + 255) & ~255LL;
-    }
+    const long long nb = (n + DNB - 1) / DNB;              // blocks of the recurrence
+    long long blocks = 2LL * nb * DNB * nk * PF_DK * 4;    // normalised q and k, fp32
+    blocks += nb * nv * (long long)sizeof(nvfp4::DnBlock); // the blocks' coefficients
+    blocks = (blocks + 255) & ~255LL;
+    // (never less than for fewer tokens: 64 of 64 heads go in one block of 64, 65 four at a time, which takes less)
+    if (nvfp4::dn_chunk_takes(n, nv) || nvfp4::dn_chunk_takes(n / 64 * 64, nv))
+        blocks = std::max(blocks, nvfp4::dn_chunk_work_bytes(n, nk, nv));
+    b += blocks;
     b += (long long)n * nv * PF_DK * 2;                    // recurrence output, fp16
     return b + 256;
 }

@@ -66,7 +66,9 @@ def reference(t, nk, nv, n, dtype):
 # one, two, three and four row groups per CTA (the last head part of three is short), and more CTAs than SMs; chunks
 # that end with a block, one token into it, one before its end
 @pytest.mark.parametrize("nk,nv,n", [(1, 1, 256), (2, 6, 257), (3, 12, 319), (5, 20, 160), (10, 20, 193), (20, 40, 100),
-                                     (8, 40, 127), (8, 40, 128), (56, 56, 64), (28, 56, 65), (10, 80, 129)])
+                                     (8, 40, 127), (8, 40, 128), (56, 56, 64), (28, 56, 65), (10, 80, 129),
+                                     # (those of them that four tokens at a time take, a little longer)
+                                     (3, 12, 321), (20, 40, 112), (28, 56, 97)])
 @pytest.mark.parametrize("decay", ["usual", "strong", "none"])
 def test_blocks_of_64_against_float64(lib, nk, nv, n, decay):
     t, ld = inputs(nk, nv, n, decay)
@@ -79,6 +81,12 @@ def test_blocks_of_64_against_float64(lib, nk, nv, n, decay):
     # without decay a state forgets little: its fp32 error is far above its roundings, and differs by the order of sums.)
     err = lambda a: (a.double() - want_S).norm() / want_S.norm()
     assert err(S) <= 3 * err(plain_S) + 2 ** -20, (err(S), err(plain_S))
+    # every head, and every head's output of every token (three fp16 steps of each value are 3 * 2^-11 of the row, halved
+    # and doubled within a binade)
+    norm = lambda a: a.flatten(1).norm(dim=1)
+    assert (norm(S.double() - want_S) <= 3 * norm(plain_S.double() - want_S) + 2 ** -20 * norm(want_S)).all()
+    rows = lambda a: a.double().view(n * nv, 128).norm(dim=1)
+    assert (rows(out.double() - want.double()) <= 2 ** -8 * rows(want)).all()
     steps = ulp_diff_f16(out.cpu().numpy(), want.cpu().numpy())
     assert (steps <= 1).mean() > 0.98 and (steps <= 3).mean() > 0.999, ((steps <= 1).mean(), steps.max())
 
@@ -111,3 +119,105 @@ def test_a_token_that_is_not_finite_stays_out_of_earlier_ones(lib):
     S3, out = run(lib, t, ld, nk, nv, n)
     assert torch.isfinite(out[:bad]).all() and not torch.isfinite(out[bad:, :128 * (nv // nk)]).any()
     assert torch.isfinite(out[:, 128 * (nv // nk):]).all()
+
+
+def real_inputs(nk, nv, n, seed):
+    """What a decoder layer meets: small conv weights, decays of e^-0.001 to e^-20 and more, a state in use."""
+    g = torch.Generator().manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g)
+    C = (2 * nk + nv) * 128
+    ld = C + nv * 128 + 2 * nv
+    t = dict(x=r(n, ld), conv_w=r(C, 4) * 0.02, conv_state=r(C, 4), A_log=torch.log(torch.rand(nv, generator=g) * 16 + 1e-3),
+             dt_bias=torch.ones(nv), norm_w=torch.ones(128))
+    t = {k: v.half().cuda() for k, v in t.items()}
+    t["state"] = (r(nv, 128, 128) * 0.1).cuda()
+    return t, ld
+
+
+def float64_state(t, ld, conv_out, nk, nv, n):
+    """The state after the chunk in 64 bits, from the fp16 conv outputs and the fp16 beta."""
+    C = (2 * nk + nv) * 128
+    x, co = t["x"].double(), conv_out.double()
+    unit = lambda v: (v / torch.sqrt((v * v).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(nv // nk, 1)
+    k = unit(co[:, nk * 128:2 * nk * 128].view(n, nk, 128))
+    v = co[:, 2 * nk * 128:].view(n, nv, 128)
+    beta = torch.sigmoid(x[:, C + nv * 128:C + nv * 129]).half().double()
+    g = -torch.exp(t["A_log"].double()) * torch.nn.functional.softplus(x[:, C + nv * 129:] + t["dt_bias"].double())
+    S = t["state"].double()
+    for i in range(n):
+        S = S * torch.exp(g[i])[:, None, None]
+        delta = beta[i][:, None] * (v[i] - torch.einsum("hrd,hd->hr", S, k[i]))
+        S = S + delta[:, :, None] * k[i][:, None, :]
+    return S
+
+
+@pytest.mark.parametrize("kind,n", [("usual", 100), ("usual", 512), ("slow", 200), ("alike", 200)])
+def test_error_is_that_of_the_token_by_token_form(lib, kind, n):
+    # The same chunk at once (blocks of 64) and in pieces that the kernel of four tokens at a time takes (64 tokens of 48 heads),
+    # both against 64 bits.  Everything that both share is exact: q, k and v are chosen, conv weights (0, 0, 0, 1) and inputs
+    # of 24 and more, or 0, pass the conv and silu unchanged; beta is 1/2 or 1.
+    nk, nv = 16, 48
+    t, ld = real_inputs(nk, nv, n, 7 + n)
+    C = (2 * nk + nv) * 128
+    g = torch.Generator().manual_seed(n)
+    t["conv_w"].zero_()
+    t["conv_w"][:, 3] = 1
+    x = torch.randint(24, 200, (n, C), generator=g).float()
+    if kind != "alike":                      # a key or query has a third of its values, so that they are far from parallel
+        x[:, :2 * nk * 128] *= (torch.rand(n, 2 * nk * 128, generator=g) < 0.33)
+    t["x"][:, :C] = x.half().cuda()
+    b = torch.where(torch.rand(n, nv, generator=g) < 0.5, 0.0, 30.0)
+    t["x"][:, C + nv * 128:C + nv * 129] = b.half().cuda()
+    if kind != "usual":
+        t["A_log"].fill_(-7.0)
+    want = float64_state(t, ld, t["x"][:, :C], nk, nv, n)
+    once, _ = run(lib, t, ld, nk, nv, n)
+    pieces = dict(t)
+    for i in range(0, n, 64):
+        m = min(64, n - i)
+        state, conv_state = pieces["state"].clone(), pieces["conv_state"].clone()
+        nbytes = lib.nvfp4_dn_prefill_work_bytes(m, nk, nv)
+        work, out = torch.empty(nbytes, dtype=torch.uint8, device="cuda"), torch.empty(m * nv * 128, dtype=torch.float16, device="cuda")
+        assert lib.launch_dn_prefill(ptr(t["x"][i:]), ld, ptr(t["conv_w"]), ptr(conv_state), ptr(t["A_log"]), ptr(t["dt_bias"]),
+                                     ptr(t["norm_w"]), ptr(state), ptr(work), nbytes, ptr(out), m, nk, nv, 1e-6, stream()) == 0
+        pieces.update(state=state, conv_state=conv_state)
+    torch.cuda.synchronize()
+    err = lambda a: ((a.double() - want).norm() / want.norm()).item()
+    # the errors are averages over 786432 values of a few dozen roundings each: 10 % is far outside their spread
+    assert err(once) <= 1.1 * err(pieces["state"]), (err(once), err(pieces["state"]))
+
+
+def test_small_tokens_beside_large_ones(lib):
+    # A token of 60000s, one that clears the state, then tokens of 2^-8 and less with hardly any decay: operands that share a
+    # row's scale with the large token, and everything that is left at the end is small.
+    nk, nv, n = 16, 48, 128
+    t, ld = real_inputs(nk, nv, n, 11)
+    C = (2 * nk + nv) * 128
+    g = torch.Generator().manual_seed(12)
+    t["conv_w"].zero_()
+    t["conv_w"][:, 3] = 1
+    x = torch.randint(24, 200, (n, C), generator=g).float()
+    x[:, :2 * nk * 128] *= (torch.rand(n, 2 * nk * 128, generator=g) < 0.33)
+    x[:, 2 * nk * 128:] = torch.randn(n, nv * 128, generator=g) * 2.0 ** -9
+    x[::64, 2 * nk * 128:] = 60000
+    t["x"][:, :C] = x.half().cuda()
+    t["x"][:, C + nv * 128:C + nv * 129] = 30.0
+    t["x"][:, C + nv * 129:] = 0.0
+    t["x"][1::64, C + nv * 129:] = 60000.0
+    t["A_log"].fill_(-7.0)
+    S, _ = run(lib, t, ld, nk, nv, n)
+    # silu of the small values as the kernel rounds it: fp32, then fp16 (a value that falls the other way is 2^-11 of itself off,
+    # and there are few: 1e-5 of the state)
+    co = t["x"][:, :C].clone()
+    v = co[:, 2 * nk * 128:].float()
+    co[:, 2 * nk * 128:] = (v / (1 + torch.exp(-v))).half()
+    want = float64_state(t, ld, co, nk, nv, n)
+    worst = ((S.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)).max().item()
+    assert worst <= 1e-5, worst
+
+
+def test_workspace_grows_with_the_chunk(lib):
+    # a workspace sized for the longest chunk serves the shorter ones, whichever of the two forms takes them
+    for nk, nv in ((16, 48), (16, 64), (14, 56), (10, 40), (8, 24), (5, 20), (4, 12), (1, 1)):
+        sizes = [lib.nvfp4_dn_prefill_work_bytes(n, nk, nv) for n in range(1, 700)]
+        assert all(a <= b for a, b in zip(sizes, sizes[1:])), (nk, nv)
