@@ -454,15 +454,17 @@ void nvfp4_gemv_tc_probe(void* device_buffer);
  * nvfp4_gemm_fp4_status: like nvfp4_gemm_status, for the FP4 kernel's bounded waits alone
  *   (nvfp4_gemm_status reports them as 100 + id).
  * nvfp4_b200_gemm_fp4_config: bit 0: shapes whose output tiles would leave more than half of the SMs
- *   idle and whose K is deep (32 tokens x 5120 rows x K 17408: 40 tiles) split K over several CTAs per
- *   tile; the CTA that arrives last adds the fp32 partial tiles in split order (split launches on one
- *   device share a workspace and must follow one another in stream order).  Bit 1: the CTA-pair kernel
+ *   idle and whose K is deep (32 tokens x 5120 rows x K 17408: 40 tiles) split K into parts whose fp32
+ *   sums are added in order: up to 64 tokens over several CTAs per tile, where the CTA that arrives
+ *   last adds (those launches share a workspace on a device and must follow one another in stream
+ *   order), from 65 tokens on one after the other within a CTA pair.  Bit 1: the CTA-pair kernel
  *   (clusters of two, tcgen05 cta_group::2, each CTA loading half of the token tile) where it is
- *   faster: more than 128 tokens but for few tiles of shallow K, and few deep tiles from 65 tokens on;
- *   bit 2: always for more than 128 tokens.  Bit 3: one CTA (pair) per output tile instead of one per
- *   SM (two SMs) that walks the tiles; bits 4, 5: tiles of 256, of 192 tokens always; bits 8..15: pairs
- *   of the walking pair kernel (0 = half the SM count).  Default 3.  Bit-identical results but for the
- *   K split. */
+ *   faster: more than 128 tokens but for few tiles of shallow K, and few deep tiles from 65 tokens on
+ *   (without it all split launches are of the first kind); bit 2: always for more than 128 tokens,
+ *   K in one part.  Bit 3: one CTA (pair) per output tile instead of one per SM (two SMs) that walks the
+ *   tiles; bits 4, 5: tiles of 256, of 192 tokens always, K in one part; bits 8..15: pairs of the
+ *   walking pair kernel (0 = half the SM count).  Default 3.  Bit-identical results but for the
+ *   parts of K. */
 void nvfp4_b200_gemm_fp4_config(int flags);
 int launch_nvfp4_gemm_fp4(const uint8_t* w_packed, const uint8_t* w_scales, const uint8_t* a_packed,
                           const uint8_t* a_scales, void* out, int M, int n_tokens, int K, int ld_out,

@@ -354,7 +354,8 @@ gemm_fp4_block_scaled_kernel(const __grid_constant__ CUtensorMap w_map,
 // issued with the MMAs that read them.  (Warps that store them there have to wait for the MMAs of two stages before.)
 // That copy wants a K block's bytes as 32 pieces of 16, piece l = 4 bytes of each of rows l, l + 32, l + 64, l + 96.
 // 192 tokens leave room in tensor memory for two accumulators, so that a tile's epilogue (four warps of its own, through
-// shared memory and TMA stores) runs under the next tile's MMAs; 256 tokens have one, and 10 % more work per stage.
+// shared memory and TMA stores) runs under the next tile's MMAs; 256 tokens have one, and 10 % more work per stage.  128
+// tokens (few deep tiles only) have two and room for a third: K in parts of kseg stages, which the epilogue warps add up.
 // 17408 x 5120 at 8192 tokens 383 -> 338 us (4.3 PFLOP/s; with the K loop's copies alone 233, its MMAs alone 292).
 //
 // Roles per CTA (352 threads): warp 0 operand copies, warp 1 MMAs (first CTA), warps 2..5 scale bytes, every fourth
@@ -370,7 +371,8 @@ constexpr int F4P_OUT = 32 * 64;                     // an epilogue warp's 32 ro
 template <int BN>
 struct F4Pair {
     static constexpr int ACCS = BN == 256 ? 1 : 2;                       // accumulators
-    static constexpr int ST = BN == 256 ? 4 : 5;                         // ring of stages
+    static constexpr bool SEGS = BN == 128;                              // K in segments, whose sums go to a third one
+    static constexpr int ST = BN == 256 ? 4 : BN == 192 ? 5 : 6;         // ring of stages
     static constexpr int A = F4_BM * 128, B = BN / 2 * 128;              // operand bytes of a stage
     static constexpr int SA = F4_BM * 16 * F4P_SK, SB = BN * 16 * F4P_SK;    // scale bytes of a box
     static constexpr int SMEM = ST * (A + B + F4P_SF) + 2 * (SA + SB) + 4 * F4P_OUT + 1024;
@@ -421,13 +423,15 @@ __global__ void __launch_bounds__(F4_PAIR_THREADS, 1)
 gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap a_map,
                      const __grid_constant__ CUtensorMap ws_map, const __grid_constant__ CUtensorMap as_map,
                      const __grid_constant__ CUtensorMap o_map, int tma_out, __half* __restrict__ out, int M,
-                     int n_tokens, int K, int ld_out) {
+                     int n_tokens, int K, int ld_out, int kseg_) {
     using T = F4Pair<BN>;
     constexpr int HALF = BN / 2, ST = T::ST, SK = F4P_SK, ACCS = T::ACCS;
+    constexpr bool SEGS = T::SEGS;
+    constexpr int PARTS = BN > 128 ? 3 : 2;          // rearranged scale bytes: weights, groups of 128 tokens
     constexpr int NB = BN / 32;                      // groups of 32 tokens
     constexpr int SFB = 8;                           // token-scale columns per MMA (a multiple of 4)
     constexpr int SF_STRIDE = 64;                    // columns of a stage (two take turns): 16 for the weights, 4 x SFB
-    static_assert(NB <= SFB && ACCS * BN + 2 * SF_STRIDE <= 512 && 16 + 4 * SFB <= SF_STRIDE, "tensor memory");
+    static_assert(NB <= SFB && (ACCS + (SEGS ? 1 : 0)) * BN + 2 * SF_STRIDE <= 512 && 16 + 4 * SFB <= SF_STRIDE, "tensor memory");
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                ~(uintptr_t)1023);
@@ -448,7 +452,7 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
     const int pairs = (int)(gridDim.x >> 1), pair0 = (int)(blockIdx.x >> 1);
     const int tiles_m = (M + 2 * F4_BM - 1) / (2 * F4_BM);
     const int ntiles = tiles_m * ((n_tokens + BN - 1) / BN);
-    const int ksteps = K / F4_BK;
+    const int ksteps = K / F4_BK, kseg = SEGS ? kseg_ : ksteps;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < ST; s++) {
@@ -472,7 +476,7 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
     cluster_sync_all();
     tcgen05_fence_after();
     const uint32_t tmem = s_tmem;
-    const uint32_t tmem_sf = tmem + ACCS * BN;
+    const uint32_t tmem_sum = tmem + ACCS * BN, tmem_sf = tmem + (ACCS + (SEGS ? 1 : 0)) * BN;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -531,38 +535,43 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
             uint32_t ph = 0, aph = 0;
             bool ok = true, ready = false;
             for (int tile = pair0; tile < ntiles; tile += pairs) {
-                // both CTAs' epilogues must have read what this accumulator held
-                if (ok) ok = f4_wait(smem_u32(&bar_acc_free[acc]), aph ^ 1u, 5);
-                const uint32_t d = tmem + (uint32_t)(acc * BN);
-                for (int it = 0; it < ksteps; it++) {
-                    if (ok && !ready) ok = f4_wait(smem_u32(&bar_full[s]), ph, 1);
-                    __syncwarp();
-                    tcgen05_fence_after();
-                    // the next stage's barrier is asked before this stage's instructions are issued, which hide the
-                    // answer's 170 cycles (16 instructions a stage are what this warp can issue in time)
-                    const bool wrap = s + 1 == ST;
-                    const bool next = mbar_test_wait_cluster(smem_u32(&bar_full[wrap ? 0 : s + 1]), wrap ? ph ^ 1u : ph);
-                    const uint64_t ad = a_desc + (uint64_t)(s * (T::A >> 4)), bd = b_desc + (uint64_t)(s * (T::B >> 4));
-                    const uint64_t sd = s_desc + (uint64_t)(s * (F4P_SF >> 4));
-                    const uint32_t sf = tmem_sf + (uint32_t)(set * SF_STRIDE);
+                int k0 = 0;
+                do {
+                    const int k1 = SEGS ? min(k0 + kseg, ksteps) : ksteps;
+                    // both CTAs' epilogues must have read what this accumulator held
+                    if (ok) ok = f4_wait(smem_u32(&bar_acc_free[acc]), aph ^ 1u, 5);
+                    const uint32_t d = tmem + (uint32_t)(acc * BN);
+                    for (int it = k0; it < k1; it++) {
+                        if (ok && !ready) ok = f4_wait(smem_u32(&bar_full[s]), ph, 1);
+                        __syncwarp();
+                        tcgen05_fence_after();
+                        // the next stage's barrier is asked before this stage's instructions are issued, which hide the
+                        // answer's 170 cycles (16 instructions a stage are what this warp can issue in time)
+                        const bool wrap = s + 1 == ST;
+                        const bool next = mbar_test_wait_cluster(smem_u32(&bar_full[wrap ? 0 : s + 1]), wrap ? ph ^ 1u : ph);
+                        const uint64_t ad = a_desc + (uint64_t)(s * (T::A >> 4)), bd = b_desc + (uint64_t)(s * (T::B >> 4));
+                        const uint64_t sd = s_desc + (uint64_t)(s * (F4P_SF >> 4));
+                        const uint32_t sf = tmem_sf + (uint32_t)(set * SF_STRIDE);
 #pragma unroll
-                    for (int kk = 0; kk < 4; kk++) {
-                        f4p_copy(sf + (uint32_t)(kk * 4), sd + 32 * kk);
-                        f4p_copy(sf + (uint32_t)(16 + kk * SFB), sd + 128 + 32 * kk);
-                        f4p_copy(sf + (uint32_t)(16 + kk * SFB + 4), sd + 256 + 32 * kk);
+                        for (int kk = 0; kk < 4; kk++) {
+                            f4p_copy(sf + (uint32_t)(kk * 4), sd + 32 * kk);
+                            f4p_copy(sf + (uint32_t)(16 + kk * SFB), sd + 128 + 32 * kk);
+                            if (PARTS == 3) f4p_copy(sf + (uint32_t)(16 + kk * SFB + 4), sd + 256 + 32 * kk);
+                        }
+#pragma unroll
+                        for (int kk = 0; kk < 4; kk++)   // 64 elements of K = 32 bytes further along the swizzled row
+                            f4p_mma(d, ad + 2 * kk, bd + 2 * kk, idesc, sf + (uint32_t)(kk * 4), sf + (uint32_t)(16 + kk * SFB),
+                                    ((SEGS ? it - k0 : it) | kk) != 0 ? 1u : 0u);
+                        f4p_commit(smem_u32(&bar_empty[s]));
+                        ready = __all_sync(0xffffffffu, next);
+                        set ^= 1;
+                        if (++s == ST) { s = 0; ph ^= 1u; }
                     }
-#pragma unroll
-                    for (int kk = 0; kk < 4; kk++)   // 64 elements of K = 32 bytes further along the swizzled row
-                        f4p_mma(d, ad + 2 * kk, bd + 2 * kk, idesc, sf + (uint32_t)(kk * 4), sf + (uint32_t)(16 + kk * SFB),
-                                (it | kk) != 0 ? 1u : 0u);
-                    f4p_commit(smem_u32(&bar_empty[s]));
-                    ready = __all_sync(0xffffffffu, next);
-                    set ^= 1;
-                    if (++s == ST) { s = 0; ph ^= 1u; }
-                }
-                f4p_commit(smem_u32(&bar_acc_full[acc]));
-                if (++acc == ACCS) acc = 0;
-                if (acc == 0) aph ^= 1u;
+                    f4p_commit(smem_u32(&bar_acc_full[acc]));
+                    if (++acc == ACCS) acc = 0;
+                    if (acc == 0) aph ^= 1u;
+                    k0 = k1;
+                } while (SEGS && k0 < ksteps);
             }
         }
     } else if (warp < 6) {
@@ -586,7 +595,7 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
                     const int c16 = lane * 64 + (j ^ ((lane >> 1) & 3)) * 16;
                     uint8_t* dst = smem_sf + s * F4P_SF + lane * 16;
 #pragma unroll
-                    for (int part = 0; part < 3; part++) { // weights, tokens 0..127, the others
+                    for (int part = 0; part < PARTS; part++) { // weights, tokens 0..127, the others
                         const uint8_t* src = part == 0 ? smem_sa + u * T::SA + c16
                                                        : smem_sb + u * T::SB + (part - 1) * 8192 + c16;
                         uint4 v[4];
@@ -616,6 +625,37 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
         uint32_t aph = 0;
         for (int tile = pair0; tile < ntiles; tile += pairs) {
             const int m0 = ((tile % tiles_m) * 2 + (int)rank) * F4_BM + q * 32, n0 = (tile / tiles_m) * BN;
+            if (SEGS) {
+                // the segments before the last: their sum, in order, beside the accumulators
+                for (int k0 = kseg; k0 < ksteps; k0 += kseg) {
+                    if (ok) ok = f4_wait(smem_u32(&bar_acc_full[acc]), aph, 4);
+                    __syncwarp();
+                    tcgen05_fence_after();
+#pragma unroll 1
+                    for (int cb = 0; cb < BN / 32; cb++) {
+                        uint32_t v[32];
+                        tcgen05_ld_32x32b_x32(tmem + lane_base + (uint32_t)(acc * BN + cb * 32), v);
+                        if (k0 != kseg) {
+                            uint32_t p[32];
+                            tcgen05_ld_32x32b_x32(tmem_sum + lane_base + (uint32_t)(cb * 32), p);
+                            tcgen05_wait_ld();
+#pragma unroll
+                            for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(p[j]) + __uint_as_float(v[j]));
+                        } else {
+                            tcgen05_wait_ld();
+                        }
+#pragma unroll
+                        for (int j = 0; j < 32; j += 8)
+                            tcgen05_st_32x32b<8>(tmem_sum + lane_base + (uint32_t)(cb * 32 + j), v + j);
+                    }
+                    tcgen05_wait_st();
+                    tcgen05_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(cluster_map_shared(smem_u32(&bar_acc_free[acc]), 0));
+                    if (++acc == ACCS) acc = 0;
+                    if (acc == 0) aph ^= 1u;
+                }
+            }
             if (ok) ok = f4_wait(smem_u32(&bar_acc_full[acc]), aph, 4);
             __syncwarp();
             tcgen05_fence_after();
@@ -623,7 +663,15 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
             for (int cb = 0; cb < BN / 32; cb++) {
                 uint32_t v[32];
                 tcgen05_ld_32x32b_x32(tmem + lane_base + (uint32_t)(acc * BN + cb * 32), v);
-                tcgen05_wait_ld();
+                if (SEGS && kseg < ksteps) {
+                    uint32_t p[32];
+                    tcgen05_ld_32x32b_x32(tmem_sum + lane_base + (uint32_t)(cb * 32), p);
+                    tcgen05_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(p[j]) + __uint_as_float(v[j]));
+                } else {
+                    tcgen05_wait_ld();
+                }
                 if (cb == BN / 32 - 1) {       // the accumulator is read: the MMAs of the tile after the next may start
                     tcgen05_fence_before();
                     __syncwarp();
@@ -690,6 +738,16 @@ static int f4_sm_count(int dev) {
     return sms[dev];
 }
 
+// K split of few deep tiles: stages per part; all of them where it does not pay.  When the output tiles leave more than
+// half of the SMs idle AND K is deep (32 tokens x 5120 rows x K 17408 is 40 tiles of 68 stages: 25.2 us unsplit, 16.3 us in
+// three parts).  Meeting in the epilogue costs about 4 us, more than a 20-stage tile saves (K = 5120: 10.0 us unsplit, 11.0
+// us split), hence the floor of 40 stages; parts keep >= 8 stages each.
+static int f4_split_stages(int tiles, int total, int sms) {
+    if (!g_f4_split || tiles * 2 > sms || total < 40) return total;
+    const int Z = std::max(1, std::min(std::min(sms / tiles, total / 8), F4_SPLIT_CTAS / tiles));
+    return (total + Z - 1) / Z;
+}
+
 static bool f4_workspace(int dev, cudaStream_t st, F4Workspace* out) {
     F4Workspace& w = g_f4_ws[dev];
     if (!w.part) {
@@ -731,20 +789,11 @@ static cudaError_t launch_fp4(const CUtensorMap& wm, const CUtensorMap& am, cons
     }
     const int ntiles = ((M + F4_BM - 1) / F4_BM) * ((n + BN - 1) / BN);
     dim3 grid((unsigned)ntiles, 1, 1);
-    // K split: when the output tiles leave more than half of the SMs idle AND K is deep (32 tokens
-    // x 5120 rows x K 17408 is 40 tiles of 68 stages: 25.2 us unsplit, 16.3 us in three splits).
-    // Meeting in the epilogue costs about 4 us, more than a 20-stage tile saves (K = 5120: 10.0 us
-    // unsplit, 11.0 us split), hence the floor of 40 stages; splits keep >= 8 stages each.
-    const int tiles = ntiles, total = K / F4_BK;
-    int Z = 1, kper = total;
+    const int tiles = ntiles, total = K / F4_BK, sms = f4_sm_count(dev);
+    int Z = 1, kper = f4_split_stages(tiles, total, sms);
     F4Workspace w = {nullptr, nullptr};
-    const int sms = f4_sm_count(dev);
-    if (g_f4_split && tiles * 2 <= sms && total >= 40 && f4_workspace(dev, st, &w)) {
-        Z = std::min(std::min(sms / tiles, total / 8), F4_SPLIT_CTAS / tiles);
-        if (Z < 1) Z = 1;
-        kper = (total + Z - 1) / Z;
-        Z = (total + kper - 1) / kper;                   // no split without stages
-    }
+    if (kper < total && f4_workspace(dev, st, &w)) Z = (total + kper - 1) / kper;      // no split without stages
+    else kper = total;
     grid.z = (unsigned)Z;
     // without a K split a CTA per SM walks the tiles (see the kernel); with one, a CTA per tile and split
     if (Z == 1 && g_f4_persistent) grid.x = (unsigned)std::min(ntiles, sms);
@@ -762,16 +811,29 @@ static int g_f4_pair = 1;           // the CTA-pair kernel: 1 = where fp4_pair_t
 //   17408 x 5120: 192 tokens 18.2 / 16.5 / 17.4, 256 tokens 17.6 / 23.4 / 18.0, 1000: 57 / 56 / 51, 2048: 106 / 95 / 92,
 //   8192: 438 / 373 / 376 (a long run; 383 / 338 apart); 6144 x 5120, 8192: 143 / 121 / 117; 5120 x 17408, 8192: 326 /
 //   336 / 306; 4096 x 1024, 8192: 42 / 30 / 34, but 129 tokens 10.6 / 11.4 / 11.8, 800: 12.5 / 13.4 / 13.0.
-// Few deep tiles used to be split over K.  The partial tiles of 128 and more tokens are what that waits for: 5120 x 17408,
-// 65 tokens 34.2 / 31.4 / 35, 129 tokens 59.6 / 32.2 / 35.7; 1024 x 17408, 129 tokens 110 / 31; at 64 tokens 21.4 / 31.1.
+// Few deep tiles are split over K by the single-CTA kernel, whose CTAs meet in memory: the partial tiles of 128 and more
+// tokens are what that waits for.  From 65 tokens on pairs of 128 tokens add the same parts in the same order (*kseg stages
+// each), one after the other and in tensor memory, so the bits are the same.  A single accumulation over all of K would do
+// as well for speed, but the tensor core truncates the sum it adds to: with scale bytes over 12 binades 1.1e-2 of the
+// results of 5120 x 17408 are not the correctly rounded ones then, 3.8e-3 in three parts; of 1024 x 17408 1.1e-2 and, in
+// eight, 1.5e-3.  us, single CTAs that meet / pairs of 192 in one accumulation / this: 5120 x 17408, 65 tokens 32.6 /
+// 29.4 / 27.3, 129: 57.5 / 30.5 / 28.5; 1024 x 17408, 65: 50.8 / 29.4 / 28.8, 129: 108 / 29.9 / 29.0; 5120 x 10240, 256:
+// 55.6 / 21.5 / 19.5.  At 64 tokens the single CTAs take 21.4.
 // Both widths run in rounds of pairs, a round costs a part per stage and a fixed part (ns, fitted to the above).
-static int fp4_pair_tokens(int M, int n, int K) {
+static int fp4_pair_tokens(int M, int n, int K, int* kseg) {
     const int st = K / F4_BK, sms = f4_sm_count(current_device_index());
     const int tiles1 = ((M + F4_BM - 1) / F4_BM) * ((n + 255) / 256);
+    *kseg = st;
     if (g_f4_pair == 0) return 0;
     if (g_f4_pair == 1) {
-        const bool few_deep = g_f4_split && tiles1 * 2 <= sms && st >= 40;
-        if (few_deep ? n <= 64 : n <= 128 || M <= F4_BM) return 0;
+        const int part = f4_split_stages(tiles1, st, sms);
+        if (part < st) {
+            if (n <= 64) return 0;
+            if (g_f4_pair_bn) return g_f4_pair_bn;
+            *kseg = part;
+            return 128;
+        }
+        if (n <= 128 || M <= F4_BM) return 0;
         if (st <= 4 && tiles1 <= sms) return 0;
     } else if (n <= 128) {
         return 0;
@@ -787,7 +849,7 @@ static int fp4_pair_tokens(int M, int n, int K) {
 template <int BN>
 static cudaError_t launch_fp4_pair(const CUtensorMap& wm, const CUtensorMap& am, const CUtensorMap& ws,
                                    const CUtensorMap& as, const CUtensorMap& om, bool tma_out, __half* out, int M, int n,
-                                   int K, int ld, cudaStream_t st) {
+                                   int K, int ld, int kseg, cudaStream_t st) {
     static bool attr[NVFP4_MAX_DEVICES] = {false};
     const int dev = current_device_index();
     if (!attr[dev]) {
@@ -813,7 +875,7 @@ static cudaError_t launch_fp4_pair(const CUtensorMap& wm, const CUtensorMap& am,
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemm_fp4_pair_kernel<BN>, wm, am, ws, as, om, tma_out ? 1 : 0, out, M, n, K, ld);
+    return cudaLaunchKernelEx(&cfg, gemm_fp4_pair_kernel<BN>, wm, am, ws, as, om, tma_out ? 1 : 0, out, M, n, K, ld, kseg);
 }
 
 static bool byte_matrix_map(EncodeTiledFn enc, CUtensorMap* map, const void* base, int rows, int K,
@@ -871,7 +933,8 @@ int launch_nvfp4_gemm_fp4(const uint8_t* w_packed, const uint8_t* w_scales, cons
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return -3;
     const int BN = n_tokens > 128 ? 256 : n_tokens > 64 ? 128 : n_tokens > 32 ? 64 : 32;
-    const int pbn = fp4_pair_tokens(M, n_tokens, K);
+    int kseg = 0;
+    const int pbn = fp4_pair_tokens(M, n_tokens, K, &kseg);
     const bool pair = pbn != 0;
     CUtensorMap wm, am, wsm, asm_, om;
     const bool tma_out = pair && (ld_out & 7) == 0;
@@ -885,8 +948,9 @@ int launch_nvfp4_gemm_fp4(const uint8_t* w_packed, const uint8_t* w_scales, cons
     cudaStream_t st = (cudaStream_t)stream;
     __half* o = static_cast<__half*>(out);
     const cudaError_t e =
-        pbn == 256 ? launch_fp4_pair<256>(wm, am, wsm, asm_, om, tma_out, o, M, n_tokens, K, ld_out, st)
-      : pbn == 192 ? launch_fp4_pair<192>(wm, am, wsm, asm_, om, tma_out, o, M, n_tokens, K, ld_out, st)
+        pbn == 256 ? launch_fp4_pair<256>(wm, am, wsm, asm_, om, tma_out, o, M, n_tokens, K, ld_out, kseg, st)
+      : pbn == 192 ? launch_fp4_pair<192>(wm, am, wsm, asm_, om, tma_out, o, M, n_tokens, K, ld_out, kseg, st)
+      : pbn == 128 ? launch_fp4_pair<128>(wm, am, wsm, asm_, om, tma_out, o, M, n_tokens, K, ld_out, kseg, st)
       : BN == 256 ? launch_fp4<256, 4>(wm, am, wsm, asm_, o, M, n_tokens, K, ld_out, st)
       : BN == 128 ? launch_fp4<128, 6>(wm, am, wsm, asm_, o, M, n_tokens, K, ld_out, st)
       : BN == 64  ? launch_fp4<64, 6>(wm, am, wsm, asm_, o, M, n_tokens, K, ld_out, st)

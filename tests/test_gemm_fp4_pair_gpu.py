@@ -45,10 +45,39 @@ def test_pairs_equal_the_single_cta_kernel(lib, M, K, n, ld, tile):
     assert lib.nvfp4_gemm_fp4_status(0) == 0
 
 
-# few deep tiles: from 65 tokens on pairs instead of the K split, also for one row tile
-@pytest.mark.parametrize("M,K,n", [(128, 10240, 65), (100, 10496, 129), (1024, 10240, 128), (5120, 10240, 256)])
-def test_few_deep_tiles_run_on_pairs(lib, M, K, n):
+# Few deep tiles: K in parts.  From 65 tokens on pairs add the parts that the single-CTA kernel's CTAs have, in the same order;
+# parts that do not divide K, one row tile, several column tiles, an output that TMA stores do not take.
+@pytest.mark.parametrize("M,K,n,ld", [(128, 10240, 65, 72), (100, 10496, 129, 136), (1024, 10240, 128, 128),
+                                      (5120, 10240, 256, 256), (5120, 17408, 200, 203), (300, 12288, 1000, 1000)])
+def test_few_deep_tiles_run_on_pairs(lib, M, K, n, ld):
     ops = operands(M, K, n)
-    ld = (n + 7) // 8 * 8
-    assert torch.equal(run(lib, ops, M, K, n, ld, 3), run(lib, ops, M, K, n, ld, 0))
+    want = run(lib, ops, M, K, n, ld, 1)
+    for _ in range(3):
+        assert torch.equal(run(lib, ops, M, K, n, ld, 3), want)
+    rows = want.view(M + 1, ld)
+    nan = torch.full((1,), float("nan"), dtype=torch.float16).view(torch.int16).item()
+    assert (rows[M] == nan).all() and (rows[:M, n:] == nan).all()
     assert lib.nvfp4_gemm_fp4_status(0) == 0
+
+
+@pytest.mark.parametrize("M,K,n", [(1024, 17408, 100), (1024, 17408, 200)])
+def test_few_deep_tiles_against_float64(lib, M, K, n):
+    # Scale bytes over 12 binades on both sides, so that sums do not fit fp32.  The tensor core truncates the sum that it
+    # adds to: eight parts of K leave an eighth of the truncations of one accumulation over all of it, so at most half
+    # of the results that are not the correctly rounded ones.
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + n)
+    r = lambda lo, hi, *s: torch.randint(lo, hi, s, dtype=torch.uint8, device="cuda", generator=g)
+    ops = r(0, 256, M, K // 2), r(110, 122, M, K // 16), r(0, 256, n, K // 2), r(110, 122, n, K // 16)
+    lut = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6], dtype=torch.float64, device="cuda")
+    lut = torch.cat([lut, -lut])
+
+    def decode(p, s):
+        w = lut[torch.stack([p & 15, p >> 4], -1).view(p.shape[0], -1).long()]
+        return w * torch.exp2(s.double() - 127).repeat_interleave(16, 1)
+
+    want = (decode(*ops[:2]) @ decode(*ops[2:]).t()).half()
+    ld = (n + 7) // 8 * 8
+    wrong = {c: (run(lib, ops, M, K, n, ld, c).view(torch.float16).view(M + 1, ld)[:M, :n] != want).double().mean().item()
+             for c in (0, 3)}
+    assert wrong[3] <= 0.5 * wrong[0], wrong
