@@ -387,7 +387,7 @@ int launch_nvfp4_decode_rows(const void* packed, const void* scales, const void*
  * allocates a workspace (do it outside stream capture).  0; -2 shape or pointer not taken; -3 no
  * tensor-map encoder / no memory; else the launch's cudaError_t.
  * nvfp4_gemv_tc_status: 0, or 1 + id of the first bounded wait in that kernel that ran out (20 + for the
- *   kernel of two activations, which launch_nvfp4_gemv2 and gemv2i hand matrices of 10 M elements to). */
+ *   kernel of two activations, see nvfp4_gemv_tc2_split). */
 int launch_nvfp4_gemv_tc(const uint8_t* weight_packed, const uint8_t* weight_scales,
                          const void* activation, void* output, int M, int K, void* stream);
 /* The same with the neighbours of launch_nvfp4_gemv_fused: prologue 1 = RMSNorm of the activation
@@ -424,6 +424,9 @@ void nvfp4_b200_gemv_tc_ctas(int per_sm);
 int nvfp4_gemv_tc_wanted(int M, int K);
 int nvfp4_gemv_tc_wanted_plain(int M, int K);
 int nvfp4_gemv_tc_wanted_step(int M, int K);
+/* CTAs that split K on the kernel of two activations where launch_nvfp4_gemv2 and gemv2i hand it an M x K matrix, 0
+ * where the register-streaming kernel is at least as fast. */
+int nvfp4_gemv_tc2_split(int M, int K);
 void nvfp4_b200_gemv_tc_config_plain(int min_mega_elements);
 int nvfp4_gemv_tc_prepare(void);
 /* Timing probe of launch_nvfp4_gemv_tc: while a device buffer of 128 int64 words is set, launch n

@@ -103,6 +103,7 @@ SIGNATURES = {
     "nvfp4_gemv_tc_wanted": ([_i, _i], _i),
     "nvfp4_gemv_tc_wanted_plain": ([_i, _i], _i),
     "nvfp4_gemv_tc_wanted_step": ([_i, _i], _i),
+    "nvfp4_gemv_tc2_split": ([_i, _i], _i),
     "nvfp4_b200_gemv_tc_config_plain": ([_i], None),
     "nvfp4_gemv_tc_prepare": ([], _i),
     "nvfp4_gemv_tc_probe": ([_vp], None),

@@ -395,7 +395,11 @@ static int few_clusters(int dev, int split) {
     const int wider = few_clusters_one_per_sm(dev, (split + 1) / 2);
     return twice > wider ? twice : wider;
 }
-int gemm_few_clusters(int dev, int split) { return few_clusters(dev, split); }
+// Of four CTAs fewer clusters are placed than the answer for two, 74: 71 run at once, and a launch of 72 takes half as
+// long again and more.  66 always fit, two layers of clusters with a CTA per SM; this is the mean of both.
+int gemm_few_clusters(int dev, int split) {
+    return split == 4 ? (few_clusters(dev, 4) + 2 * few_clusters_one_per_sm(dev, 4)) / 2 : few_clusters(dev, split);
+}
 
 template <int BN, bool IN_TM>
 static cudaError_t few_launch(const CUtensorMap& wm, const CUtensorMap& sm, const CUtensorMap& am, __half* out,
@@ -404,10 +408,12 @@ static cudaError_t few_launch(const CUtensorMap& wm, const CUtensorMap& sm, cons
     const cudaError_t opt = few_opt_in<BN, IN_TM>(dev);
     if (opt != cudaSuccess) return opt;
     const int rows = (M + FEW_BM - 1) / FEW_BM, cols = (N + BN - 1) / BN, nk = K / FEW_BK;
-    // K split: the fewest stages per CTA among the splits whose clusters all run at once
+    // K split: the fewest stages per CTA among the splits whose clusters all run at once.  (One column tile keeps to four
+    // parts for 71 to 74 row tiles too: 9216 x 5120 at 26 tokens takes 15.8 us with them and 11.9 with three, but with
+    // fewer parts the sums in them are longer, and a third more of the results are not the correctly rounded ones.)
     int split = 1;
     for (int s = 2; s <= FEW_MAX_SPLIT && s <= nk; s++)
-        if ((long long)rows * cols <= few_clusters(dev, s) && (nk + s - 1) / s < (nk + split - 1) / split) split = s;
+        if ((long long)rows * cols <= (cols == 1 ? few_clusters(dev, s) : gemm_few_clusters(dev, s)) && (nk + s - 1) / s < (nk + split - 1) / split) split = s;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(rows * split), (unsigned)cols, 1);
     cfg.blockDim = dim3(FEW_THREADS, 1, 1);
@@ -435,12 +441,13 @@ bool gemm_few_takes(const uint8_t* packed, const uint8_t* scales, int N, int K) 
 // / 9.9 and 19.7 / 11.8, 5120 x 6144 23.7 / 19.3 and 24.8 / 19.5, 5120 x 17408 53.7 / 39.3 and 56.1 / 41.6, 1024 x 17408
 // 51.4 / 18.2 and 51.4 / 20.5.  Wider ones are split less and read their weights twice (6144 x 5120 21.0 / 20.0,
 // feature-major 22.7 / 24.8; 10240 x 5120 23.3 / 31.4), and a short K leaves a CTA too little
-// (5120 x 1024 9.2 / 9.7 at 256, feature-major 9.3 / 10.4; 2048 x 1024 8.7 / 7.0).
+// (5120 x 1024 9.2 / 9.7 at 256, feature-major 9.3 / 10.4; 2048 x 1024 8.7 / 7.0).  The line is at 42 row tiles of 148 SMs:
+// 84 of the 90 clusters of three CTAs that run at once; with more, K is split over two, and 48 row tiles already lose.
 bool gemm_few_takes_two(const uint8_t* packed, const uint8_t* scales, int M, int N, int K) {
     const int rows = (M + FEW_BM - 1) / FEW_BM;
     return N > GEMM_FEW_MAX_TOKENS && N <= 2 * GEMM_FEW_MAX_TOKENS && K % FEW_BK == 0 &&
            (((uintptr_t)packed | (uintptr_t)scales) & 15) == 0 && (K >= 12 * FEW_BK || rows <= 20) &&
-           2LL * rows * 7 <= 4LL * device_sms(current_device_index());
+           rows * 7 <= 2 * device_sms(current_device_index());
 }
 
 int gemm_few_launch(const uint8_t* packed, const uint8_t* scales, const __half* act, long long ld_act,

@@ -18,7 +18,7 @@
 // plain fp32 from global memory.
 // Every wait is bounded and reported through nvfp4_gemv_tc_status (20 + id).
 //
-// Measured: at gemv_tc2_takes.
+// Measured: at gemv_tc2_faster.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -294,20 +294,37 @@ static int t2_split(int M, int K) {
     return best;
 }
 
-// us, weights cold, chain of launches, register-streaming kernel / this one:
-//   17408 x 5120  17.0 / 11.3      34816 x 5120  28.0 / 19.1      6144 x 5120  6.5 / 6.2      1024 x 5120  3.8 / 4.4
-//   5120 x 17408  17.7 / 11.5      16480 x 5120  16.8 / 10.9      2048 x 5120  5.1 / 4.7      12000 x 2048  5.0 / 5.6
-// Fixed cost (digits, the cluster's meeting) is higher here, so small matrices and shallow K keep the other.
-static bool gemv_tc2_takes(int M, int K) { return K >= 12 * TC_BK && (long long)M * K >= 10000000; }
+// us of a chain of launches with the weights cold / in L2, register-streaming kernel and this one:
+//    2048 x 5120   5.3 / 4.1   4.6 / 4.6       9216 x 3072   6.2 / 5.9   6.1 / 5.9       19456 x 4096  13.5 / 12.8  13.8 / 13.4
+//    6144 x 3072   4.6 / 4.5   4.8 / 4.7      10240 x 4096   8.1 / 7.5   7.4 / 7.0       19456 x 6144  18.9 / 17.8  19.1 / 18.3
+//    4096 x 4096   4.9 / 4.5   5.3 / 5.2      12288 x 4096   8.8 / 7.9   8.5 / 8.1       24576 x 4096  16.1 / 15.0  14.2 / 13.4
+//    2560 x 5120   5.5 / 5.1   4.6 / 4.7      12288 x 5120  10.8 / 9.3  10.1 / 9.3       17408 x 5120  17.1 / 16.5  11.4 /  9.5
+//    6144 x 5120   6.6 / 6.2   6.2 / 5.9      12288 x 6144  12.9 / 11.2 11.6 / 10.6       5120 x 17408 17.2 / 14.9  11.5 / 10.8
+// A stage of a CTA costs this kernel 0.6 us on top of 3.4, whichever way the tiles are split.  The other one goes in rounds of
+// three 16-row tiles an SM, each as long as K, but is there sooner; so the line is by its rounds, where this kernel is the
+// faster one with the weights cold and with them in L2 (launched one by one, three matrices of 12288 x 5120 in turn: 9.7
+// and 10.4).
+static bool gemv_tc2_faster(int M, int K, int split) {
+    const int sms = device_sms(current_device_index()), tiles = (M + 15) / 16, rounds = (tiles + 3 * sms - 1) / (3 * sms);
+    if (K < 12 * TC_BK) return false;
+    if (rounds == 1) return tiles > sms && K >= 20 * TC_BK;
+    if (rounds == 2) return K >= (split > 2 ? 16 : 24) * TC_BK;
+    return rounds > 3 || split > 1;
+}
+// CTAs that split K, 0 where the other kernel takes the problem
+int gemv_tc2_split(int M, int K) {
+    if (M <= 0 || K <= 0 || K % TC_BK != 0) return 0;
+    const int split = t2_split(M, K);
+    return split > 0 && gemv_tc2_faster(M, K, split) ? split : 0;
+}
 
 int gemv_tc2_launch(const uint8_t* packed, const uint8_t* scales, const void* act0, const void* act1, bool interleaved,
                     void* out, int M, int K, cudaStream_t st) {
     if (K % TC_BK != 0 || (((uintptr_t)packed | (uintptr_t)scales) & 15) != 0) return NVFP4_ERR_SHAPE;
-    if (!gemv_tc2_takes(M, K)) return NVFP4_ERR_SHAPE;
+    const int split = gemv_tc2_split(M, K);
+    if (split == 0) return NVFP4_ERR_SHAPE;
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return -3;
-    const int split = t2_split(M, K);
-    if (split == 0) return NVFP4_ERR_SHAPE;
     CUtensorMap wm, sm;
     const cuuint32_t estr[2] = {1, 1};
     for (int i = 0; i < 2; i++) {
@@ -325,6 +342,12 @@ int gemv_tc2_launch(const uint8_t* packed, const uint8_t* scales, const void* ac
                                       : t2_launch<false>(wm, sm, packed, scales, x0, x1, static_cast<__half*>(out), M, K, split, st);
     return (int)e;
 }
+
+}  // namespace nvfp4
+
+extern "C" int nvfp4_gemv_tc2_split(int M, int K) { return nvfp4::gemv_tc2_split(M, K); }
+
+namespace nvfp4 {
 
 int gemv_tc2_status(int reset) {
     int v = 0;

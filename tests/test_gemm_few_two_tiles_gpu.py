@@ -12,6 +12,7 @@ pytestmark = pytest.mark.gpu
     (300, 200, 512),        # ragged rows and tokens
     (2560, 193, 1024),      # the widest with a short K; a token past 64 in the second tile
     (5120, 136, 6144),      # K split over three
+    (4608, 200, 3072),      # 72 tiles, which clusters of four CTAs do not hold
     (5376, 255, 3072),      # the widest of all
     (1000, 256, 17408),     # K split over eight
 ])

@@ -20,11 +20,18 @@ def check(y, p, s, a):
     assert oc.rel_error_floored(y, ref).max() <= 1e-3       # the fp16 rounding of the output is 4.9e-4
 
 
-# K splits of 1 to 8 CTAs, ragged row tiles, splits that do not divide the stages; then shapes around the line to the other
-# kernel (K of 11 and 12 stages, too many tiles for one round)
-@pytest.mark.parametrize("M,K", [(3000, 3584), (6144, 5120), (5120, 6144), (700, 17408), (5120, 17408), (10240, 3072),
-                                 (13000, 3072), (20000, 3072), (37000, 3072), (4000, 2816), (40000, 3072), (1, 256), (1000, 768)])
-def test_two_activations(lib, M, K):
+# K splits of 1 to 8 CTAs on the tensor-core kernel, ragged row tiles, splits that do not divide the stages; then shapes that
+# the other kernel keeps (split 0): one round of row tiles with a short K, one tile an SM, two rounds, three with no split,
+# K of 11 stages, too many tiles for one round of clusters, the smallest
+@pytest.mark.parametrize("M,K,split", [(3000, 8192, 8), (3000, 5376, 7), (5500, 6144, 6), (6144, 5120, 5), (5120, 6144, 6),
+                                       (5120, 17408, 6), (8000, 5120, 4), (8900, 4096, 4), (9216, 4096, 3), (10240, 4096, 3),
+                                       (13000, 6144, 2), (17000, 3072, 2), (28000, 3072, 1), (37000, 3072, 1),
+                                       (3000, 3584, 0), (6144, 3072, 0), (700, 17408, 0), (2368, 5120, 0), (10240, 3072, 0),
+                                       (12288, 5120, 0), (20000, 3072, 0), (25000, 2816, 0), (40000, 3072, 0), (1, 256, 0),
+                                       (1000, 768, 0)])
+def test_two_activations(lib, M, K, split):
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert lib.nvfp4_gemv_tc2_split(M, K) == split
     p, s = weights(M, K)
     rng = np.random.default_rng(1)
     a0 = rng.standard_normal(K).astype(np.float16)
@@ -47,7 +54,8 @@ def test_two_activations(lib, M, K):
 @pytest.mark.parametrize("at", [0, 777, 5119])
 def test_an_activation_that_is_not_finite(lib, bad, at):
     # what IEEE arithmetic gives: a row is +-inf or NaN by its weight there, the other activation is untouched
-    M, K = 2050, 5120
+    M, K = 2450, 5120
+    assert lib.nvfp4_gemv_tc2_split(M, K) > 0
     p, s = weights(M, K)
     rng = np.random.default_rng(2)
     a0, a1 = rng.standard_normal(K).astype(np.float16), rng.standard_normal(K).astype(np.float16)
@@ -68,6 +76,7 @@ def test_an_activation_that_is_not_finite(lib, bad, at):
 def test_streams_share_nothing(lib):
     jobs = []
     for i, (M, K) in enumerate([(5120, 17408), (1024, 5120), (17408, 5120), (6144, 5120)]):
+        assert (lib.nvfp4_gemv_tc2_split(M, K) > 0) == (M > 1024)
         p, s = weights(M, K, i)
         x = np.random.default_rng(i).standard_normal((2, K)).astype(np.float16)
         jobs.append((M, K, dev(p), dev(s), dev(x), torch.zeros((2, M), dtype=torch.float16, device="cuda"), torch.cuda.Stream()))
