@@ -223,7 +223,7 @@ int launch_nvfp4_gemv_fused(const void* weight_packed, const void* weight_scales
                             const void* norm_w1, float eps, int epilogue, const void* residual,
                             void* stream);
 /* The same for calls that follow one another on one stream, like those of a decode step: the tensor-core kernel, whose
- * workspace belongs to the device, takes matrices from 30 instead of 35 * 2^20 elements
+ * workspace belongs to the device, takes matrices from 22 instead of 35 * 2^20 elements
  * (nvfp4_gemv_tc_wanted_step). */
 int launch_nvfp4_gemv_step(const void* weight_packed, const void* weight_scales,
                            const void* activation, void* output, int M, int K, int prologue,

@@ -1184,7 +1184,7 @@ int launch_nvfp4_gemv_fused(const void* weight_packed, const void* weight_scales
 }
 
 // The same for a caller whose other projections use the tensor-core GEMV's workspace anyway (a decode step): matrices
-// of 30 M elements go there too.  Not for everybody: the register-streaming kernel that they otherwise get has no
+// of 22 M elements go there too.  Not for everybody: the register-streaming kernel that they otherwise get has no
 // workspace, so calls on several streams may run side by side.
 int launch_nvfp4_gemv_step(const void* weight_packed, const void* weight_scales, const void* activation, void* output,
                            int M, int K, int prologue, const void* norm_w1, float eps, int epilogue,

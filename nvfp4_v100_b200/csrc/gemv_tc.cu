@@ -1206,11 +1206,15 @@ void nvfp4_b200_gemv_tc_config_plain(int min_mega_elements) {
 int nvfp4_gemv_tc_wanted(int M, int K) {
     return g_tc_route_min > 0 && (long long)M * K >= g_tc_route_min && K % nvfp4::TC_BK == 0;
 }
-// launch_nvfp4_gemv_step: 30 by default.  The output projections of the 27B decoder (5120 x 6144, residual added) take
-// 6.0 us on the register-streaming kernel and 6.3 here, back to back; in a decode step, between other launches of
-// this kernel, they are the faster ones here: 3597 -> 3558 us a step (3546 to 3578 with 25, 20, 15 and 10).
+// launch_nvfp4_gemv_step: 22 by default (22 / 35 of the fused entry's).  Back to back an output projection of 5120 x 6144 takes
+// 6.0 us on the register-streaming kernel and 6.3 here; in a decode step, between other launches of this kernel, it is the
+// faster one here.  us of in-projection, output projection (residual added), gate/up and down in turn, the output
+// projection there / here, by its elements in 2^20:
+//   30: 5120 x 6144  46.8 / 45.5    25: 5120 x 5120  46.3 / 45.2    20: 2560 x 8192  32.2 / 31.2    16: 8192 x 2048  38.4 / 37.7
+//   24: 8192 x 3072  40.4 / 38.2    24: 3072 x 8192  32.7 / 31.7    20: 5120 x 4096  45.7 / 45.7    16: 4096 x 4096  35.0 / 36.1
+//   24: 6144 x 4096  47.9 / 47.5    24: 4096 x 6144  36.6 / 36.7    16: 2048 x 8192  32.5 / 32.6    10: 5120 x 2048  43.4 / 44.3
 int nvfp4_gemv_tc_wanted_step(int M, int K) {
-    return g_tc_route_min > 0 && (long long)M * K >= g_tc_route_min / 7 * 6 && K % nvfp4::TC_BK == 0;
+    return g_tc_route_min > 0 && (long long)M * K >= g_tc_route_min / 35 * 22 && K % nvfp4::TC_BK == 0;
 }
 int nvfp4_gemv_tc_wanted_plain(int M, int K) {
     return g_tc_route_min_plain > 0 && (long long)M * K >= g_tc_route_min_plain && K % nvfp4::TC_BK == 0;

@@ -244,8 +244,10 @@ def test_mlp_block_rejects_bad_arguments(lib):
 
 
 def test_routing_of_a_decode_step(lib):
-    # 30 M elements: the output projections; the public entry leaves them to the kernel without a workspace
-    assert lib.nvfp4_gemv_tc_wanted_step(5120, 6144) == 1 and lib.nvfp4_gemv_tc_wanted_step(5119, 6144) == 0
+    # from 22 M elements on, the 30 M of the output projections among them; the public entry leaves those to the kernel
+    # without a workspace
+    assert lib.nvfp4_gemv_tc_wanted_step(5120, 6144) == 1 and lib.nvfp4_gemv_tc_wanted_step(5119, 6144) == 1
+    assert lib.nvfp4_gemv_tc_wanted_step(5632, 4096) == 1 and lib.nvfp4_gemv_tc_wanted_step(5631, 4096) == 0
     assert lib.nvfp4_gemv_tc_wanted(5120, 6144) == 0
     lib.nvfp4_b200_gemv_tc_config(0)
     assert lib.nvfp4_gemv_tc_wanted_step(34816, 5120) == 0
