@@ -985,6 +985,7 @@ int gemv2i_dispatch(const void* packed, const void* scales, const void* act_i, v
 int gemv_ex_dispatch(const void* packed, const void* scales, const void* act, void* out, int M,
                      int K, int prologue, const void* norm_w1, float eps, int epilogue,
                      const void* residual, void* stream, bool step) {
+    const char* who = step ? "launch_nvfp4_gemv_step" : "launch_nvfp4_gemv_fused";
     if (K <= 0 || K % 128 != 0 || M <= 0) return NVFP4_ERR_SHAPE;
     if (!packed || !scales || !act || !out) return NVFP4_ERR_SHAPE;
     if (!aligned(packed, 32) || !aligned(scales, 8) || !aligned(act, 16) || !aligned(out, 2))
@@ -1002,7 +1003,7 @@ int gemv_ex_dispatch(const void* packed, const void* scales, const void* act, vo
                                                   M, K, prologue, norm_w1, eps, epilogue, residual, stream);
         if (rc == 0) return NVFP4_OK;
         if (rc != NVFP4_ERR_SHAPE && rc != -3) {
-            fprintf(stderr, "launch_nvfp4_gemv_fused (tensor-core kernel): error %d\n", rc);
+            fprintf(stderr, "%s (tensor-core kernel): error %d\n", who, rc);
             return NVFP4_ERR_LAUNCH;
         }
     }
@@ -1016,7 +1017,7 @@ int gemv_ex_dispatch(const void* packed, const void* scales, const void* act, vo
         const cudaError_t es = launch_stream(packed, scales, act, out, M, K, prologue, norm_w1, eps,
                                              epilogue, residual, sp, st, !g_cfg.no_pdl);
         if (es != cudaSuccess) {
-            fprintf(stderr, "launch_nvfp4_gemv_fused (ring): %s\n", cudaGetErrorString(es));
+            fprintf(stderr, "%s (ring): %s\n", who, cudaGetErrorString(es));
             return NVFP4_ERR_LAUNCH;
         }
         return NVFP4_OK;
@@ -1044,7 +1045,7 @@ int gemv_ex_dispatch(const void* packed, const void* scales, const void* act, vo
     }
 #undef NVFP4_EX_CASE
     if (e != cudaSuccess) {
-        fprintf(stderr, "launch_nvfp4_gemv_fused: %s\n", cudaGetErrorString(e));
+        fprintf(stderr, "%s: %s\n", who, cudaGetErrorString(e));
         return NVFP4_ERR_LAUNCH;
     }
     return NVFP4_OK;

@@ -446,13 +446,14 @@ class DecodeEngine:
         # where gate/up uses the tensor-core GEMV's workspace, the projections a little smaller may too
         gu = self.layers[0].w_gu
         step = self.lib.nvfp4_gemv_tc_wanted(gu.M, gu.K)
-        rc = (self.lib.launch_nvfp4_gemv_step if step else self.lib.launch_nvfp4_gemv_fused)(
+        entry = "launch_nvfp4_gemv_step" if step else "launch_nvfp4_gemv_fused"
+        rc = getattr(self.lib, entry)(
             vp(m.packed.data_ptr()), vp(m.scales.data_ptr()), vp(x.data_ptr()), vp(out_ptr),
             m.M, m.K, 0 if pro_w1 is None else 1,
             vp(0 if pro_w1 is None else pro_w1.data_ptr()), float(self.cfg.rms_eps), epi,
             vp(0 if residual is None else residual.data_ptr()), st)
         if rc != 0:
-            raise RuntimeError(f"launch_nvfp4_gemv_fused rc={rc} (M={m.M}, K={m.K})")
+            raise RuntimeError(f"{entry} rc={rc} (M={m.M}, K={m.K})")
         self.n_launch += 1
 
     def _mlp_one_launch(self, st, L) -> bool:
