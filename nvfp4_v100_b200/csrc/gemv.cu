@@ -827,7 +827,7 @@ static cudaError_t launch_mma(const void* packed, const void* scales, const void
     // the opt-in to more than 48 KB of dynamic shared memory applies to the current device only
     static int max_smem_set[MAX_DEVICES] = {0};
     const int dev = current_device();
-    if (smem > 48 * 1024 && smem > max_smem_set[dev]) {
+    if (smem > 40 * 1024 && smem > max_smem_set[dev]) {          // (the 48 KB are with the static part)
         if (cudaFuncSetAttribute(gemv_mma_kernel<WARPS, NACT, PRO, EPI>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return cudaErrorInvalidValue;

@@ -199,3 +199,15 @@ def test_config1_full_size(lib):
     rc, y = gemv(lib, p, s, a)
     assert rc == 0
     check(y, p, s, a)
+
+
+@pytest.mark.parametrize("K", [11904, 12032, 12160, 12288, 12416])
+def test_interleaved_activations_that_just_fill_48_kilobytes(lib, K):
+    # the activations take K * 4 bytes of shared memory beside the kernel's own: one launch limit lies in between
+    p, s = (np.random.default_rng(K).integers(0, 256, (256, K // 2), dtype=np.uint8),
+            np.random.default_rng(K).integers(118, 123, (256, K // 16), dtype=np.uint8))
+    a = np.random.default_rng(1).standard_normal((2, K)).astype(np.float16)
+    rc, y = gemv2i(lib, p, s, a[0], a[1])
+    assert rc == 0
+    for t in range(2):
+        assert oc.rel_error_floored(y[t], oc.gemv_f64(p, s, a[t])).max() <= 1e-3
