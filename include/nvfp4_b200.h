@@ -109,8 +109,10 @@ int nvfp4_gemm_status(int reset);
  * dequantises 128 rows and loads half of a token tile): the one with the weights in tensor memory
  * (K % 256 == 0, 16-byte aligned scales) except where 256-row tiles are faster (K below some 1000 to
  * 4000, depending on the output layout), the other (K % 128 == 0) where 256-row tiles are not used.
- * Bit 2: CTA-pair kernels wherever they can run.  Default 3.  All of them give bit-identical results;
- * at most 128 tokens have a kernel of their own, which splits K and adds in another order. */
+ * Bit 2: CTA-pair kernels wherever they can run.  Default 3.  All of them give bit-identical results.
+ * The few-token kernel, which splits K and so adds in another order, takes at most 128 tokens whatever
+ * the flags, and with bit 1 set and bit 2 clear (as by default) 129 to 256 tokens of narrow matrices
+ * (up to 5376 rows; K >= 3072 or up to 2560 rows): for those 2 and 3 differ from the other settings. */
 void nvfp4_b200_gemm_config(int flags);
 
 /* Tuning hook; no counterpart in the reference.  warps per CTA (0 = auto, 2, 4 or 8), resident

@@ -73,7 +73,37 @@ assert codes == {keys: [0] * 20 for keys in CONTEXTS}, codes
 """
 
 
-@pytest.mark.parametrize("program", [DELTANET, ATTENTION], ids=["deltanet", "attention"])
+GEMM = """
+import threading
+import torch
+from nvfp4_v100_b200 import _lib
+from tests.gpu_util import ptr
+
+lib = _lib.load()
+TOKENS = [1, 20, 40, 100, 130, 300, 600, 1100]      # every kernel has tensor maps made for it, by an encoder looked up once
+start, codes = threading.Barrier(len(TOKENS)), {}
+
+def call(n):
+    M, K = 512, 1024
+    z = lambda *s: torch.zeros(s, dtype=torch.float16, device="cuda")
+    p, s = (torch.zeros(M * K // d, dtype=torch.uint8, device="cuda") for d in (2, 16))
+    x, out, side = z(n, K), z(n, M), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    start.wait()
+    codes[n] = [lib.launch_nvfp4_gemm_w4a16_ex(ptr(p), ptr(s), ptr(x), K, ptr(out), M, M, n, K, 3, side.cuda_stream)
+                for _ in range(20)]
+    side.synchronize()
+
+threads = [threading.Thread(target=call, args=(n,)) for n in TOKENS]
+for t in threads:
+    t.start()
+for t in threads:
+    t.join()
+assert codes == {n: [0] * 20 for n in TOKENS}, codes
+"""
+
+
+@pytest.mark.parametrize("program", [DELTANET, ATTENTION, GEMM], ids=["deltanet", "attention", "gemm"])
 def test_no_call_fails(program):
     for _ in range(4):
         subprocess.run([sys.executable, "-c", program], cwd=ROOT, check=True, timeout=120)

@@ -221,7 +221,8 @@ def test_fp4_prefill_size_8192_tokens(lib):
 def test_fp4_batched_decode_splits_k(lib, M, n, K):
     # batched decode (32 tokens) of a down projection: 40 output tiles of 68 K stages would leave
     # two thirds of the SMs idle, so K (>= 40 stages of 256) is split over several CTAs per tile
-    # and the last to arrive adds the fp32 partial tiles in split order.  Oracle as above over the whole output; the split result is reproducible bit
+    # and the last to arrive adds the fp32 partial tiles in split order (from 65 tokens on a CTA pair adds the same
+    # parts; tests/test_gemm_fp4_pair_gpu.py compares the two).  Oracle as above over the whole output; the split result is reproducible bit
     # for bit (the order of the sum does not depend on which CTA comes last), and differs from
     # the unsplit kernel's only by the fp32 association of the K sum.
     rng = np.random.default_rng(M + n)
@@ -470,7 +471,7 @@ def test_fp4_cta_pair_kernel_equals_the_single_cta_kernel(lib, M, n, K):
     outs = []
     lib.nvfp4_gemm_fp4_status(1)
     try:
-        for cfg in (1, 7):                       # single-CTA kernel, then the pair kernel for every K
+        for cfg in (0, 7):                       # single-CTA kernel, K in one part; then the pair kernel for every K
             lib.nvfp4_b200_gemm_fp4_config(cfg)
             out = torch.full((M * ld + 16,), float("nan"), dtype=torch.float16, device="cuda")
             assert lib.launch_nvfp4_gemm_fp4(ptr(d_p), ptr(d_s), ptr(d_ap), ptr(d_as), ptr(out), M, n, K,
