@@ -70,6 +70,12 @@ __device__ __forceinline__ uint4 ld_stream_u4(const void* p) {
 
 __device__ __forceinline__ float round_f16(float x) { return __half2float(__float2half(x)); }
 __device__ __forceinline__ float silu_pf(float x) { return x / (1.0f + expf(-x)); }
+__device__ __forceinline__ float softplus_pf(float x) { return (x > 20.0f) ? x : log1pf(expf(x)); }
+// 16 bytes of global memory into shared memory, without registers
+__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gsrc) : "memory");
+}
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

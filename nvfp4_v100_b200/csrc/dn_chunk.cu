@@ -79,10 +79,6 @@ __device__ __forceinline__ void dc_ldsm_t(uint32_t (&r)[4], const void* p) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
 }
-__device__ __forceinline__ void dc_cp16(void* smem_dst, const void* gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)),
-                 "l"(gsrc) : "memory");
-}
 
 // Power of two that brings a row's largest magnitude to 2^14..2^15, and its inverse.  (Zero rows and rows below
 // 2^-111 take the scale of 2^-111; infinite ones give NaN products, which the caller notices.)
@@ -137,7 +133,6 @@ __device__ __forceinline__ double dc_rsqrt(double s) {
     const double y = (double)rsqrtf((float)s);
     return s < 1e38 ? fma(0.5 * y, fma(-s * y, y, 1.0), y) : y;
 }
-__device__ __forceinline__ float dc_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
 // One CTA per (value head, block): X and D with their scales, the scales of the other products, and (first value
 // head of a key head) the block's keys and queries.  k.k and q.k are tensor-core products of the raw fp16 numbers.  The
@@ -246,7 +241,7 @@ dn_chunk_prep_kernel(const __half* __restrict__ conv_out, int conv_dim, const __
             float gt = 0.0f, beta = 0.0f;
             if (t0 + 2 * lane + e < n) {
                 beta = round_f16(1.0f / (1.0f + expf(-__half2float(gb[e]))));
-                gt = decay * dc_softplus(__half2float(ga[e]) + dt);
+                gt = decay * softplus_pf(__half2float(ga[e]) + dt);
                 // e^g is 0 either way, but differences of the sums must exist and not lose the other tokens' decays
                 if (gt < -200.0f) gt = -200.0f;
             }
@@ -573,16 +568,16 @@ dn_chunk_scan_kernel(const DcKQ* __restrict__ kq, const DcHead* __restrict__ hea
         const uint8_t* d = reinterpret_cast<const uint8_t*>(hp + c);
         uint8_t* sa = reinterpret_cast<uint8_t*>(&s.kq);
 #pragma unroll 4
-        for (int i = tid; i < (int)sizeof(DcKQ) / 16; i += T) dc_cp16(sa + i * 16, a + i * 16);
+        for (int i = tid; i < (int)sizeof(DcKQ) / 16; i += T) cp_async_16(sa + i * 16, a + i * 16);
 #pragma unroll 4
-        for (int i = tid; i < DC_HEAD_COPY / 16; i += T) dc_cp16(s.head + i * 16, d + i * 16);
+        for (int i = tid; i < DC_HEAD_COPY / 16; i += T) cp_async_16(s.head + i * 16, d + i * 16);
         // values: pieces of 8 rows per token; rows past the head's end and tokens past the chunk's end are not there
         const int rows = min(W * 16, DC - part * W * 16);
         for (int i = tid; i < CH * W * 2; i += T) {
             const int t = i / (W * 2), p = i - t * (W * 2);
             if (p * 8 >= rows) continue;
             __half* dst = &s.v[t][p * 8];
-            if (c * CH + t < n) dc_cp16(dst, vbase + (size_t)(c * CH + t) * conv_dim + part * W * 16 + p * 8);
+            if (c * CH + t < n) cp_async_16(dst, vbase + (size_t)(c * CH + t) * conv_dim + part * W * 16 + p * 8);
             else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");

@@ -654,15 +654,8 @@ int launch_nvfp4_gemmtc_v5(const uint8_t* d_weight_packed, const uint8_t* d_weig
     EncodeTiledFn enc = tc_ok ? encode_tiled_fn() : nullptr;
     if (enc) {
         CUtensorMap map;
-        const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)K};        // inner = tokens
-        const cuuint64_t strides[1] = {(cuuint64_t)N * sizeof(__half)};   // bytes between k rows
-        const cuuint32_t box[2] = {64, (cuuint32_t)GEMM_BK};
-        const cuuint32_t estr[2] = {1, 1};
-        const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)d_activation, dims,
-                               strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r == CUDA_SUCCESS) {
+        if (tile_map(enc, &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, d_activation, N, K, N * (long long)sizeof(__half), 64, GEMM_BK,
+                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)) {      // inner = tokens
             const cudaError_t e = launch_tc_any<false>(map, d_weight_packed, d_weight_scales, d_output, M,
                                                        N, K, N, GEMM_OUT_FM, N, st);
             return (e == cudaSuccess) ? 0 : (int)e;
@@ -713,25 +706,11 @@ int launch_nvfp4_gemm_w4a16_ex(const uint8_t* d_weight_packed, const uint8_t* d_
         return gemm_pair_launch(d_weight_packed, d_weight_scales, static_cast<const __half*>(act), ld_act, in_tm,
                                 o, (int)ld_out, M, N, n_tokens, K, mode, st);
     CUtensorMap map;
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult r;
-    if (in_tm) {
-        const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)n_tokens};       // inner = K
-        const cuuint64_t strides[1] = {(cuuint64_t)ld_act * sizeof(__half)};
-        const cuuint32_t box[2] = {(cuuint32_t)GEMM_BK,
-                                   (cuuint32_t)(gemm_use_pair(M, N, K) ? PAIR_HALF : gemm_tile_bn(N))};
-        r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(act), dims, strides, box, estr,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else {
-        const cuuint64_t dims[2] = {(cuuint64_t)N8, (cuuint64_t)K};
-        const cuuint64_t strides[1] = {(cuuint64_t)N8 * sizeof(__half)};
-        const cuuint32_t box[2] = {64, (cuuint32_t)GEMM_BK};
-        r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(act), dims, strides, box, estr,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    }
-    if (r != CUDA_SUCCESS) return -3;
+    if (!tile_map(enc, &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, act, in_tm ? K : N8, in_tm ? n_tokens : K,
+                  (in_tm ? ld_act : N8) * (long long)sizeof(__half), in_tm ? GEMM_BK : 64,
+                  in_tm ? (gemm_use_pair(M, N, K) ? PAIR_HALF : gemm_tile_bn(N)) : GEMM_BK, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B))
+        return -3;
     const cudaError_t e = in_tm ? launch_tc_any<true>(map, d_weight_packed, d_weight_scales, o, M, N, K,
                                                       (int)ld_out, mode, n_tokens, st)
                                 : launch_tc_any<false>(map, d_weight_packed, d_weight_scales, o, M, N, K,

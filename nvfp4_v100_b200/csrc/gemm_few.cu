@@ -458,34 +458,12 @@ int gemm_few_launch(const uint8_t* packed, const uint8_t* scales, const __half* 
     // token tile: the narrowest that holds all tokens; token-minor boxes are 64 tokens wide
     const int bn = N > 64 ? 128 : (!in_tm || N > 32) ? 64 : N > 16 ? 32 : 16;
     CUtensorMap wm, sm, am;
-    const cuuint32_t estr[2] = {1, 1};
-    {
-        const cuuint64_t dims[2] = {(cuuint64_t)(K / 2), (cuuint64_t)M};
-        const cuuint64_t strides[1] = {(cuuint64_t)(K / 2)};
-        const cuuint32_t box[2] = {128, FEW_BM};
-        if (enc(&wm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(packed), dims, strides, box, estr,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return -3;
-    }
-    {
-        const cuuint64_t dims[2] = {(cuuint64_t)(K / 16), (cuuint64_t)M};
-        const cuuint64_t strides[1] = {(cuuint64_t)(K / 16)};
-        const cuuint32_t box[2] = {16, FEW_BM};
-        if (enc(&sm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(scales), dims, strides, box, estr,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return -3;
-    }
-    {
-        const cuuint64_t dims[2] = {(cuuint64_t)(in_tm ? K : N), (cuuint64_t)(in_tm ? n_tokens : K)};
-        const cuuint64_t strides[1] = {(cuuint64_t)ld_act * sizeof(__half)};
-        const cuuint32_t box[2] = {64, (cuuint32_t)(in_tm ? bn : 64)};
-        if (enc(&am, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(act), dims, strides, box, estr,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return -3;
-    }
+    if (!packed_map(enc, &wm, packed, M, K, FEW_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
+        !scales_map(enc, &sm, scales, M, K, FEW_BM) ||
+        !tile_map(enc, &am, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, act, in_tm ? K : N, in_tm ? n_tokens : K,
+                  ld_act * (long long)sizeof(__half), 64, in_tm ? bn : 64, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B))
+        return -3;
     cudaError_t e;
 #define FEW_CASE(B) \
     if (bn == B) e = in_tm ? few_launch<B, true>(wm, sm, am, out, M, N, K, ld_out, out_mode, n_tokens, st) \

@@ -878,38 +878,13 @@ static cudaError_t launch_fp4_pair(const CUtensorMap& wm, const CUtensorMap& am,
     return cudaLaunchKernelEx(&cfg, gemm_fp4_pair_kernel<BN>, wm, am, ws, as, om, tma_out ? 1 : 0, out, M, n, K, ld, kseg);
 }
 
-static bool byte_matrix_map(EncodeTiledFn enc, CUtensorMap* map, const void* base, int rows, int K,
-                            int box_rows) {
-    const cuuint64_t dims[2] = {(cuuint64_t)(K / 2), (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)(K / 2)};
-    const cuuint32_t box[2] = {128, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // scale bytes [rows][K/16]: boxes of 16 bytes (one 256-element stage, unswizzled) or 64 bytes (four of them, 64-byte
 // swizzle) x box_rows rows
 static bool scale_matrix_map(EncodeTiledFn enc, CUtensorMap* map, const void* base, int rows, int K,
                              int box_rows, int box_bytes) {
-    const cuuint64_t dims[2] = {(cuuint64_t)(K / 16), (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)(K / 16)};
-    const cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
-               CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// the output [M][ld] as boxes of 32 rows x 32 tokens (what lies past row M or token n is not written)
-static bool out_matrix_map(EncodeTiledFn enc, CUtensorMap* map, void* base, int M, int n, int ld) {
-    const cuuint64_t dims[2] = {(cuuint64_t)n, (cuuint64_t)M};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(__half)};
-    const cuuint32_t box[2] = {32, 32};
-    const cuuint32_t estr[2] = {1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    if (box_bytes == 16) return scales_map(enc, map, base, rows, K, box_rows);
+    return tile_map(enc, map, CU_TENSOR_MAP_DATA_TYPE_UINT8, base, K / 16, rows, K / 16, box_bytes, box_rows,
+                    CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
 }
 
 }  // namespace nvfp4
@@ -938,11 +913,13 @@ int launch_nvfp4_gemm_fp4(const uint8_t* w_packed, const uint8_t* w_scales, cons
     const bool pair = pbn != 0;
     CUtensorMap wm, am, wsm, asm_, om;
     const bool tma_out = pair && (ld_out & 7) == 0;
-    if (!byte_matrix_map(enc, &wm, w_packed, M, K, F4_BM) ||
-        !byte_matrix_map(enc, &am, a_packed, n_tokens, K, pair ? pbn / 2 : BN) ||
+    if (!packed_map(enc, &wm, w_packed, M, K, F4_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
+        !packed_map(enc, &am, a_packed, n_tokens, K, pair ? pbn / 2 : BN, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
         !scale_matrix_map(enc, &wsm, w_scales, M, K, F4_BM, pair ? 64 : 16) ||
         !scale_matrix_map(enc, &asm_, a_scales, n_tokens, K, pair ? pbn : BN, pair ? 64 : 16) ||
-        (tma_out && !out_matrix_map(enc, &om, out, M, n_tokens, ld_out)))
+        // the output [M][ld] as boxes of 32 rows x 32 tokens (what lies past row M or token n is not written)
+        (tma_out && !tile_map(enc, &om, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, out, n_tokens, M, ld_out * (long long)sizeof(__half),
+                              32, 32, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE)))
         return -3;
     if (!tma_out) om = am;                           // not used by the kernel
     cudaStream_t st = (cudaStream_t)stream;

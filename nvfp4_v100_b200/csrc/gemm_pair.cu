@@ -531,20 +531,11 @@ int gemm_pair_launch(const uint8_t* packed, const uint8_t* scales, const __half*
     if (!enc) return -3;
     const int bn = gp_tile_tokens(current_device_index(), M, N);
     CUtensorMap wm, sm, am;
-    const cuuint32_t estr[2] = {1, 1};
-    auto encode = [&](CUtensorMap& m, CUtensorMapDataType type, const void* p, cuuint64_t d0, cuuint64_t d1,
-                      cuuint64_t stride, cuuint32_t b0, cuuint32_t b1, CUtensorMapSwizzle swizzle) {
-        const cuuint64_t dims[2] = {d0, d1}, strides[1] = {stride};
-        const cuuint32_t box[2] = {b0, b1};
-        return enc(&m, type, 2, const_cast<void*>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    };
-    if (!encode(wm, CU_TENSOR_MAP_DATA_TYPE_UINT8, packed, (cuuint64_t)(K / 2), (cuuint64_t)M, (cuuint64_t)(K / 2), 128,
-                GP_BM, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !encode(sm, CU_TENSOR_MAP_DATA_TYPE_UINT8, scales, (cuuint64_t)(K / 16), (cuuint64_t)M, (cuuint64_t)(K / 16), 16,
-                GP_BM, CU_TENSOR_MAP_SWIZZLE_NONE) ||
-        !encode(am, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, act, (cuuint64_t)(in_tm ? K : N), (cuuint64_t)(in_tm ? n_tokens : K),
-                (cuuint64_t)ld_act * sizeof(__half), 64, (cuuint32_t)(in_tm ? bn / 2 : 64), CU_TENSOR_MAP_SWIZZLE_128B))
+    if (!packed_map(enc, &wm, packed, M, K, GP_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
+        !scales_map(enc, &sm, scales, M, K, GP_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
+        !tile_map(enc, &am, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, act, in_tm ? K : N, in_tm ? n_tokens : K,
+                  ld_act * (long long)sizeof(__half), 64, in_tm ? bn / 2 : 64, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B))
         return -3;
     const int slots = gp_slots(current_device_index());
     const long long tiles = (long long)((M + 2 * GP_BM - 1) / (2 * GP_BM)) * ((N + bn - 1) / bn);

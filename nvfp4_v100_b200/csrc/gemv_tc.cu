@@ -1048,25 +1048,9 @@ static int tc_launch(const uint8_t* weight_packed, const uint8_t* weight_scales,
     if (!tc_workspace(dev, (size_t)ntiles + G, (size_t)ntiles, &ws)) return -3;
 
     CUtensorMap wm, sm;
-    const cuuint32_t estr[2] = {1, 1};
-    {
-        const cuuint64_t dims[2] = {(cuuint64_t)(K / 2), (cuuint64_t)M};
-        const cuuint64_t strides[1] = {(cuuint64_t)(K / 2)};
-        const cuuint32_t box[2] = {128, TC_BM};
-        if (enc(&wm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(weight_packed), dims, strides,
-                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return -3;
-    }
-    {
-        const cuuint64_t dims[2] = {(cuuint64_t)(K / 16), (cuuint64_t)M};
-        const cuuint64_t strides[1] = {(cuuint64_t)(K / 16)};
-        const cuuint32_t box[2] = {16, TC_BM};
-        if (enc(&sm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(weight_scales), dims, strides,
-                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return -3;
-    }
+    if (!packed_map(enc, &wm, weight_packed, M, K, TC_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
+        !scales_map(enc, &sm, weight_scales, M, K, TC_BM))
+        return -3;
     const TcFuse fz = {norm_w1, eps, static_cast<const __half*>(residual), g_tc_pre, weight_packed, weight_scales};
     const __half* x = static_cast<const __half*>(activation);
     __half* y = static_cast<__half*>(output);
@@ -1137,22 +1121,11 @@ int launch_nvfp4_mlp_tc(const uint8_t* gu_packed, const uint8_t* gu_scales, cons
     TcWorkspace* ws = nullptr;
     if (!tc_workspace(dev, (size_t)(nt0 + nt1 + 2 * G), 1, &ws)) return -3;
     CUtensorMap m[4];
-    const cuuint32_t estr[2] = {1, 1};
-    const uint8_t* bases[4] = {gu_packed, gu_scales, down_packed, down_scales};
-    const int rows[4] = {M0, M0, M1, M1}, ks[4] = {K0, K0, K1, K1};
-    for (int i = 0; i < 4; i++) {
-        const bool sc = (i & 1) != 0;
-        const cuuint64_t inner = (cuuint64_t)(sc ? ks[i] / 16 : ks[i] / 2);
-        const cuuint64_t dims[2] = {inner, (cuuint64_t)rows[i]};
-        const cuuint64_t strides[1] = {inner};
-        const cuuint32_t box[2] = {(cuuint32_t)(sc ? 16 : 128), TC_BM};
-        if (enc(&m[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(bases[i]), dims, strides, box,
-                estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                sc ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
-                sc ? CU_TENSOR_MAP_L2_PROMOTION_NONE : CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return -3;
-    }
+    if (!packed_map(enc, &m[0], gu_packed, M0, K0, TC_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
+        !scales_map(enc, &m[1], gu_scales, M0, K0, TC_BM) ||
+        !packed_map(enc, &m[2], down_packed, M1, K1, TC_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
+        !scales_map(enc, &m[3], down_scales, M1, K1, TC_BM))
+        return -3;
     TcMlpArgs a;
     a.h = static_cast<__half*>(h);
     a.act = static_cast<__half*>(act);

@@ -326,16 +326,9 @@ int gemv_tc2_launch(const uint8_t* packed, const uint8_t* scales, const void* ac
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return -3;
     CUtensorMap wm, sm;
-    const cuuint32_t estr[2] = {1, 1};
-    for (int i = 0; i < 2; i++) {
-        const cuuint64_t inner = (cuuint64_t)(i ? K / 16 : K / 2), dims[2] = {inner, (cuuint64_t)M}, strides[1] = {inner};
-        const cuuint32_t box[2] = {(cuuint32_t)(i ? 16 : 128), TC_BM};
-        if (enc(i ? &sm : &wm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(i ? scales : packed), dims, strides, box,
-                estr, CU_TENSOR_MAP_INTERLEAVE_NONE, i ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
-                i ? CU_TENSOR_MAP_L2_PROMOTION_NONE : CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return -3;
-    }
+    if (!packed_map(enc, &wm, packed, M, K, TC_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
+        !scales_map(enc, &sm, scales, M, K, TC_BM))
+        return -3;
     const __half* x0 = static_cast<const __half*>(act0);
     const __half* x1 = static_cast<const __half*>(act1);
     const cudaError_t e = interleaved ? t2_launch<true>(wm, sm, packed, scales, x0, x0, static_cast<__half*>(out), M, K, split, st)

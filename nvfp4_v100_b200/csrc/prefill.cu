@@ -27,7 +27,6 @@
 
 namespace nvfp4 {
 
-__device__ __forceinline__ float softplus_pf(float x) { return (x > 20.0f) ? x : log1pf(expf(x)); }
 
 // dst[c][r] = src[r][c] for r < R, c < C; dst rows are ld_dst long and columns R .. ld_dst-1 are
 // zero-filled (the GEMM reads whole rows).  src rows are ld_src long.
@@ -392,10 +391,6 @@ __device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
     return d;
 }
 
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gsrc) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {

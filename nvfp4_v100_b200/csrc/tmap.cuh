@@ -24,4 +24,26 @@ static inline EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
+// A matrix of `rows` rows of `inner` elements, `pitch` bytes apart, as boxes of box_rows x box_inner; what lies outside is
+// read as zero and not written.
+static inline bool tile_map(EncodeTiledFn enc, CUtensorMap* map, CUtensorMapDataType type, const void* base, long long inner,
+                            long long rows, long long pitch, int box_inner, int box_rows, CUtensorMapSwizzle swizzle,
+                            CUtensorMapL2promotion promotion) {
+    const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch};
+    const cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows}, estr[2] = {1, 1};
+    return enc(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+               promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// Stages of 256 k: packed bytes [rows][K / 2] in 128-byte swizzled boxes of 128, scale bytes [rows][K / 16] in boxes of 16.
+static inline bool packed_map(EncodeTiledFn enc, CUtensorMap* map, const void* base, int rows, int K, int box_rows,
+                              CUtensorMapL2promotion promotion) {
+    return tile_map(enc, map, CU_TENSOR_MAP_DATA_TYPE_UINT8, base, K / 2, rows, K / 2, 128, box_rows,
+                    CU_TENSOR_MAP_SWIZZLE_128B, promotion);
+}
+static inline bool scales_map(EncodeTiledFn enc, CUtensorMap* map, const void* base, int rows, int K, int box_rows,
+                              CUtensorMapL2promotion promotion = CU_TENSOR_MAP_L2_PROMOTION_NONE) {
+    return tile_map(enc, map, CU_TENSOR_MAP_DATA_TYPE_UINT8, base, K / 16, rows, K / 16, 16, box_rows,
+                    CU_TENSOR_MAP_SWIZZLE_NONE, promotion);
+}
+
 }  // namespace nvfp4
