@@ -110,13 +110,15 @@ __device__ __forceinline__ bool tc_not_finite(float sum) { return !(fabsf(sum) <
 // activation that is not; a scale byte of 255, which is infinity here and NaN to the tensor core).  load(k): the
 // activations k .. k + 7.
 template <typename LOAD>
-__device__ __noinline__ float tc_plain_row(const uint8_t* packed, const uint8_t* scales, const LOAD load, int row, int K) {
+__device__ __forceinline__ float tc_plain_row(const uint8_t* packed, const uint8_t* scales, const LOAD load, int row, int K) {
     const uint8_t* w = packed + (size_t)row * (K / 2);
     const uint8_t* sc = scales + (size_t)row * (K / 16);
     float sum = 0.0f;
+#pragma unroll 1
     for (int b = 0; b < K / 16; b++) {
         const uint2 p = *reinterpret_cast<const uint2*>(w + b * 8);
         float acc = 0.0f;
+#pragma unroll 1
         for (int half = 0; half < 2; half++) {
             uint32_t h[4];
             e2m1x8_to_half2x4(half ? p.y : p.x, h[0], h[1], h[2], h[3]);
