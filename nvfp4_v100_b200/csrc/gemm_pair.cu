@@ -207,11 +207,16 @@ gemm_w4a16_pair_tm_kernel(const __grid_constant__ CUtensorMap w_map, const __gri
         tma_load_2d(smem_u32(smem_w + s * GP_W_BYTES), &w_map, i * 128, m0, bar);
         tma_load_2d(smem_u32(smem_s + s * GP_S_BYTES), &s_map, i * 16, m0, bar);
     };
-    // (ONE: straight from the grid; gp_tile's divisions ahead of the first copies made 10240 x 5120 at 256 tokens 32.3 us
-    // instead of 31.8)
+    // (ONE, at most a hundred tiles or so: by a reciprocal.  gp_tile's divisions ahead of the first copies made 10240 x 5120
+    // at 256 tokens 32.3 us instead of 31.8.  Not as a grid of rows x columns, whose clusters land elsewhere: 5120 x 17408
+    // at 300 tokens 56.9 us instead of 54.2)
     auto place = [&](int t, int& row, int& col) {
-        if (ONE) { row = (int)blockIdx.x >> 1; col = (int)blockIdx.y; }
-        else gp_tile(t, rows, cols, row, col);
+        if (ONE) {
+            row = (int)__fdividef((float)t + 0.5f, (float)cols);
+            col = t - row * cols;
+        } else {
+            gp_tile(t, rows, cols, row, col);
+        }
     };
     auto rows_of = [&](int t) {                          // first row of this CTA's half of tile t
         int row, col;
@@ -490,7 +495,7 @@ static cudaError_t gp_launch(const CUtensorMap& wm, const CUtensorMap& sm, const
     }
     cudaLaunchConfig_t cfg = {};
     const int rows = (M + 2 * GP_BM - 1) / (2 * GP_BM), cols = (N + bn - 1) / bn;
-    cfg.gridDim = ONE ? dim3((unsigned)(2 * rows), (unsigned)cols, 1) : dim3((unsigned)(2 * pairs), 1, 1);
+    cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
     cfg.blockDim = dim3(ONE ? GP_THREADS_ONE : GP_THREADS, 1, 1);
     cfg.dynamicSmemBytes = GP_SMEM;
     cfg.stream = st;
