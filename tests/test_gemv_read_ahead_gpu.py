@@ -32,19 +32,22 @@ def fused(entry):
                                   fused("launch_nvfp4_gemv_step")],
                          ids=["gemv2", "gemv2i", "v8", "fused", "step"])
 def test_weights_written_by_the_kernel_in_front(lib, call):
-    # the quantiser lets its successor start at once; without the bit the first stages of weights would be the old ones
+    # A row copy (launch_embed_rows) lets its successor start at once; without the bit the GEMV's first stages of weights
+    # would be those that were there before.
     g = torch.Generator(device="cuda")
     g.manual_seed(5)
-    w = [(torch.randn((M, K), device="cuda", generator=g) * 0.02).half() for _ in range(2)]
+    weights = torch.randint(0, 256, (2 * M, K // 2), dtype=torch.uint8, device="cuda", generator=g)     # two matrices
+    rows = [torch.arange(i * M, (i + 1) * M, dtype=torch.int64, device="cuda") for i in range(2)]
     x = torch.randn((2, K), device="cuda", generator=g).half()
-    p = torch.empty(M * K // 2, dtype=torch.uint8, device="cuda")
-    s = torch.empty(M * K // 16, dtype=torch.uint8, device="cuda")
-    encode = lambda i: lib.launch_nvfp4_encode(ptr(w[i]), ptr(p), ptr(s), M, K, stream())
+    p = torch.zeros((M, K // 2), dtype=torch.uint8, device="cuda")
+    s = torch.randint(118, 123, (M * K // 16,), dtype=torch.uint8, device="cuda", generator=g)
+    write = lambda i: lib.launch_embed_rows(ptr(weights), ptr(rows[i]), ptr(p), M, K // 4, 2 * M, stream())
     y = torch.zeros((2, M), dtype=torch.float16, device="cuda")
     want = []
     for i in range(2):
-        assert encode(i) == 0
+        assert write(i) == 0
         torch.cuda.synchronize()
+        assert torch.equal(p, weights[i * M:(i + 1) * M])
         assert call(lib, p, s, x, y) == 0
         torch.cuda.synchronize()
         want.append(y.clone())
@@ -52,7 +55,7 @@ def test_weights_written_by_the_kernel_in_front(lib, call):
     assert lib.nvfp4_b200_gemv_config(0, 0, 2) == 0
     try:
         for i in (0, 1, 0, 1):
-            assert encode(i) == 0 and call(lib, p, s, x, y) == 0
+            assert write(i) == 0 and call(lib, p, s, x, y) == 0
             torch.cuda.synchronize()
             assert torch.equal(y, want[i])
     finally:
